@@ -2289,10 +2289,17 @@ struct Planner {
   }
 
   // stablehlo.cholesky (src/pjrt_plugin/ops/linalg.cc:553-570 of the reference hands it to LAPACK on the host). One
-  // block per matrix factors it in place in the result, column by column: the square root of the pivot, the column
-  // scaled by it, then the trailing triangle updated with the column's outer product; every element is written by one
-  // thread per step, so the result does not depend on scheduling. Only the named triangle of the input is read; the
-  // other triangle of the result is zero. A matrix that is not positive definite gives NaN from its first bad pivot on.
+  // block per matrix, right-looking over panels of NB columns held in shared memory. The time is the chain of n pivots
+  // (square root, reciprocal, a few multiply-adds each), not arithmetic or memory, so a panel is arranged around it: warp 0
+  // factors the NB x NB diagonal block with a row per lane in registers, knows the next pivot before the column it comes
+  // from is finished (from two values fetched ahead) and subtracts a column from those behind it while the next root is
+  // on its way; then every row below is a thread that substitutes through the diagonal block; then all threads subtract
+  // the panel's product from the trailing triangle, which stays in the result (L2), in tiles of 4 x 4 or, near the end,
+  // 2 x 2. Panels pass between memory and shared memory by rows, so that both sides are coalesced. 160 x 160, eight
+  // matrices: 756 us for a block that updated the trailing triangle element by element after each column, 43 us now
+  // (per panel 3.0 us diagonal, 1.4 us rows below, 1 - 6 us triangle). NB is 32 while NB columns fit static shared memory.
+  // Only the named triangle of the input is read; the other triangle of the result is zero. A matrix that is not
+  // positive definite gives NaN from its first bad pivot on.
   void lower_cholesky(Op* op, Plan& plan, BlockState& st) {
     if (op->operands.size() != 1 || op->results.size() != 1) throw CompileError("stablehlo.cholesky: malformed operands");
     Value *a = op->operands[0], *out = op->results[0];
@@ -2308,36 +2315,222 @@ struct Planner {
     const bool lower = !op->has("lower") || attr_bool(op->attr("lower"));
     const std::string T = c_type(a->type.dt);
     const std::string at = lower ? "(i) * N + (j)" : "(j) * N + (i)";        // element (i, j) of the lower factor
+    // column stride of the panel: 16-byte rows of four, four banks apart from the next column's
+    const int64_t np = (n + 27) / 32 * 32 + 4, es = (int64_t)dt_size(a->type.dt);
+    int64_t nb = 32;
+    while (nb > 1 && nb * np * es + nb * (nb + 2) * es > 46 * 1024) nb /= 2;
+    const bool paneled = nb >= 4;                          // narrower panels than that (n above 2800 in f32): column by column
+    const int threads = !paneled ? kThreads : n <= 32 ? 64 : n <= 96 || es > 4 ? 256 : 640;
     std::ostringstream src;
-    src << "extern \"C\" __global__ void __launch_bounds__(" << kThreads << ") @NAME@(" << signature({out}, {a}) << ") {\n";
+    src << "extern \"C\" __global__ void __launch_bounds__(" << threads << ") @NAME@(" << signature({out}, {a}) << ") {\n";
     src << "#define AT(i, j) (" << at << ")\n";
     src << "  const int N = " << n << ";\n";
     src << "  " << T << "* o = out0 + (long long)blockIdx.x * N * N;\n  const " << T << "* a = in0 + (long long)blockIdx.x * N * N;\n";
-    src << "  for (int e = threadIdx.x; e < N * N; e += " << kThreads << ") { const int i = e / N, j = e % N; o[AT(i, j)] = i >= j ? a[AT(i, j)] : (" << T << ")0; }\n";
-    src << "  __syncthreads();\n";
-    src << "  for (int j = 0; j < N; ++j) {\n";
-    src << "    if (threadIdx.x == 0) o[AT(j, j)] = op_sqrt(o[AT(j, j)]);\n    __syncthreads();\n";
-    src << "    const " << T << " d = o[AT(j, j)];\n";
-    src << "    for (int i = j + 1 + threadIdx.x; i < N; i += " << kThreads << ") o[AT(i, j)] = o[AT(i, j)] / d;\n    __syncthreads();\n";
-    src << "    const int m = N - j - 1;\n";
-    src << "    for (int e = threadIdx.x; e < m * m; e += " << kThreads << ") {\n      const int i = j + 1 + e / m, k = j + 1 + e % m;\n";
-    src << "      if (k <= i) o[AT(i, k)] = o[AT(i, k)] - o[AT(i, j)] * o[AT(k, j)];\n    }\n    __syncthreads();\n  }\n";
-    src << "#undef AT\n}\n";
+    if (paneled) {
+      src << "  typedef " << T << " T;\n  const int NB = " << nb << ", NP = " << np << ", TH = " << threads << ";\n";
+      src << "  const bool LOWER = " << (lower ? "true" : "false") << ", ALIGNED = " << (n % 4 == 0 ? "true" : "false") << ";\n";
+      src << R"SRC(  struct alignas(4 * sizeof(T)) V4 { T v[4]; };
+  struct alignas(2 * sizeof(T)) V2 { T v[2]; };
+  __shared__ V4 panel4[NB * NP / 4];                 // [column of the panel][row]
+  __shared__ V4 diag4[NB * NB / 4];                  // [column][row] of the diagonal block's factor
+  __shared__ T pivot[NB], inverse[NB];
+  __shared__ int regular;                            // every pivot of the panel is a positive number far from both ends of the range
+  T *P = (T*)panel4, *D = (T*)diag4;
+  const int tid = threadIdx.x, lane = tid & 31;
+  for (int e = tid; e < N * N; e += TH) { const int i = e / N, j = e % N; if (j > i) o[AT(i, j)] = (T)0; }
+  // (row, column) of tile e of a triangle of tiles
+  auto tile_of = [](int e, int& ti, int& tk) {
+    ti = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);
+    while (ti * (ti + 1) / 2 > e) --ti;
+    while ((ti + 1) * (ti + 2) / 2 <= e) ++ti;
+    tk = e - ti * (ti + 1) / 2;
+  };
+  for (int c0 = 0; c0 < N; c0 += NB) {
+    const T* s = c0 == 0 ? a : (const T*)o;          // the first panel reads the input, the trailing triangle lives in the result
+    const int m = N - c0, nb = m < NB ? m : NB;
+    for (int q = tid; q < m * NB; q += TH) {
+      const int k = LOWER ? q % NB : q / m, i = LOWER ? q / NB : q % m;
+      if (k < nb) P[k * NP + c0 + i] = s[AT(c0 + i, c0 + k)];
+    }
+    __syncthreads();
+    if (tid < 32) {
+      // columns past the matrix are those of the identity, so that the chain below has no branches
+      T r[NB], d = P[c0], l = (T)0, lv = (T)0;
+      bool fine = true;
+#pragma unroll
+      for (int k = 0; k < NB; ++k) r[k] = (lane < nb && k <= lane) ? P[k * NP + c0 + lane] : (T)(lane == k ? 1 : 0);
+#pragma unroll
+      for (int j = 0; j < NB; ++j) {
+        T root, inv;
+        fine = lin_pivot(d, root, inv) && fine;
+        if (j > 0) {                                 // what column j - 1 takes from the columns behind it, while the root is on its way
+#pragma unroll
+          for (int k4 = j / 4; k4 < NB / 4; ++k4) {
+            const V4 c = diag4[(j - 1) * (NB / 4) + k4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (4 * k4 + e >= j) r[4 * k4 + e] = r[4 * k4 + e] - l * (4 * k4 + e == j ? lv : c.v[e]);
+          }
+        }
+        const T v = __shfl_sync(0xFFFFFFFFu, r[j], j + 1 < NB ? j + 1 : 0);
+        const T w = __shfl_sync(0xFFFFFFFFu, r[j + 1 < NB ? j + 1 : 0], j + 1 < NB ? j + 1 : 0);
+        l = lin_quotient(r[j], root, inv);
+        lv = lin_quotient(v, root, inv);
+        if (lane == j) l = root;
+        d = w - lv * lv;                             // the next pivot
+        r[j] = l;
+        if (lane < NB) D[j * NB + lane] = l;
+        if (lane == j) { pivot[j] = root; inverse[j] = inv; }
+        __syncwarp();
+      }
+      if (!fine) {                                   // the same with plain roots and divisions, from the panel as it was loaded
+#pragma unroll
+        for (int k = 0; k < NB; ++k) r[k] = (lane < nb && k <= lane) ? P[k * NP + c0 + lane] : (T)(lane == k ? 1 : 0);
+#pragma unroll
+        for (int j = 0; j < NB; ++j) {
+          const T root = op_sqrt(__shfl_sync(0xFFFFFFFFu, r[j], j));
+          r[j] = lane == j ? root : r[j] / root;
+          __syncwarp();
+          if (lane < NB) D[j * NB + lane] = r[j];
+          if (lane == j) pivot[j] = root;
+          __syncwarp();
+#pragma unroll
+          for (int k = j + 1; k < NB; ++k) r[k] = r[k] - r[j] * D[j * NB + k];
+        }
+      }
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < NB; ++j)
+        if (lane >= j && lane < nb) P[j * NP + c0 + lane] = r[j];
+      if (lane == 0) regular = fine ? 1 : 0;
+    }
+    __syncthreads();
+    const bool reg = regular != 0;
+    for (int i = c0 + nb + tid; i < N; i += TH) {
+      T x[NB];
+#pragma unroll
+      for (int k = 0; k < NB; ++k) x[k] = P[k * NP + i];
+#pragma unroll
+      for (int j = 0; j < NB; ++j) {
+        x[j] = reg ? lin_quotient(x[j], pivot[j], inverse[j]) : x[j] / pivot[j];
+#pragma unroll
+        for (int k4 = (j + 1) / 4; k4 < NB / 4; ++k4) {
+          const V4 c = diag4[j * (NB / 4) + k4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (4 * k4 + e > j) x[4 * k4 + e] = x[4 * k4 + e] - x[j] * c.v[e];
+        }
+        P[j * NP + i] = x[j];
+      }
+    }
+    __syncthreads();
+    for (int q = tid; q < m * NB; q += TH) {
+      const int k = LOWER ? q % NB : q / m, i = LOWER ? q / NB : q % m;
+      if (k < nb && i >= k) o[AT(c0 + i, c0 + k)] = P[k * NP + c0 + i];
+    }
+    const int r0 = c0 + nb, nt = (N - r0 + 3) / 4;   // rows below exist only under a full panel, so r0 is a multiple of 4
+    if (nt <= 16) {                                  // few rows left: 2 x 2 tiles, so that the block still has work for its warps
+      const int n2 = (N - r0 + 1) / 2;
+      for (int e = tid; e < n2 * (n2 + 1) / 2; e += TH) {
+        int ti, tk;
+        tile_of(e, ti, tk);
+        const int i0 = r0 + 2 * ti, k0 = r0 + 2 * tk;
+        T c[2][2];
+#pragma unroll
+        for (int y = 0; y < 2; ++y)
+#pragma unroll
+          for (int x = 0; x < 2; ++x) c[y][x] = (i0 + y < N && k0 + x <= i0 + y) ? s[AT(i0 + y, k0 + x)] : (T)0;
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
+          const V2 pi = *(const V2*)&P[q * NP + i0], pk = *(const V2*)&P[q * NP + k0];
+#pragma unroll
+          for (int y = 0; y < 2; ++y)
+#pragma unroll
+            for (int x = 0; x < 2; ++x) c[y][x] = c[y][x] - pi.v[y] * pk.v[x];
+        }
+#pragma unroll
+        for (int y = 0; y < 2; ++y)
+#pragma unroll
+          for (int x = 0; x < 2; ++x)
+            if (i0 + y < N && k0 + x <= i0 + y) o[AT(i0 + y, k0 + x)] = c[y][x];
+      }
+    } else {
+      for (int e = tid; e < nt * (nt + 1) / 2; e += TH) {
+        int ti, tk;
+        tile_of(e, ti, tk);
+        const int i0 = r0 + 4 * ti, k0 = r0 + 4 * tk;
+        const bool inner = ALIGNED && ti != tk && i0 + 4 <= N;      // whole vectors of four along memory
+        T c[4][4];                                   // [line][element of the line]
+#pragma unroll
+        for (int y = 0; y < 4; ++y) {
+          if (inner) {
+            const V4 t = *(const V4*)&s[LOWER ? AT(i0 + y, k0) : AT(i0, k0 + y)];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) c[y][x] = t.v[x];
+          } else {
+#pragma unroll
+            for (int x = 0; x < 4; ++x) { const int i = i0 + (LOWER ? y : x), k = k0 + (LOWER ? x : y); c[y][x] = (i < N && k <= i) ? s[AT(i, k)] : (T)0; }
+          }
+        }
+#pragma unroll 8
+        for (int q = 0; q < NB; ++q) {
+          const V4 pl = *(const V4*)&P[q * NP + (LOWER ? i0 : k0)], pe = *(const V4*)&P[q * NP + (LOWER ? k0 : i0)];
+#pragma unroll
+          for (int y = 0; y < 4; ++y)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) c[y][x] = c[y][x] - pl.v[y] * pe.v[x];
+        }
+#pragma unroll
+        for (int y = 0; y < 4; ++y) {
+          if (inner) {
+            V4 t;
+#pragma unroll
+            for (int x = 0; x < 4; ++x) t.v[x] = c[y][x];
+            *(V4*)&o[LOWER ? AT(i0 + y, k0) : AT(i0, k0 + y)] = t;
+          } else {
+#pragma unroll
+            for (int x = 0; x < 4; ++x) { const int i = i0 + (LOWER ? y : x), k = k0 + (LOWER ? x : y); if (i < N && k <= i) o[AT(i, k)] = c[y][x]; }
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+#undef AT
+}
+)SRC";
+    } else {
+      src << "  for (int e = threadIdx.x; e < N * N; e += " << kThreads << ") { const int i = e / N, j = e % N; o[AT(i, j)] = i >= j ? a[AT(i, j)] : (" << T << ")0; }\n";
+      src << "  __syncthreads();\n";
+      src << "  for (int j = 0; j < N; ++j) {\n";
+      src << "    if (threadIdx.x == 0) o[AT(j, j)] = op_sqrt(o[AT(j, j)]);\n    __syncthreads();\n";
+      src << "    const " << T << " d = o[AT(j, j)];\n";
+      src << "    for (int i = j + 1 + threadIdx.x; i < N; i += " << kThreads << ") o[AT(i, j)] = o[AT(i, j)] / d;\n    __syncthreads();\n";
+      src << "    const int m = N - j - 1;\n";
+      src << "    for (int e = threadIdx.x; e < m * m; e += " << kThreads << ") {\n      const int i = j + 1 + e / m, k = j + 1 + e % m;\n";
+      src << "      if (k <= i) o[AT(i, k)] = o[AT(i, k)] - o[AT(i, j)] * o[AT(k, j)];\n    }\n    __syncthreads();\n  }\n";
+      src << "#undef AT\n}\n";
+    }
     Step s;
     s.kind = Step::KERNEL;
     s.kernel = add_kernel(src.str(), "cholesky");
     s.label = op->name;
     s.grid[0] = (unsigned)batch; s.grid[1] = s.grid[2] = 1;
-    s.block[0] = kThreads; s.block[1] = s.block[2] = 1;
+    s.block[0] = (unsigned)threads; s.block[1] = s.block[2] = 1;
     s.args = {slot_of.at(out), slot_of.at(a)};
     s.n_outs = 1;
     plan.steps.push_back(std::move(s));
   }
 
   // stablehlo.triangular_solve (src/pjrt_plugin/ops/linalg.cc:573-660 of the reference): op(A) X = B or X op(A) = B for a
-  // batch of triangular A. One thread per right-hand-side vector (a column of B on the left side, a row on the right)
-  // substitutes forwards or backwards through its matrix, reading its earlier unknowns back from the result. As in the
-  // reference, a matrix with a zero on a diagonal that counts gives NaN for its whole solution.
+  // batch of triangular A. A warp per right-hand-side vector: lane l owns the unknowns l, l + 32, ... in registers, and
+  // step j hands unknown j to all lanes by a shuffle, which subtract its column from the rows they own. The chain per
+  // unknown is one shuffle and four dependent multiply-adds, whatever n is, as long as the matrix is at hand: its
+  // columns come in panels of NB through shared memory, the next panel in flight in registers meanwhile. A block holds
+  // four or eight vectors of one matrix: more would queue for shared memory (n / 32 reads a step and warp). 160 x 160,
+  // eight matrices, twelve vectors: 712 us for a thread per vector that read the matrix and its unknowns back from
+  // memory, 15 us now. Above n = 1024 (32 unknowns in a lane) the thread per vector stays. As in the reference, a
+  // matrix with a zero on a diagonal that counts gives NaN for its whole solution.
   void lower_triangular_solve(Op* op, Plan& plan, BlockState& st) {
     if (op->operands.size() != 2 || op->results.size() != 1) throw CompileError("stablehlo.triangular_solve: malformed operands");
     Value *a = op->operands[0], *bv = op->operands[1], *out = op->results[0];
@@ -2362,27 +2555,120 @@ struct Planner {
     const bool fwd = lower != flip;                        // ... and it is lower triangular: substitute forwards
     const std::string T = c_type(a->type.dt);
     std::ostringstream src;
+    const bool by_warp = n <= 1024;
+    // eight vectors a block once that still makes a wave of blocks, four below
+    const int64_t per_block = batch * ((vecs_per + 7) / 8) >= 148 ? 8 : 4;
     src << "extern \"C\" __global__ void __launch_bounds__(" << kThreads << ") @NAME@(" << signature({out}, {a, bv}) << ") {\n";
-    src << "  const long long t = (long long)blockIdx.x * " << kThreads << " + threadIdx.x;\n";
-    src << "  if (t >= " << batch * vecs_per << "LL) return;\n";
     src << "  const int N = " << n << ";\n";
-    src << "  const long long g = t / " << vecs_per << "LL, v = t % " << vecs_per << "LL;\n";
-    src << "  const " << T << "* A = in0 + g * N * N;\n";
-    src << "#define M(i, j) A[" << (flip ? "(long long)(j) * N + (i)" : "(long long)(i) * N + (j)") << "]\n";
-    src << "#define X(i) (g * " << rows * cols << "LL + " << (left ? "(long long)(i) * " + std::to_string(cols) + " + v" : "v * " + std::to_string(cols) + " + (i)") << ")\n";
-    src << "  bool singular = false;\n";
-    if (!unit) src << "  for (int i = 0; i < N; ++i) singular = singular || A[(long long)i * N + i] == (" << T << ")0;\n";
-    src << "  for (int q = 0; q < N; ++q) {\n    const int i = " << (fwd ? "q" : "N - 1 - q") << ";\n";
-    src << "    " << T << " acc = in1[X(i)];\n";
-    src << "    for (int j = " << (fwd ? "0; j < i" : "i + 1; j < N") << "; ++j) acc = acc - M(i, j) * out0[X(j)];\n";
-    src << "    out0[X(i)] = " << (unit ? "acc" : "acc / M(i, i)") << ";\n  }\n";
-    src << "  if (singular) for (int i = 0; i < N; ++i) out0[X(i)] = (" << T << ")__uint_as_float(0x7FC00000u);\n";
-    src << "#undef M\n#undef X\n}\n";
+    if (by_warp) {
+      const int64_t es = (int64_t)dt_size(a->type.dt), np = n | 1;            // an odd stride: no bank conflicts either way
+      int64_t nb = 32;
+      while (nb > 1 && nb * np * es > 46 * 1024) nb /= 2;
+      const int64_t groups = (vecs_per + per_block - 1) / per_block;
+      src << "  typedef " << T << " T;\n  const int NB = " << nb << ", NP = " << np << ", NR = " << (n + 31) / 32 << ", VB = " << per_block << ", TH = " << kThreads << ";\n";
+      src << "  const long long g = blockIdx.x / " << groups << "u;\n  const int v = (int)(blockIdx.x % " << groups << "u) * VB + (int)(threadIdx.x >> 5);\n";
+      src << "  const T* A = in0 + g * N * N;\n";
+      // unknowns in the order they are found: U(i) is the row of unknown i
+      src << "#define U(i) (" << (fwd ? "(i)" : "N - 1 - (i)") << ")\n";
+      src << "#define X(i) (g * " << rows * cols << "LL + " << (left ? "(long long)U(i) * " + std::to_string(cols) + " + v" : "(long long)v * " + std::to_string(cols) + " + U(i)") << ")\n";
+      // element q of the panel at column c0: consecutive threads read consecutive memory
+      src << "#define COL(q) " << (flip ? "((q) / N)" : "((q) % NB)") << "\n#define ROW(q) " << (flip ? "((q) % N)" : "((q) / NB)") << "\n";
+      src << "#define M(i, j) A[" << (flip ? "(long long)U(j) * N + U(i)" : "(long long)U(i) * N + U(j)") << "]\n";
+      src << "  const bool UNIT = " << (unit ? "true" : "false") << ";\n";
+      src << R"SRC(  __shared__ T panel[NB * NP];                       // [column of the panel][row]
+  const int tid = threadIdx.x, lane = tid & 31;
+  const bool mine = (tid >> 5) < VB && v < )SRC" << vecs_per << R"SRC(;
+  __shared__ int singular;
+  if (tid == 0) singular = 0;
+  bool zero = false;
+  if (!UNIT)
+    for (int i = tid; i < N; i += TH) zero = zero || A[(long long)i * N + i] == (T)0;
+  T acc[NR];
+#pragma unroll
+  for (int r = 0; r < NR; ++r) acc[r] = (mine && lane + 32 * r < N) ? in1[X(lane + 32 * r)] : (T)0;
+  const int PF = (NB * N + TH - 1) / TH;             // elements of a panel per thread
+  T next[PF];
+  auto fetch = [&](int c0) {
+#pragma unroll
+    for (int k = 0; k < PF; ++k) {
+      const int q = tid + k * TH, c = c0 + COL(q), i = ROW(q);
+      next[k] = (q < NB * N && c < N && i >= c) ? M(i, c) : (T)0;
+    }
+  };
+  fetch(0);
+  __syncthreads();
+  if (zero) singular = 1;                            // read behind the barriers of the panels
+#pragma unroll
+  for (int p = 0; p < NR; ++p) {
+    T x = acc[p];                                    // the unknown of this lane among 32 p ..
+#pragma unroll
+    for (int h = 0; h < 32 / NB; ++h) {
+      const int c0 = 32 * p + h * NB;
+      if (c0 < N) {
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < PF; ++k) {
+          const int q = tid + k * TH;
+          if (q < NB * N) panel[COL(q) * NP + ROW(q)] = next[k];
+        }
+        __syncthreads();
+        if (c0 + NB < N) fetch(c0 + NB);
+        if (mine) {
+          const int own = lane - h * NB;             // column of the panel that holds this lane's pivot
+          const T d = (!UNIT && own >= 0 && own < NB && 32 * p + lane < N) ? panel[own * NP + 32 * p + lane] : (T)1;
+          const T inv = (T)1 / d;
+          const bool reg = lin_regular(inv);
+          const int cols = N - c0 < NB ? N - c0 : NB;
+#pragma unroll 4
+          for (int j = 0; j < cols; ++j) {
+            const T* col = panel + j * NP;
+            const T sol = UNIT ? acc[p] : lin_div(acc[p], d, inv, reg);
+            const T xj = __shfl_sync(0xFFFFFFFFu, sol, h * NB + j);
+            if (lane == h * NB + j) x = xj;
+            if (32 * p + lane < N) acc[p] = acc[p] - (lane > h * NB + j ? col[32 * p + lane] : (T)0) * xj;
+#pragma unroll
+            for (int r = p + 1; r < NR; ++r)
+              if (32 * r + lane < N) acc[r] = acc[r] - col[32 * r + lane] * xj;
+          }
+        }
+      }
+    }
+    acc[p] = x;
+  }
+  if (mine)
+#pragma unroll
+    for (int r = 0; r < NR; ++r)
+      if (lane + 32 * r < N) out0[X(lane + 32 * r)] = singular ? (T)__uint_as_float(0x7FC00000u) : acc[r];
+#undef M
+#undef X
+#undef U
+#undef COL
+#undef ROW
+}
+)SRC";
+    } else {
+      src << "  const long long t = (long long)blockIdx.x * " << kThreads << " + threadIdx.x;\n";
+      src << "  if (t >= " << batch * vecs_per << "LL) return;\n";
+      src << "  const long long g = t / " << vecs_per << "LL, v = t % " << vecs_per << "LL;\n";
+      src << "  const " << T << "* A = in0 + g * N * N;\n";
+      src << "#define M(i, j) A[" << (flip ? "(long long)(j) * N + (i)" : "(long long)(i) * N + (j)") << "]\n";
+      src << "#define X(i) (g * " << rows * cols << "LL + " << (left ? "(long long)(i) * " + std::to_string(cols) + " + v" : "v * " + std::to_string(cols) + " + (i)") << ")\n";
+      src << "  bool singular = false;\n";
+      if (!unit) src << "  for (int i = 0; i < N; ++i) singular = singular || A[(long long)i * N + i] == (" << T << ")0;\n";
+      src << "  for (int q = 0; q < N; ++q) {\n    const int i = " << (fwd ? "q" : "N - 1 - q") << ";\n";
+      src << "    " << T << " acc = in1[X(i)];\n";
+      src << "    for (int j = " << (fwd ? "0; j < i" : "i + 1; j < N") << "; ++j) acc = acc - M(i, j) * out0[X(j)];\n";
+      src << "    out0[X(i)] = " << (unit ? "acc" : "acc / M(i, i)") << ";\n  }\n";
+      src << "  if (singular) for (int i = 0; i < N; ++i) out0[X(i)] = (" << T << ")__uint_as_float(0x7FC00000u);\n";
+      src << "#undef M\n#undef X\n}\n";
+    }
     Step s;
     s.kind = Step::KERNEL;
     s.kernel = add_kernel(src.str(), "triangular_solve");
     s.label = op->name;
-    s.grid[0] = (unsigned)((batch * vecs_per + kThreads - 1) / kThreads); s.grid[1] = s.grid[2] = 1;
+    const int64_t blocks = by_warp ? batch * ((vecs_per + per_block - 1) / per_block) : (batch * vecs_per + kThreads - 1) / kThreads;
+    if (blocks >= (1LL << 31)) throw CompileError("stablehlo.triangular_solve: too many right-hand sides");
+    s.grid[0] = (unsigned)blocks; s.grid[1] = s.grid[2] = 1;
     s.block[0] = kThreads; s.block[1] = s.block[2] = 1;
     s.args = {slot_of.at(out), slot_of.at(a), slot_of.at(bv)};
     s.n_outs = 1;
