@@ -123,6 +123,15 @@ bool dot16_geometry(Op* op, Dot16& d) {
   return gemm16_plan(g, true);
 }
 
+// chlo.top_k that one block per row selects (lower_top_k): rows long enough that a full sort costs more than a pass over
+// them, and few enough results that the maxima of the block's threads bound them (at least k of the threads' maxima
+// reach the k-th largest element, and twice as many threads keep that bound tight).
+int top_k_threads(int64_t n) { return n >= 8192 ? 1024 : n >= 2048 ? 512 : 256; }
+bool few_of_many(const TensorType& t, int64_t k) {
+  const int64_t n = t.dims.empty() ? 0 : t.dims.back();
+  return n >= 512 && n < (1LL << 30) && k >= 1 && k <= top_k_threads(n) / 2 && dt_size(t.dt) <= 4 && t.numel() > 0;
+}
+
 // ---------------------------------------------------------------------------
 // pass 1: inlining and pass-through removal
 // ---------------------------------------------------------------------------
@@ -454,7 +463,8 @@ struct Inliner {
     // and the multiply are evaluated inside the reduction kernel; nothing of the large shape is stored.
     // chlo.top_k (src/pjrt_plugin/ops/sort_fft_complex.cc:41-88): a stable descending sort of the values together with
     // their positions along the last dimension, of which the first k are kept. NaN goes after every number.
-    if (op->name == "chlo.top_k" && op->operands.size() == 1 && op->results.size() == 2) {
+    if (op->name == "chlo.top_k" && op->operands.size() == 1 && op->results.size() == 2 &&
+        !few_of_many(op->operands[0]->type, op->results[0]->type.dims.empty() ? 0 : op->results[0]->type.dims.back())) {
       Value* x = op->operands[0];
       const TensorType xt = x->type;
       const int R = xt.rank();
@@ -1194,7 +1204,7 @@ Cat categorize(Op* op) {
   if (sh == "reduce_window" || sh == "select_and_scatter") return Cat::WINDOW;
   if (sh == "sort") return Cat::SORT;
   if (sh == "rng_bit_generator") return Cat::RNG;
-  if (sh == "cholesky" || sh == "triangular_solve") return Cat::LINALG;
+  if (sh == "cholesky" || sh == "triangular_solve" || sh == "top_k") return Cat::LINALG;
   if (sh == "while") return Cat::WHILE;
   if (sh == "case") return Cat::CASE;
   if (sh == "all_reduce") return Cat::ALL_REDUCE;
@@ -1906,6 +1916,373 @@ struct Planner {
     return L;
   }
 
+  // A comparator that orders by one operand alone, in an order that the bits of a 32-bit key can be mapped to: floats in
+  // their total order, integers. `key`: that operand.
+  static bool radix_order(Op* op, size_t& key, bool& descending) {
+    Block* b = op->regions[0].get();
+    if (b->ops.size() != 2 || b->ops[0]->short_name() != "compare" || b->ops[1]->operands.size() != 1 || b->ops[0]->operands.size() != 2 ||
+        b->ops[1]->operands[0] != b->ops[0]->results[0])
+      return false;
+    Op* c = b->ops[0].get();
+    const std::string dir = attr_enum(c->attr("comparison_direction"));
+    if (dir != "LT" && dir != "GT") return false;
+    for (size_t q = 0; 2 * q + 1 < b->args.size(); q++) {
+      if (c->operands[0] != b->args[2 * q] || c->operands[1] != b->args[2 * q + 1]) continue;
+      const DT dt = op->operands[q]->type.dt;
+      const std::string ct = c->has("compare_type") ? attr_enum(c->attr("compare_type")) : "";
+      if (!(dt == DT::I32 || dt == DT::U32 || (dt == DT::F32 && ct == "TOTALORDER"))) return false;
+      key = q;
+      descending = dir == "GT";
+      return true;
+    }
+    return false;
+  }
+
+  // Stable ascending radix sort of the mapped keys of rows that are contiguous in memory, eight bits a pass. A warp takes
+  // 256 consecutive elements in eight rounds of 32; equal digits of a round find one another by eight ballots, and the
+  // ranks add up over rounds, warps and tiles in element order, so equal keys keep their order. What bounds the work is
+  // latency (a tile has a few thousand elements and a pass is a chain of ballots, two scans and a scatter), which is why
+  // a row of up to kRadixTile elements is sorted by one block that keeps it in shared memory through all four passes, and
+  // a longer row takes one launch per pass: a tile adds up the digit counts of the tiles in front of it itself instead of
+  // waiting for a scan kernel, and counts the next pass's digits where its elements land. Floats and integers of 32 bits
+  // with any riders; the merge sort below takes every other comparator. 16 rows of 30522 keys with positions: 114 us as
+  // a merge sort, 73 us here; 32 rows of 64000: 377 and 173; 8 rows of 4000: 45 and 28. (One row of 8000 is 57 us both
+  // ways, which is where the rule in lower_sort draws the line.)
+  static constexpr int kRadixTile = 4096;
+  bool lower_radix_sort(Op* op, size_t key, bool descending, int64_t rows, int64_t N, Plan& plan, BlockState& st) {
+    std::vector<Value*> ins(op->operands.begin(), op->operands.end()), outs(op->results.begin(), op->results.end());
+    const int64_t tiles = (N + kRadixTile - 1) / kRadixTile, numel = rows * N;
+    if (numel >= (1LL << 31) || rows * tiles * 1024 >= (1LL << 31)) return false;
+    const DT kd = ins[key]->type.dt;
+    const bool one = tiles == 1;
+    const int threads = one ? (int)std::min<int64_t>(512, (N + 255) / 256 * 32) : 512;
+    const std::string K = std::to_string(key);
+    auto head = [&](std::ostringstream& src) {
+      src << "  const int N = " << N << ", TH = " << threads << ", NW = TH / 32, TILES = " << tiles << ", T = " << kRadixTile << ";\n";
+      src << "  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;\n";
+      src << "  const u32 flip = " << (descending ? "0xFFFFFFFFu" : "0u") << ";\n";
+      if (kd == DT::F32)
+        src << "  auto map = [&](float v) -> u32 { const u32 u = __float_as_uint(v); return (u ^ ((u >> 31) ? 0xFFFFFFFFu : 0x80000000u)) ^ flip; };\n"
+               "  auto unmap = [&](u32 m) -> float { m ^= flip; return __uint_as_float(m ^ ((m >> 31) ? 0x80000000u : 0xFFFFFFFFu)); };\n";
+      else
+        src << "  auto map = [&](" << s_type(kd) << " v) -> u32 { return (u32)v ^ " << (kd == DT::I32 ? "0x80000000u" : "0u") << " ^ flip; };\n"
+            << "  auto unmap = [&](u32 m) -> " << s_type(kd) << " { return (" << s_type(kd) << ")(m ^ flip ^ " << (kd == DT::I32 ? "0x80000000u" : "0u") << "); };\n";
+    };
+    // ranks of this thread's eight elements among the equal digits of their warp, and the warp's digit counts
+    const char* rank = R"SRC(
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const bool ok = w * 256 + r * 32 + lane < cnt;
+      const u32 d = (kk[r] >> shift) & 255u;
+      u32 peers = __ballot_sync(0xFFFFFFFFu, ok);
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        const u32 vote = __ballot_sync(0xFFFFFFFFu, (d >> b) & 1u);
+        peers &= ((d >> b) & 1u) ? vote : ~vote;
+      }
+      const int before = __popc(peers & ((1u << lane) - 1u)), base = ok ? warps[w * 256 + d] : 0;
+      __syncwarp();
+      if (ok && before == 0) warps[w * 256 + d] = (u16)(base + __popc(peers));
+      __syncwarp();
+      rk[r] = base + before;
+    }
+)SRC";
+    // exclusive scan of 256 totals in `start` by the first warp, eight digits a lane
+    const char* scan = R"SRC(
+    if (w == 0) {
+      int c[8], sum = 0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) { c[q] = start[lane * 8 + q]; sum += c[q]; }
+      int incl = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xFFFFFFFFu, incl, o); if (lane >= o) incl += v; }
+      int run = incl - sum;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) { start[lane * 8 + q] = run; run += c[q]; }
+    }
+)SRC";
+    auto launch = [&](std::ostringstream& src, const char* stem, const std::string& label, std::vector<int> args, int n_outs) {
+      Step s;
+      s.kind = Step::KERNEL;
+      s.kernel = add_kernel(src.str(), stem);
+      s.label = label;
+      s.grid[0] = (unsigned)(rows * tiles); s.grid[1] = s.grid[2] = 1;
+      s.block[0] = (unsigned)threads; s.block[1] = s.block[2] = 1;
+      s.args = std::move(args);
+      s.n_outs = n_outs;
+      plan.steps.push_back(std::move(s));
+    };
+    std::vector<int> in_slots, out_slots;
+    for (auto* v : ins) in_slots.push_back(slot_of.at(v));
+    for (auto* v : outs) out_slots.push_back(slot_of.at(v));
+    if (one) {
+      std::ostringstream src;
+      src << "extern \"C\" __global__ void __launch_bounds__(" << threads << ") @NAME@(" << signature(outs, ins) << ") {\n";
+      head(src);
+      src << "  __shared__ u16 warps[NW * 256], sidx[NW * 256];\n  __shared__ u32 skey[NW * 256];\n  __shared__ int start[256];\n";
+      src << "  const long long base = (long long)blockIdx.x * N;\n  const int cnt = N;\n  u32 kk[8];\n  int ii[8], rk[8];\n";
+      src << "#pragma unroll\n  for (int r = 0; r < 8; ++r) { const int i = w * 256 + r * 32 + lane; ii[r] = i; kk[r] = i < N ? map(in" << K << "[base + i]) : 0u; }\n";
+      src << "  for (int shift = 0; shift < 32; shift += 8) {\n    for (int q = tid; q < NW * 256; q += TH) warps[q] = 0;\n    __syncthreads();\n" << rank;
+      src << R"SRC(    __syncthreads();
+    for (int d = tid; d < 256; d += TH) {
+      int run = 0;
+#pragma unroll
+      for (int q = 0; q < NW; ++q) { const int c = warps[q * 256 + d]; warps[q * 256 + d] = (u16)run; run += c; }
+      start[d] = run;
+    }
+    __syncthreads();)SRC" << scan << R"SRC(    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+      if (w * 256 + r * 32 + lane < cnt) {
+        const u32 d = (kk[r] >> shift) & 255u;
+        const int to = start[d] + warps[w * 256 + d] + rk[r];
+        skey[to] = kk[r];
+        sidx[to] = (u16)ii[r];
+      }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 8; ++r) { const int i = w * 256 + r * 32 + lane; if (i < cnt) { kk[r] = skey[i]; ii[r] = sidx[i]; } }
+  }
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    const int i = w * 256 + r * 32 + lane;
+    if (i < cnt) {
+)SRC";
+      for (size_t q = 0; q < ins.size(); q++)
+        src << "      out" << q << "[base + i] = " << (q == key ? "unmap(kk[r])" : "in" + std::to_string(q) + "[base + ii[r]]") << ";\n";
+      src << "    }\n  }\n}\n";
+      std::vector<int> args = out_slots;
+      args.insert(args.end(), in_slots.begin(), in_slots.end());
+      launch(src, "sort_tile", "sort (tile)", args, (int)ins.size());
+      return true;
+    }
+    TensorType et, ht;
+    et.dt = ht.dt = DT::U32;
+    et.dims = {numel};
+    ht.dims = {4 * rows * tiles * 256};
+    const int kbuf[2] = {new_slot(Slot::TEMP, et, st.arena), new_slot(Slot::TEMP, et, st.arena)};
+    const int ibuf[2] = {new_slot(Slot::TEMP, et, st.arena), new_slot(Slot::TEMP, et, st.arena)};
+    const int hist = new_slot(Slot::TEMP, ht, st.arena);
+    {
+      std::ostringstream src;
+      src << "extern \"C\" __global__ void __launch_bounds__(" << threads << ") @NAME@(int* __restrict__ hist, " << signature({}, {ins[key]}) << ") {\n";
+      head(src);
+      src << "  const long long HS = " << rows * tiles * 256 << "LL;\n";
+      src << R"SRC(  __shared__ int h[256];
+  if (tid < 256) h[tid] = 0;
+  __syncthreads();
+  const int row = blockIdx.x / TILES, t0 = (blockIdx.x % TILES) * T;
+#pragma unroll
+  for (int r = 0; r < T / TH; ++r) { const int i = t0 + r * TH + tid; if (i < N) atomicAdd(&h[map(in0[(long long)row * N + i]) & 255u], 1); }
+  __syncthreads();
+  if (tid < 256) {
+    int* to = hist + (long long)blockIdx.x * 256 + tid;
+    to[0] = h[tid];
+    to[HS] = 0; to[2 * HS] = 0; to[3 * HS] = 0;      // counted by the passes in front of theirs
+  }
+}
+)SRC";
+      launch(src, "sort_count", "sort (digit counts)", {hist, in_slots[key]}, 1);
+    }
+    for (int pass = 0; pass < 4; pass++) {
+      const bool first = pass == 0, last = pass == 3;
+      std::ostringstream src;
+      src << "extern \"C\" __global__ void __launch_bounds__(" << threads << ") @NAME@(";
+      if (last) src << signature(outs, ins);
+      else src << "u32* __restrict__ kout, u32* __restrict__ iout" << (first ? ", " + signature({}, ins) : "");
+      src << ", int* __restrict__ hist" << (first ? "" : ", const u32* __restrict__ kin, const u32* __restrict__ iin") << ") {\n";
+      head(src);
+      src << "  const int shift = " << 8 * pass << ";\n  const long long HS = " << rows * tiles * 256 << "LL;\n";
+      src << R"SRC(  __shared__ u16 warps[NW * 256];
+  __shared__ int start[256], ahead[256];
+  const int row = blockIdx.x / TILES, tile = blockIdx.x % TILES, t0 = tile * T;
+  const int cnt = N - t0 < T ? N - t0 : T;
+  const long long base = (long long)row * N;
+  u32 kk[8];
+  int ii[8], rk[8];
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    const int i = w * 256 + r * 32 + lane;
+)SRC";
+      if (first) src << "    kk[r] = i < cnt ? map(in" << K << "[base + t0 + i]) : 0u;\n    ii[r] = t0 + i;\n";
+      else src << "    kk[r] = i < cnt ? kin[base + t0 + i] : 0u;\n    ii[r] = i < cnt ? (int)iin[base + t0 + i] : 0;\n";
+      src << R"SRC(  }
+  if (tid < 256) {                                   // digits of the whole row, and of the tiles in front of this one
+    const int* h = hist + )SRC" << pass << R"SRC( * HS + (long long)row * TILES * 256 + tid;
+    int all = 0, front = 0;
+#pragma unroll 4
+    for (int t = 0; t < TILES; ++t) { const int c = h[t * 256]; front += t < tile ? c : 0; all += c; }
+    start[tid] = all;
+    ahead[tid] = front;
+  }
+  for (int q = tid; q < NW * 256; q += TH) warps[q] = 0;
+  __syncthreads();
+)SRC" << scan << rank << R"SRC(
+  __syncthreads();
+  if (tid < 256) {
+    int run = start[tid] + ahead[tid];
+    start[tid] = run;
+    run = 0;
+#pragma unroll
+    for (int q = 0; q < NW; ++q) { const int c = warps[q * 256 + tid]; warps[q * 256 + tid] = (u16)run; run += c; }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < 8; ++r)
+    if (w * 256 + r * 32 + lane < cnt) {
+      const u32 d = (kk[r] >> shift) & 255u;
+      const int to = start[d] + warps[w * 256 + d] + rk[r];
+)SRC";
+      if (last) {
+        for (size_t q = 0; q < ins.size(); q++)
+          src << "      out" << q << "[base + to] = " << (q == key ? "unmap(kk[r])" : "in" + std::to_string(q) + "[base + ii[r]]") << ";\n";
+      } else {
+        src << "      kout[base + to] = kk[r];\n      iout[base + to] = (u32)ii[r];\n";
+        src << "      atomicAdd(hist + " << pass + 1 << " * HS + ((long long)row * TILES + to / T) * 256 + ((kk[r] >> " << 8 * (pass + 1) << ") & 255u), 1);\n";
+      }
+      src << "    }\n}\n";
+      std::vector<int> args;
+      if (last) { args = out_slots; args.insert(args.end(), in_slots.begin(), in_slots.end()); }
+      else { args = {kbuf[pass & 1], ibuf[pass & 1]}; if (first) args.insert(args.end(), in_slots.begin(), in_slots.end()); }
+      args.push_back(hist);
+      if (!first) { args.push_back(kbuf[(pass & 1) ^ 1]); args.push_back(ibuf[(pass & 1) ^ 1]); }
+      launch(src, last ? "sort_pass_out" : "sort_pass", "sort (radix pass " + std::to_string(pass) + ")", args, last ? (int)ins.size() : 2);
+    }
+    return true;
+  }
+
+  // chlo.top_k of a few out of many (the rule is few_of_many). A block per row. The k-th largest of the threads'
+  // own maxima is a threshold that at least k elements reach, and for keys in no particular order hardly more do: it is
+  // found by a search over the key's bits, two at a time, that ends as soon as the number of maxima above is between k and
+  // about 1.5 k. The elements that reach it are collected in shared memory and each finds its place by counting the
+  // candidates in front of it (larger, or equal and earlier), so the result does not depend on the order of collection.
+  // More candidates than there is room for (rows of few distinct values, or whose large values share threads): the search
+  // goes on over all elements to the k-th largest itself, and the elements equal to it are taken in order of position.
+  // Bound by one pass over the row by one SM plus a chain of about 15 block barriers: 16 rows of 30522 floats, k = 50,
+  // took 111 us as a full sort and two slices, 12 us here.
+  void lower_top_k(Op* op, Plan& plan, BlockState& st) {
+    Value *x = op->operands[0], *vals = op->results[0], *pos = op->results[1];
+    if (!slot_of.count(x)) throw CompileError("internal: operand of top_k has no storage");
+    ensure_slot(vals, st);
+    ensure_slot(pos, st);
+    const int64_t N = x->type.dims.back(), rows = x->type.numel() / N, k = vals->type.dims.back();
+    if (rows >= (1LL << 31)) throw CompileError("chlo.top_k: too many rows");
+    const int threads = top_k_threads(N);
+    const int64_t per = (N + threads - 1) / threads;
+    const bool held = per <= 32;                           // the row's keys stay in registers
+    const DT dt = x->type.dt;
+    std::ostringstream src;
+    src << "extern \"C\" __global__ void __launch_bounds__(" << threads << ") @NAME@(" << signature({vals, pos}, {x}) << ") {\n";
+    src << "  const int N = " << N << ", K = " << k << ", TH = " << threads << ", PER = " << per << ", CAP = 2048;\n";
+    src << "  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;\n";
+    src << "  const long long base = (long long)blockIdx.x * N;\n";
+    // larger keys go first; NaN goes after every number and is equal to itself, -0 is equal to +0
+    src << "  auto key_at = [&](int i) -> u32 { const " << c_type(dt) << " v = " << load_expr(x, "in0", "base + i") << ";\n";
+    if (dt_is_float(dt)) src << "    if (v != v) return 0u;\n    const u32 u = __float_as_uint(v + 0.0f);\n    return u ^ ((u >> 31) ? 0xFFFFFFFFu : 0x80000000u); };\n";
+    else src << "    return (u32)v" << (dt_is_signed(dt) ? " ^ 0x80000000u" : "") << "; };\n";
+    src << R"SRC(  __shared__ u32 ckey[CAP];
+  __shared__ int cidx[CAP], total[64], found, share[TH / 32];
+  if (tid < 64) total[tid] = 0;
+  if (tid == 0) found = 0;
+)SRC";
+    if (held) src << "  u32 key[PER];\n#pragma unroll\n  for (int j = 0; j < PER; ++j) key[j] = tid + j * TH < N ? key_at(tid + j * TH) : 0u;\n#define KEY(j) key[j]\n";
+    else src << "#define KEY(j) (tid + (j) * TH < N ? key_at(tid + (j) * TH) : 0u)\n";
+    src << "#define EACH " << (held ? "_Pragma(\"unroll\")" : "_Pragma(\"unroll 8\")") << " for (int j = 0; j < PER; ++j)\n";
+    src << R"SRC(  u32 most = 0u;
+  EACH { const u32 v = KEY(j); most = v > most ? v : most; }
+  __syncthreads();
+  u32 least = 0u;                                    // at least K maxima reach it
+  for (int b = 30, q = 0; b >= 0; b -= 2, q += 3) {
+#pragma unroll
+    for (int s = 1; s < 4; ++s) {
+      const u32 vote = __ballot_sync(0xFFFFFFFFu, most >= (least | ((u32)s << b)));
+      if (lane == 0 && vote) atomicAdd(&total[q + s - 1], __popc(vote));
+    }
+    __syncthreads();
+    int reached = TH;
+#pragma unroll
+    for (int s = 3; s > 0; --s)
+      if (total[q + s - 1] >= K) { least |= (u32)s << b; reached = total[q + s - 1]; break; }
+    if (reached <= K + K / 2 + 8) break;
+  }
+  EACH {
+    const int i = tid + j * TH;
+    if (i < N) {
+      const u32 v = KEY(j);
+      if (v >= least) {
+        const int at = atomicAdd(&found, 1);
+        if (at < CAP) { ckey[at] = v; cidx[at] = i; }
+      }
+    }
+  }
+  __syncthreads();
+  int count = found;
+  if (count > CAP) {
+    // the K-th largest key of the row, bit by bit
+    u32 kth = 0u;
+    for (int b = 31; b >= 0; --b) {
+      const u32 trial = kth | (1u << b);
+      __syncthreads();
+      if (tid == 0) found = 0;
+      __syncthreads();
+      int mine = 0;
+      EACH mine += (tid + j * TH < N && KEY(j) >= trial) ? 1 : 0;
+      if (mine) atomicAdd(&found, mine);
+      __syncthreads();
+      if (found >= K) kth = trial;
+    }
+    __syncthreads();
+    if (tid == 0) found = 0;
+    __syncthreads();
+    EACH {
+      const int i = tid + j * TH;
+      if (i < N) {
+        const u32 v = KEY(j);
+        if (v > kth) { const int at = atomicAdd(&found, 1); ckey[at] = v; cidx[at] = i; }
+      }
+    }
+    __syncthreads();
+    int taken = found;                               // below K; the rest are the first positions whose key is the K-th largest
+    for (int j = 0; j < PER && taken < K; ++j) {
+      const int i = tid + j * TH;
+      const bool eq = i < N && key_at(i) == kth;
+      const u32 vote = __ballot_sync(0xFFFFFFFFu, eq);
+      if (lane == 0) share[w] = __popc(vote);
+      __syncthreads();
+      int front = taken, all = 0;
+      for (int q = 0; q < TH / 32; ++q) { front += q < w ? share[q] : 0; all += share[q]; }
+      const int at = front + __popc(vote & ((1u << lane) - 1u));
+      if (eq && at < K) { ckey[at] = kth; cidx[at] = i; }
+      taken += all;
+      __syncthreads();
+    }
+    count = K;
+  }
+  for (int c = tid; c < count; c += TH) {
+    const u32 v = ckey[c];
+    const int i = cidx[c];
+    int place = 0;
+    for (int o = 0; o < count; ++o) { const u32 u = ckey[o]; place += (u > v || (u == v && cidx[o] < i)) ? 1 : 0; }
+    if (place < K) {
+      out0[(long long)blockIdx.x * K + place] = in0[base + i];
+      out1[(long long)blockIdx.x * K + place] = i;
+    }
+  }
+#undef KEY
+#undef EACH
+}
+)SRC";
+    Step s;
+    s.kind = Step::KERNEL;
+    s.kernel = add_kernel(src.str(), "top_k");
+    s.label = "top_k";
+    s.grid[0] = (unsigned)rows; s.grid[1] = s.grid[2] = 1;
+    s.block[0] = (unsigned)threads; s.block[1] = s.block[2] = 1;
+    s.args = {slot_of.at(vals), slot_of.at(pos), slot_of.at(x)};
+    s.n_outs = 2;
+    plan.steps.push_back(std::move(s));
+  }
+
   // stablehlo.sort (src/pjrt_plugin/ops/sort_fft_complex.cc:135-250 of the reference, which recognises ascending and
   // descending comparators; here the comparator region is compiled as it stands). A stable merge sort over a
   // permutation: a block sorts a tile of up to kSortTile elements of one row in shared memory, starting from runs of
@@ -1942,6 +2319,12 @@ struct Planner {
     const int64_t tiles = (N + kSortTile - 1) / kSortTile;
     if (rows * tiles >= (1LL << 31)) throw CompileError("stablehlo.sort: too many rows");
     const bool one_tile = tiles == 1;
+
+    if (inner == 1 && N >= 128 && (N <= kRadixTile || N * rows >= 16384)) {
+      size_t key = 0;
+      bool descending = false;
+      if (radix_order(op, key, descending) && lower_radix_sort(op, key, descending, rows, N, plan, st)) return;
+    }
 
     // shared pieces of source text
     auto comparator = [&](Emitter& e) {
@@ -4820,6 +5203,7 @@ struct Planner {
         }
         case Cat::LINALG: {
           if (op->short_name() == "cholesky") lower_cholesky(op, plan, st);
+          else if (op->short_name() == "top_k") lower_top_k(op, plan, st);
           else lower_triangular_solve(op, plan, st);
           break;
         }
