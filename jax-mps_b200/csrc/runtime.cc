@@ -270,14 +270,28 @@ Completion& completion() {
 
 }  // namespace
 
-// Error counter of the device as one execution saw it: the word before its first kernel and after its last, copied
-// into pinned memory on the compute stream. The execution failed (a bounded device-side wait ran out) when the two
-// differ once the copies have landed.
+// One pinned word that a copy of the device's error counter lands in, from the client's block of them.
+struct StatusWord {
+  b200_client* client;
+  int index;
+  volatile int* word;
+  ~StatusWord();
+};
+
+// Error counter of the device as one execution saw it: before its first kernel and after its last. The execution failed
+// (a bounded device-side wait ran out) when the two differ once the copies have landed. Executions follow one another on
+// the compute stream, so the counter behind one is the counter in front of the next: one copy per execution. Plans
+// whose kernels wait for nothing are not watched at all.
 struct ExecStatus {
-  volatile int* pair = nullptr;   // pinned: [0] before, [1] after
-  std::function<void(volatile int*)> release;
-  ~ExecStatus() { if (release && pair) release(pair); }
-  bool failed() const { return pair && pair[1] != pair[0]; }
+  std::shared_ptr<StatusWord> before, after;
+  bool failed() const { return before && after && *after->word != *before->word; }
+};
+
+// An event from the client's pool, recorded once; all results of an execution share theirs.
+struct ReadyEvent {
+  b200_client* client;
+  cudaEvent_t ev;
+  ~ReadyEvent();
 };
 
 struct b200_event {
@@ -294,8 +308,7 @@ struct b200_event {
 struct PinnedBlock {
   void* ptr = nullptr;
   size_t size = 0;
-  cudaEvent_t ev = nullptr;
-  bool in_flight = false;
+  std::shared_ptr<ReadyEvent> reader;   // the copy that reads it
 };
 
 struct LoadedProgram {
@@ -315,10 +328,18 @@ struct LoadedProgram {
   // Graphs of data-dependent loops and cases (conditional nodes), per step and per set of addresses of the slots the
   // step and everything below it touches.
   std::vector<LoopGraph> cond_graphs;
+  // Graphs of the whole plan, per set of argument and result addresses that came back (replay_plan).
+  struct PlanGraph { std::vector<void*> ptrs; cudaGraphExec_t exec; int launches; uint64_t used; };
+  std::vector<PlanGraph> plan_graphs;
+  bool replayable = false;                     // the plan only launches kernels and device copies, and enough of them
+  uint64_t calls = 0, replays = 0, recordings = 0;
+  bool watched = false;                        // some kernel of the plan has a bounded wait that can run out
   ~LoadedProgram() {
     for (auto& g : loop_graphs)
       if (g.exec) cudaGraphExecDestroy(g.exec);
     for (auto& g : cond_graphs)
+      if (g.exec) cudaGraphExecDestroy(g.exec);
+    for (auto& g : plan_graphs)
       if (g.exec) cudaGraphExecDestroy(g.exec);
     for (auto* a : arenas)
       if (a) cudaFree(a);
@@ -353,12 +374,28 @@ struct b200_client {
   bool profiling = false;
   // debugging switches of the contraction kernels and the loop executor, read from the environment once at creation
   struct Switches { bool no_vec_gather = false, no_seg_gather = false, no_tmem_a = false, no_half_ctas = false, narrow_tiles = false,
-                    no_loop_graphs = false, no_tma_a = false, no_pdl = false, no_device_cf = false; } sw;
+                    no_loop_graphs = false, no_tma_a = false, no_pdl = false, no_device_cf = false, no_plan_graphs = false; } sw;
   int reported_errors = 0;              // value of the error word at the last b200_client_synchronize
   int armed_wait_polls = 0;             // test hook: the next execution starts with a wait that runs out
-  int* status_block = nullptr;          // pinned pairs handed to executions
-  std::vector<int> free_status;         // free pair indices
-  static constexpr int kStatusPairs = 4096;
+  int* status_block = nullptr;          // pinned words handed to executions
+  static constexpr int kStatusWords = 8192;
+  std::shared_ptr<StatusWord> last_status;      // the counter behind the last watched execution; null: not known
+  // Small parts that executions and buffers hand back and forth: free status words and events (under a lock of their
+  // own, taken by destructors on any thread).
+  std::mutex parts_mu;
+  std::vector<int> free_status;
+  std::vector<cudaEvent_t> free_events;
+  static constexpr size_t kEventPool = 1024;
+  // Device blocks of up to kBlockMax bytes that were freed on the compute stream and go back to allocations of the same
+  // size on it, oldest out first. A call to the stream-ordered pool costs about as much as a kernel launch, which is
+  // what a small program is made of.
+  struct FreeBlock { size_t bytes; void* ptr; };
+  std::deque<FreeBlock> free_blocks;
+  static constexpr size_t kBlockMax = 1 << 20, kBlockPool = 64;
+  // Copies to the device carry a number in the order of the copy stream; the compute stream is behind all copies up to
+  // h2d_waited, so that a program waits once for the newest of its arguments and not again in its next call.
+  uint64_t h2d_seq = 0, h2d_waited = 0;
+  const ReadyEvent* tail = nullptr;     // the event at the end of the compute stream; null when something went in behind it
   struct ProfEntry { std::string kind; double ms = 0; long long count = 0; };
   std::map<std::string, ProfEntry> profile;
   int64_t total_mem = 0;
@@ -381,13 +418,25 @@ struct b200_buffer {
   size_t bytes = 0;
   b200_dtype dtype = B200_INVALID;
   std::vector<int64_t> dims;
-  cudaEvent_t ready = nullptr;                 // recorded on the producing stream
+  std::shared_ptr<ReadyEvent> ready;           // recorded on the producing stream
   cudaStream_t ready_on = nullptr;             // that stream: work issued to it later needs no wait
-  struct Block { void* base; int refs; };      // one device allocation shared by several results of an execution
+  uint64_t ready_seq = 0;                      // on the copy stream: the number of the copy
+  struct Block { void* base; size_t bytes; int refs; };      // one device allocation shared by several results of an execution
   Block* block = nullptr;                      // non-null: ptr lies inside block->base, freed with its last buffer
-  std::vector<cudaEvent_t> reads;              // pending reads on other streams
+  std::vector<std::shared_ptr<ReadyEvent>> reads;   // pending reads on other streams
   bool deleted = false;
 };
+
+StatusWord::~StatusWord() {
+  std::lock_guard<std::mutex> l(client->parts_mu);
+  client->free_status.push_back(index);
+}
+ReadyEvent::~ReadyEvent() {
+  if (!ev) return;
+  std::lock_guard<std::mutex> l(client->parts_mu);
+  if (client->free_events.size() < b200_client::kEventPool) client->free_events.push_back(ev);
+  else cudaEventDestroy(ev);
+}
 
 struct b200_profiler {
   bool running = false;
@@ -405,9 +454,51 @@ b200_error* set_device(b200_client* c) {
   return nullptr;
 }
 
+// Host copies up to here are made on the compute stream and through pinned staging.
+constexpr size_t kSmallCopy = 64 << 10;
+
+size_t block_bytes(size_t bytes) { return (std::max<size_t>(bytes, 16) + 511) & ~(size_t)511; }
+
+void release_blocks(b200_client* c) {
+  for (auto& f : c->free_blocks) cudaFreeAsync(f.ptr, c->compute);
+  c->free_blocks.clear();
+}
+
+// A block on the compute stream or, for `stream` the copy stream, from the pool itself (whose blocks the compute stream
+// may still be using are not for other streams). Not counted as an allocation of the client.
+cudaError_t block_alloc(b200_client* c, size_t bytes, cudaStream_t stream, void** out) {
+  const size_t n = block_bytes(bytes);
+  if (stream == c->compute && n <= b200_client::kBlockMax)
+    for (auto it = c->free_blocks.rbegin(); it != c->free_blocks.rend(); ++it)
+      if (it->bytes == n) {
+        *out = it->ptr;
+        c->free_blocks.erase(std::next(it).base());
+        return cudaSuccess;
+      }
+  cudaError_t e = cudaMallocAsync(out, n, stream);
+  if (e != cudaSuccess && !c->free_blocks.empty()) {     // give what is kept back and try once more
+    cudaGetLastError();
+    release_blocks(c);
+    cudaStreamSynchronize(c->compute);
+    e = cudaMallocAsync(out, n, stream);
+  }
+  return e;
+}
+
+// Frees a block in the order of the compute stream.
+void block_free(b200_client* c, void* ptr, size_t bytes) {
+  const size_t n = block_bytes(bytes);
+  if (n > b200_client::kBlockMax) { cudaFreeAsync(ptr, c->compute); return; }
+  c->free_blocks.push_back({n, ptr});
+  if (c->free_blocks.size() > b200_client::kBlockPool) {
+    cudaFreeAsync(c->free_blocks.front().ptr, c->compute);
+    c->free_blocks.pop_front();
+  }
+}
+
 b200_error* device_alloc(b200_client* c, size_t bytes, cudaStream_t stream, void** out) {
   size_t n = std::max<size_t>(bytes, 16);
-  cudaError_t e = cudaMallocAsync(out, n, stream);
+  cudaError_t e = block_alloc(c, n, stream, out);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return make_error(B200_RESOURCE_EXHAUSTED, "device allocation of " + std::to_string(n) + " bytes failed: " +
@@ -415,6 +506,27 @@ b200_error* device_alloc(b200_client* c, size_t bytes, cudaStream_t stream, void
   }
   c->note_alloc(n);
   return nullptr;
+}
+
+std::shared_ptr<StatusWord> new_status_word(b200_client* c) {
+  std::lock_guard<std::mutex> l(c->parts_mu);
+  if (c->free_status.empty()) return nullptr;
+  const int k = c->free_status.back();
+  c->free_status.pop_back();
+  return std::shared_ptr<StatusWord>(new StatusWord{c, k, c->status_block + k});
+}
+
+// A pooled event recorded at the end of `stream`.
+cudaError_t record_ready(b200_client* c, cudaStream_t stream, std::shared_ptr<ReadyEvent>* out) {
+  cudaEvent_t ev = nullptr;
+  {
+    std::lock_guard<std::mutex> l(c->parts_mu);
+    if (!c->free_events.empty()) { ev = c->free_events.back(); c->free_events.pop_back(); }
+  }
+  if (!ev)
+    if (cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) return e;
+  *out = std::shared_ptr<ReadyEvent>(new ReadyEvent{c, ev});
+  return cudaEventRecord(ev, stream);
 }
 
 b200_event* new_event_on(b200_client* c, cudaStream_t stream, b200_error** err) {
@@ -430,14 +542,22 @@ b200_event* new_event_on(b200_client* c, cudaStream_t stream, b200_error** err) 
   return e;
 }
 
+// The compute stream waits for a buffer that the copy stream produced, unless it is behind that copy already.
+cudaError_t wait_for_copy(b200_client* c, const b200_buffer* b) {
+  if (b->ready_on == c->compute || b->ready_seq <= c->h2d_waited) return cudaSuccess;
+  c->h2d_waited = b->ready_seq;
+  c->tail = nullptr;
+  return cudaStreamWaitEvent(c->compute, b->ready->ev, 0);
+}
+
 // Pinned staging blocks are reused once the copy that read them has finished.
 void* acquire_pinned(b200_client* c, size_t bytes, int* index) {
   for (size_t i = 0; i < c->pinned.size(); i++) {
     PinnedBlock& b = c->pinned[i];
     if (b.size < bytes) continue;
-    if (b.in_flight) {
-      if (cudaEventQuery(b.ev) != cudaSuccess) continue;
-      b.in_flight = false;
+    if (b.reader) {
+      if (cudaEventQuery(b.reader->ev) != cudaSuccess) continue;
+      b.reader.reset();
     }
     *index = (int)i;
     return b.ptr;
@@ -450,7 +570,6 @@ void* acquire_pinned(b200_client* c, size_t bytes, int* index) {
     return nullptr;
   }
   nb.size = sz;
-  cudaEventCreateWithFlags(&nb.ev, cudaEventDisableTiming);
   c->pinned.push_back(nb);
   *index = (int)c->pinned.size() - 1;
   return nb.ptr;
@@ -571,18 +690,29 @@ struct ExecCtx {
 
 b200_error* run_plan(ExecCtx& x, const Plan& plan);
 
+// Whether a kernel of the plan has a bounded wait (tensor-core pipelines; data-dependent loops, which are bounded in time).
+bool waits_inside(const Plan& plan) {
+  for (const Step& s : plan.steps) {
+    if (s.kind == Step::IGEMM || s.kind == Step::GEMM16 || (s.kind == Step::WHILE && s.trip_count < 0)) return true;
+    for (auto& p : s.sub)
+      if (p && waits_inside(*p)) return true;
+  }
+  return false;
+}
+
 // A plan can be recorded into a CUDA graph when it only launches kernels and device copies: no host round trip
 // (data-dependent loops, case), no collective.
-bool graph_safe(const Plan& plan) {
-  for (const Step& s : plan.steps) {
-    switch (s.kind) {
-      case Step::KERNEL: case Step::IGEMM: case Step::MEMCPY: case Step::GEMM16: case Step::REPACK16: case Step::TRANSPOSE: break;
-      case Step::WHILE:
-        if (s.trip_count < 0 || !graph_safe(*s.sub[1])) return false;
-        break;
-      default: return false;
-    }
+bool graph_safe(const Plan& plan);
+bool graph_safe_step(const Step& s) {
+  switch (s.kind) {
+    case Step::KERNEL: case Step::IGEMM: case Step::MEMCPY: case Step::GEMM16: case Step::REPACK16: case Step::TRANSPOSE: return true;
+    case Step::WHILE: return s.trip_count >= 0 && graph_safe(*s.sub[1]);
+    default: return false;
   }
+}
+bool graph_safe(const Plan& plan) {
+  for (const Step& s : plan.steps)
+    if (!graph_safe_step(s)) return false;
   return true;
 }
 
@@ -1186,6 +1316,69 @@ b200_error* run_plan(ExecCtx& x, const Plan& plan) {
   return nullptr;
 }
 
+// A plan of many small kernels is bound by the host: a launch costs it two to four microseconds, a graph of all of them a
+// few. The addresses of arguments and results are part of a recording, and programs that run in a loop come back to the
+// same few sets of them (results return to the pool and are handed out again), so a set is recorded when it is seen for
+// the second time and replayed from then on; everything else is launched step by step as before. Bounded: at most
+// kPlanGraphs recordings are kept, the least recently used goes first, and a program whose addresses keep changing stops
+// recording (a recording has to pay for itself in replays).
+constexpr size_t kPlanGraphs = 12;
+constexpr int kReplayLaunches = 6;
+
+b200_error* run_main(ExecCtx& x) {
+  LoadedProgram& lp = *x.lp;
+  b200_client* c = x.c;
+  const Plan& plan = lp.prog->main;
+  if (!lp.replayable || c->profiling || c->sw.no_plan_graphs) return run_plan(x, plan);
+  lp.calls++;
+  std::vector<void*> key;
+  for (size_t s = 0; s < lp.prog->slots.size(); s++)
+    if (lp.prog->slots[s].kind == Slot::ARG || lp.prog->slots[s].kind == Slot::RESULT) key.push_back(x.ptrs[s]);
+  LoadedProgram::PlanGraph* hit = nullptr;
+  for (auto& g : lp.plan_graphs)
+    if (g.ptrs == key) { hit = &g; break; }
+  if (hit && hit->exec) {
+    hit->used = lp.calls;
+    lp.replays++;
+    CUDA_TRY(cudaGraphLaunch(hit->exec, c->compute));
+    x.launches += hit->launches;
+    return nullptr;
+  }
+  if (!hit) {
+    if (lp.plan_graphs.size() >= kPlanGraphs) {
+      auto old = std::min_element(lp.plan_graphs.begin(), lp.plan_graphs.end(), [](auto& a, auto& b) { return a.used < b.used; });
+      if (old->exec) {
+        CUDA_TRY(cudaStreamSynchronize(c->compute));
+        cudaGraphExecDestroy(old->exec);
+      }
+      lp.plan_graphs.erase(old);
+    }
+    lp.plan_graphs.push_back({std::move(key), nullptr, 0, lp.calls});
+    return run_plan(x, plan);
+  }
+  hit->used = lp.calls;
+  if (lp.recordings > 2 * kPlanGraphs + lp.replays / 16) return run_plan(x, plan);
+  lp.recordings++;
+  const int before = x.launches;
+  CUDA_TRY(cudaStreamBeginCapture(c->compute, cudaStreamCaptureModeRelaxed));
+  b200_error* err = run_plan(x, plan);
+  cudaGraph_t graph = nullptr;
+  cudaError_t ce = cudaStreamEndCapture(c->compute, &graph);
+  if (err) {
+    if (graph) cudaGraphDestroy(graph);
+    return err;
+  }
+  CUDA_TRY(ce);
+  cudaGraphExec_t exec = nullptr;
+  ce = cudaGraphInstantiate(&exec, graph, 0);
+  cudaGraphDestroy(graph);
+  CUDA_TRY(ce);
+  hit->exec = exec;
+  hit->launches = x.launches - before;
+  CUDA_TRY(cudaGraphLaunch(exec, c->compute));
+  return nullptr;
+}
+
 uint64_t hash_text(const char* s, size_t n, uint64_t seed) {
   uint64_t h = 1469598103934665603ull ^ seed;
   for (size_t i = 0; i < n; i++) { h ^= (unsigned char)s[i]; h *= 1099511628211ull; }
@@ -1269,9 +1462,9 @@ b200_error* create_client(const b200_client_options* o, ncclComm_t given_comm, b
   CUDA_TRY(cudaMalloc((void**)&c->error_flag, sizeof(int)));
   CUDA_TRY(cudaMalloc((void**)&c->loop_guard, sizeof(unsigned long long)));
   CUDA_TRY(cudaMemset(c->error_flag, 0, sizeof(int)));
-  CUDA_TRY(cudaMallocHost((void**)&c->status_block, 2 * sizeof(int) * b200_client::kStatusPairs));
-  memset(c->status_block, 0, 2 * sizeof(int) * b200_client::kStatusPairs);
-  for (int k = b200_client::kStatusPairs - 1; k >= 0; k--) c->free_status.push_back(k);
+  CUDA_TRY(cudaMallocHost((void**)&c->status_block, sizeof(int) * b200_client::kStatusWords));
+  memset(c->status_block, 0, sizeof(int) * b200_client::kStatusWords);
+  for (int k = b200_client::kStatusWords - 1; k >= 0; k--) c->free_status.push_back(k);
   if (const char* e2 = getenv("B200_NO_TENSOR_CORES")) c->tensor_cores = atoi(e2) == 0;
   c->sw.no_vec_gather = getenv("B200_NO_VEC_GATHER") != nullptr;
   c->sw.no_seg_gather = getenv("B200_NO_SEG_GATHER") != nullptr;
@@ -1282,6 +1475,7 @@ b200_error* create_client(const b200_client_options* o, ncclComm_t given_comm, b
   c->sw.no_tma_a = getenv("B200_NO_TMA_A") != nullptr;
   c->sw.no_pdl = getenv("B200_NO_PDL") != nullptr;
   c->sw.no_device_cf = getenv("B200_NO_DEVICE_CONTROL_FLOW") != nullptr;
+  c->sw.no_plan_graphs = getenv("B200_NO_PLAN_GRAPHS") != nullptr;
   if (const char* lim = getenv("B200_WHILE_TIME_LIMIT_S")) c->while_limit_s = std::max(0.001, atof(lim));
   set_programmatic_launch(!c->sw.no_pdl);
   set_igemm_programmatic_launch(!c->sw.no_pdl && !getenv("B200_NO_IGEMM_PDL"));
@@ -1326,11 +1520,15 @@ b200_error* b200_client_destroy(b200_client* c) {
   cudaSetDevice(c->ordinal);
   cudaDeviceSynchronize();
   c->cache.clear();
+  c->last_status.reset();
+  release_blocks(c);
   if (c->comm) nccl().CommDestroy(c->comm);
   for (auto& b : c->pinned) {
+    b.reader.reset();
     cudaFreeHost(b.ptr);
-    cudaEventDestroy(b.ev);
   }
+  for (auto ev : c->free_events) cudaEventDestroy(ev);
+  c->free_events.clear();
   if (c->pred_host) cudaFreeHost(c->pred_host);
   if (c->loop_guard) cudaFree(c->loop_guard);
   if (c->status_block) cudaFreeHost(c->status_block);
@@ -1475,6 +1673,9 @@ b200_error* b200_client_compile(b200_client* c, const char* code, size_t code_si
       else fputs(lp->prog->dump.c_str(), stderr);
     }
     if (auto* e = build_kernels(*lp)) return e;
+    lp->watched = waits_inside(lp->prog->main);
+    lp->replayable = (int)lp->prog->main.steps.size() >= kReplayLaunches;
+    for (const Step& st : lp->prog->main.steps) lp->replayable = lp->replayable && st.kind != Step::WHILE && (graph_safe_step(st) || st.kind == Step::SCATTER);
     // constants: one device block, uploaded once
     CompiledProgram& p = *lp->prog;
     size_t total = 0;
@@ -1680,24 +1881,29 @@ b200_error* b200_buffer_from_host(b200_client* c, const void* data, b200_dtype d
   b->dtype = dtype;
   b->dims.assign(dims, dims + nd);
   b->bytes = bytes;
-  if (auto* e = device_alloc(c, bytes, c->h2d, &b->ptr)) return e;
+  // A small array goes through pinned staging on the compute stream itself: what uses it comes later on that stream
+  // anyway, and the copy takes less than making another stream's copy a dependency of the program would.
+  const bool small = bytes <= kSmallCopy;
+  const cudaStream_t stream = small ? c->compute : c->h2d;
+  if (auto* e = device_alloc(c, bytes, stream, &b->ptr)) return e;
   bool host_ready_now = true;
+  int staged = -1;
   if (bytes) {
-    cudaPointerAttributes attr;
-    bool pinned = dense && cudaPointerGetAttributes(&attr, data) == cudaSuccess && attr.type == cudaMemoryTypeHost;
-    cudaGetLastError();
+    bool pinned = false;
+    if (!small && dense) {
+      cudaPointerAttributes attr;
+      pinned = cudaPointerGetAttributes(&attr, data) == cudaSuccess && attr.type == cudaMemoryTypeHost;
+      cudaGetLastError();
+    }
     if (pinned) {
       CUDA_TRY(cudaMemcpyAsync(b->ptr, data, bytes, cudaMemcpyHostToDevice, c->h2d));
       host_ready_now = false;
     } else if (bytes <= (256u << 20)) {
-      int idx = -1;
-      void* stage = acquire_pinned(c, bytes, &idx);
+      void* stage = acquire_pinned(c, bytes, &staged);
       if (!stage) return make_error(B200_RESOURCE_EXHAUSTED, "cannot allocate pinned staging memory");
       if (dense) memcpy(stage, data, bytes);
       else pack_strided((const char*)data, (char*)stage, dims, byte_strides, nd, es);
-      CUDA_TRY(cudaMemcpyAsync(b->ptr, stage, bytes, cudaMemcpyHostToDevice, c->h2d));
-      CUDA_TRY(cudaEventRecord(c->pinned[idx].ev, c->h2d));
-      c->pinned[idx].in_flight = true;
+      CUDA_TRY(cudaMemcpyAsync(b->ptr, stage, bytes, cudaMemcpyHostToDevice, stream));
     } else {
       std::vector<char> tmp;
       const void* src = data;
@@ -1710,9 +1916,11 @@ b200_error* b200_buffer_from_host(b200_client* c, const void* data, b200_dtype d
       CUDA_TRY(cudaStreamSynchronize(c->h2d));
     }
   }
-  CUDA_TRY(cudaEventCreateWithFlags(&b->ready, cudaEventDisableTiming));
-  CUDA_TRY(cudaEventRecord(b->ready, c->h2d));
-  b->ready_on = c->h2d;
+  CUDA_TRY(record_ready(c, stream, &b->ready));
+  b->ready_on = stream;
+  if (small) c->tail = nullptr;
+  else b->ready_seq = ++c->h2d_seq;
+  if (staged >= 0) c->pinned[staged].reader = b->ready;
   if (done) {
     if (host_ready_now) *done = new b200_event();
     else {
@@ -1737,27 +1945,40 @@ b200_error* b200_buffer_to_host(b200_buffer* b, void* dst, size_t* dst_size, b20
   b200_client* c = b->client;
   std::lock_guard<std::recursive_mutex> lock(c->mu);
   if (auto* e = set_device(c)) return e;
-  CUDA_TRY(cudaStreamWaitEvent(c->d2h, b->ready, 0));
-  if (b->bytes) CUDA_TRY(cudaMemcpyAsync(dst, b->ptr, b->bytes, cudaMemcpyDeviceToHost, c->d2h));
-  cudaEvent_t rd;
-  CUDA_TRY(cudaEventCreateWithFlags(&rd, cudaEventDisableTiming));
-  CUDA_TRY(cudaEventRecord(rd, c->d2h));
-  // drop finished read markers, keep this one so deletion waits for the copy
-  for (auto it = b->reads.begin(); it != b->reads.end();) {
-    if (cudaEventQuery(*it) == cudaSuccess) { cudaEventDestroy(*it); it = b->reads.erase(it); }
-    else ++it;
-  }
-  b->reads.push_back(rd);
-  if (event) {
-    b200_error* err = nullptr;
-    *event = new_event_on(c, c->d2h, &err);
-    if (err) return err;
-    (*event)->status = b->status;
-  } else {
-    CUDA_TRY(cudaStreamSynchronize(c->d2h));
+  if (!event) {
+    // The caller waits. The end of the compute stream is as good a place for the copy as the copy stream when nothing
+    // has gone in behind the buffer's producer, and saves the hop between streams; a small result lands in pinned staging
+    // first, which is quicker than the driver's own handling of pageable memory.
+    const bool inline_copy = b->ready_on == c->compute && c->tail == b->ready.get();
+    const cudaStream_t stream = inline_copy ? c->compute : c->d2h;
+    if (!inline_copy) CUDA_TRY(cudaStreamWaitEvent(c->d2h, b->ready->ev, 0));
+    if (b->bytes) {
+      int idx = -1;
+      void* stage = b->bytes <= kSmallCopy ? acquire_pinned(c, b->bytes, &idx) : nullptr;
+      CUDA_TRY(cudaMemcpyAsync(stage ? stage : dst, b->ptr, b->bytes, cudaMemcpyDeviceToHost, stream));
+      CUDA_TRY(cudaStreamSynchronize(stream));
+      if (stage) memcpy(dst, stage, b->bytes);
+    } else {
+      CUDA_TRY(cudaStreamSynchronize(stream));
+    }
     if (b->status && b->status->failed())
       return make_error(B200_INTERNAL, "the execution that produced this buffer gave up on a bounded device-side wait; its results are invalid");
+    return nullptr;
   }
+  CUDA_TRY(cudaStreamWaitEvent(c->d2h, b->ready->ev, 0));
+  if (b->bytes) CUDA_TRY(cudaMemcpyAsync(dst, b->ptr, b->bytes, cudaMemcpyDeviceToHost, c->d2h));
+  // drop finished read markers, keep one for this copy so that deletion waits for it
+  for (auto it = b->reads.begin(); it != b->reads.end();) {
+    if (cudaEventQuery((*it)->ev) == cudaSuccess) it = b->reads.erase(it);
+    else ++it;
+  }
+  std::shared_ptr<ReadyEvent> rd;
+  CUDA_TRY(record_ready(c, c->d2h, &rd));
+  b->reads.push_back(std::move(rd));
+  b200_error* err = nullptr;
+  *event = new_event_on(c, c->d2h, &err);
+  if (err) return err;
+  (*event)->status = b->status;
   return nullptr;
 }
 
@@ -1776,7 +1997,7 @@ b200_error* b200_buffer_ready_event(b200_buffer* b, b200_event** event) {
   std::lock_guard<std::recursive_mutex> lock(c->mu);
   if (auto* e = set_device(c)) return e;
   // a fresh event on the d2h stream ordered after the buffer's producer
-  CUDA_TRY(cudaStreamWaitEvent(c->d2h, b->ready, 0));
+  CUDA_TRY(cudaStreamWaitEvent(c->d2h, b->ready->ev, 0));
   b200_error* err = nullptr;
   *event = new_event_on(c, c->d2h, &err);
   if (*event) (*event)->status = b->status;
@@ -1791,20 +2012,17 @@ b200_error* b200_buffer_delete(b200_buffer* b) {
   b->deleted = true;
   if (b->ptr) {
     // the free is ordered on the compute stream: only a producer on another stream needs a wait
-    if (b->ready && b->ready_on != c->compute) cudaStreamWaitEvent(c->compute, b->ready, 0);
-    for (auto ev : b->reads) {
-      cudaStreamWaitEvent(c->compute, ev, 0);
-      cudaEventDestroy(ev);
-    }
+    if (b->ready) wait_for_copy(c, b);
+    for (auto& r : b->reads) cudaStreamWaitEvent(c->compute, r->ev, 0);
     b->reads.clear();
     if (b->block) {
       if (--b->block->refs == 0) {
-        cudaFreeAsync(b->block->base, c->compute);
+        block_free(c, b->block->base, b->block->bytes);
         delete b->block;
       }
       b->block = nullptr;
     } else {
-      cudaFreeAsync(b->ptr, c->compute);
+      block_free(c, b->ptr, b->bytes);
     }
     c->note_free(std::max<size_t>(b->bytes, 16));
     b->ptr = nullptr;
@@ -1815,8 +2033,6 @@ b200_error* b200_buffer_delete(b200_buffer* b) {
 b200_error* b200_buffer_destroy(b200_buffer* b) {
   if (!b) return nullptr;
   b200_error* e = b200_buffer_delete(b);
-  if (b->ready) cudaEventDestroy(b->ready);
-  for (auto ev : b->reads) cudaEventDestroy(ev);
   delete b;
   return e;
 }
@@ -1833,11 +2049,11 @@ b200_error* b200_buffer_copy(b200_buffer* b, b200_buffer** out) {
   n->dims = b->dims;
   n->bytes = b->bytes;
   if (auto* e = device_alloc(c, b->bytes, c->compute, &n->ptr)) return e;
-  CUDA_TRY(cudaStreamWaitEvent(c->compute, b->ready, 0));
+  CUDA_TRY(wait_for_copy(c, b));
   if (b->bytes) CUDA_TRY(cudaMemcpyAsync(n->ptr, b->ptr, b->bytes, cudaMemcpyDeviceToDevice, c->compute));
-  CUDA_TRY(cudaEventCreateWithFlags(&n->ready, cudaEventDisableTiming));
-  CUDA_TRY(cudaEventRecord(n->ready, c->compute));
+  CUDA_TRY(record_ready(c, c->compute, &n->ready));
   n->ready_on = c->compute;
+  c->tail = nullptr;
   *out = n.release();
   return nullptr;
 }
@@ -1870,23 +2086,25 @@ b200_error* b200_executable_execute(b200_executable* exe, b200_buffer* const* ar
   x.lp = exe->lp.get();
   x.ptrs.assign(p.slots.size(), nullptr);
   // arguments produced on the compute stream itself (the outputs of earlier executions) are ordered already
+  const b200_buffer* newest = nullptr;
   for (size_t k = 0; k < num_args; k++)
-    if (args[k]->ready_on != c->compute) CUDA_TRY(cudaStreamWaitEvent(c->compute, args[k]->ready, 0));
+    if (args[k]->ready_on != c->compute && (!newest || args[k]->ready_seq > newest->ready_seq)) newest = args[k];
+  if (newest) CUDA_TRY(wait_for_copy(c, newest));
+  c->tail = nullptr;
   std::vector<std::unique_ptr<b200_buffer>> outs(p.results.size());
   // Donation (tf.aliasing_output on an argument): the argument is consumed. Its buffer is left deleted and its memory
   // goes back to the stream-ordered pool behind this execution, where the next allocation of the stream finds it; the
   // results themselves are fresh allocations (the kernels are free to write a result before they have read all of
   // the argument, so the two never share storage).
   std::vector<bool> arg_taken(num_args, false);
-  // the error counter as this execution sees it before its first and after its last kernel
-  auto status = std::make_shared<ExecStatus>();
-  if (!c->free_status.empty()) {
-    const int slot = c->free_status.back();
-    c->free_status.pop_back();
-    status->pair = c->status_block + 2 * slot;
-    status->pair[0] = status->pair[1] = 0;
-    status->release = [c, slot](volatile int*) { std::lock_guard<std::recursive_mutex> l(c->mu); c->free_status.push_back(slot); };
-    CUDA_TRY(cudaMemcpyAsync((void*)&status->pair[0], c->error_flag, sizeof(int), cudaMemcpyDeviceToHost, c->compute));
+  std::shared_ptr<ExecStatus> status;
+  if (exe->lp->watched || c->armed_wait_polls > 0) {
+    status = std::make_shared<ExecStatus>();
+    status->before = c->last_status;
+    status->after = new_status_word(c);
+    if (!status->before && (status->before = new_status_word(c)))
+      CUDA_TRY(cudaMemcpyAsync((void*)status->before->word, c->error_flag, sizeof(int), cudaMemcpyDeviceToHost, c->compute));
+    c->last_status.reset();              // known again once this execution's copy is on its way
   }
   if (c->armed_wait_polls > 0) {
     cudaError_t he = b200::launch_expiring_wait(c->armed_wait_polls, c->error_flag, c->compute);
@@ -1917,14 +2135,14 @@ b200_error* b200_executable_execute(b200_executable* exe, b200_buffer* const* ar
     for (int g = 0; g < 2; g++) {
       if (count[g] < 2) continue;
       void* base = nullptr;
-      cudaError_t e = cudaMallocAsync(&base, total[g], c->compute);
+      cudaError_t e = block_alloc(c, total[g], c->compute, &base);
       if (e != cudaSuccess) {
         cudaGetLastError();
-        if (blocks[0]) { cudaFreeAsync(blocks[0]->base, c->compute); delete blocks[0]; }
+        if (blocks[0]) { block_free(c, blocks[0]->base, blocks[0]->bytes); delete blocks[0]; }
         return make_error(B200_RESOURCE_EXHAUSTED, "device allocation of " + std::to_string(total[g]) + " bytes for " +
                                                        std::to_string(count[g]) + " results failed: " + cudaGetErrorString(e));
       }
-      blocks[g] = new b200_buffer::Block{base, 0};
+      blocks[g] = new b200_buffer::Block{base, total[g], 0};
     }
     size_t at[2] = {0, 0};
     for (auto& b : outs) {
@@ -1954,7 +2172,7 @@ b200_error* b200_executable_execute(b200_executable* exe, b200_buffer* const* ar
       case Slot::RESULT: x.ptrs[s] = outs[sl.index]->ptr; break;
     }
   }
-  b200_error* err = run_plan(x, p.main);
+  b200_error* err = run_main(x);
   if (x.coll_pending) cudaStreamWaitEvent(c->compute, c->coll_done, 0);   // a plan that ended early still joins
   c->launches += x.launches;
   if (!x.timed.empty()) {
@@ -1975,18 +2193,24 @@ b200_error* b200_executable_execute(b200_executable* exe, b200_buffer* const* ar
       if (b && b->ptr) b200_buffer_delete(b.get());
     return err;
   }
-  for (size_t k = 0; k < outs.size(); k++) {
-    CUDA_TRY(cudaEventCreateWithFlags(&outs[k]->ready, cudaEventDisableTiming));
-    CUDA_TRY(cudaEventRecord(outs[k]->ready, c->compute));
-    outs[k]->ready_on = c->compute;
+  if (status && status->after) {
+    CUDA_TRY(cudaMemcpyAsync((void*)status->after->word, c->error_flag, sizeof(int), cudaMemcpyDeviceToHost, c->compute));
+    c->last_status = status->after;
+  }
+  if (!outs.empty()) {
+    std::shared_ptr<ReadyEvent> ready;
+    CUDA_TRY(record_ready(c, c->compute, &ready));
+    for (auto& b : outs) {
+      b->ready = ready;
+      b->ready_on = c->compute;
+    }
+    c->tail = ready.get();
   }
   if (donate) {
     // donated arguments are consumed (PJRT semantics): their memory returns to the pool in stream order
     for (size_t k = 0; k < num_args; k++)
       if (arg_taken[k]) b200_buffer_delete(args[k]);
   }
-  if (status->pair)
-    CUDA_TRY(cudaMemcpyAsync((void*)&status->pair[1], c->error_flag, sizeof(int), cudaMemcpyDeviceToHost, c->compute));
   if (done) {
     b200_error* e2 = nullptr;
     *done = new_event_on(c, c->compute, &e2);
@@ -2304,6 +2528,7 @@ b200_error* b200_client_probe_tf32_mma_rate(b200_client* c, double* tflops) {
   if (!c || !tflops) return make_error(B200_INVALID_ARGUMENT, "null argument");
   std::lock_guard<std::recursive_mutex> lock(c->mu);
   if (auto* e = set_device(c)) return e;
+  c->last_status.reset();                // a probe's kernels may count too
   cudaError_t e = b200::probe_tf32_mma_rate(c->error_flag, c->compute, tflops);
   if (e != cudaSuccess) return make_error(B200_INTERNAL, std::string("tensor-core rate probe failed: ") + cudaGetErrorString(e));
   return nullptr;
