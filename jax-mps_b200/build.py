@@ -11,7 +11,7 @@ from pathlib import Path
 HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 OUT = HERE / "b200" / "libb200core.so"
-SOURCES = ["parser.cc", "codegen.cc", "compiler.cc", "runtime.cc", "kernels.cu", "gemm16.cu"]
+SOURCES = ["parser.cc", "codegen.cc", "compiler.cc", "runtime.cc", "kernels.cu", "gemm16.cu", "gemm32.cu"]
 
 
 def _nccl_include() -> str:

@@ -47,6 +47,22 @@ struct Dot16 {
   struct Repack { bool needed = false; long long rows = 0, cols = 0, src_ld = 0, dst_ld = 0; } ra, rb;
 };
 
+// the row-major multi-index over `which` as extent and a single stride (false when it does not collapse)
+bool collapse_dims(const std::vector<int64_t>& dims, const std::vector<int64_t>& s, const std::vector<int64_t>& which, long long& extent,
+                   long long& stride) {
+  extent = 1;
+  stride = 0;
+  bool have = false;
+  for (int q = (int)which.size() - 1; q >= 0; q--) {
+    const int64_t dsz = dims[which[q]];
+    if (dsz == 1) continue;
+    if (!have) { stride = s[which[q]]; have = true; }
+    else if (s[which[q]] != stride * extent) return false;
+    extent *= dsz;
+  }
+  return true;
+}
+
 bool dot16_geometry(Op* op, Dot16& d) {
   if (op->operands.size() != 2 || op->results.size() != 1 || getenv("B200_NO_GEMM16")) return false;
   Value *lhs = op->operands[0], *rhs = op->operands[1], *out = op->results[0];
@@ -67,27 +83,12 @@ bool dot16_geometry(Op* op, Dot16& d) {
     for (int k = (int)dims.size() - 1; k >= 0; k--) { s[k] = st; st *= dims[k]; }
     return s;
   };
-  // the row-major multi-index over `which` as extent and a single stride (false when it does not collapse)
-  auto collapse = [](const std::vector<int64_t>& dims, const std::vector<int64_t>& s, const std::vector<int64_t>& which,
-                     long long& extent, long long& stride) {
-    extent = 1;
-    stride = 0;
-    bool have = false;
-    for (int q = (int)which.size() - 1; q >= 0; q--) {
-      const int64_t dsz = dims[which[q]];
-      if (dsz == 1) continue;
-      if (!have) { stride = s[which[q]]; have = true; }
-      else if (s[which[q]] != stride * extent) return false;
-      extent *= dsz;
-    }
-    return true;
-  };
   auto sl = strides(lhs->type.dims), sr = strides(rhs->type.dims);
   long long G, G2, M, N, K, K2;
   Gemm16Launch& g = d.g;
-  if (!collapse(lhs->type.dims, sl, lbd, G, g.a_gs) || !collapse(rhs->type.dims, sr, rbd, G2, g.b_gs) ||
-      !collapse(lhs->type.dims, sl, lfree, M, g.a_ms) || !collapse(rhs->type.dims, sr, rfree, N, g.b_ns) ||
-      !collapse(lhs->type.dims, sl, lcd, K, g.a_ks) || !collapse(rhs->type.dims, sr, rcd, K2, g.b_ks))
+  if (!collapse_dims(lhs->type.dims, sl, lbd, G, g.a_gs) || !collapse_dims(rhs->type.dims, sr, rbd, G2, g.b_gs) ||
+      !collapse_dims(lhs->type.dims, sl, lfree, M, g.a_ms) || !collapse_dims(rhs->type.dims, sr, rfree, N, g.b_ns) ||
+      !collapse_dims(lhs->type.dims, sl, lcd, K, g.a_ks) || !collapse_dims(rhs->type.dims, sr, rcd, K2, g.b_ks))
     return false;
   if (G != G2 || K != K2 || G <= 0 || M <= 0 || N <= 0 || K < 8) return false;
   if (G > 65535 || M >= (1LL << 31) || N >= (1LL << 31) || K >= (1LL << 31)) return false;
@@ -1646,7 +1647,9 @@ struct Planner {
         default: return 0;
       }
     };
-    bool two_byte_out = false, wide_ok = n >= 4096;
+    // A wide thread does the work of W one after the other: worth it once the blocks fill the SMs, not before (the cell of
+    // a recurrent network, 16384 elements of exponentials, took twice as long in 16 blocks as in 64)
+    bool two_byte_out = false, wide_ok = n >= 148LL * kThreads * 4;
     for (auto* o : outs) {
       wide_ok = wide_ok && esize(o->type.dt) != 0;
       two_byte_out = two_byte_out || esize(o->type.dt) == 2;
@@ -1683,14 +1686,15 @@ struct Planner {
       int64_t blocks = std::max<int64_t>(1, (n / W + kThreads - 1) / kThreads);
       L.grid[0] = (unsigned)blocks; L.grid[1] = L.grid[2] = 1;
     } else {
-      src << "  #pragma unroll\n  for (int e = 0; e < " << kEPT << "; ++e) {\n";
-      src << "    const " << em.idx_t << " lin = ((" << em.idx_t << ")blockIdx.x * " << kEPT << " + e) * " << kThreads
+      const int ept = n >= 148LL * kThreads * kEPT ? kEPT : 1;
+      src << "  #pragma unroll\n  for (int e = 0; e < " << ept << "; ++e) {\n";
+      src << "    const " << em.idx_t << " lin = ((" << em.idx_t << ")blockIdx.x * " << ept << " + e) * " << kThreads
           << " + threadIdx.x;\n";
       src << "    if (lin >= (" << em.idx_t << ")" << n << "LL) break;\n";
       src << em.str();
       src << "  }\n}\n";
       L.kernel = add_kernel(src.str(), "fused");
-      int64_t blocks = std::max<int64_t>(1, (n + (int64_t)kThreads * kEPT - 1) / ((int64_t)kThreads * kEPT));
+      int64_t blocks = std::max<int64_t>(1, (n + (int64_t)kThreads * ept - 1) / ((int64_t)kThreads * ept));
       L.grid[0] = (unsigned)blocks; L.grid[1] = L.grid[2] = 1;
     }
     L.block[0] = kThreads; L.block[1] = L.block[2] = 1;
@@ -3433,7 +3437,8 @@ struct Planner {
   // (measured on the ResNet layer shapes: about 0.6 us per 128 x 64 x 32 k-tile, 0.9 us per 128 x 128 x 32 one,
   // 6 us of fixed cost per wave of CTAs, partial sums written and re-read at about 3 TB/s) picks the split
   // that minimises waves * time per CTA + reduction time.
-  void choose_split_k(IGemmParams& p) {
+  // Returns the modelled time in microseconds.
+  static double choose_split_k(IGemmParams& p) {
     const int bn = p.N >= 128 ? 128 : 64;
     const long long tiles = (long long)((p.M + 127) / 128) * ((p.N + bn - 1) / bn) * p.groups;
     const long long ktiles = (p.K + 31) / 32;
@@ -3457,6 +3462,36 @@ struct Planner {
       if (cost < best_cost * 0.97) { best_cost = cost; best = split; }
     }
     p.split_k = best;
+    return best_cost;
+  }
+
+  // Whether a dense fp32 product is faster on the FMA pipe (gemm32.cu) than on the tensor cores, and in which tile and
+  // split. Cycles of an SM, fitted to products from 64 x 64 x 64 to 512 x 8003 x 462: 1.7 per row of four warps' FMA
+  // instructions and k when a CTA is alone on its SM (one warp per scheduler) and 1.25 when others fill its stalls, 1500
+  // (900) to fill and drain a CTA, 2500 for the launch, 700 for the sum of warps, 1000 for that of a
+  // cluster. The lines against choose_split_k's model: 462 x 512 x 512 is 7 us here and 19 there, 462 x 2048 x 512 about
+  // 27 both ways, 4096 x 1000 x 784 stays on the tensor cores.
+  static bool fma_product(Gemm32Launch& g) {
+    if (g.G > 65535 || getenv("B200_NO_GEMM32")) return false;
+    double best = 1e30;
+    for (int tile = 2; tile >= 0; tile--) {
+      const int tm = tile == 0 ? 32 : 64, tn = tile == 2 ? 128 : 64;
+      const long long tiles = (long long)((g.M + tm - 1) / tm) * ((g.N + tn - 1) / tn) * g.G;
+      for (int split = 1; split <= 4; split *= 2) {
+        if (split > 1 && g.K < 32 * split) break;
+        const long long per_sm = tiles * split <= gemm32_resident(split) ? 1 : (tiles * split + 147) / 148;
+        const long long chunk = ((g.K + split - 1) / split + 3) / 4 * 4;
+        const double row = per_sm == 1 ? 1.7 : 1.25, edge = per_sm == 1 ? 1500.0 : 900.0;
+        const double us = ((double)per_sm * (tm * tn / 128 * row * (double)chunk + edge) + 2500.0 + (split > 1 || tile < 2 ? 700.0 : 0.0) +
+                           (split > 1 ? 1000.0 : 0.0)) / 1850.0;
+        if (us < best * 0.97) { best = us; g.split = split; g.tile = tile; }
+      }
+    }
+    IGemmParams t;
+    t.M = g.M; t.N = g.N; t.K = g.K; t.groups = g.G;
+    t.vec = g.a_vec && g.b_vec;
+    t.seg = t.vec && g.K % 32 == 0 && (g.a_kc || g.M % 32 == 0) && (g.b_kc || g.N % 32 == 0);
+    return best < choose_split_k(t);
   }
 
   Step lower_conv(Op* op, BlockState& st) {
@@ -3696,6 +3731,38 @@ struct Planner {
     IGemmParams p;
     p.M = (int)M; p.N = (int)N; p.K = (int)K; p.groups = (int)G;
     p.needs_mask = 0;
+    {
+      // a strided matrix per group on both sides, with one of its two indices contiguous
+      long long mv, kv, nv, kv2, gv, gv2;
+      long long ms = 0, ks = 0, ns = 0, ks2 = 0;
+      Gemm32Launch g;
+      if (M > 0 && N > 0 && K > 0 && G > 0 && collapse_dims(lhs->type.dims, sl, lfree, mv, ms) && collapse_dims(lhs->type.dims, sl, lcd, kv, ks) &&
+          collapse_dims(rhs->type.dims, sr, rfree, nv, ns) && collapse_dims(rhs->type.dims, sr, rcd, kv2, ks2) &&
+          collapse_dims(lhs->type.dims, sl, lbd, gv, g.a_gs) && collapse_dims(rhs->type.dims, sr, rbd, gv2, g.b_gs) &&
+          (ks == 1 || ms == 1 || K == 1 || M == 1) && (ks2 == 1 || ns == 1 || K == 1 || N == 1)) {
+        g.M = (int)M; g.N = (int)N; g.K = (int)K; g.G = (int)G;
+        // an index of extent one is contiguous whatever its stride
+        g.a_kc = (ks == 1 || K == 1) ? 1 : 0;
+        g.a_ld = g.a_kc ? ms : ks;
+        g.b_kc = (ns == 1 || N == 1) ? 0 : 1;
+        g.b_ld = g.b_kc ? ns : ks2;
+        auto rows16 = [](int extent, long long ld, long long gs) { return extent % 4 == 0 && ld % 4 == 0 && gs % 4 == 0; };
+        g.a_vec = rows16(g.a_kc ? g.K : g.M, g.a_ld, g.a_gs);
+        g.b_vec = rows16(g.b_kc ? g.K : g.N, g.b_ld, g.b_gs);
+        if (fma_product(g)) {
+          p.fma = g;
+          p.a_contig = g.a_kc ? 0 : 1;
+          p.b_contig = g.b_kc;
+          p.vec = g.a_vec && g.b_vec;
+          Step s;
+          s.kind = Step::IGEMM;
+          s.label = op->name;
+          s.ig = p;
+          s.args = {slot_of.at(lhs), slot_of.at(rhs), slot_of.at(out)};
+          return s;
+        }
+      }
+    }
     auto am = offsets(lhs->type.dims, sl, lfree, M), ak = offsets(lhs->type.dims, sl, lcd, K);
     auto bk = offsets(rhs->type.dims, sr, rcd, K), bn = offsets(rhs->type.dims, sr, rfree, N);
     auto ag = offsets(lhs->type.dims, sl, lbd, G), bg = offsets(rhs->type.dims, sr, rbd, G);
@@ -5569,7 +5636,9 @@ void dump_plan(const CompiledProgram& prog, const Plan& p, std::ostringstream& o
         break;
       case Step::IGEMM:
         os << "igemm M=" << s.ig.M << " N=" << s.ig.N << " K=" << s.ig.K << " G=" << s.ig.groups << " splitK=" << s.ig.split_k
-           << " a_contig=" << s.ig.a_contig << " b_contig=" << s.ig.b_contig << " vec=" << s.ig.vec << " seg=" << s.ig.seg << (s.ig.kt_stride ? " ktlist" : "") << (s.ig.a_tma ? " tmaA" : "") << " " << s.label;
+           << " a_contig=" << s.ig.a_contig << " b_contig=" << s.ig.b_contig << " vec=" << s.ig.vec << " seg=" << s.ig.seg << (s.ig.kt_stride ? " ktlist" : "") << (s.ig.a_tma ? " tmaA" : "");
+        if (s.ig.fma.split) os << " fma tile=" << s.ig.fma.tile << " cluster=" << s.ig.fma.split;
+        os << " " << s.label;
         break;
       case Step::MEMCPY: os << "memcpy " << s.bytes; break;
       case Step::GEMM16:

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include "gemm16.h"
+#include "gemm32.h"
 
 namespace b200 {
 
@@ -68,6 +69,10 @@ void set_igemm_programmatic_launch(bool on);
 cudaError_t launch_while_handle(unsigned long long handle, const void* pred, unsigned long long* started, double limit_seconds,
                                 bool first, int* error_flag, cudaStream_t stream);
 cudaError_t launch_switch_handle(unsigned long long handle, const void* index, int branches, cudaStream_t stream);
+
+// fp32 product on the FMA pipe (gemm32.cu): C dense [G][M][N].
+cudaError_t launch_gemm32(const Gemm32Launch& p, const void* A, const void* B, void* C, cudaStream_t stream, int* launches);
+void set_gemm32_programmatic_launch(bool on);
 
 // Test hook: one kernel whose bounded mbarrier wait (budget `polls`) runs out and counts up *error_flag.
 cudaError_t launch_expiring_wait(int polls, int* error_flag, cudaStream_t stream);

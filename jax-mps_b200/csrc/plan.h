@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "gemm16.h"
+#include "gemm32.h"
 #include "ir.h"
 
 namespace b200 {
@@ -52,6 +53,7 @@ struct IGemmParams {
   int tma_c = 0, tma_w = 0, tma_h = 0, tma_n = 0;        // input extents (channels, width, height, images)
   int tma_ow = 0, tma_oh = 0, tma_box_h = 0, tma_box_n = 0;
   int tma_kw = 0, tma_pad_h = 0, tma_pad_w = 0, tma_rdil_h = 1, tma_rdil_w = 1;
+  Gemm32Launch fma;                          // split > 0: a dense product on the FMA pipe, args are {A, B, C} alone
 };
 
 struct Plan;
@@ -70,7 +72,7 @@ struct Step {
   unsigned grid[3] = {1, 1, 1}, block[3] = {1, 1, 1};
   std::vector<int> args;              // slot ids, in kernel-parameter order
   int n_outs = 0;                     // KERNEL: the first n_outs args are written, the rest only read
-  // IGEMM: args = {A, B, C, a_row, a_col, b_row(k), b_col(n), c_row(m), c_col(n), a_grp, b_grp, c_grp, [split-K scratch]}
+  // IGEMM (ig.fma.split == 0): args = {A, B, C, a_row, a_col, b_row(k), b_col(n), c_row(m), c_col(n), a_grp, b_grp, c_grp, [split-K scratch]}
   IGemmParams ig;
   // GEMM16: args = {A, B, C, [fp32 scratch], [counters]}; iparams = {has scratch, has counters}
   // REPACK16: args = {dst, src}; iparams = {rows, cols, dst_ld, src_ld}

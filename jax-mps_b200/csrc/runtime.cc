@@ -321,9 +321,9 @@ struct LoadedProgram {
   std::vector<void*> const_ptrs;
   std::vector<void*> arenas;
   void* const_block = nullptr;
-  // Instantiated CUDA graphs of counted-loop bodies (two iterations each), per loop step and per set of slot
+  // Instantiated CUDA graphs of counted-loop bodies (an even number of iterations each), per loop step and per set of slot
   // addresses the graph was captured with.
-  struct LoopGraph { const void* step; std::vector<void*> ptrs; cudaGraphExec_t exec; int launches; };
+  struct LoopGraph { const void* step; std::vector<void*> ptrs; cudaGraphExec_t exec; int launches; long long iterations; };
   std::vector<LoopGraph> loop_graphs;
   // Graphs of data-dependent loops and cases (conditional nodes), per step and per set of addresses of the slots the
   // step and everything below it touches.
@@ -454,6 +454,9 @@ b200_error* set_device(b200_client* c) {
   return nullptr;
 }
 
+// Nodes that a recording of a counted loop aims at.
+constexpr long long kLoopGraphNodes = 384;
+
 // Host copies up to here are made on the compute stream and through pinned staging.
 constexpr size_t kSmallCopy = 64 << 10;
 
@@ -468,13 +471,18 @@ void release_blocks(b200_client* c) {
 // may still be using are not for other streams). Not counted as an allocation of the client.
 cudaError_t block_alloc(b200_client* c, size_t bytes, cudaStream_t stream, void** out) {
   const size_t n = block_bytes(bytes);
-  if (stream == c->compute && n <= b200_client::kBlockMax)
-    for (auto it = c->free_blocks.rbegin(); it != c->free_blocks.rend(); ++it)
-      if (it->bytes == n) {
-        *out = it->ptr;
-        c->free_blocks.erase(std::next(it).base());
-        return cudaSuccess;
-      }
+  if (stream == c->compute && n <= b200_client::kBlockMax) {
+    // the lowest address that fits: programs that repeat themselves then see the same addresses again, which recordings
+    // of loops and plans are made for
+    auto best = c->free_blocks.end();
+    for (auto it = c->free_blocks.begin(); it != c->free_blocks.end(); ++it)
+      if (it->bytes == n && (best == c->free_blocks.end() || it->ptr < best->ptr)) best = it;
+    if (best != c->free_blocks.end()) {
+      *out = best->ptr;
+      c->free_blocks.erase(best);
+      return cudaSuccess;
+    }
+  }
   cudaError_t e = cudaMallocAsync(out, n, stream);
   if (e != cudaSuccess && !c->free_blocks.empty()) {     // give what is kept back and try once more
     cudaGetLastError();
@@ -693,7 +701,7 @@ b200_error* run_plan(ExecCtx& x, const Plan& plan);
 // Whether a kernel of the plan has a bounded wait (tensor-core pipelines; data-dependent loops, which are bounded in time).
 bool waits_inside(const Plan& plan) {
   for (const Step& s : plan.steps) {
-    if (s.kind == Step::IGEMM || s.kind == Step::GEMM16 || (s.kind == Step::WHILE && s.trip_count < 0)) return true;
+    if ((s.kind == Step::IGEMM && !s.ig.fma.split) || s.kind == Step::GEMM16 || (s.kind == Step::WHILE && s.trip_count < 0)) return true;
     for (auto& p : s.sub)
       if (p && waits_inside(*p)) return true;
   }
@@ -768,6 +776,11 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
       return nullptr;
     }
     case Step::IGEMM: {
+      if (s.ig.fma.split) {
+        cudaError_t e = launch_gemm32(s.ig.fma, x.ptrs[s.args[0]], x.ptrs[s.args[1]], x.ptrs[s.args[2]], st, &x.launches);
+        if (e != cudaSuccess) return make_error(B200_INTERNAL, "launch of " + s.label + " failed: " + cudaGetErrorString(e));
+        return nullptr;
+      }
       IGemmLaunch p;
       p.M = s.ig.M; p.N = s.ig.N; p.K = s.ig.K; p.groups = s.ig.groups; p.split_k = s.ig.split_k;
       p.Hd = s.ig.Hd; p.Wd = s.ig.Wd; p.ldh = s.ig.ldh; p.ldw = s.ig.ldw;
@@ -908,16 +921,18 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
         CUDA_TRY(cudaStreamIsCapturing(st, &capturing));
         if (s.trip_count >= 4 && !c->profiling && capturing == cudaStreamCaptureStatusNone && graph_safe(*s.sub[1]) &&
             !c->sw.no_loop_graphs) {
-          // Two iterations (after which exchanged pointers are back where they started) are recorded once as a
-          // CUDA graph and replayed: the host issues one launch per pair instead of one per kernel, and the
-          // dependent kernels of a latency-bound body follow each other without a host round trip.
-          const long long pairs = s.trip_count / 2;
-          long long replayed = 0;
+          // An even number of iterations (after which exchanged pointers are back where they started) is recorded once as
+          // a CUDA graph and replayed: the host issues one launch for all of them. As many iterations as make about
+          // kLoopGraphNodes nodes: kernels inside a graph start while their predecessors drain, but a graph waits for the
+          // whole graph in front of it, which costs about 1 us (a loop of one small kernel took 2.1 us an iteration in
+          // graphs of two and takes 0.9 us in long ones).
+          std::vector<void*> touched;                  // what the recording depends on: not the program's other arguments and results
+          touched_addresses(x, s, touched);
           LoadedProgram::LoopGraph* hit = nullptr;
           for (auto& g : x.lp->loop_graphs)
-            if (g.step == &s && g.ptrs == x.ptrs) { hit = &g; break; }
+            if (g.step == &s && g.ptrs == touched) { hit = &g; break; }
           if (!hit) {
-            if (x.lp->loop_graphs.size() >= 16) {
+            if (x.lp->loop_graphs.size() >= 24) {
               // bounded cache: let the device finish with the oldest graph before it goes
               CUDA_TRY(cudaStreamSynchronize(st));
               cudaGraphExecDestroy(x.lp->loop_graphs.front().exec);
@@ -926,13 +941,16 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
             const std::vector<void*> at_start = x.ptrs;
             // the first pair runs directly, so that every kernel of the body has been loaded and configured
             // before anything is recorded
+            const int first = x.launches;
             if (auto* e = iterate()) return e;
             if (auto* e = iterate()) return e;
-            replayed = 1;
+            done = 2;
+            const int per_pair = std::max(1, x.launches - first);
+            const long long pairs = std::max<long long>(1, std::min<long long>((s.trip_count - done) / 2, kLoopGraphNodes / per_pair));
             const int before = x.launches;
             CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
-            b200_error* err = iterate();
-            if (!err) err = iterate();
+            b200_error* err = nullptr;
+            for (long long i = 0; i < 2 * pairs && !err; i++) err = iterate();
             cudaGraph_t graph = nullptr;
             cudaError_t ce = cudaStreamEndCapture(st, &graph);
             if (err) {
@@ -946,15 +964,16 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
             CUDA_TRY(ce);
             if (x.ptrs != at_start) {
               cudaGraphExecDestroy(exec);
-              return make_error(B200_INTERNAL, "loop state pointers did not return after two iterations");
+              return make_error(B200_INTERNAL, "loop state pointers did not return after an even number of iterations");
             }
-            x.lp->loop_graphs.push_back({&s, at_start, exec, x.launches - before});
+            x.lp->loop_graphs.push_back({&s, std::move(touched), exec, x.launches - before, 2 * pairs});
             x.launches = before;
             hit = &x.lp->loop_graphs.back();
           }
-          for (long long i = replayed; i < pairs; i++) CUDA_TRY(cudaGraphLaunch(hit->exec, st));
-          x.launches += (int)(hit->launches * (pairs - replayed));
-          done = 2 * pairs;
+          for (; done + hit->iterations <= s.trip_count; done += hit->iterations) {
+            CUDA_TRY(cudaGraphLaunch(hit->exec, st));
+            x.launches += hit->launches;
+          }
         }
         for (long long i = done; i < s.trip_count; i++)
           if (auto* e = iterate()) return e;
@@ -1009,6 +1028,7 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
         x.plain_launch = true;
         set_programmatic_launch(false);
         set_igemm_programmatic_launch(false);
+        set_gemm32_programmatic_launch(false);
         cudaError_t ce = cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed);
         if (ce != cudaSuccess) fail(ce, "begin capture");
         else {
@@ -1062,6 +1082,7 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
         x.plain_launch = false;
         set_programmatic_launch(!c->sw.no_pdl);
         set_igemm_programmatic_launch(!c->sw.no_pdl && !getenv("B200_NO_IGEMM_PDL"));
+        set_gemm32_programmatic_launch(!c->sw.no_pdl);
         if (graph) cudaGraphDestroy(graph);
         const int recorded = x.launches - before;
         x.launches = before;
@@ -1071,7 +1092,7 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
           b200_error_destroy(err);
           cudaGetLastError();
         } else {
-          x.lp->cond_graphs.push_back({&s, touched, exec, recorded});
+          x.lp->cond_graphs.push_back({&s, touched, exec, recorded, 0});
         }
       }
       return nullptr;
@@ -1180,7 +1201,7 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
           b200_error_destroy(err);
           cudaGetLastError();
         } else {
-          x.lp->cond_graphs.push_back({&s, touched, exec, recorded});
+          x.lp->cond_graphs.push_back({&s, touched, exec, recorded, 0});
         }
       }
       return nullptr;
@@ -1291,7 +1312,8 @@ b200_error* run_plan(ExecCtx& x, const Plan& plan) {
                   " G=" + std::to_string(s.ig.groups) + " splitK=" + std::to_string(s.ig.split_k) + " a_mcontig=" +
                   std::to_string(s.ig.a_contig) + " b_kcontig=" + std::to_string(s.ig.b_contig) + " mask=" +
                   std::to_string(s.ig.needs_mask) + " ld=" + std::to_string(s.ig.ldh) + "x" + std::to_string(s.ig.ldw) + " vec=" + std::to_string(s.ig.vec) + " seg=" + std::to_string(s.ig.seg);
-          if (!(x.c->tensor_cores && (long long)s.ig.M * s.ig.N * s.ig.K * s.ig.groups >= (1LL << 18) && s.ig.K >= 16))
+          if (s.ig.fma.split) t.kind = "gemm32", t.key += " fma cluster=" + std::to_string(s.ig.fma.split);
+          else if (!(x.c->tensor_cores && (long long)s.ig.M * s.ig.N * s.ig.K * s.ig.groups >= (1LL << 18) && s.ig.K >= 16))
             t.kind = "igemm_fma";
           break;
         case Step::ALL_REDUCE: t.kind = "all_reduce"; t.key = "all_reduce " + std::to_string(s.bytes); break;
@@ -1479,6 +1501,7 @@ b200_error* create_client(const b200_client_options* o, ncclComm_t given_comm, b
   if (const char* lim = getenv("B200_WHILE_TIME_LIMIT_S")) c->while_limit_s = std::max(0.001, atof(lim));
   set_programmatic_launch(!c->sw.no_pdl);
   set_igemm_programmatic_launch(!c->sw.no_pdl && !getenv("B200_NO_IGEMM_PDL"));
+  set_gemm32_programmatic_launch(!c->sw.no_pdl);
   if (!driver().ok) return make_error(B200_FAILED_PRECONDITION, driver().error);
   if (c->nprocs > 1) {
     NcclApi& n = nccl();
@@ -1640,7 +1663,7 @@ b200_error* b200_client_compile(b200_client* c, const char* code, size_t code_si
     static const char* names[] = {"B200_NO_WINDOW_UPDATE", "B200_NO_FLAT_ALL_REDUCE", "B200_NO_GEMM16", "B200_NO_ROW_FUSION",
                                   "B200_NO_WEIGHT_HOIST", "B200_NO_LICM", "B200_NO_CSE", "B200_NO_HOIST", "B200_NO_BUNDLES",
                                   "B200_NO_TILED_TRANSPOSE", "B200_NO_ALL_REDUCE_OVERLAP", "B200_DEBUG_NO_REUSE", "B200_NO_COL4",
-                                  "B200_NO_ATTENTION_FUSION", "B200_NO_WIDE_POINTWISE", "B200_NO_WIDE_ROWS"};
+                                  "B200_NO_ATTENTION_FUSION", "B200_NO_WIDE_POINTWISE", "B200_NO_WIDE_ROWS", "B200_NO_GEMM32"};
     for (size_t k = 0; k < sizeof names / sizeof names[0]; k++)
       if (getenv(names[k])) env_bits |= 1u << k;
   }
