@@ -213,6 +213,11 @@ void b200_string_free(char* s);
 b200_error* b200_buffer_from_host(b200_client* client, const void* data, b200_dtype dtype, const int64_t* dims,
                                   size_t num_dims, const int64_t* byte_strides, b200_buffer** buffer,
                                   b200_event** done_with_host_buffer);
+/* Page-locked host memory that b200_buffer_to_host copies into at link speed, from a bounded process-wide pool. Null for
+ * sizes outside 64 KB .. 16 MB, or when enough of it is out already: use memory of your own then. Thread-safe. */
+void* b200_host_alloc(size_t bytes);
+void b200_host_free(void* ptr);
+
 /* dst == NULL: only *dst_size is written (bytes needed). Otherwise starts an asynchronous copy; *event
  * (may be NULL: then the call blocks) is ready when dst holds the data. */
 b200_error* b200_buffer_to_host(b200_buffer* buffer, void* dst, size_t* dst_size, b200_event** event);

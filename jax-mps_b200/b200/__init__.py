@@ -16,6 +16,11 @@ from pathlib import Path
 
 import numpy as np
 
+try:
+    from . import _hot                  # the calls of an inner loop (csrc/hot.c); built beside the library
+except ImportError:
+    _hot = None
+
 _LIB_NAME = "libb200core.so"
 
 
@@ -105,6 +110,8 @@ SIGNATURES = {
     "b200_string_free": (None, [_P]),
     "b200_buffer_from_host": (_P, [_P, _P, C.c_int, C.POINTER(C.c_int64), C.c_size_t, C.POINTER(C.c_int64), C.POINTER(_P), C.POINTER(_P)]),
     "b200_buffer_to_host": (_P, [_P, _P, C.POINTER(C.c_size_t), C.POINTER(_P)]),
+    "b200_host_alloc": (_P, [C.c_size_t]),
+    "b200_host_free": (None, [_P]),
     "b200_buffer_dtype": (C.c_int, [_P]),
     "b200_buffer_num_dims": (C.c_size_t, [_P]),
     "b200_buffer_dims": (C.POINTER(C.c_int64), [_P]),
@@ -194,6 +201,11 @@ def load_library():
         fn = getattr(lib, name)
         fn.restype = res
         fn.argtypes = args
+    if _hot is None:
+        raise B200Error(f"b200._hot not found beside {p}: build both with `python jax-mps_b200/build.py`", FAILED_PRECONDITION)
+    _hot.bind([C.cast(getattr(lib, n), _P).value for n in (
+        "b200_executable_execute", "b200_buffer_from_host", "b200_buffer_to_host", "b200_buffer_destroy", "b200_error_destroy",
+        "b200_host_alloc", "b200_host_free")], lambda err: _check(err), Buffer)
     _lib = lib
     return lib
 
@@ -347,11 +359,8 @@ class Event:
             self._h = None
 
 
-class Buffer:
-    """A device array (PJRT_Buffer)."""
-
-    def __init__(self, client: "Client", handle):
-        self.client, self._h = client, handle
+class Buffer(_hot.Handle if _hot else object):
+    """A device array (PJRT_Buffer), made from its client and its handle (`_h`), which it owns."""
 
     @property
     def dtype_code(self) -> int:
@@ -402,6 +411,12 @@ class Buffer:
     def to_numpy(self) -> np.ndarray:
         """bf16 buffers come back as float32 (exactly representable)."""
         code = self.dtype_code
+        nbytes = self.nbytes
+        if 65536 <= nbytes <= 1 << 24:
+            block = _hot.to_block(self, nbytes)              # page-locked memory, given back with the array
+            if block is not None:
+                out = np.frombuffer(block, dtype=_DT_TO_NP[code]).reshape(self.shape)
+                return (out.astype(np.uint32) << 16).view(np.float32) if code == BF16 else out
         out = np.empty(self.shape, dtype=_DT_TO_NP[code])
         size = C.c_size_t(out.nbytes)
         _check(load_library().b200_buffer_to_host(self._h, out.ctypes.data_as(_P), C.byref(size), None))
@@ -412,14 +427,6 @@ class Buffer:
     def __array__(self, dtype=None, copy=None):
         a = self.to_numpy()
         return a.astype(dtype) if dtype is not None else a
-
-    def __del__(self):
-        if getattr(self, "_h", None) and load_library is not None:
-            try:
-                load_library().b200_buffer_destroy(self._h)
-            except Exception:
-                pass
-            self._h = None
 
 
 class Executable:
@@ -476,15 +483,8 @@ class Executable:
     def execute(self, args, donate: bool = False, with_event: bool = False):
         """Enqueue one execution; returns the output buffers without waiting (with `with_event`: the buffers and the
         completion event of the execution)."""
-        lib = load_library()
-        n = len(args)
-        arr = (_P * max(n, 1))(*[a._h for a in args])
-        outs = (_P * max(self.num_outputs, 1))()
-        opts = _ExecuteOptions(C.sizeof(_ExecuteOptions), 1 if donate else 0)
-        done = _P()
-        _check(lib.b200_executable_execute(self._h, arr, n, outs, C.byref(done) if with_event else None, C.byref(opts)))
-        bufs = [Buffer(self.client, outs[k]) for k in range(self.num_outputs)]
-        return (bufs, Event(done.value)) if with_event else bufs
+        r = _hot.execute(self._h, args, self.num_outputs, donate, with_event, self.client)
+        return (r[0], Event(r[1])) if with_event else r
 
     def __call__(self, *arrays):
         bufs = [a if isinstance(a, Buffer) else self.client.buffer_from_host(a) for a in arrays]
@@ -560,6 +560,10 @@ class Client:
     def buffer_from_host(self, array, dtype: str | None = None) -> Buffer:
         """Host array -> device buffer. `dtype='bf16'` converts float32 input to bfloat16 on the host (a uint16 array
         is taken as bfloat16 bit patterns as it is)."""
+        if dtype is None and type(array) is np.ndarray:
+            buf = _hot.from_host(self._h, array, self)
+            if buf is not None:
+                return buf
         a = np.asarray(array)
         if dtype == "bf16":
             if a.dtype != np.uint16:                      # uint16 input is taken as bfloat16 bit patterns
