@@ -2093,8 +2093,8 @@ struct Planner {
       std::ostringstream src;
       src << "extern \"C\" __global__ void __launch_bounds__(" << threads << ") @NAME@(";
       if (last) src << signature(outs, ins);
-      else src << "u32* __restrict__ kout, u32* __restrict__ iout" << (first ? ", " + signature({}, ins) : "");
-      src << ", int* __restrict__ hist" << (first ? "" : ", const u32* __restrict__ kin, const u32* __restrict__ iin") << ") {\n";
+      else src << "u32* __restrict__ kout, u32* __restrict__ iout, int* __restrict__ hist" << (first ? ", " + signature({}, ins) : "");
+      src << (last ? ", const int* __restrict__ hist" : "") << (first ? "" : ", const u32* __restrict__ kin, const u32* __restrict__ iin") << ") {\n";
       head(src);
       src << "  const int shift = " << 8 * pass << ";\n  const long long HS = " << rows * tiles * 256 << "LL;\n";
       src << R"SRC(  __shared__ u16 warps[NW * 256];
@@ -2146,11 +2146,10 @@ struct Planner {
       }
       src << "    }\n}\n";
       std::vector<int> args;
-      if (last) { args = out_slots; args.insert(args.end(), in_slots.begin(), in_slots.end()); }
-      else { args = {kbuf[pass & 1], ibuf[pass & 1]}; if (first) args.insert(args.end(), in_slots.begin(), in_slots.end()); }
-      args.push_back(hist);
+      if (last) { args = out_slots; args.insert(args.end(), in_slots.begin(), in_slots.end()); args.push_back(hist); }
+      else { args = {kbuf[pass & 1], ibuf[pass & 1], hist}; if (first) args.insert(args.end(), in_slots.begin(), in_slots.end()); }
       if (!first) { args.push_back(kbuf[(pass & 1) ^ 1]); args.push_back(ibuf[(pass & 1) ^ 1]); }
-      launch(src, last ? "sort_pass_out" : "sort_pass", "sort (radix pass " + std::to_string(pass) + ")", args, last ? (int)ins.size() : 2);
+      launch(src, last ? "sort_pass_out" : "sort_pass", "sort (radix pass " + std::to_string(pass) + ")", args, last ? (int)ins.size() : 3);
     }
     return true;
   }
@@ -5391,6 +5390,7 @@ struct Planner {
       for (size_t k = i; k < j; k++) {
         b.label += (k > i ? " + " : "") + plan.steps[k].label;
         b.args.insert(b.args.end(), plan.steps[k].args.begin(), plan.steps[k].args.end());
+        for (size_t a = 0; a < plan.steps[k].args.size(); a++) b.writes.push_back((int)a < plan.steps[k].n_outs ? 1 : 0);
       }
       out.push_back(std::move(b));
       i = j;
@@ -5501,6 +5501,9 @@ struct Planner {
   int partition_id = 0;
 
   // ---- arena layout ---------------------------------------------------------------
+  // Memory goes to another temporary only so many steps after its last use: recordings run steps side by side that do not
+  // depend on one another, and steps that share memory do.
+  static constexpr int kReuseDistance = 8;
   void layout_arena(Plan& plan) {
     const int arena = plan.arena;
     // liveness over the step sequence of this plan
@@ -5598,7 +5601,7 @@ struct Planner {
         for (int m : pk->second) need += (prog.slots[m].bytes + 255) & ~(size_t)255;
       }
       // drop blocks that ended before `first`
-      active.erase(std::remove_if(active.begin(), active.end(), [&](const Blk& b) { return b.last < first; }), active.end());
+      active.erase(std::remove_if(active.begin(), active.end(), [&](const Blk& b) { return b.last + kReuseDistance < first; }), active.end());
       std::sort(active.begin(), active.end(), [](const Blk& a, const Blk& b) { return a.off < b.off; });
       size_t off = 0;
       for (auto& b : active) {

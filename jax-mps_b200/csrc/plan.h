@@ -72,6 +72,7 @@ struct Step {
   unsigned grid[3] = {1, 1, 1}, block[3] = {1, 1, 1};
   std::vector<int> args;              // slot ids, in kernel-parameter order
   int n_outs = 0;                     // KERNEL: the first n_outs args are written, the rest only read
+  std::vector<char> writes;           // KERNEL of several parts (n_outs 0): per argument, whether it is written
   // IGEMM (ig.fma.split == 0): args = {A, B, C, a_row, a_col, b_row(k), b_col(n), c_row(m), c_col(n), a_grp, b_grp, c_grp, [split-K scratch]}
   IGemmParams ig;
   // GEMM16: args = {A, B, C, [fp32 scratch], [counters]}; iparams = {has scratch, has counters}

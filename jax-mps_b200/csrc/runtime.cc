@@ -330,6 +330,15 @@ struct LoadedProgram {
   std::vector<LoopGraph> cond_graphs;
   // Graphs of the whole plan, per set of argument and result addresses that came back (replay_plan).
   struct PlanGraph { std::vector<void*> ptrs; cudaGraphExec_t exec; int launches; uint64_t used; };
+  // Sets of addresses met once, newest last: recording costs some 15 us a node, so it is for what comes back.
+  std::deque<std::pair<const void*, std::vector<void*>>> met;
+  bool met_before(const void* step, const std::vector<void*>& ptrs) {
+    for (auto it = met.begin(); it != met.end(); ++it)
+      if (it->first == step && it->second == ptrs) { met.erase(it); return true; }
+    met.emplace_back(step, ptrs);
+    if (met.size() > 48) met.pop_front();
+    return false;
+  }
   std::vector<PlanGraph> plan_graphs;
   bool replayable = false;                     // the plan only launches kernels and device copies, and enough of them
   uint64_t calls = 0, replays = 0, recordings = 0;
@@ -735,6 +744,144 @@ void touched_addresses(const ExecCtx& x, const Step& s, std::vector<void*>& out,
     if (p) for (const Step& t : p->steps) touched_addresses(x, t, out, false);
 }
 
+// Records steps into a CUDA graph whose edges are the dependences between them instead of the order they were planned in,
+// so that independent kernels (the two products of a gradient, the branches of a bundle of heads) run side by side. A
+// small program is a chain of kernels that fill a fraction of the chip each; what it gains is the branches of that chain.
+// Dependences are found from the memory that the steps read and write; the plan hands out memory so that neighbouring
+// steps do not meet by reuse alone (kReuseDistance in the plan compiler).
+b200_error* run_step(ExecCtx& x, const Step& s);
+
+class Recorder {
+ public:
+  Recorder(ExecCtx& x, cudaGraph_t graph) : x_(x), graph_(graph) {}
+
+  b200_error* step(const Step& s) {
+    reads_.clear();
+    writes_.clear();
+    const bool all = !accesses(s);
+    return record(all, [&]() { return run_step(x_, s); });
+  }
+  b200_error* copy(void* dst, const void* src, size_t bytes) {
+    reads_.assign(1, {(uintptr_t)src, (uintptr_t)src + bytes});
+    writes_.assign(1, {(uintptr_t)dst, (uintptr_t)dst + bytes});
+    return record(false, [&]() -> b200_error* {
+      CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, x_.c->compute));
+      return nullptr;
+    });
+  }
+
+ private:
+  struct Range { uintptr_t lo, hi; };
+  struct Memory { Range at; int writer; std::vector<int> readers; };
+  struct Node { std::vector<cudaGraphNode_t> ends; std::vector<bool> before; };
+
+  void add(std::vector<Range>& to, int slot) {
+    if (slot < 0) return;
+    const Slot& sl = x_.lp->prog->slots[slot];
+    const uintptr_t p = (uintptr_t)x_.ptrs[slot];
+    const size_t n = std::max(sl.bytes, sl.type.bytes());
+    if (p && n) to.push_back({p, p + n});
+  }
+  // Memory that a step reads and writes; false: not known, it depends on everything and everything on it.
+  bool accesses(const Step& s) {
+    auto is_const = [&](int slot) { return x_.lp->prog->slots[slot].kind == Slot::CONST; };
+    switch (s.kind) {
+      case Step::KERNEL:
+        for (size_t k = 0; k < s.args.size(); k++) {
+          if (s.writes.empty() ? (int)k < s.n_outs : s.writes[k] != 0) add(writes_, s.args[k]);
+          else if (!is_const(s.args[k])) add(reads_, s.args[k]);
+        }
+        return s.n_outs > 0 || !s.writes.empty();
+      case Step::IGEMM:
+        add(reads_, s.args[0]);
+        add(reads_, s.args[1]);
+        add(writes_, s.args[2]);
+        if (!s.ig.fma.split && s.ig.split_k > 1) add(writes_, s.args[12]);
+        return true;
+      case Step::GEMM16:
+        add(reads_, s.args[0]);
+        add(reads_, s.args[1]);
+        for (size_t k = 2; k < s.args.size(); k++) add(writes_, s.args[k]);       // result, scratch, counters
+        return true;
+      case Step::MEMCPY: case Step::REPACK16: case Step::TRANSPOSE:
+        add(writes_, s.args[0]);
+        add(reads_, s.args[1]);
+        return true;
+      case Step::SCATTER:
+        for (size_t k = 0; k < s.args.size(); k++) add(k < 3 ? reads_ : writes_, s.args[k]);
+        return true;
+      default: return false;
+    }
+  }
+
+  template <typename F>
+  b200_error* record(bool all, F&& launch) {
+    const int me = (int)nodes_.size();
+    std::vector<int> deps;
+    if (all) {
+      for (int k = 0; k < me; k++) deps.push_back(k);
+      memory_.clear();
+      barrier_ = me;
+    } else {
+      if (barrier_ >= 0) deps.push_back(barrier_);
+      for (auto& m : memory_) {
+        auto meets = [&](const std::vector<Range>& rs) {
+          for (auto& r : rs) if (r.lo < m.at.hi && m.at.lo < r.hi) return true;
+          return false;
+        };
+        const bool written = meets(writes_);
+        if ((written || meets(reads_)) && m.writer >= 0) deps.push_back(m.writer);
+        if (written) deps.insert(deps.end(), m.readers.begin(), m.readers.end());
+      }
+    }
+    // keep what no other dependence implies
+    std::sort(deps.begin(), deps.end());
+    deps.erase(std::unique(deps.begin(), deps.end()), deps.end());
+    Node node;
+    node.before.assign(me, false);
+    std::vector<cudaGraphNode_t> from;
+    for (size_t k = deps.size(); k-- > 0;) {
+      const int d = deps[k];
+      if (node.before[d]) continue;
+      from.insert(from.end(), nodes_[d].ends.begin(), nodes_[d].ends.end());
+      node.before[d] = true;
+      for (size_t q = 0; q < nodes_[d].before.size(); q++) if (nodes_[d].before[q]) node.before[q] = true;
+    }
+    const cudaStream_t st = x_.c->compute;
+    CUDA_TRY(cudaStreamBeginCaptureToGraph(st, graph_, from.data(), nullptr, from.size(), cudaStreamCaptureModeRelaxed));
+    // launches stay programmatic: the capture makes every edge into such a kernel a programmatic one, and its first
+    // statement waits for all of the kernels those come from
+    b200_error* err = launch();
+    cudaStreamCaptureStatus status;
+    const cudaGraphNode_t* ends = nullptr;
+    size_t count = 0;
+    cudaError_t ce = cudaStreamGetCaptureInfo(st, &status, nullptr, nullptr, &ends, &count);
+    if (ce == cudaSuccess) node.ends.assign(ends, ends + count);
+    cudaError_t ee = cudaStreamEndCapture(st, nullptr);
+    if (err) return err;
+    CUDA_TRY(ce);
+    CUDA_TRY(ee);
+    // what this step wrote supersedes what was known about memory inside it
+    for (auto& w : writes_)
+      memory_.erase(std::remove_if(memory_.begin(), memory_.end(), [&](const Memory& m) { return w.lo <= m.at.lo && m.at.hi <= w.hi; }), memory_.end());
+    for (auto& w : writes_) memory_.push_back({w, me, {}});
+    for (auto& r : reads_) {
+      Memory* found = nullptr;
+      for (auto& m : memory_) if (m.at.lo == r.lo && m.at.hi == r.hi) { found = &m; break; }
+      if (found) { if (found->writer != me) found->readers.push_back(me); }
+      else memory_.push_back({r, -1, {me}});
+    }
+    nodes_.push_back(std::move(node));
+    return nullptr;
+  }
+  ExecCtx& x_;
+  cudaGraph_t graph_;
+  std::vector<Node> nodes_;
+  std::vector<Memory> memory_;
+  std::vector<Range> reads_, writes_;
+  int barrier_ = -1;
+};
+
 b200_error* run_step(ExecCtx& x, const Step& s) {
   b200_client* c = x.c;
   cudaStream_t st = c->compute;
@@ -931,7 +1078,16 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
           LoadedProgram::LoopGraph* hit = nullptr;
           for (auto& g : x.lp->loop_graphs)
             if (g.step == &s && g.ptrs == touched) { hit = &g; break; }
-          if (!hit) {
+          bool record = !hit;
+          if (record && !x.lp->met_before(&s, touched)) {
+            // addresses that are new: a loop of many recordings' length is worth one all the same
+            const int first = x.launches;
+            if (auto* e = iterate()) return e;
+            if (auto* e = iterate()) return e;
+            done = 2;
+            record = (s.trip_count - done) / 2 * std::max(1, x.launches - first) >= 16 * kLoopGraphNodes;
+          }
+          if (record) {
             if (x.lp->loop_graphs.size() >= 24) {
               // bounded cache: let the device finish with the oldest graph before it goes
               CUDA_TRY(cudaStreamSynchronize(st));
@@ -939,25 +1095,36 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
               x.lp->loop_graphs.erase(x.lp->loop_graphs.begin());
             }
             const std::vector<void*> at_start = x.ptrs;
-            // the first pair runs directly, so that every kernel of the body has been loaded and configured
-            // before anything is recorded
+            // a pair runs directly, so that every kernel of the body has been loaded and configured before anything is
+            // recorded, and its launches are known
             const int first = x.launches;
             if (auto* e = iterate()) return e;
             if (auto* e = iterate()) return e;
-            done = 2;
+            done += 2;
             const int per_pair = std::max(1, x.launches - first);
             const long long pairs = std::max<long long>(1, std::min<long long>((s.trip_count - done) / 2, kLoopGraphNodes / per_pair));
             const int before = x.launches;
-            CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
-            b200_error* err = nullptr;
-            for (long long i = 0; i < 2 * pairs && !err; i++) err = iterate();
             cudaGraph_t graph = nullptr;
-            cudaError_t ce = cudaStreamEndCapture(st, &graph);
+            CUDA_TRY(cudaGraphCreate(&graph, 0));
+            b200_error* err = nullptr;
+            {
+              Recorder recorder(x, graph);
+              for (long long i = 0; i < 2 * pairs && !err; i++) {
+                for (const Step& t : s.sub[1]->steps)
+                  if (!err) err = recorder.step(t);
+                for (size_t k = 0; k < n && !err; k++) {
+                  void *&d = x.ptrs[s.state[k]], *&src = x.ptrs[s.next[k]];
+                  const size_t b = x.lp->prog->slots[s.state[k]].type.bytes();
+                  if (k < s.swap.size() && s.swap[k]) std::swap(d, src);
+                  else if (d != src && b) err = recorder.copy(d, src, b);
+                }
+              }
+            }
             if (err) {
-              if (graph) cudaGraphDestroy(graph);
+              cudaGraphDestroy(graph);
               return err;
             }
-            CUDA_TRY(ce);
+            cudaError_t ce;
             cudaGraphExec_t exec = nullptr;
             ce = cudaGraphInstantiate(&exec, graph, 0);
             cudaGraphDestroy(graph);
@@ -970,7 +1137,7 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
             x.launches = before;
             hit = &x.lp->loop_graphs.back();
           }
-          for (; done + hit->iterations <= s.trip_count; done += hit->iterations) {
+          for (; hit && done + hit->iterations <= s.trip_count; done += hit->iterations) {
             CUDA_TRY(cudaGraphLaunch(hit->exec, st));
             x.launches += hit->launches;
           }
@@ -1356,47 +1523,41 @@ b200_error* run_main(ExecCtx& x) {
   std::vector<void*> key;
   for (size_t s = 0; s < lp.prog->slots.size(); s++)
     if (lp.prog->slots[s].kind == Slot::ARG || lp.prog->slots[s].kind == Slot::RESULT) key.push_back(x.ptrs[s]);
-  LoadedProgram::PlanGraph* hit = nullptr;
   for (auto& g : lp.plan_graphs)
-    if (g.ptrs == key) { hit = &g; break; }
-  if (hit && hit->exec) {
-    hit->used = lp.calls;
-    lp.replays++;
-    CUDA_TRY(cudaGraphLaunch(hit->exec, c->compute));
-    x.launches += hit->launches;
-    return nullptr;
-  }
-  if (!hit) {
-    if (lp.plan_graphs.size() >= kPlanGraphs) {
-      auto old = std::min_element(lp.plan_graphs.begin(), lp.plan_graphs.end(), [](auto& a, auto& b) { return a.used < b.used; });
-      if (old->exec) {
-        CUDA_TRY(cudaStreamSynchronize(c->compute));
-        cudaGraphExecDestroy(old->exec);
-      }
-      lp.plan_graphs.erase(old);
+    if (g.ptrs == key) {
+      g.used = lp.calls;
+      lp.replays++;
+      CUDA_TRY(cudaGraphLaunch(g.exec, c->compute));
+      x.launches += g.launches;
+      return nullptr;
     }
-    lp.plan_graphs.push_back({std::move(key), nullptr, 0, lp.calls});
-    return run_plan(x, plan);
+  if (!lp.met_before(&plan, key) || lp.recordings > 2 * kPlanGraphs + lp.replays / 16) return run_plan(x, plan);
+  if (lp.plan_graphs.size() >= kPlanGraphs) {
+    auto old = std::min_element(lp.plan_graphs.begin(), lp.plan_graphs.end(), [](auto& a, auto& b) { return a.used < b.used; });
+    CUDA_TRY(cudaStreamSynchronize(c->compute));
+    cudaGraphExecDestroy(old->exec);
+    lp.plan_graphs.erase(old);
   }
-  hit->used = lp.calls;
-  if (lp.recordings > 2 * kPlanGraphs + lp.replays / 16) return run_plan(x, plan);
   lp.recordings++;
   const int before = x.launches;
-  CUDA_TRY(cudaStreamBeginCapture(c->compute, cudaStreamCaptureModeRelaxed));
-  b200_error* err = run_plan(x, plan);
   cudaGraph_t graph = nullptr;
-  cudaError_t ce = cudaStreamEndCapture(c->compute, &graph);
+  CUDA_TRY(cudaGraphCreate(&graph, 0));
+  b200_error* err = nullptr;
+  {
+    Recorder recorder(x, graph);
+    for (const Step& st : plan.steps)
+      if (!err) err = recorder.step(st);
+  }
   if (err) {
-    if (graph) cudaGraphDestroy(graph);
+    cudaGraphDestroy(graph);
     return err;
   }
-  CUDA_TRY(ce);
+  cudaError_t ce;
   cudaGraphExec_t exec = nullptr;
   ce = cudaGraphInstantiate(&exec, graph, 0);
   cudaGraphDestroy(graph);
   CUDA_TRY(ce);
-  hit->exec = exec;
-  hit->launches = x.launches - before;
+  lp.plan_graphs.push_back({std::move(key), exec, x.launches - before, lp.calls});
   CUDA_TRY(cudaGraphLaunch(exec, c->compute));
   return nullptr;
 }
