@@ -13,7 +13,7 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 OUT = HERE / "b200" / "libb200core.so"
 HOT = HERE / "b200" / "_hot.so"
-SOURCES = ["parser.cc", "codegen.cc", "compiler.cc", "runtime.cc", "kernels.cu", "gemm16.cu", "gemm32.cu"]
+SOURCES = ["parser.cc", "codegen.cc", "compiler.cc", "runtime.cc", "kernels.cu", "gemm16.cu", "gemm32.cu", "tile32.cu"]
 
 
 def _nccl_include() -> str:

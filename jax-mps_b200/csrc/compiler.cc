@@ -3464,14 +3464,38 @@ struct Planner {
     return best_cost;
   }
 
-  // Whether a dense fp32 product is faster on the FMA pipe (gemm32.cu) than on the tensor cores, and in which tile and
-  // split. Cycles of an SM, fitted to products from 64 x 64 x 64 to 512 x 8003 x 462: 1.7 per row of four warps' FMA
+  // Tile width and K split of a contraction by tiled copies (tile32.cu), and its modelled time in microseconds. Cycles: 450 per
+  // 64-wide and 800 per 128-wide k-tile, 500 per tile of C, 3000 to launch, fill and drain; a split adds the pass that sums it.
+  // A k-tile really takes 830 and 960, but the table-driven kernels take as much longer than choose_split_k says, and the two are
+  // compared. At the measured values the 462-row encoder step ran 1540 us, at these 1330; ResNet-18 steps differed by 1 %.
+  // `b_is_weight`: B is a program input, whose split image is made beside what is in front of the product.
+  static double tile_product(Tile32Launch& t, bool b_is_weight) {
+    const long long ktiles = (t.K + 31) / 32, tm = (t.M + 127) / 128;
+    double best = 1e30;
+    for (int bn : {128, 64}) {
+      if (bn == 128 && t.N <= 64) continue;
+      const long long tiles = tm * ((t.N + bn - 1) / bn) * t.G;
+      for (long long want = 1; want <= std::min<long long>(ktiles, 160); want++) {
+        const long long kps = (ktiles + want - 1) / want, split = (ktiles + kps - 1) / kps;
+        if (split != want) continue;
+        if (split > 1 && (tiles * split > 2 * 148 || split * t.G * t.M * t.N > (64LL << 20))) break;
+        double cycles = (double)((tiles * split + 147) / 148) * ((double)kps * (bn == 64 ? 450.0 : 800.0) + 500.0) + 3000.0;
+        if (split > 1) cycles += 4000.0 + (double)split * t.G * t.M * t.N * 8.0 / 3000.0;
+        if (cycles < best * 0.98) { best = cycles; t.bn = bn; t.split = (int)split; }
+      }
+    }
+    const double image = (double)t.G * t.K * t.N * 12.0;
+    return best / 1850.0 + (b_is_weight ? 0.3 : 2.0 + image / 5e6);
+  }
+
+  // Modelled time of a dense fp32 product on the FMA pipe (gemm32.cu), with its tile and split. Cycles of an SM, fitted to
+  // products from 64 x 64 x 64 to 512 x 8003 x 462: 1.7 per row of four warps' FMA
   // instructions and k when a CTA is alone on its SM (one warp per scheduler) and 1.25 when others fill its stalls, 1500
   // (900) to fill and drain a CTA, 2500 for the launch, 700 for the sum of warps, 1000 for that of a
   // cluster. The lines against choose_split_k's model: 462 x 512 x 512 is 7 us here and 19 there, 462 x 2048 x 512 about
   // 27 both ways, 4096 x 1000 x 784 stays on the tensor cores.
-  static bool fma_product(Gemm32Launch& g) {
-    if (g.G > 65535 || getenv("B200_NO_GEMM32")) return false;
+  static double fma_product(Gemm32Launch& g) {
+    if (g.G > 65535 || getenv("B200_NO_GEMM32")) return 1e30;
     double best = 1e30;
     for (int tile = 2; tile >= 0; tile--) {
       const int tm = tile == 0 ? 32 : 64, tn = tile == 2 ? 128 : 64;
@@ -3486,12 +3510,18 @@ struct Planner {
         if (us < best * 0.97) { best = us; g.split = split; g.tile = tile; }
       }
     }
+    return best;
+  }
+  // ... and in the table-driven kernels (choose_split_k).
+  static double table_product(const Gemm32Launch& g) {
     IGemmParams t;
     t.M = g.M; t.N = g.N; t.K = g.K; t.groups = g.G;
     t.vec = g.a_vec && g.b_vec;
     t.seg = t.vec && g.K % 32 == 0 && (g.a_kc || g.M % 32 == 0) && (g.b_kc || g.N % 32 == 0);
-    return best < choose_split_k(t);
+    return choose_split_k(t);
   }
+
+  std::vector<Step> before_product;          // steps that go in front of the product being lowered
 
   Step lower_conv(Op* op, BlockState& st) {
     Value *lhs = op->operands[0], *rhs = op->operands[1], *out = op->results[0];
@@ -3629,6 +3659,16 @@ struct Planner {
         p.tma_ow = (int)OW; p.tma_oh = (int)OH; p.tma_box_h = (int)box_h; p.tma_box_n = (int)box_n;
         p.tma_kw = (int)KW; p.tma_pad_h = (int)pad[0]; p.tma_pad_w = (int)pad[2];
         p.tma_rdil_h = (int)rdil[0]; p.tma_rdil_w = (int)rdil[1];
+        if (!getenv("B200_NO_TILE32")) {
+          Tile32Launch& t = p.tile;
+          t.mode = 1;
+          t.M = p.M; t.N = p.N; t.K = p.K;
+          t.dims[0] = Cin; t.dims[1] = W; t.dims[2] = H; t.dims[3] = Nb;
+          t.strides[0] = Cin; t.strides[1] = W * Cin; t.strides[2] = H * W * Cin;
+          t.box[0] = 32; t.box[1] = (unsigned)OW; t.box[2] = (unsigned)box_h; t.box[3] = (unsigned)box_n;
+          t.ow = (int)OW; t.oh = (int)OH; t.kw = (int)KW; t.cin = (int)Cin;
+          t.dil_h = (int)rdil[0]; t.dil_w = (int)rdil[1]; t.pad_h = (int)pad[0]; t.pad_w = (int)pad[2];
+        }
       }
     }
     return make_igemm(op, p, lhs, rhs, out, arow, acol, bcol, bn, crow, cn, ag, bg, cg, st);
@@ -3748,7 +3788,23 @@ struct Planner {
         auto rows16 = [](int extent, long long ld, long long gs) { return extent % 4 == 0 && ld % 4 == 0 && gs % 4 == 0; };
         g.a_vec = rows16(g.a_kc ? g.K : g.M, g.a_ld, g.a_gs);
         g.b_vec = rows16(g.b_kc ? g.K : g.N, g.b_ld, g.b_gs);
-        if (fma_product(g)) {
+        // three ways: the FMA pipe, tiled copies, the table-driven kernels
+        Tile32Launch t;
+        t.M = g.M; t.N = g.N; t.K = g.K; t.G = g.G;
+        const double us_fma = fma_product(g), us_table = table_product(g);
+        double us_tile = 1e30;
+        if (g.a_vec && g.M * g.G >= 64 && !getenv("B200_NO_TILE32")) {
+          t.mode = g.a_kc ? 2 : 3;
+          const long long inner = g.a_kc ? g.K : g.M, outer = g.a_kc ? g.M : g.K;
+          t.dims[0] = inner; t.dims[1] = outer; t.dims[2] = g.G; t.dims[3] = 1;
+          t.strides[0] = outer > 1 ? g.a_ld : (inner + 3) / 4 * 4;
+          t.strides[1] = g.G > 1 ? g.a_gs : t.strides[0] * outer;
+          t.strides[2] = t.strides[1] * g.G;
+          t.box[0] = 32; t.box[1] = g.a_kc ? 128 : 32; t.box[2] = t.box[3] = 1;
+          us_tile = tile_product(t, !rhs->def && rhs->owner && rhs->owner->parent_op == nullptr);
+        }
+        if (us_tile < us_fma && us_tile < us_table) p.tile = t;
+        else if (us_fma < us_table) {
           p.fma = g;
           p.a_contig = g.a_kc ? 0 : 1;
           p.b_contig = g.b_kc;
@@ -3868,12 +3924,37 @@ struct Planner {
       if (al) p.c_vec = 2;
     }
     if (!(p.seg && p.a_contig == 0)) p.a_tma = 0;
-    choose_split_k(p);
+    const double us_table = choose_split_k(p);
     Step s;
     s.kind = Step::IGEMM;
     s.label = op->name;
-    s.ig = p;
     auto tab = [&](const void* d, size_t n) { return table_slot(d, std::max<size_t>(n, 1)); };
+    if (p.tile.mode && op->short_name() != "dot_general") {
+      const bool weight = !rhs->def && rhs->owner && rhs->owner->parent_op == nullptr;
+      if (tile_product(p.tile, weight) >= us_table) p.tile.mode = 0;
+    }
+    if (p.tile.mode) {
+      p.tile.c_vec = p.c_vec;
+      s.ig = p;
+      TensorType it;
+      it.dt = DT::F32;
+      it.dims = {(int64_t)p.tile.image_floats()};
+      Step b;
+      b.kind = Step::SPLIT_B;
+      b.label = "split of an operand of " + op->name;
+      b.ig = p;
+      b.args = {new_slot(Slot::TEMP, it, st.arena), slot_of.at(rhs), tab(bcol.data(), bcol.size() * 8), tab(bn.data(), bn.size() * 8), tab(bg.data(), bg.size() * 8)};
+      s.args = {slot_of.at(lhs), b.args[0], slot_of.at(out), tab(crow.data(), crow.size() * 8), tab(cn.data(), cn.size() * 8), tab(cg.data(), cg.size() * 8)};
+      if (p.tile.split > 1) {
+        TensorType t;
+        t.dt = DT::F32;
+        t.dims = {p.tile.split, p.tile.G, p.tile.M, p.tile.N};
+        s.args.push_back(new_slot(Slot::TEMP, t, st.arena));
+      }
+      before_product.push_back(std::move(b));
+      return s;
+    }
+    s.ig = p;
     s.args = {slot_of.at(lhs), slot_of.at(rhs), slot_of.at(out),
               tab(arow.data(), arow.size() * sizeof(RowEnt)), tab(acol.data(), acol.size() * sizeof(ColEnt)),
               tab(bcol.data(), bcol.size() * 8), tab(bn.data(), bn.size() * 8), tab(crow.data(), crow.size() * 8),
@@ -5043,6 +5124,8 @@ struct Planner {
           Dot16 native;
           if (c == Cat::DOT && dot16_geometry(op, native)) { lower_dot16(op, native, plan, st); break; }
           Step s = c == Cat::CONV ? lower_conv(op, st) : lower_dot(op, st);
+          for (auto& b : before_product) plan.steps.push_back(std::move(b));
+          before_product.clear();
           plan.steps.push_back(std::move(s));
           break;
         }
@@ -5640,9 +5723,11 @@ void dump_plan(const CompiledProgram& prog, const Plan& p, std::ostringstream& o
       case Step::IGEMM:
         os << "igemm M=" << s.ig.M << " N=" << s.ig.N << " K=" << s.ig.K << " G=" << s.ig.groups << " splitK=" << s.ig.split_k
            << " a_contig=" << s.ig.a_contig << " b_contig=" << s.ig.b_contig << " vec=" << s.ig.vec << " seg=" << s.ig.seg << (s.ig.kt_stride ? " ktlist" : "") << (s.ig.a_tma ? " tmaA" : "");
+        if (s.ig.tile.mode) os << " tile mode=" << s.ig.tile.mode << " bn=" << s.ig.tile.bn << " split=" << s.ig.tile.split;
         if (s.ig.fma.split) os << " fma tile=" << s.ig.fma.tile << " cluster=" << s.ig.fma.split;
         os << " " << s.label;
         break;
+      case Step::SPLIT_B: os << "split_b N=" << s.ig.tile.N << " K=" << s.ig.tile.K << " bn=" << s.ig.tile.bn << " " << s.label; break;
       case Step::MEMCPY: os << "memcpy " << s.bytes; break;
       case Step::GEMM16:
         os << (s.g16.path == 0 ? "gemm16" : s.g16.path == 1 ? "gemv16_nc" : s.g16.path == 3 ? "gemv16_nc_small" : "gemv16_kc") << " M=" << s.g16.M << " N=" << s.g16.N
@@ -5771,7 +5856,8 @@ std::unique_ptr<CompiledProgram> compile_module(Module& m, const CompileOptions&
       for (auto& s : p.steps) {
         if (s.kind == Step::KERNEL || s.kind == Step::ALL_REDUCE || s.kind == Step::ALL_GATHER) n += 1;
         else if (s.kind == Step::SCATTER) n += (s.iparams.size() > 5 && s.iparams[5] == 1) ? scatter_elems_launches(s.iparams[0]) - (s.iparams[4] < 0 ? 1 : 0) : scatter_rows_launches(s.iparams[0], s.iparams[2]);
-        else if (s.kind == Step::IGEMM) n += s.ig.split_k > 1 ? 2 : 1;
+        else if (s.kind == Step::IGEMM) n += (s.ig.tile.mode ? s.ig.tile.split : s.ig.split_k) > 1 ? 2 : 1;
+        else if (s.kind == Step::SPLIT_B) n += 1;
         else if (s.kind == Step::GEMM16) n += (s.g16.path == 0 && s.g16.split_k > 1) ? 2 : 1;
         else if (s.kind == Step::REPACK16) n += (s.iparams[0] + 65534) / 65535;
         else if (s.kind == Step::TRANSPOSE) n += 1;

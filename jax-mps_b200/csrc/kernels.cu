@@ -1068,27 +1068,6 @@ struct TaCfg {
   static constexpr int THREADS = HALF ? 416 : 800;
 };
 
-__device__ __forceinline__ void umma_tf32_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-__device__ __forceinline__ void tmem_store32(uint32_t taddr, const uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, "
-      "%25, %26, %27, %28, %29, %30, %31, %32};"
-      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-        "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]),
-        "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
-        "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-      : "memory");
-}
-
 template <int BN, bool A_MCONTIG, bool B_KCONTIG, bool MASK, bool HALF>
 __global__ void __launch_bounds__((TaCfg<BN, HALF>::THREADS), (HALF ? 2 : 1)) igemm_tf32x3_ta_kernel(
     const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C, const RowEnt* __restrict__ a_row,
@@ -1560,6 +1539,23 @@ __global__ void __launch_bounds__(256) scatter_apply_elems_kernel(T* __restrict_
 
 }  // namespace
 
+cudaError_t launch_splitk_reduce(const float* partial, float* C, const long long* c_row, const long long* c_col, const long long* c_grp, int M, int N,
+                                 int groups, int split_k, int c_vec, cudaStream_t stream, int* launches) {
+  const long long total = (long long)groups * M * N;
+  // four consecutive n per thread when they are four consecutive, 16-byte aligned floats of C; the splits are
+  // spread over 8 thread rows when there are many of them and few outputs
+  const bool vec = c_vec == 2 && N % 4 == 0 && (((uintptr_t)C) & 15) == 0 && (((uintptr_t)partial) & 15) == 0;
+  const long long items = vec ? total / 4 : total;
+  const bool tall = split_k >= 16;
+  const unsigned blocks = (unsigned)(tall ? (items + 31) / 32 : (items + 255) / 256);
+  if (vec && tall) launch_k(splitk_reduce_kernel<8, true>, blocks, dim3(32, 8), 0, stream, partial, C, c_row, c_col, c_grp, M, N, groups, split_k);
+  else if (vec) launch_k(splitk_reduce_kernel<1, true>, blocks, dim3(256, 1), 0, stream, partial, C, c_row, c_col, c_grp, M, N, groups, split_k);
+  else if (tall) launch_k(splitk_reduce_kernel<8, false>, blocks, dim3(32, 8), 0, stream, partial, C, c_row, c_col, c_grp, M, N, groups, split_k);
+  else launch_k(splitk_reduce_kernel<1, false>, blocks, dim3(256, 1), 0, stream, partial, C, c_row, c_col, c_grp, M, N, groups, split_k);
+  if (launches) (*launches)++;
+  return cudaGetLastError();
+}
+
 cudaError_t launch_igemm_f32(const IGemmLaunch& p, const void* A, const void* B, void* C, const void* const* tables,
                              void* partial, const int* kt_table, int* error_flag, cudaStream_t stream, int* launches) {
   auto a_row = (const RowEnt*)tables[0];
@@ -1689,23 +1685,7 @@ cudaError_t launch_igemm_f32(const IGemmLaunch& p, const void* A, const void* B,
   if (launches) (*launches)++;
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  if (p.split_k > 1) {
-    long long total = (long long)p.groups * p.M * p.N;
-    // four consecutive n per thread when they are four consecutive, 16-byte aligned floats of C; the splits are
-    // spread over 8 thread rows when there are many of them and few outputs
-    const float* pp = (const float*)partial;
-    float* cc = (float*)C;
-    const bool vec = p.c_vec == 2 && p.N % 4 == 0 && (((uintptr_t)C) & 15) == 0 && (((uintptr_t)partial) & 15) == 0;
-    const long long items = vec ? total / 4 : total;
-    const bool tall = p.split_k >= 16;
-    const unsigned blocks = (unsigned)(tall ? (items + 31) / 32 : (items + 255) / 256);
-    if (vec && tall) launch_k(splitk_reduce_kernel<8, true>, blocks, dim3(32, 8), 0, stream, pp, cc, c_row, c_col, c_grp, p.M, p.N, p.groups, p.split_k);
-    else if (vec) launch_k(splitk_reduce_kernel<1, true>, blocks, dim3(256, 1), 0, stream, pp, cc, c_row, c_col, c_grp, p.M, p.N, p.groups, p.split_k);
-    else if (tall) launch_k(splitk_reduce_kernel<8, false>, blocks, dim3(32, 8), 0, stream, pp, cc, c_row, c_col, c_grp, p.M, p.N, p.groups, p.split_k);
-    else launch_k(splitk_reduce_kernel<1, false>, blocks, dim3(256, 1), 0, stream, pp, cc, c_row, c_col, c_grp, p.M, p.N, p.groups, p.split_k);
-    if (launches) (*launches)++;
-    e = cudaGetLastError();
-  }
+  if (p.split_k > 1) e = launch_splitk_reduce((const float*)partial, (float*)C, c_row, c_col, c_grp, p.M, p.N, p.groups, p.split_k, p.c_vec, stream, launches);
   return e;
 }
 

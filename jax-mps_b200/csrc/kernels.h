@@ -4,6 +4,7 @@
 
 #include "gemm16.h"
 #include "gemm32.h"
+#include "tile32.h"
 
 namespace b200 {
 
@@ -69,6 +70,16 @@ void set_igemm_programmatic_launch(bool on);
 cudaError_t launch_while_handle(unsigned long long handle, const void* pred, unsigned long long* started, double limit_seconds,
                                 bool first, int* error_flag, cudaStream_t stream);
 cudaError_t launch_switch_handle(unsigned long long handle, const void* index, int branches, cudaStream_t stream);
+
+// fp32 contraction by tiled copies (tile32.cu): B split into its image (b_tables: b_row, b_col, b_grp; `lanes_n`: n is the
+// contiguous index of B), then the product (c_tables: c_row, c_col, c_grp; `partial`: [split][G][M][N] floats for split > 1).
+cudaError_t launch_split_b(const Tile32Launch& t, bool lanes_n, const void* B, void* image, const void* const* b_tables, cudaStream_t stream, int* launches);
+cudaError_t launch_tile32(const Tile32Launch& t, const void* A, const void* image, void* C, void* partial, const void* const* c_tables, int* error_flag,
+                          cudaStream_t stream, int* launches);
+void set_tile32_programmatic_launch(bool on);
+// Sum of split-K partial tiles in a fixed order.
+cudaError_t launch_splitk_reduce(const float* partial, float* C, const long long* c_row, const long long* c_col, const long long* c_grp, int M, int N,
+                                 int groups, int split_k, int c_vec, cudaStream_t stream, int* launches);
 
 // fp32 product on the FMA pipe (gemm32.cu): C dense [G][M][N].
 cudaError_t launch_gemm32(const Gemm32Launch& p, const void* A, const void* B, void* C, cudaStream_t stream, int* launches);

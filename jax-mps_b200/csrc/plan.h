@@ -14,6 +14,7 @@
 
 #include "gemm16.h"
 #include "gemm32.h"
+#include "tile32.h"
 #include "ir.h"
 
 namespace b200 {
@@ -53,6 +54,7 @@ struct IGemmParams {
   int tma_c = 0, tma_w = 0, tma_h = 0, tma_n = 0;        // input extents (channels, width, height, images)
   int tma_ow = 0, tma_oh = 0, tma_box_h = 0, tma_box_n = 0;
   int tma_kw = 0, tma_pad_h = 0, tma_pad_w = 0, tma_rdil_h = 1, tma_rdil_w = 1;
+  Tile32Launch tile;                         // mode > 0: by tiled copies, args are {A, image of B, C, c_row, c_col, c_grp, [partial sums]}
   Gemm32Launch fma;                          // split > 0: a dense product on the FMA pipe, args are {A, B, C} alone
 };
 
@@ -65,7 +67,7 @@ long long scatter_elems_scratch_ints(long long updates);
 int scatter_elems_launches(long long numel);
 
 struct Step {
-  enum Kind { KERNEL, IGEMM, MEMCPY, MEMSET, WHILE, CASE, ALL_REDUCE, SCATTER, JOIN, GEMM16, REPACK16, TRANSPOSE, ALL_GATHER } kind = KERNEL;
+  enum Kind { KERNEL, IGEMM, MEMCPY, MEMSET, WHILE, CASE, ALL_REDUCE, SCATTER, JOIN, GEMM16, REPACK16, TRANSPOSE, ALL_GATHER, SPLIT_B } kind = KERNEL;
   std::string label;                  // op names, for profiling and error text
   // KERNEL
   int kernel = -1;                    // index into Executable::kernels
@@ -75,6 +77,7 @@ struct Step {
   std::vector<char> writes;           // KERNEL of several parts (n_outs 0): per argument, whether it is written
   // IGEMM (ig.fma.split == 0): args = {A, B, C, a_row, a_col, b_row(k), b_col(n), c_row(m), c_col(n), a_grp, b_grp, c_grp, [split-K scratch]}
   IGemmParams ig;
+  // SPLIT_B: args = {image, B, b_row, b_col, b_grp}, ig.tile as in the product that reads the image; ig.b_contig
   // GEMM16: args = {A, B, C, [fp32 scratch], [counters]}; iparams = {has scratch, has counters}
   // REPACK16: args = {dst, src}; iparams = {rows, cols, dst_ld, src_ld}
   // TRANSPOSE: args = {dst, src}; iparams = {element bytes, batch, rows, cols, dst_ld, dst batch stride, dst offset (elements)}

@@ -722,7 +722,7 @@ bool waits_inside(const Plan& plan) {
 bool graph_safe(const Plan& plan);
 bool graph_safe_step(const Step& s) {
   switch (s.kind) {
-    case Step::KERNEL: case Step::IGEMM: case Step::MEMCPY: case Step::GEMM16: case Step::REPACK16: case Step::TRANSPOSE: return true;
+    case Step::KERNEL: case Step::IGEMM: case Step::MEMCPY: case Step::GEMM16: case Step::REPACK16: case Step::TRANSPOSE: case Step::SPLIT_B: return true;
     case Step::WHILE: return s.trip_count >= 0 && graph_safe(*s.sub[1]);
     default: return false;
   }
@@ -796,14 +796,15 @@ class Recorder {
         add(reads_, s.args[0]);
         add(reads_, s.args[1]);
         add(writes_, s.args[2]);
-        if (!s.ig.fma.split && s.ig.split_k > 1) add(writes_, s.args[12]);
+        if (s.ig.tile.mode) { if (s.ig.tile.split > 1) add(writes_, s.args[6]); }
+        else if (!s.ig.fma.split && s.ig.split_k > 1) add(writes_, s.args[12]);
         return true;
       case Step::GEMM16:
         add(reads_, s.args[0]);
         add(reads_, s.args[1]);
         for (size_t k = 2; k < s.args.size(); k++) add(writes_, s.args[k]);       // result, scratch, counters
         return true;
-      case Step::MEMCPY: case Step::REPACK16: case Step::TRANSPOSE:
+      case Step::MEMCPY: case Step::REPACK16: case Step::TRANSPOSE: case Step::SPLIT_B:
         add(writes_, s.args[0]);
         add(reads_, s.args[1]);
         return true;
@@ -923,6 +924,13 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
       return nullptr;
     }
     case Step::IGEMM: {
+      if (s.ig.tile.mode) {
+        const void* tables[3] = {x.ptrs[s.args[3]], x.ptrs[s.args[4]], x.ptrs[s.args[5]]};
+        cudaError_t e = launch_tile32(s.ig.tile, x.ptrs[s.args[0]], x.ptrs[s.args[1]], x.ptrs[s.args[2]], s.ig.tile.split > 1 ? x.ptrs[s.args[6]] : nullptr,
+                                      tables, c->error_flag, st, &x.launches);
+        if (e != cudaSuccess) return make_error(B200_INTERNAL, "launch of " + s.label + " failed: " + cudaGetErrorString(e));
+        return nullptr;
+      }
       if (s.ig.fma.split) {
         cudaError_t e = launch_gemm32(s.ig.fma, x.ptrs[s.args[0]], x.ptrs[s.args[1]], x.ptrs[s.args[2]], st, &x.launches);
         if (e != cudaSuccess) return make_error(B200_INTERNAL, "launch of " + s.label + " failed: " + cudaGetErrorString(e));
@@ -953,6 +961,12 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
       const int* kt_table = s.ig.kt_stride > 0 ? (const int*)x.ptrs[s.args.back()] : nullptr;
       cudaError_t e = launch_igemm_f32(p, x.ptrs[s.args[0]], x.ptrs[s.args[1]], x.ptrs[s.args[2]], tables, partial,
                                        kt_table, c->error_flag, st, &x.launches);
+      if (e != cudaSuccess) return make_error(B200_INTERNAL, "launch of " + s.label + " failed: " + cudaGetErrorString(e));
+      return nullptr;
+    }
+    case Step::SPLIT_B: {
+      const void* tables[3] = {x.ptrs[s.args[2]], x.ptrs[s.args[3]], x.ptrs[s.args[4]]};
+      cudaError_t e = launch_split_b(s.ig.tile, s.ig.b_contig == 0, x.ptrs[s.args[1]], x.ptrs[s.args[0]], tables, st, &x.launches);
       if (e != cudaSuccess) return make_error(B200_INTERNAL, "launch of " + s.label + " failed: " + cudaGetErrorString(e));
       return nullptr;
     }
@@ -1196,6 +1210,7 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
         set_programmatic_launch(false);
         set_igemm_programmatic_launch(false);
         set_gemm32_programmatic_launch(false);
+        set_tile32_programmatic_launch(false);
         cudaError_t ce = cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed);
         if (ce != cudaSuccess) fail(ce, "begin capture");
         else {
@@ -1250,6 +1265,7 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
         set_programmatic_launch(!c->sw.no_pdl);
         set_igemm_programmatic_launch(!c->sw.no_pdl && !getenv("B200_NO_IGEMM_PDL"));
         set_gemm32_programmatic_launch(!c->sw.no_pdl);
+        set_tile32_programmatic_launch(!c->sw.no_pdl);
         if (graph) cudaGraphDestroy(graph);
         const int recorded = x.launches - before;
         x.launches = before;
@@ -1479,7 +1495,8 @@ b200_error* run_plan(ExecCtx& x, const Plan& plan) {
                   " G=" + std::to_string(s.ig.groups) + " splitK=" + std::to_string(s.ig.split_k) + " a_mcontig=" +
                   std::to_string(s.ig.a_contig) + " b_kcontig=" + std::to_string(s.ig.b_contig) + " mask=" +
                   std::to_string(s.ig.needs_mask) + " ld=" + std::to_string(s.ig.ldh) + "x" + std::to_string(s.ig.ldw) + " vec=" + std::to_string(s.ig.vec) + " seg=" + std::to_string(s.ig.seg);
-          if (s.ig.fma.split) t.kind = "gemm32", t.key += " fma cluster=" + std::to_string(s.ig.fma.split);
+          if (s.ig.tile.mode) t.key += " tile bn=" + std::to_string(s.ig.tile.bn) + " split=" + std::to_string(s.ig.tile.split);
+          else if (s.ig.fma.split) t.kind = "gemm32", t.key += " fma cluster=" + std::to_string(s.ig.fma.split);
           else if (!(x.c->tensor_cores && (long long)s.ig.M * s.ig.N * s.ig.K * s.ig.groups >= (1LL << 18) && s.ig.K >= 16))
             t.kind = "igemm_fma";
           break;
@@ -1663,6 +1680,7 @@ b200_error* create_client(const b200_client_options* o, ncclComm_t given_comm, b
   set_programmatic_launch(!c->sw.no_pdl);
   set_igemm_programmatic_launch(!c->sw.no_pdl && !getenv("B200_NO_IGEMM_PDL"));
   set_gemm32_programmatic_launch(!c->sw.no_pdl);
+        set_tile32_programmatic_launch(!c->sw.no_pdl);
   if (!driver().ok) return make_error(B200_FAILED_PRECONDITION, driver().error);
   if (c->nprocs > 1) {
     NcclApi& n = nccl();
@@ -1824,7 +1842,7 @@ b200_error* b200_client_compile(b200_client* c, const char* code, size_t code_si
     static const char* names[] = {"B200_NO_WINDOW_UPDATE", "B200_NO_FLAT_ALL_REDUCE", "B200_NO_GEMM16", "B200_NO_ROW_FUSION",
                                   "B200_NO_WEIGHT_HOIST", "B200_NO_LICM", "B200_NO_CSE", "B200_NO_HOIST", "B200_NO_BUNDLES",
                                   "B200_NO_TILED_TRANSPOSE", "B200_NO_ALL_REDUCE_OVERLAP", "B200_DEBUG_NO_REUSE", "B200_NO_COL4",
-                                  "B200_NO_ATTENTION_FUSION", "B200_NO_WIDE_POINTWISE", "B200_NO_WIDE_ROWS", "B200_NO_GEMM32"};
+                                  "B200_NO_ATTENTION_FUSION", "B200_NO_WIDE_POINTWISE", "B200_NO_WIDE_ROWS", "B200_NO_GEMM32", "B200_NO_TILE32"};
     for (size_t k = 0; k < sizeof names / sizeof names[0]; k++)
       if (getenv(names[k])) env_bits |= 1u << k;
   }
