@@ -56,7 +56,7 @@ struct G16Cfg {
   static constexpr int A_BYTES = G_BM * G_BK * 2, B_BYTES = BN * G_BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGES = BN == 256 ? 4 : (BN == 128 ? 6 : 8);       // 192 KB of operand stages
-  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256;
+  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256 + 8 * 4096;      // barriers, 4 KB for each read-back warp
   static constexpr int TMEM_COLS = 2 * BN;                                 // two accumulators
 };
 
@@ -126,42 +126,44 @@ __device__ __forceinline__ uint32_t to_bf16_bits(float v) {
 __device__ __forceinline__ uint32_t to_f16_bits(float v) { return (uint32_t)__half_as_ushort(__float2half_rn(v)); }
 __device__ __forceinline__ uint32_t to16(float v, int c_kind) { return c_kind == 1 ? to_bf16_bits(v) : to_f16_bits(v); }
 
-// Stores 32 consecutive columns (n0 ..) of row `row` of a dense [rows][N] result: fp32 as it is, 16-bit rounded. The
-// widest store the row's address allows is used (a row of an odd-sized result starts 4 or 8 bytes off a 16-byte line).
-__device__ __forceinline__ void store_row32(void* C, long long row, int N, int n0, const uint32_t (&v)[32], int c_kind) {
-  if (n0 >= N) return;
-  const bool full = n0 + 32 <= N;
-  if (c_kind == 2) {
-    float* out = (float*)C + row * N + n0;
-    if (full && (((uintptr_t)out) & 15) == 0) {
+// Two fp32 values as a pair of 16-bit ones, rounded to nearest even.
+__device__ __forceinline__ uint32_t pack16(uint32_t lo, uint32_t hi, int c_kind) {
+  uint32_t d;
+  if (c_kind == 1) asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(__uint_as_float(hi)), "f"(__uint_as_float(lo)));
+  else asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(__uint_as_float(hi)), "f"(__uint_as_float(lo)));
+  return d;
+}
+
+// 32 rows of up to 128 bytes from a warp's staging buffer (16-byte pieces permuted by the row) to rows `pitch` bytes apart,
+// in whole lines: a store of the warp covers four rows, or one where the rows start off 16 bytes (4-byte or 2-byte lanes).
+// Stored from registers, a row a lane, every instruction touched 32 lines: the read-back of a 128 x 256 tile took 7900
+// cycles and set the pace of products with K below about 1000.
+__device__ __forceinline__ void store_lines(char* out, long long pitch, int rows, int bytes, const uint8_t* stage, int lane) {
+  const uintptr_t a = (uintptr_t)out | (uintptr_t)pitch;
+  if ((a & 15) == 0) {
+    const int c = lane & 7;
 #pragma unroll
-      for (int q = 0; q < 32; q += 4)
-        *reinterpret_cast<uint4*>(out + q) = make_uint4(v[q], v[q + 1], v[q + 2], v[q + 3]);
-    } else {
-#pragma unroll
-      for (int q = 0; q < 32; ++q)
-        if (n0 + q < N) out[q] = __uint_as_float(v[q]);
+    for (int i = 0; i < 8; ++i) {
+      const int r = i * 4 + (lane >> 3);
+      if (r < rows && c * 16 < bytes)
+        *reinterpret_cast<uint4*>(out + r * pitch + c * 16) = *reinterpret_cast<const uint4*>(stage + r * 128 + ((c ^ (r & 7)) << 4));
     }
-    return;
-  }
-  uint16_t* out = (uint16_t*)C + row * N + n0;
-  uint32_t w[16];
-#pragma unroll
-  for (int q = 0; q < 16; ++q) w[q] = to16(__uint_as_float(v[2 * q]), c_kind) | (to16(__uint_as_float(v[2 * q + 1]), c_kind) << 16);
-  const uintptr_t a = (uintptr_t)out;
-  if (full && (a & 15) == 0) {
-#pragma unroll
-    for (int q = 0; q < 16; q += 4) *reinterpret_cast<uint4*>(out + 2 * q) = make_uint4(w[q], w[q + 1], w[q + 2], w[q + 3]);
-  } else if (full && (a & 7) == 0) {
-#pragma unroll
-    for (int q = 0; q < 16; q += 2) *reinterpret_cast<uint2*>(out + 2 * q) = make_uint2(w[q], w[q + 1]);
-  } else if (full && (a & 3) == 0) {
-#pragma unroll
-    for (int q = 0; q < 16; ++q) *reinterpret_cast<uint32_t*>(out + 2 * q) = w[q];
+  } else if ((a & 3) == 0) {
+#pragma unroll 8
+    for (int r = 0; r < 32; ++r)
+      if (r < rows && lane * 4 < bytes)
+        *reinterpret_cast<uint32_t*>(out + r * pitch + lane * 4) =
+            *reinterpret_cast<const uint32_t*>(stage + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4);
   } else {
+#pragma unroll 4
+    for (int r = 0; r < 32; ++r)
 #pragma unroll
-    for (int q = 0; q < 32; ++q)
-      if (n0 + q < N) out[q] = (uint16_t)((q & 1) ? (w[q >> 1] >> 16) : (w[q >> 1] & 0xFFFFu));
+      for (int h = 0; h < 2; ++h) {
+        const int e = lane + 32 * h;
+        if (r < rows && e * 2 < bytes)
+          *reinterpret_cast<uint16_t*>(out + r * pitch + e * 2) =
+              *reinterpret_cast<const uint16_t*>(stage + r * 128 + (((e >> 3) ^ (r & 7)) << 4) + (e & 7) * 2);
+      }
   }
 }
 
@@ -170,7 +172,6 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm16_tma_kernel(const __grid_c
                                                                   const __grid_constant__ CUtensorMap tm_b,
                                                                   void* __restrict__ C, float* __restrict__ partial,
                                                                   int* __restrict__ error_flag, Gemm16Params p) {
-  pdl_prologue();
   using Cfg = G16Cfg<BN>;
   constexpr int S = Cfg::STAGES;
   extern __shared__ uint8_t smem_raw[];
@@ -179,7 +180,8 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm16_tma_kernel(const __grid_c
   uint64_t* empty = full + S;                                    // the MMAs that read a stage have retired
   uint64_t* acc_full = empty + S;                                // all MMAs of a tile have retired
   uint64_t* acc_empty = acc_full + 2;                            // the read-back warps are done with an accumulator
-  uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
+  uint64_t* drained = acc_empty + 2;
+  uint32_t* tmem_slot = (uint32_t*)(drained + 1);
   volatile int* failed = (volatile int*)(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -192,6 +194,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm16_tma_kernel(const __grid_c
       mbar_init(smem_u32(&acc_full[b]), 1);
       mbar_init(smem_u32(&acc_empty[b]), 8);
     }
+    mbar_init(smem_u32(drained), 1);
     *failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -204,6 +207,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm16_tma_kernel(const __grid_c
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  pdl_prologue();
 
   const int ktiles = (p.K + G_BK - 1) / G_BK;
   const long long tiles = (long long)p.mtiles * p.ntiles * p.G * p.split_k;
@@ -216,39 +220,34 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm16_tma_kernel(const __grid_c
   };
 
   if (warp == 0) {
-    // ------------------------------ TMA producer (whole warp loops, one elected lane issues) -----------------
+    // ------------------------------ TMA producer (one lane) --------------------------------------------------
     uint32_t it = 0;
     bool ok = true;
-    for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+    if (lane == 0) for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
       int mt, nt, g, sp;
       decode(t, mt, nt, g, sp);
       const int m0 = mt * G_BM, n0 = nt * BN;
       const int kt_end = min(ktiles, (sp + 1) * p.kt_per_split);
       for (int kt = sp * p.kt_per_split; kt < kt_end; ++kt, ++it) {
         const int s = it % S;
-        ok = !*failed && mbar_wait(smem_u32(&empty[s]), ((it / S) & 1) ^ 1);
-        ok = __all_sync(0xFFFFFFFFu, ok);
-        if (!ok) { *failed = 1; break; }
-        if (elect_one()) {
-          const uint32_t bar = smem_u32(&full[s]);
-          mbar_expect_tx(bar, Cfg::STAGE_BYTES);
-          const uint32_t a_dst = smem_u32(smem + s * Cfg::STAGE_BYTES), b_dst = a_dst + Cfg::A_BYTES;
-          const int k0 = kt * G_BK;
-          if (!p.a_mn) tma_load_3d(a_dst, &tm_a, bar, k0, m0, g);                 // box 64 k x 128 m
-          else {
-            tma_load_3d(a_dst, &tm_a, bar, m0, k0, g);                            // boxes 64 m x 64 k
-            tma_load_3d(a_dst + 8192, &tm_a, bar, m0 + 64, k0, g);
-          }
-          if (!p.b_mn) tma_load_3d(b_dst, &tm_b, bar, k0, n0, g);                 // box 64 k x BN n
-          else {
-#pragma unroll
-            for (int j = 0; j < BN / 64; ++j) tma_load_3d(b_dst + j * 8192, &tm_b, bar, n0 + 64 * j, k0, g);
-          }
+        if (it >= S && !(ok = role_wait(smem_u32(&empty[s]), ((it / S) & 1) ^ 1, failed))) break;
+        const uint32_t bar = smem_u32(&full[s]);
+        mbar_expect_tx(bar, Cfg::STAGE_BYTES);
+        const uint32_t a_dst = smem_u32(smem + s * Cfg::STAGE_BYTES), b_dst = a_dst + Cfg::A_BYTES;
+        const int k0 = kt * G_BK;
+        if (!p.a_mn) tma_load_3d(a_dst, &tm_a, bar, k0, m0, g);                 // box 64 k x 128 m
+        else {
+          tma_load_3d(a_dst, &tm_a, bar, m0, k0, g);                            // boxes 64 m x 64 k
+          tma_load_3d(a_dst + 8192, &tm_a, bar, m0 + 64, k0, g);
         }
-        __syncwarp();
+        if (!p.b_mn) tma_load_3d(b_dst, &tm_b, bar, k0, n0, g);                 // box 64 k x BN n
+        else {
+#pragma unroll
+          for (int j = 0; j < BN / 64; ++j) tma_load_3d(b_dst + j * 8192, &tm_b, bar, n0 + 64 * j, k0, g);
+        }
       }
     }
-    if (*failed) {
+    if (lane == 0 && (!ok || *failed)) {
       // copies issued into stages nobody consumed any more: wait for them before the shared memory goes away
       const uint32_t pending = it < (uint32_t)S ? it : (uint32_t)S;
       for (uint32_t j = it - pending; j < it; ++j) mbar_wait(smem_u32(&full[j % S]), (j / S) & 1);
@@ -263,77 +262,90 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm16_tma_kernel(const __grid_c
     const uint64_t d_b = p.b_mn ? umma_desc_mn16(base0 + Cfg::A_BYTES, 8192) : umma_desc(base0 + Cfg::A_BYTES);
     // one k-step of 16: 32 bytes along the swizzled row (k contiguous) or two 8-row groups (m / n contiguous)
     const uint64_t a_step = (uint64_t)((p.a_mn ? 2048 : 32) >> 4), b_step = (uint64_t)((p.b_mn ? 2048 : 32) >> 4);
-    uint32_t it = 0, tl = 0;
-    bool ok = true;
-    for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++tl) {
+    // Between two k-tiles this loop has to be short (the tensor core queues only a few instructions): one wait, asked for
+    // before the MMAs in front of it. A wait that gives up leaves `failed` set; what follows then only runs out its loops.
+    uint32_t tl = 0, ph = 0;
+    int s = 0;
+    bool ready = false;
+    for (long long t = blockIdx.x; t < tiles; t += gridDim.x, ++tl) {
       int mt, nt, g, sp;
       decode(t, mt, nt, g, sp);
       const uint32_t ab = tl & 1;
-      ok = !*failed && mbar_wait(smem_u32(&acc_empty[ab]), ((tl >> 1) & 1) ^ 1);
-      ok = __all_sync(0xFFFFFFFFu, ok);
-      if (!ok) { *failed = 1; break; }
+      if (tl >= 2) role_wait(smem_u32(&acc_empty[ab]), ((tl >> 1) & 1) ^ 1, failed);
+      __syncwarp();
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t d_tmem = tmem + ab * BN;
       const int kt_beg = sp * p.kt_per_split, kt_end = min(ktiles, kt_beg + p.kt_per_split);
-      for (int kt = kt_beg; kt < kt_end; ++kt, ++it) {
-        const int s = it % S;
-        ok = !*failed && mbar_wait(smem_u32(&full[s]), (it / S) & 1);
-        ok = __all_sync(0xFFFFFFFFu, ok);
-        if (!ok) { *failed = 1; break; }
+      for (int kt = kt_beg; kt < kt_end; ++kt) {
+        if (!ready) role_wait(smem_u32(&full[s]), ph, failed);
+        __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const int s1 = s + 1 < S ? s + 1 : 0;
+        const uint32_t ph1 = s + 1 < S ? ph : ph ^ 1u;
+        ready = phase_done(smem_u32(&full[s1]), ph1);
         const uint64_t st = (uint64_t)((s * Cfg::STAGE_BYTES) >> 4);
         if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < G_BK / 16; ++kk)
             umma_f16(d_tmem, d_a + st + kk * a_step, d_b + st + kk * b_step, idesc, (kt > kt_beg || kk > 0) ? 1u : 0u);
           umma_commit(smem_u32(&empty[s]));
+          if (kt + 1 == kt_end) umma_commit(smem_u32(&acc_full[ab]));
         }
         __syncwarp();
+        s = s1, ph = ph1;
       }
-      if (ok && elect_one()) umma_commit(smem_u32(&acc_full[ab]));
+    }
+    if (*failed) {                                   // tensor memory goes back only when no MMA is left
+      if (elect_one()) umma_commit(smem_u32(drained));
       __syncwarp();
+      mbar_wait(smem_u32(drained), 0);
     }
   } else {
     // ------------------------------ accumulator read-back (warps 2-9: lane quadrant warp % 4, two warps per quadrant,
     // each with one half of the tile's columns: with four warps the read-back of a 128 x 256 tile took longer than the
     // 12 k-tiles of a K = 768 product and set that product's time) ------------------------------------------------
     const int quad = warp & 3, half = (warp - 2) >> 2;
+    uint8_t* stage = smem + S * Cfg::STAGE_BYTES + 256 + (warp - 2) * 4096;
+    const bool split = p.split_k > 1;
+    const int kind = split ? 2 : p.c_kind, elt = kind == 2 ? 4 : 2;
+    const int cols = kind == 2 || BN < 128 ? 32 : 64;                // columns staged at a time
     uint32_t tl = 0;
-    bool ok = true;
-    for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++tl) {
+    for (long long t = blockIdx.x; t < tiles; t += gridDim.x, ++tl) {
       int mt, nt, g, sp;
       decode(t, mt, nt, g, sp);
       const uint32_t ab = tl & 1;
-      ok = !*failed && mbar_wait(smem_u32(&acc_full[ab]), (tl >> 1) & 1);
-      ok = __all_sync(0xFFFFFFFFu, ok);
-      if (!ok) { *failed = 1; break; }
+      role_wait(smem_u32(&acc_full[ab]), (tl >> 1) & 1, failed);
+      __syncwarp();
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int m = mt * G_BM + 32 * quad + lane;
-      const int n0 = nt * BN;
-      const bool split = p.split_k > 1;
-      void* out = split ? (void*)partial : C;
-      const long long row = split ? ((long long)sp * p.G + g) * p.M + m : (long long)g * p.M + m;
-      const int kind = split ? 2 : p.c_kind;
-#pragma unroll 1
-      // rows of C that start off 16-byte lines (N not a multiple of 8) go out in narrow stores: there the second warp
-      // of a quadrant only adds pressure, the first one takes every column
-      const bool shared_cols = split || (p.N & 7) == 0;
-      const int c_begin = shared_cols ? half * (BN / 2) : 0, c_end = shared_cols ? (half + 1) * (BN / 2) : (half == 0 ? BN : 0);
-      if (c_begin >= c_end) {
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&acc_empty[ab]));
-      }
-      for (int c0 = c_begin; c0 < c_end; c0 += 32) {
-        uint32_t v[32];
-        tmem_load32(tmem + ((uint32_t)(32 * quad) << 16) + ab * BN + (uint32_t)c0, v);
-        if (c0 + 32 == c_end) {
-          // the accumulator is in registers: hand it back to the MMA warp before storing
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&acc_empty[ab]));
+      const int m0 = mt * G_BM + 32 * quad, n0 = nt * BN;
+      const long long row = (split ? ((long long)sp * p.G + g) * p.M : (long long)g * p.M) + m0;
+      char* out = (split ? (char*)partial : (char*)C) + (row * p.N + n0) * elt;
+      for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += cols) {
+        for (int part = 0; part < cols; part += 32) {
+          uint32_t v[32];
+          tmem_load32(tmem + ((uint32_t)(32 * quad) << 16) + ab * BN + (uint32_t)(c0 + part), v);
+          if (c0 + part + 32 == (half + 1) * (BN / 2)) {
+            // the accumulator is in registers: hand it back to the MMA warp before storing
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&acc_empty[ab]));
+          }
+          uint8_t* mine = stage + lane * 128;
+          if (kind == 2) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+              *reinterpret_cast<uint4*>(mine + ((q ^ (lane & 7)) << 4)) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+          } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              *reinterpret_cast<uint4*>(mine + (((part / 8 + q) ^ (lane & 7)) << 4)) =
+                  make_uint4(pack16(v[8 * q], v[8 * q + 1], kind), pack16(v[8 * q + 2], v[8 * q + 3], kind),
+                             pack16(v[8 * q + 4], v[8 * q + 5], kind), pack16(v[8 * q + 6], v[8 * q + 7], kind));
+          }
         }
-        if (m < p.M) store_row32(out, row, p.N, n0 + c0, v, kind);
+        __syncwarp();
+        store_lines(out + (long long)c0 * elt, (long long)p.N * elt, p.M - m0, min(cols, p.N - n0 - c0) * elt, stage, lane);
+        __syncwarp();
       }
     }
   }

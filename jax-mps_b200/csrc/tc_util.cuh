@@ -28,6 +28,25 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   return false;
 }
 
+// Whether a phase has completed, without waiting.
+__device__ __forceinline__ bool phase_done(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  return done != 0;
+}
+
+// Bounded wait of a role. One that runs out sets `failed`, after which every other wait of the block gives up too.
+__device__ __forceinline__ bool role_wait(uint32_t bar, uint32_t parity, volatile int* failed) {
+  for (int spin = 0; spin < (1 << 22); ++spin) {
+    uint32_t done;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    if (done) return true;
+    if ((spin & 15) == 15 && *failed) return false;
+  }
+  *failed = 1;
+  return false;
+}
+
 // First statement of a kernel that may be launched with programmatic stream serialization: the kernel is scheduled
 // while the one in front of it drains, and waits here until everything in front of it has completed and its memory
 // is visible. Without the launch attribute this is a no-op. (Letting dependents start earlier still, with

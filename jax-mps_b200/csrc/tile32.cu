@@ -87,24 +87,6 @@ __global__ void __launch_bounds__(256) split_b_kernel(const float* __restrict__ 
   *reinterpret_cast<float4*>(tile + bn * 32 + at) = make_float4(low_part(v[0]), low_part(v[1]), low_part(v[2]), low_part(v[3]));
 }
 
-__device__ __forceinline__ bool phase_done(uint32_t bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-  return done != 0;
-}
-
-// Bounded wait of a role. One that runs out sets `failed`, after which every other wait of the block gives up too.
-__device__ __forceinline__ bool role_wait(uint32_t bar, uint32_t parity, volatile int* failed) {
-  for (int spin = 0; spin < (1 << 22); ++spin) {
-    uint32_t done;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-    if (done) return true;
-    if ((spin & 15) == 15 && *failed) return false;
-  }
-  *failed = 1;
-  return false;
-}
-
 template <int BN, bool A_MC>
 __global__ void __launch_bounds__(VTHREADS, 1) tile32_kernel(const __grid_constant__ CUtensorMap tm_a, const float* __restrict__ image, float* __restrict__ C,
                                                             float* __restrict__ partial, const long long* __restrict__ c_row,
