@@ -913,6 +913,61 @@ __global__ void __launch_bounds__(256) gemv16_kc_kernel(const uint16_t* __restri
   }
 }
 
+// One row of A, k contiguous in B, K too long for a warp per column: the eight warps of a block take an eighth of K each and
+// go through the block's columns together. A warp keeps its part of A in registers and has two columns' loads in flight; a
+// block reads one column from end to end, where a warp per column had every warp of the chip at the same offset of its
+// column. Bound by HBM; 2048 columns of 16384 inside a decode loop: 15.0 -> 12.7 us (5.3 TB/s).
+constexpr int KW_UNR = 8, KW_COLS = 32;               // chunks of 256 k per warp, columns per block at most
+template <bool BF16>
+__global__ void __launch_bounds__(256, 2) gemv16_kw_kernel(const uint16_t* __restrict__ A, const uint16_t* __restrict__ B, void* __restrict__ C,
+                                                          GemvParams p) {
+  __shared__ float red[8][KW_COLS];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = blockIdx.y;
+  const uint16_t* Ag = A + (long long)g * p.a_gs;
+  const uint16_t* Bg = B + (long long)g * p.b_gs;
+  const int slice = (p.K + 2047) / 2048 * 256, kbeg = warp * slice + lane * 8, kend = min(p.K, (warp + 1) * slice);
+  uint4 a[KW_UNR], b[KW_UNR], next[KW_UNR];
+  auto load_col = [&](uint4 (&v)[KW_UNR], int n) {
+#pragma unroll
+    for (int u = 0; u < KW_UNR; ++u) {
+      const int k = kbeg + 256 * u;
+      v[u] = n < p.N && k < kend ? __ldcs(reinterpret_cast<const uint4*>(Bg + (long long)n * p.b_ld + k)) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  if (p.b_static) load_col(b, blockIdx.x);            // nothing in flight writes B: asked for before the wait for the kernel in front
+  pdl_prologue();
+  if (!p.b_static) load_col(b, blockIdx.x);
+#pragma unroll
+  for (int u = 0; u < KW_UNR; ++u) {
+    const int k = kbeg + 256 * u;
+    a[u] = k < kend ? *reinterpret_cast<const uint4*>(Ag + k) : make_uint4(0, 0, 0, 0);
+  }
+  int i = 0;
+  for (int n = blockIdx.x; n < p.N; n += gridDim.x, ++i) {
+    load_col(next, n + gridDim.x);
+    float s = 0.f;
+#pragma unroll
+    for (int u = 0; u < KW_UNR; ++u) {
+      s = fmaf(lo16<BF16>(a[u].x), lo16<BF16>(b[u].x), s); s = fmaf(hi16<BF16>(a[u].x), hi16<BF16>(b[u].x), s);
+      s = fmaf(lo16<BF16>(a[u].y), lo16<BF16>(b[u].y), s); s = fmaf(hi16<BF16>(a[u].y), hi16<BF16>(b[u].y), s);
+      s = fmaf(lo16<BF16>(a[u].z), lo16<BF16>(b[u].z), s); s = fmaf(hi16<BF16>(a[u].z), hi16<BF16>(b[u].z), s);
+      s = fmaf(lo16<BF16>(a[u].w), lo16<BF16>(b[u].w), s); s = fmaf(hi16<BF16>(a[u].w), hi16<BF16>(b[u].w), s);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+    if (lane == 0) red[warp][i] = s;
+#pragma unroll
+    for (int u = 0; u < KW_UNR; ++u) b[u] = next[u];
+  }
+  __syncthreads();
+  if (tid < i) {
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) s += red[w][tid];
+    store_c(C, (long long)g * p.N + blockIdx.x + (long long)tid * gridDim.x, s, p.c_kind);
+  }
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -1154,6 +1209,17 @@ cudaError_t launch_gemm16(const Gemm16Launch& g, const void* A, const void* B, v
       }
       const int tasks = (g.N + g.nw - 1) / g.nw;
       dim3 grid((unsigned)std::max(1, std::min((tasks + 7) / 8, sm_count() * 8)), g.G);
+      // a warp per column reads K in steps of 2048; from 8192 the chain of these steps sets the time, up to 16384 a warp's eighth
+      // of A fits registers
+      const int blocks = std::min(g.N, 2 * sm_count());
+      if (g.M == 1 && g.K >= 8192 && g.K <= 2048 * KW_UNR && g.a_ks == 1 && (g.a_gs & 7) == 0 && (((uintptr_t)A) & 15) == 0 &&
+          (g.N + blocks - 1) / blocks <= KW_COLS) {
+        dim3 grid(blocks, g.G);
+        if (bf16) launch_k(gemv16_kw_kernel<true>, grid, 256, 0, stream, (const uint16_t*)A, (const uint16_t*)B, C, p);
+        else launch_k(gemv16_kw_kernel<false>, grid, 256, 0, stream, (const uint16_t*)A, (const uint16_t*)B, C, p);
+        if (launches) (*launches)++;
+        return cudaGetLastError();
+      }
       const size_t smem = (size_t)g.M * g.K * 2;
 #define LAUNCHKC(MM, BF, NW_) launch_k(gemv16_kc_kernel<MM, BF, NW_>, grid, 256, smem, stream, (const uint16_t*)A, (const uint16_t*)B, C, p)
       if (maxm == 1) {
