@@ -3482,17 +3482,20 @@ struct Planner {
   // 64-wide and 800 per 128-wide k-tile, 500 per tile of C, 3000 to launch, fill and drain; a split adds the pass that sums it.
   // A k-tile really takes 830 and 960, but the table-driven kernels take as much longer than choose_split_k says, and the two are
   // compared. At the measured values the 462-row encoder step ran 1540 us, at these 1330; ResNet-18 steps differed by 1 %.
-  // `b_is_weight`: B is a program input, whose split image is made beside what is in front of the product.
-  static double tile_product(Tile32Launch& t, bool b_is_weight) {
-    const long long ktiles = (t.K + 31) / 32, tm = (t.M + 127) / 128;
+  // `b_is_weight`: B is a program input, whose split image is made beside what is in front of the product. The tensor core
+  // truncates its sums, so an error grows with the k-tiles one accumulator takes in (36 of them 8e-6, 12 of them 3e-6): a
+  // product is split at least as finely as the table-driven kernels would (`split_k`), a convolution exactly so, which gives
+  // the same bits.
+  static double tile_product(Tile32Launch& t, bool b_is_weight, int split_k) {
+    const long long ktiles = (t.K + 31) / 32, tm = (t.M + 127) / 128, longest = (ktiles + split_k - 1) / split_k;
     double best = 1e30;
     for (int bn : {128, 64}) {
       if (bn == 128 && t.N <= 64) continue;
       const long long tiles = tm * ((t.N + bn - 1) / bn) * t.G;
       for (long long want = 1; want <= std::min<long long>(ktiles, 160); want++) {
         const long long kps = (ktiles + want - 1) / want, split = (ktiles + kps - 1) / kps;
-        if (split != want) continue;
-        if (split > 1 && (tiles * split > 2 * 148 || split * t.G * t.M * t.N > (64LL << 20))) break;
+        if (split != want || kps > longest || (t.mode == 1 && kps != longest)) continue;
+        if (split > 1 && kps < longest && (tiles * split > 2 * 148 || split * t.G * t.M * t.N > (64LL << 20))) break;
         double cycles = (double)((tiles * split + 147) / 148) * ((double)kps * (bn == 64 ? 450.0 : 800.0) + 500.0) + 3000.0;
         if (split > 1) cycles += 4000.0 + (double)split * t.G * t.M * t.N * 8.0 / 3000.0;
         if (cycles < best * 0.98) { best = cycles; t.bn = bn; t.split = (int)split; }
@@ -3527,12 +3530,14 @@ struct Planner {
     return best;
   }
   // ... and in the table-driven kernels (choose_split_k).
-  static double table_product(const Gemm32Launch& g) {
+  static double table_product(const Gemm32Launch& g, int& split_k) {
     IGemmParams t;
     t.M = g.M; t.N = g.N; t.K = g.K; t.groups = g.G;
     t.vec = g.a_vec && g.b_vec;
     t.seg = t.vec && g.K % 32 == 0 && (g.a_kc || g.M % 32 == 0) && (g.b_kc || g.N % 32 == 0);
-    return choose_split_k(t);
+    const double us = choose_split_k(t);
+    split_k = t.split_k;
+    return us;
   }
 
   std::vector<Step> before_product;          // steps that go in front of the product being lowered
@@ -3805,7 +3810,8 @@ struct Planner {
         // three ways: the FMA pipe, tiled copies, the table-driven kernels
         Tile32Launch t;
         t.M = g.M; t.N = g.N; t.K = g.K; t.G = g.G;
-        const double us_fma = fma_product(g), us_table = table_product(g);
+        int split_k = 1;
+        const double us_fma = fma_product(g), us_table = table_product(g, split_k);
         double us_tile = 1e30;
         if (g.a_vec && g.M * g.G >= 64 && !getenv("B200_NO_TILE32")) {
           t.mode = g.a_kc ? 2 : 3;
@@ -3815,7 +3821,7 @@ struct Planner {
           t.strides[1] = g.G > 1 ? g.a_gs : t.strides[0] * outer;
           t.strides[2] = t.strides[1] * g.G;
           t.box[0] = 32; t.box[1] = g.a_kc ? 128 : 32; t.box[2] = t.box[3] = 1;
-          us_tile = tile_product(t, !rhs->def && rhs->owner && rhs->owner->parent_op == nullptr);
+          us_tile = tile_product(t, !rhs->def && rhs->owner && rhs->owner->parent_op == nullptr, split_k);
         }
         if (us_tile < us_fma && us_tile < us_table) p.tile = t;
         else if (us_fma < us_table) {
@@ -3945,7 +3951,7 @@ struct Planner {
     auto tab = [&](const void* d, size_t n) { return table_slot(d, std::max<size_t>(n, 1)); };
     if (p.tile.mode && op->short_name() != "dot_general") {
       const bool weight = !rhs->def && rhs->owner && rhs->owner->parent_op == nullptr;
-      if (tile_product(p.tile, weight) >= us_table) p.tile.mode = 0;
+      if (tile_product(p.tile, weight, p.split_k) >= us_table) p.tile.mode = 0;
     }
     if (p.tile.mode) {
       p.tile.c_vec = p.c_vec;
