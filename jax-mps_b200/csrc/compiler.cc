@@ -3478,10 +3478,11 @@ struct Planner {
     return best_cost;
   }
 
-  // Tile width and K split of a contraction by tiled copies (tile32.cu), and its modelled time in microseconds. Cycles: 450 per
-  // 64-wide and 800 per 128-wide k-tile, 500 per tile of C, 3000 to launch, fill and drain; a split adds the pass that sums it.
+  // Tile width and K split of a contraction by tiled copies (tile32.cu), and its modelled time in microseconds. Cycles: 300 per
+  // 64-wide and 500 per 128-wide k-tile, 500 per tile of C, 2000 to launch, fill and drain; a split adds the pass that sums it.
   // A k-tile really takes 830 and 960, but the table-driven kernels take as much longer than choose_split_k says, and the two are
-  // compared. At the measured values the 462-row encoder step ran 1540 us, at these 1330; ResNet-18 steps differed by 1 %.
+  // compared; the constants are those at which encoder steps of 150 to 2048 rows and classifier steps ran fastest (462 rows:
+  // 1540 us without tiled copies, 1400 now).
   // `b_is_weight`: B is a program input, whose split image is made beside what is in front of the product. The tensor core
   // truncates its sums, so an error grows with the k-tiles one accumulator takes in (36 of them 8e-6, 12 of them 3e-6): a
   // product is split at least as finely as the table-driven kernels would (`split_k`), a convolution exactly so, which gives
@@ -3496,8 +3497,8 @@ struct Planner {
         const long long kps = (ktiles + want - 1) / want, split = (ktiles + kps - 1) / kps;
         if (split != want || kps > longest || (t.mode == 1 && kps != longest)) continue;
         if (split > 1 && kps < longest && (tiles * split > 2 * 148 || split * t.G * t.M * t.N > (64LL << 20))) break;
-        double cycles = (double)((tiles * split + 147) / 148) * ((double)kps * (bn == 64 ? 450.0 : 800.0) + 500.0) + 3000.0;
-        if (split > 1) cycles += 4000.0 + (double)split * t.G * t.M * t.N * 8.0 / 3000.0;
+        double cycles = (double)((tiles * split + 147) / 148) * ((double)kps * (bn == 64 ? 300.0 : 500.0) + 500.0) + 2000.0;
+        if (split > 1) cycles += 2000.0 + (double)split * t.G * t.M * t.N * 8.0 / 3000.0;
         if (cycles < best * 0.98) { best = cycles; t.bn = bn; t.split = (int)split; }
       }
     }
