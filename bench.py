@@ -337,14 +337,14 @@ def run_b200(args):
     roofline = {"bound": "tensor", "achieved": achieved, "peak": tens, "unit": "TFLOP/s", "frac": achieved / tens,
                 # DRAM bytes of one such launch (input 33.6 MB read once, the 33.6 MB output still in L2 when the kernel
                 # ends); algorithmic bytes are 67.3 MB
-                "traffic": 37.6e6,
-                "traffic_source": "ncu capture of this kernel on this shape, profiles/igemm_tf32x3_ta_kernel_conv3x3_stage1_stage3.md "
+                "traffic": 35.1e6,
+                "traffic_source": "ncu capture of this kernel on this shape, profiles/tile32_kernel_conv3x3_stage1_stage3.md "
                                   "(dram__bytes_read.sum + dram__bytes_write.sum per launch); not re-measured by this run",
                 "own_ceiling": {"tf32_mma_tflops": tf32_rate, "fp32_accurate_tflops": tf32_rate / 3.0 if tf32_rate else None,
                                 "frac": achieved / (tf32_rate / 3.0) if tf32_rate else None,
                                 "how": "tcgen05.mma.kind::tf32 issue loop, one CTA per SM, measured in this run; the kernel "
                                        "issues three such MMAs per fp32 product"},
-                "kernel": "igemm_tf32x3_ta_kernel<64,...> on M=131072 N=64 K=576 (stage-1 3x3 convolutions, forward "
+                "kernel": "tile32_kernel<64> on M=131072 N=64 K=576 (stage-1 3x3 convolutions, forward "
                           "and input gradient), algorithmic fp32 flop 2*M*N*K per launch",
                 "launches_per_step": dom_n // psteps, "us_per_launch": 1e3 * dom_ms / max(dom_n, 1),
                 "peak_source": f"bf16 sustained, {which}; the fp32-accurate path issues three TF32 MMAs per product, "
