@@ -2540,14 +2540,12 @@ struct Planner {
     plan.steps.push_back(std::move(s));
   }
 
-  // b200.decode_attention (DecodeAttentionFusion): attention of M <= 8 query rows per group over T cached positions in
-  // one kernel. A block takes 32 positions of one group: it stages their K and V rows and the queries in shared
-  // memory, its warps form the scores (rounded like the product they replace), the region's pointwise code (scale,
-  // mask) runs on each score, a warp per query row takes the chunk's maximum and exponentials and multiplies them into
-  // its part of the V rows. With more than one chunk, the chunk's unnormalised result, maximum and sum go to scratch,
-  // and the last block of the group to arrive (a counter that it sets back to zero) rescales and adds the chunks in
-  // chunk order and divides by the total. Unlike the chain it replaces, the probabilities are not rounded to 16 bits
-  // on their way into the second product.
+  // b200.decode_attention (DecodeAttentionFusion): attention of M <= 8 query rows per group over T cached positions. A block
+  // takes 32 positions of one group: its warps form the scores (rounded like the product they replace), a warp per query row
+  // runs the region's pointwise code (scale, mask) on its scores and takes the chunk's maximum, exponentials and their sum,
+  // then a thread per column multiplies them into the block's V rows. With more than one chunk, the chunk's unnormalised
+  // result, maximum and sum go to scratch, and a second kernel rescales and adds the chunks in chunk order and divides by the
+  // total. Unlike the chain it replaces, the probabilities are not rounded to 16 bits on their way into the second product.
   void lower_decode_attention(Op* op, Plan& plan, BlockState& st) {
     Value *Q = op->operands[0], *K = op->operands[1], *V = op->operands[2], *out = op->results[0];
     Block* body = op->regions[0].get();
@@ -2590,105 +2588,116 @@ struct Planner {
       }
       return o;
     };
+    // The time is the chain of phases, so each is spread over the block: a warp takes its positions' K rows straight into
+    // registers and keeps its part of the queries there (read from shared memory for every position they cost 2 000 cycles),
+    // eight rows' sums are halved across the lanes instead of reduced one by one, a thread owns a column of the second product.
+    // Everything the block reads is asked for at once. 8 rows over 640 positions of 256, per layer of a decode loop:
+    // 12.9 us with copy loops and the last block adding the parts alone (4.4 us of it), 4.3 us now and 2.0 for the kernel that adds them.
+    const long long KW = TC / 8, VN = (TC * N8 + 255) / 256;
+    const bool one = CH == 1;
     std::ostringstream src;
-    src << "extern \"C\" __global__ void __launch_bounds__(256) @NAME@(" << s_type(out->type.dt) << "* __restrict__ out0, float* __restrict__ part, "
-        << "int* __restrict__ cnt, const u16* __restrict__ qp, const u16* __restrict__ kp, const u16* __restrict__ vp";
+    src << "extern \"C\" __global__ void __launch_bounds__(256) @NAME@(" << (one ? s_type(out->type.dt) : std::string("float")) << "* __restrict__ out0, "
+        << "const u16* __restrict__ qp, const u16* __restrict__ kp, const u16* __restrict__ vp";
     if (!em.inputs.empty()) src << ", " << signature({}, em.inputs);
     src << ") {\n";
-    src << "  __shared__ __align__(16) u16 ks[" << TC * D << "];\n  __shared__ __align__(16) u16 vs[" << TC * N << "];\n";
-    src << "  __shared__ __align__(16) float qs[" << M * D << "];\n  __shared__ float sc[" << M * TC << "];\n  __shared__ int last_flag;\n";
+    src << "  __shared__ __align__(16) u16 vs[" << TC * N << "];\n  __shared__ float sc[" << M * TC << "];\n";
+    src << "  __shared__ __align__(16) float pt[" << TC * 8 << "];\n  __shared__ float sums[8];\n";
     src << "  const int c = blockIdx.x, g = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;\n";
     src << "  const int t0 = c * " << TC << ";\n  const int nt = " << T << " - t0 < " << TC << " ? " << T << " - t0 : " << TC << ";\n";
     src << "  const float NEG_INF = __uint_as_float(0xFF800000u);\n";
-    // Everything the block reads is asked for before anything is used (one round trip where copy loops made a dozen); V stays in
-    // registers past the scores. 8 rows over 640 positions of 256, 20 blocks: 12.9 -> 10.2 us. The time is the chain of phases;
-    // 16 positions a block were slower (11.9 us), the last block then has twice as many parts to add.
-    const long long KN = (TC * D8 + 255) / 256, VN = (TC * N8 + 255) / 256, QN = (M * D8 + 255) / 256;
-    src << "  uint4 kr[" << KN << "], vr[" << VN << "], qr[" << QN << "];\n  {\n    const uint4 none = {0u, 0u, 0u, 0u};\n";
-    src << "    const uint4* ksrc = (const uint4*)(kp + ((long long)g * " << T << " + t0) * " << D << ");\n";
-    src << "    const uint4* vsrc = (const uint4*)(vp + ((long long)g * " << T << " + t0) * " << N << ");\n";
-    src << "    const uint4* qsrc = (const uint4*)(qp + (long long)g * " << M * D << ");\n";
-    auto batch = [&](long long n, const char* reg, const char* from, const std::string& limit) {
-      src << "#pragma unroll\n    for (int j = 0; j < " << n << "; ++j) " << reg << "[j] = tid + 256 * j < " << limit << " ? " << from << "[tid + 256 * j] : none;\n";
-    };
-    batch(KN, "kr", "ksrc", "nt * " + std::to_string(D8));
-    batch(QN, "qr", "qsrc", std::to_string(M * D8));
-    batch(VN, "vr", "vsrc", "nt * " + std::to_string(N8));
-    src << "#pragma unroll\n    for (int j = 0; j < " << KN << "; ++j)\n      if (tid + 256 * j < nt * " << D8 << ") ((uint4*)ks)[tid + 256 * j] = kr[j];\n";
-    src << "#pragma unroll\n    for (int j = 0; j < " << QN << "; ++j)\n      if (tid + 256 * j < " << M * D8 << ") {\n        float qf[8];\n        const uint4 qq = qr[j];\n";
-    src << unpack("qq", "qf");
-    src << "        float4* qd = (float4*)(qs + (tid + 256 * j) * 8);\n        qd[0] = make_float4(qf[0], qf[1], qf[2], qf[3]);\n        qd[1] = make_float4(qf[4], qf[5], qf[6], qf[7]);\n      }\n  }\n";
-    src << "  __syncthreads();\n";
+    src << "  const uint4 none = {0u, 0u, 0u, 0u};\n  uint4 kr[" << KW << "], vr[" << VN << "], qr[" << M << "];\n";
+    src << "  const uint4* ksrc = (const uint4*)(kp + ((long long)g * " << T << " + t0) * " << D << ");\n";
+    src << "  const uint4* vsrc = (const uint4*)(vp + ((long long)g * " << T << " + t0) * " << N << ");\n";
+    src << "  const uint4* qsrc = (const uint4*)(qp + (long long)g * " << M * D << ");\n";
+    src << "#pragma unroll\n  for (int j = 0; j < " << KW << "; ++j) kr[j] = warp + 8 * j < nt && lane < " << D8 << " ? ksrc[(warp + 8 * j) * " << D8 << " + lane] : none;\n";
+    src << "#pragma unroll\n  for (int m = 0; m < " << M << "; ++m) qr[m] = lane < " << D8 << " ? qsrc[m * " << D8 << " + lane] : none;\n";
+    src << "#pragma unroll\n  for (int j = 0; j < " << VN << "; ++j) vr[j] = tid + 256 * j < nt * " << N8 << " ? vsrc[tid + 256 * j] : none;\n";
     // scores
-    src << "  for (int tl = warp; tl < nt; tl += 8) {\n    float acc[" << M << "];\n";
-    src << "#pragma unroll\n    for (int m = 0; m < " << M << "; ++m) acc[m] = 0.f;\n";
-    src << "    for (int p = lane; p < " << D8 << "; p += 32) {\n      const uint4 kk = ((const uint4*)ks)[tl * " << D8 << " + p];\n      float kf[8];\n";
-    src << unpack("kk", "kf");
-    src << "#pragma unroll\n      for (int m = 0; m < " << M << "; ++m) {\n        const float4 qa = *(const float4*)(qs + m * " << D << " + p * 8), qb = *(const float4*)(qs + m * " << D << " + p * 8 + 4);\n";
-    src << "        acc[m] = fmaf(kf[0], qa.x, acc[m]); acc[m] = fmaf(kf[1], qa.y, acc[m]); acc[m] = fmaf(kf[2], qa.z, acc[m]); acc[m] = fmaf(kf[3], qa.w, acc[m]);\n";
-    src << "        acc[m] = fmaf(kf[4], qb.x, acc[m]); acc[m] = fmaf(kf[5], qb.y, acc[m]); acc[m] = fmaf(kf[6], qb.z, acc[m]); acc[m] = fmaf(kf[7], qb.w, acc[m]);\n      }\n    }\n";
-    src << "    float mine = 0.f;\n#pragma unroll\n    for (int m = 0; m < " << M << "; ++m) {\n      float r = acc[m];\n";
-    src << "#pragma unroll\n      for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xFFFFFFFFu, r, o);\n      if (lane == m) mine = r;\n    }\n";
-    src << "    if (lane < " << M << ") sc[lane * " << TC << " + tl] = mine;\n  }\n";
+    src << "#pragma unroll\n  for (int j = 0; j < " << KW << "; ++j) {\n    const int tl = warp + 8 * j;\n    if (tl < nt) {\n";
+    src << "      float kf[8], acc[" << M << "];\n      const uint4 kk = kr[j];\n" << unpack("kk", "kf");
+    src << "#pragma unroll\n      for (int m = 0; m < " << M << "; ++m) {\n        float qf[8];\n        const uint4 qq = qr[m];\n" << unpack("qq", "qf");
+    src << "        acc[m] = 0.f;\n#pragma unroll\n        for (int e = 0; e < 8; ++e) acc[m] = fmaf(kf[e], qf[e], acc[m]);\n      }\n";
+    if (M == 8) {
+      src << "      float r4[4], r2[2];\n      const bool h16 = (lane & 16) != 0, h8 = (lane & 8) != 0, h4 = (lane & 4) != 0;\n";
+      src << "#pragma unroll\n      for (int i = 0; i < 4; ++i) { const float send = h16 ? acc[i] : acc[i + 4], keep = h16 ? acc[i + 4] : acc[i]; r4[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, 16); }\n";
+      src << "#pragma unroll\n      for (int i = 0; i < 2; ++i) { const float send = h8 ? r4[i] : r4[i + 2], keep = h8 ? r4[i + 2] : r4[i]; r2[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, 8); }\n";
+      src << "      float r = (h4 ? r2[1] : r2[0]) + __shfl_xor_sync(0xFFFFFFFFu, h4 ? r2[0] : r2[1], 4);\n";
+      src << "      r += __shfl_xor_sync(0xFFFFFFFFu, r, 2);\n      r += __shfl_xor_sync(0xFFFFFFFFu, r, 1);\n";
+      src << "      if ((lane & 3) == 0) sc[(lane >> 2) * " << TC << " + tl] = r;\n";
+    } else {
+      src << "      float mine = 0.f;\n#pragma unroll\n      for (int m = 0; m < " << M << "; ++m) {\n        float r = acc[m];\n";
+      src << "#pragma unroll\n        for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xFFFFFFFFu, r, o);\n        if (lane == m) mine = r;\n      }\n";
+      src << "      if (lane < " << M << ") sc[lane * " << TC << " + tl] = mine;\n";
+    }
+    src << "    }\n  }\n";
     src << "#pragma unroll\n  for (int j = 0; j < " << VN << "; ++j)\n    if (tid + 256 * j < nt * " << N8 << ") ((uint4*)vs)[tid + 256 * j] = vr[j];\n  __syncthreads();\n";
-    // the pointwise part on every score of the chunk at once (its loads, a mask for instance, go out together)
-    src << "  for (int i = tid; i < " << M * TC << "; i += 256) {\n    const int mrow = i / " << TC << ", tl = i % " << TC << ";\n    if (tl < nt) {\n";
-    src << "      const float mine = sc[i];\n      const float sval = " << round_s << ";\n";
+    // a warp per query row: the pointwise part on each score, the chunk's maximum, exponentials and their sum
+    src << "  if (warp < " << M << ") {\n    const int mrow = warp, tl = lane;\n    float x = NEG_INF;\n    if (tl < nt) {\n";
+    src << "      const float mine = sc[mrow * " << TC << " + tl];\n      const float sval = " << round_s << ";\n";
     src << "      const " << I << " lin = ((" << I << ")g * " << M << " + mrow) * " << T << " + t0 + tl;\n";
     src << em.str();
-    src << "      sc[i] = " << rexpr << ";\n    }\n  }\n  __syncthreads();\n";
-    // softmax of the chunk and the second product, a warp per query row
-    src << "  if (warp < " << M << ") {\n    const int mrow = warp;\n    float mx = NEG_INF;\n";
-    src << "    for (int tl = lane; tl < nt; tl += 32) mx = fmaxf(mx, sc[mrow * " << TC << " + tl]);\n";
+    src << "      x = " << rexpr << ";\n    }\n    float mx = x;\n";
     src << "#pragma unroll\n    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));\n";
     src << "    const float mref = mx == NEG_INF ? 0.f : mx;\n    float sum = 0.f;\n";
-    src << "    for (int tl = lane; tl < nt; tl += 32) { const float pz = expf(sc[mrow * " << TC << " + tl] - mref); sc[mrow * " << TC << " + tl] = pz; sum += pz; }\n";
-    src << "#pragma unroll\n    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);\n    __syncwarp();\n";
-    src << "    for (int p = lane; p < " << N8 << "; p += 32) {\n      float o8[8];\n#pragma unroll\n      for (int e = 0; e < 8; ++e) o8[e] = 0.f;\n";
-    src << "      for (int tl = 0; tl < nt; ++tl) {\n        const float pz = sc[mrow * " << TC << " + tl];\n        const uint4 vv = ((const uint4*)vs)[tl * " << N8 << " + p];\n        float vf[8];\n";
-    src << unpack("vv", "vf");
-    src << "#pragma unroll\n        for (int e = 0; e < 8; ++e) o8[e] = fmaf(pz, vf[e], o8[e]);\n      }\n";
-    if (CH == 1) {
-      src << "#pragma unroll\n      for (int e = 0; e < 8; ++e) out0[((long long)g * " << M << " + mrow) * " << N << " + p * 8 + e] = " << store_expr(out->type.dt, "(o8[e] / sum)") << ";\n";
-      src << "    }\n  }\n}\n";
-    } else {
-      src << "      float* dst = part + (((long long)g * " << CH << " + c) * " << M << " + mrow) * " << PS << " + p * 8;\n";
-      src << "      *(float4*)dst = make_float4(o8[0], o8[1], o8[2], o8[3]);\n      *(float4*)(dst + 4) = make_float4(o8[4], o8[5], o8[6], o8[7]);\n    }\n";
-      src << "    if (lane == 0) {\n      float* dst = part + (((long long)g * " << CH << " + c) * " << M << " + mrow) * " << PS << " + " << N << ";\n      dst[0] = mx;\n      dst[1] = sum;\n    }\n  }\n";
-      src << "  __threadfence();\n  __syncthreads();\n";
-      src << "  if (tid == 0) last_flag = atomicAdd(cnt + g, 1) == " << (CH - 1) << ";\n  __syncthreads();\n  if (!last_flag) return;\n  __threadfence();\n";
-      src << "  if (warp < " << M << ") {\n    const int mrow = warp;\n    const float* base = part + ((long long)g * " << CH * M << " + mrow) * " << PS << ";\n";
-      // lanes take the chunks' maxima and sums side by side: the row's maximum, then every chunk's weight and the total
-      src << "    float gm = NEG_INF;\n    for (int cc = lane; cc < " << CH << "; cc += 32) gm = fmaxf(gm, __ldcg(base + (long long)cc * " << M * PS << " + " << N << "));\n";
-      src << "#pragma unroll\n    for (int o = 16; o > 0; o >>= 1) gm = fmaxf(gm, __shfl_xor_sync(0xFFFFFFFFu, gm, o));\n";
-      src << "    float den = 0.f, wl = 0.f;\n    for (int cc = lane; cc < " << CH << "; cc += 32) {\n      const float mc = __ldcg(base + (long long)cc * " << M * PS << " + " << N << ");\n";
-      src << "      wl = mc == NEG_INF ? 0.f : expf(mc - gm);\n      den += wl * __ldcg(base + (long long)cc * " << M * PS << " + " << (N + 1) << ");\n    }\n";
-      src << "#pragma unroll\n    for (int o = 16; o > 0; o >>= 1) den += __shfl_xor_sync(0xFFFFFFFFu, den, o);\n";
-      src << "    for (int p = lane; p < " << ((N8 + 31) / 32 * 32) << "; p += 32) {\n      const bool mine = p < " << N8 << ";\n      float o8[8];\n#pragma unroll\n      for (int e = 0; e < 8; ++e) o8[e] = 0.f;\n";
-      src << "#pragma unroll " << std::min<long long>(CH, 10) << "\n      for (int cc = 0; cc < " << CH << "; ++cc) {\n        const float* row = base + (long long)cc * " << M * PS << ";\n";
-      if (CH <= 32) src << "        const float w = __shfl_sync(0xFFFFFFFFu, wl, cc);\n";
-      else src << "        const float mc = __ldcg(row + " << N << ");\n        const float w = mc == NEG_INF ? 0.f : expf(mc - gm);\n";
-      src << "        if (!mine) continue;\n";
-      src << "        const float4 a = __ldcg((const float4*)(row + p * 8)), b4 = __ldcg((const float4*)(row + p * 8 + 4));\n";
-      src << "        o8[0] = fmaf(w, a.x, o8[0]); o8[1] = fmaf(w, a.y, o8[1]); o8[2] = fmaf(w, a.z, o8[2]); o8[3] = fmaf(w, a.w, o8[3]);\n";
-      src << "        o8[4] = fmaf(w, b4.x, o8[4]); o8[5] = fmaf(w, b4.y, o8[5]); o8[6] = fmaf(w, b4.z, o8[6]); o8[7] = fmaf(w, b4.w, o8[7]);\n      }\n";
-      src << "      if (!mine) continue;\n";
-      src << "#pragma unroll\n      for (int e = 0; e < 8; ++e) out0[((long long)g * " << M << " + mrow) * " << N << " + p * 8 + e] = " << store_expr(out->type.dt, "(o8[e] / den)") << ";\n";
-      src << "    }\n  }\n  if (tid == 0) cnt[g] = 0;\n}\n";
-    }
+    src << "    if (tl < nt) { const float pz = expf(x - mref); pt[tl * 8 + mrow] = pz; sum = pz; }\n";
+    src << "#pragma unroll\n    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);\n";
+    if (one) src << "    if (lane == 0) sums[mrow] = sum;\n";
+    else src << "    if (lane == 0) {\n      float* dst = out0 + (((long long)g * " << CH << " + c) * " << M << " + mrow) * " << PS << " + " << N << ";\n      dst[0] = mx;\n      dst[1] = sum;\n    }\n";
+    src << "  }\n  __syncthreads();\n";
+    // second product, a thread per column
+    src << "  if (tid < " << N << ") {\n    float o[" << M << "];\n#pragma unroll\n    for (int m = 0; m < " << M << "; ++m) o[m] = 0.f;\n";
+    src << "#pragma unroll 8\n    for (int tl = 0; tl < nt; ++tl) {\n      const float v = " << H2F << "(vs[tl * " << N << " + tid]);\n";
+    src << "#pragma unroll\n      for (int m = 0; m < " << M << "; ++m) o[m] = fmaf(pt[tl * 8 + m], v, o[m]);\n    }\n";
+    src << "#pragma unroll\n    for (int m = 0; m < " << M << "; ++m) ";
+    if (one) src << "out0[((long long)g * " << M << " + m) * " << N << " + tid] = " << store_expr(out->type.dt, "(o[m] / sums[m])") << ";\n";
+    else src << "out0[(((long long)g * " << CH << " + c) * " << M << " + m) * " << PS << " + tid] = o[m];\n";
+    src << "  }\n}\n";
+    const std::string label = op->has("label") ? attr_str(op->attr("label")) : op->name;
     Step s;
     s.kind = Step::KERNEL;
     s.kernel = add_kernel(src.str(), "attention");
-    s.label = op->has("label") ? attr_str(op->attr("label")) : op->name;
+    s.label = label;
     s.grid[0] = (unsigned)CH; s.grid[1] = (unsigned)G; s.grid[2] = 1;
     s.block[0] = 256; s.block[1] = s.block[2] = 1;
-    TensorType pt;
-    pt.dt = DT::F32;
-    pt.dims = {std::max<long long>(1, CH > 1 ? G * CH * M * PS : 1)};
-    std::vector<int> zeros((size_t)G, 0);
-    s.args = {slot_of.at(out), new_slot(Slot::TEMP, pt, st.arena), table_slot(zeros.data(), zeros.size() * sizeof(int)), slot_of.at(Q), slot_of.at(K), slot_of.at(V)};
+    int parts = slot_of.at(out);
+    if (!one) {
+      TensorType pt;
+      pt.dt = DT::F32;
+      pt.dims = {G * CH * M * PS};
+      parts = new_slot(Slot::TEMP, pt, st.arena);
+    }
+    s.args = {parts, slot_of.at(Q), slot_of.at(K), slot_of.at(V)};
     for (Value* v : em.inputs) s.args.push_back(slot_of.at(v));
-    s.n_outs = 3;
+    s.n_outs = 1;
+    if (one) { plan.steps.push_back(std::move(s)); return; }
+    plan.steps.push_back(std::move(s));
+    // The chunks' parts added in chunk order, a block per query row and group, a thread per column. A kernel of its own: read by
+    // the one block that arrives last, 160 KB of parts took longer than the launch does.
+    std::ostringstream cs;
+    cs << "extern \"C\" __global__ void __launch_bounds__(256) @NAME@(" << s_type(out->type.dt) << "* __restrict__ out0, const float* __restrict__ part) {\n";
+    cs << "  const int mrow = blockIdx.x, g = blockIdx.y, tid = threadIdx.x, lane = tid & 31;\n  const float NEG_INF = __uint_as_float(0xFF800000u);\n";
+    cs << "  const float* base = part + ((long long)g * " << CH * M << " + mrow) * " << PS << ";\n  const int col = tid < " << N << " ? tid : 0;\n";
+    const long long U = std::min<long long>(CH, 32);
+    cs << "  float pv[" << U << "];\n#pragma unroll\n  for (int cc = 0; cc < " << U << "; ++cc) pv[cc] = base[(long long)cc * " << M * PS << " + col];\n";
+    cs << "  float gm = NEG_INF;\n  for (int cc = lane; cc < " << CH << "; cc += 32) gm = fmaxf(gm, base[(long long)cc * " << M * PS << " + " << N << "]);\n";
+    cs << "#pragma unroll\n  for (int o = 16; o > 0; o >>= 1) gm = fmaxf(gm, __shfl_xor_sync(0xFFFFFFFFu, gm, o));\n";
+    cs << "  float den = 0.f, wl = 0.f;\n  for (int cc = lane; cc < " << CH << "; cc += 32) {\n    const float mc = base[(long long)cc * " << M * PS << " + " << N << "];\n";
+    cs << "    const float w = mc == NEG_INF ? 0.f : expf(mc - gm);\n    if (cc < 32) wl = w;\n    den += w * base[(long long)cc * " << M * PS << " + " << (N + 1) << "];\n  }\n";
+    cs << "#pragma unroll\n  for (int o = 16; o > 0; o >>= 1) den += __shfl_xor_sync(0xFFFFFFFFu, den, o);\n";
+    cs << "  float o1 = 0.f;\n#pragma unroll\n  for (int cc = 0; cc < " << U << "; ++cc) o1 = fmaf(__shfl_sync(0xFFFFFFFFu, wl, cc), pv[cc], o1);\n";
+    if (CH > 32) {
+      cs << "  for (int cc = 32; cc < " << CH << "; ++cc) {\n    const float mc = base[(long long)cc * " << M * PS << " + " << N << "];\n";
+      cs << "    const float w = mc == NEG_INF ? 0.f : expf(mc - gm);\n    o1 = fmaf(w, base[(long long)cc * " << M * PS << " + col], o1);\n  }\n";
+    }
+    cs << "  if (tid < " << N << ") out0[((long long)g * " << M << " + mrow) * " << N << " + tid] = " << store_expr(out->type.dt, "(o1 / den)") << ";\n}\n";
+    s = Step();
+    s.kind = Step::KERNEL;
+    s.kernel = add_kernel(cs.str(), "combine");
+    s.label = label + " sum";
+    s.grid[0] = (unsigned)M; s.grid[1] = (unsigned)G; s.grid[2] = 1;
+    s.block[0] = 256; s.block[1] = s.block[2] = 1;
+    s.args = {slot_of.at(out), parts};
+    s.n_outs = 1;
     plan.steps.push_back(std::move(s));
   }
 
