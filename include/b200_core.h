@@ -193,6 +193,10 @@ b200_error* b200_executable_arg_info(const b200_executable* exe, size_t index, b
 int64_t b200_executable_launches_per_execute(const b200_executable* exe);
 int64_t b200_executable_num_kernels(const b200_executable* exe);
 int64_t b200_executable_temp_bytes(const b200_executable* exe);
+/* CUDA graphs recorded for the plan and its counted loops so far (once each, whatever buffers the calls were given), and how
+ * often one of them was given the addresses of other arguments or results. */
+int64_t b200_executable_recordings(const b200_executable* exe);
+int64_t b200_executable_relocations(const b200_executable* exe);
 /* Text of the kernel plan (what B200_DUMP_PLAN prints); owned by the executable. */
 const char* b200_executable_plan_text(const b200_executable* exe);
 

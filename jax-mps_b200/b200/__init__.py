@@ -102,6 +102,8 @@ SIGNATURES = {
     "b200_executable_output_info": (_P, [_P, C.c_size_t, C.POINTER(C.c_int), C.POINTER(C.POINTER(C.c_int64)), C.POINTER(C.c_size_t)]),
     "b200_executable_arg_info": (_P, [_P, C.c_size_t, C.POINTER(C.c_int), C.POINTER(C.POINTER(C.c_int64)), C.POINTER(C.c_size_t)]),
     "b200_executable_launches_per_execute": (C.c_int64, [_P]),
+    "b200_executable_recordings": (C.c_int64, [_P]),
+    "b200_executable_relocations": (C.c_int64, [_P]),
     "b200_executable_num_kernels": (C.c_int64, [_P]),
     "b200_executable_temp_bytes": (C.c_int64, [_P]),
     "b200_executable_plan_text": (C.c_char_p, [_P]),
@@ -449,6 +451,16 @@ class Executable:
     @property
     def launches_per_execute(self) -> int:
         return load_library().b200_executable_launches_per_execute(self._h)
+
+    @property
+    def recordings(self) -> int:
+        """CUDA graphs recorded for the plan and its counted loops so far."""
+        return load_library().b200_executable_recordings(self._h)
+
+    @property
+    def relocations(self) -> int:
+        """How often a recording was given the addresses of other arguments or results."""
+        return load_library().b200_executable_relocations(self._h)
 
     @property
     def num_kernels(self) -> int:

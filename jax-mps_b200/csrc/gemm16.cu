@@ -22,6 +22,7 @@
 #include <mutex>
 
 #include "kernels.h"
+#include "launch.h"
 #include "tc_util.cuh"
 
 namespace b200 {
@@ -45,7 +46,7 @@ cudaError_t launch_k(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, c
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = g_programmatic_launch ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+  return launch_kernel(cfg, kernel, std::forward<A>(args)...);
 }
 
 

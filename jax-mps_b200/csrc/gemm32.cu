@@ -18,6 +18,7 @@
 #include <cstdint>
 
 #include "kernels.h"
+#include "launch.h"
 #include "tc_util.cuh"
 
 namespace b200 {
@@ -249,7 +250,7 @@ cudaError_t launch(const Gemm32Launch& p, const float* A, const float* B, float*
   }
   cfg.attrs = attr;
   cfg.numAttrs = (unsigned)n;
-  return cudaLaunchKernelEx(&cfg, kernel, A, B, C, p);
+  return launch_kernel(cfg, kernel, A, B, C, p);
 }
 
 template <class Cfg, bool AKC, bool BKC>

@@ -23,6 +23,7 @@
 #include <cstring>
 
 #include "kernels.h"
+#include "launch.h"
 #include "tc_util.cuh"
 
 namespace b200 {
@@ -43,7 +44,7 @@ cudaError_t launch_k(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, c
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = g_igemm_programmatic_launch ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+  return launch_kernel(cfg, kernel, std::forward<A>(args)...);
 }
 
 
@@ -1948,9 +1949,9 @@ cudaError_t launch_scatter_rows(int elem_kind, int index_bytes, int kind, long l
   const unsigned rb = (unsigned)((updates + 255) / 256);
   if (updates <= kScatterAllPairsMax) {
     if (index_bytes == 8)
-      scatter_rank_kernel<long long><<<rb, 256, 0, stream>>>((const long long*)indices, updates, rows, key, order);
+      launch_plain(scatter_rank_kernel<long long>, rb, 256, 0, stream, (const long long*)indices, updates, rows, key, order);
     else
-      scatter_rank_kernel<int><<<rb, 256, 0, stream>>>((const int*)indices, updates, rows, key, order);
+      launch_plain(scatter_rank_kernel<int>, rb, 256, 0, stream, (const int*)indices, updates, rows, key, order);
     *launches += 1;
   } else {
     int* key_b = scratch + 2 * (long long)updates;
@@ -1958,14 +1959,14 @@ cudaError_t launch_scatter_rows(int elem_kind, int index_bytes, int kind, long l
     int* hist = scratch + 4 * (long long)updates;
     const int nblocks = (updates + 1023) / 1024;
     if (index_bytes == 8)
-      scatter_keys_kernel<long long><<<rb, 256, 0, stream>>>((const long long*)indices, updates, rows, key, order);
+      launch_plain(scatter_keys_kernel<long long>, rb, 256, 0, stream, (const long long*)indices, updates, rows, key, order);
     else
-      scatter_keys_kernel<int><<<rb, 256, 0, stream>>>((const int*)indices, updates, rows, key, order);
+      launch_plain(scatter_keys_kernel<int>, rb, 256, 0, stream, (const int*)indices, updates, rows, key, order);
     const int passes = scatter_radix_passes(rows);
     for (int pass = 0; pass < passes; ++pass) {
-      radix_hist_kernel<<<nblocks, 1024, 0, stream>>>(key, updates, 8 * pass, hist, nblocks);
-      radix_scan_kernel<<<1, 1024, 0, stream>>>(hist, 256 * nblocks);
-      radix_scatter_kernel<<<nblocks, 1024, 0, stream>>>(key, order, key_b, order_b, updates, 8 * pass, hist, nblocks);
+      launch_plain(radix_hist_kernel, nblocks, 1024, 0, stream, key, updates, 8 * pass, hist, nblocks);
+      launch_plain(radix_scan_kernel, 1, 1024, 0, stream, hist, 256 * nblocks);
+      launch_plain(radix_scatter_kernel, nblocks, 1024, 0, stream, key, order, key_b, order_b, updates, 8 * pass, hist, nblocks);
       std::swap(key, key_b);
       std::swap(order, order_b);
     }
@@ -1975,12 +1976,12 @@ cudaError_t launch_scatter_rows(int elem_kind, int index_bytes, int kind, long l
   if (e != cudaSuccess) return e;
   dim3 grid((unsigned)updates, (unsigned)std::min<long long>(64, (row_elems + 255) / 256));
   if (elem_kind == 0)
-    scatter_apply_kernel<float, float><<<grid, 256, 0, stream>>>((float*)out, (const float*)upd, key, order, updates, rows, row_elems, kind);
+    launch_plain(scatter_apply_kernel<float, float>, grid, 256, 0, stream, (float*)out, (const float*)upd, key, order, updates, rows, row_elems, kind);
   else if (elem_kind == 1)
-    scatter_apply_kernel<unsigned short, float><<<grid, 256, 0, stream>>>((unsigned short*)out, (const unsigned short*)upd, key, order,
-                                                                          updates, rows, row_elems, kind);
+    launch_plain(scatter_apply_kernel<unsigned short, float>, grid, 256, 0, stream, (unsigned short*)out, (const unsigned short*)upd, key, order,
+                 updates, rows, row_elems, kind);
   else
-    scatter_apply_kernel<int, int><<<grid, 256, 0, stream>>>((int*)out, (const int*)upd, key, order, updates, rows, row_elems, kind);
+    launch_plain(scatter_apply_kernel<int, int>, grid, 256, 0, stream, (int*)out, (const int*)upd, key, order, updates, rows, row_elems, kind);
   *launches += 1;
   return cudaGetLastError();
 }
@@ -1993,9 +1994,9 @@ cudaError_t launch_scatter_elems(int elem_kind, int kind, long long numel, int u
   const int nblocks = (updates + 1023) / 1024;
   const int passes = scatter_radix_passes(numel);
   for (int pass = 0; pass < passes; ++pass) {
-    radix_hist_kernel<<<nblocks, 1024, 0, stream>>>(key, updates, 8 * pass, hist, nblocks);
-    radix_scan_kernel<<<1, 1024, 0, stream>>>(hist, 256 * nblocks);
-    radix_scatter_kernel<<<nblocks, 1024, 0, stream>>>(key, order, key_b, order_b, updates, 8 * pass, hist, nblocks);
+    launch_plain(radix_hist_kernel, nblocks, 1024, 0, stream, key, updates, 8 * pass, hist, nblocks);
+    launch_plain(radix_scan_kernel, 1, 1024, 0, stream, hist, 256 * nblocks);
+    launch_plain(radix_scatter_kernel, nblocks, 1024, 0, stream, key, order, key_b, order_b, updates, 8 * pass, hist, nblocks);
     std::swap(key, key_b);
     std::swap(order, order_b);
   }
@@ -2007,12 +2008,12 @@ cudaError_t launch_scatter_elems(int elem_kind, int kind, long long numel, int u
   }
   const unsigned grid = (unsigned)((updates + 255) / 256);
   if (elem_kind == 0)
-    scatter_apply_elems_kernel<float, float><<<grid, 256, 0, stream>>>((float*)out, (const float*)upd, key, order, updates, numel, kind);
+    launch_plain(scatter_apply_elems_kernel<float, float>, grid, 256, 0, stream, (float*)out, (const float*)upd, key, order, updates, numel, kind);
   else if (elem_kind == 1)
-    scatter_apply_elems_kernel<unsigned short, float><<<grid, 256, 0, stream>>>((unsigned short*)out, (const unsigned short*)upd, key, order,
-                                                                                updates, numel, kind);
+    launch_plain(scatter_apply_elems_kernel<unsigned short, float>, grid, 256, 0, stream, (unsigned short*)out, (const unsigned short*)upd, key, order,
+                 updates, numel, kind);
   else
-    scatter_apply_elems_kernel<int, int><<<grid, 256, 0, stream>>>((int*)out, (const int*)upd, key, order, updates, numel, kind);
+    launch_plain(scatter_apply_elems_kernel<int, int>, grid, 256, 0, stream, (int*)out, (const int*)upd, key, order, updates, numel, kind);
   *launches += 3 * passes + 1;
   return cudaGetLastError();
 }

@@ -31,6 +31,7 @@
 
 #include "../../include/b200_core.h"
 #include "kernels.h"
+#include "launch.h"
 #include "plan.h"
 
 using namespace b200;
@@ -77,6 +78,7 @@ struct DriverApi {
   CUresult (*LaunchKernel)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, CUstream,
                            void**, void**) = nullptr;
   CUresult (*LaunchKernelEx)(const CUlaunchConfig*, CUfunction, void**, void**) = nullptr;   // optional
+  CUresult (*GraphExecKernelNodeSetParams)(CUgraphExec, CUgraphNode, const CUDA_KERNEL_NODE_PARAMS*) = nullptr;   // optional
   CUresult (*GetErrorString)(CUresult, const char**) = nullptr;
   std::string error;
   bool ok = false;
@@ -101,6 +103,7 @@ DriverApi& driver() {
     if (api.ok) {
       const std::string keep = api.error;
       if (!get("cuLaunchKernelEx", (void**)&api.LaunchKernelEx)) { api.LaunchKernelEx = nullptr; api.error = keep; }
+      if (!get("cuGraphExecKernelNodeSetParams", (void**)&api.GraphExecKernelNodeSetParams)) { api.GraphExecKernelNodeSetParams = nullptr; api.error = keep; }
     }
   });
   return api;
@@ -311,6 +314,33 @@ struct PinnedBlock {
   std::shared_ptr<ReadyEvent> reader;   // the copy that reads it
 };
 
+// Steps of a plan as a CUDA graph. The nodes of steps that use arguments or results hold their addresses, which are others
+// from call to call; before a launch those nodes, and no others, are given the addresses of the call (Relocator). One
+// recording serves every call: nothing depends on which buffers a program is given, or on where the pool puts results.
+struct Recording {
+  cudaGraph_t graph = nullptr;                 // kept: the nodes below are its handles
+  cudaGraphExec_t exec = nullptr;
+  int launches = 0;
+  long long iterations = 0;                    // of a counted loop
+  bool off = false;                            // cannot be recorded: step by step for good
+  struct Node { cudaGraphNode_t node; const void* func; dim3 grid, block; size_t bytes; };      // func null: a copy; bytes: shared memory, or copied
+  struct Issue { std::vector<void*> at; std::vector<Node> nodes; };
+  std::vector<int> order;                      // steps and copies as recorded: index into issues, or -1 for temporaries alone
+  std::vector<Issue> issues;
+  std::vector<void*> outer;                    // arguments and results that the nodes have the addresses of
+  void clear() {
+    if (exec) cudaGraphExecDestroy(exec);
+    if (graph) cudaGraphDestroy(graph);
+    exec = nullptr;
+    graph = nullptr;
+    order.clear();
+    issues.clear();
+  }
+  Recording() = default;
+  Recording(const Recording&) = delete;
+  ~Recording() { clear(); }
+};
+
 struct LoadedProgram {
   std::unique_ptr<CompiledProgram> prog;
   std::string text;                            // the module this plan was compiled from
@@ -321,34 +351,18 @@ struct LoadedProgram {
   std::vector<void*> const_ptrs;
   std::vector<void*> arenas;
   void* const_block = nullptr;
-  // Instantiated CUDA graphs of counted-loop bodies (an even number of iterations each), per loop step and per set of slot
-  // addresses the graph was captured with.
-  struct LoopGraph { const void* step; std::vector<void*> ptrs; cudaGraphExec_t exec; int launches; long long iterations; };
-  std::vector<LoopGraph> loop_graphs;
+  // The main plan, and iterations of counted loops (an even number each), as CUDA graphs.
+  Recording main_graph;
+  std::map<const void*, Recording> loop_graphs;
   // Graphs of data-dependent loops and cases (conditional nodes), per step and per set of addresses of the slots the
   // step and everything below it touches.
-  std::vector<LoopGraph> cond_graphs;
-  // Graphs of the whole plan, per set of argument and result addresses that came back (replay_plan).
-  struct PlanGraph { std::vector<void*> ptrs; cudaGraphExec_t exec; int launches; uint64_t used; };
-  // Sets of addresses met once, newest last: recording costs some 15 us a node, so it is for what comes back.
-  std::deque<std::pair<const void*, std::vector<void*>>> met;
-  bool met_before(const void* step, const std::vector<void*>& ptrs) {
-    for (auto it = met.begin(); it != met.end(); ++it)
-      if (it->first == step && it->second == ptrs) { met.erase(it); return true; }
-    met.emplace_back(step, ptrs);
-    if (met.size() > 48) met.pop_front();
-    return false;
-  }
-  std::vector<PlanGraph> plan_graphs;
-  bool replayable = false;                     // the plan only launches kernels and device copies, and enough of them
-  uint64_t calls = 0, replays = 0, recordings = 0;
+  struct CondGraph { const void* step; std::vector<void*> ptrs; cudaGraphExec_t exec; int launches; };
+  std::vector<CondGraph> cond_graphs;
+  bool replayable = false;                     // the main plan only launches kernels and device copies, and enough of them
+  int64_t recordings = 0, relocations = 0;     // graphs recorded; calls whose graph was given other memory
   bool watched = false;                        // some kernel of the plan has a bounded wait that can run out
   ~LoadedProgram() {
-    for (auto& g : loop_graphs)
-      if (g.exec) cudaGraphExecDestroy(g.exec);
     for (auto& g : cond_graphs)
-      if (g.exec) cudaGraphExecDestroy(g.exec);
-    for (auto& g : plan_graphs)
       if (g.exec) cudaGraphExecDestroy(g.exec);
     for (auto* a : arenas)
       if (a) cudaFree(a);
@@ -481,8 +495,8 @@ void release_blocks(b200_client* c) {
 cudaError_t block_alloc(b200_client* c, size_t bytes, cudaStream_t stream, void** out) {
   const size_t n = block_bytes(bytes);
   if (stream == c->compute && n <= b200_client::kBlockMax) {
-    // the lowest address that fits: programs that repeat themselves then see the same addresses again, which recordings
-    // of loops and plans are made for
+    // the lowest address that fits: a program that repeats itself then sees the same addresses again, and its recording
+    // has fewer nodes to give new ones
     auto best = c->free_blocks.end();
     for (auto it = c->free_blocks.begin(); it != c->free_blocks.end(); ++it)
       if (it->bytes == n && (best == c->free_blocks.end() || it->ptr < best->ptr)) best = it;
@@ -701,6 +715,7 @@ struct ExecCtx {
   bool plain_launch = false;            // while the bodies of conditional graph nodes are recorded: no programmatic launches
   bool coll_pending = false;            // work on the collective stream that the compute stream has not waited for yet
   cudaStream_t coll_stream = nullptr;   // set while the members of an all-reduce group are issued
+  class NodeObserver* nodes = nullptr;  // set while steps go into a recording instead of to the device
   struct Timed { std::string kind, key; cudaEvent_t a, b; };
   std::vector<Timed> timed;
 };
@@ -751,26 +766,139 @@ void touched_addresses(const ExecCtx& x, const Step& s, std::vector<void*>& out,
 // steps do not meet by reuse alone (kReuseDistance in the plan compiler).
 b200_error* run_step(ExecCtx& x, const Step& s);
 
+// Addresses of all arguments and results of a call.
+std::vector<void*> outer_addresses(const ExecCtx& x) {
+  std::vector<void*> v;
+  const auto& slots = x.lp->prog->slots;
+  for (size_t k = 0; k < slots.size(); k++)
+    if (slots[k].kind == Slot::ARG || slots[k].kind == Slot::RESULT) v.push_back(x.ptrs[k]);
+  return v;
+}
+
+// Receives what steps launch while they go into a recording: `nodes` gets the graph node behind each launch on the
+// capturing stream, or, with `exec`, the launch becomes the new parameters of the next of those nodes. In the second case
+// the kernel, its grid and its shared memory have to be what they were; otherwise `failed`, and the recording is void.
+class NodeObserver final : public LaunchObserver {
+ public:
+  NodeObserver(ExecCtx& x, cudaGraphExec_t exec) : x_(x), exec_(exec) {
+    x_.nodes = this;
+    launch_observer = this;
+  }
+  ~NodeObserver() {
+    x_.nodes = nullptr;
+    launch_observer = nullptr;
+  }
+  std::vector<Recording::Node>* nodes = nullptr;       // null: of no interest
+  size_t next = 0;
+  bool failed = false;
+
+  cudaError_t kernel(const void* func, const cudaLaunchConfig_t& cfg, void** args) override {
+    const Recording::Node n{nullptr, func, cfg.gridDim, cfg.blockDim, cfg.dynamicSmemBytes};
+    if (!exec_) return noted(cudaLaunchKernelExC(&cfg, func, args), n);
+    const Recording::Node* old = expect(n);
+    if (!old) return cudaSuccess;
+    cudaKernelNodeParams p = {};
+    p.func = (void*)func;
+    p.gridDim = cfg.gridDim;
+    p.blockDim = cfg.blockDim;
+    p.sharedMemBytes = (unsigned)cfg.dynamicSmemBytes;
+    p.kernelParams = args;
+    return set(cudaGraphExecKernelNodeSetParams(exec_, old->node, &p));
+  }
+  cudaError_t copy(void* dst, const void* src, size_t bytes, cudaStream_t stream) override {
+    const Recording::Node n{nullptr, nullptr, dim3(), dim3(), bytes};
+    if (!exec_) return noted(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, stream), n);
+    const Recording::Node* old = expect(n);
+    return old ? set(cudaGraphExecMemcpyNodeSetParams1D(exec_, old->node, dst, src, bytes, cudaMemcpyDeviceToDevice)) : cudaSuccess;
+  }
+  // a generated kernel, launched through the driver
+  template <typename F>
+  CUresult generated(CUfunction func, const dim3& grid, const dim3& block, void** args, F&& launch) {
+    const Recording::Node n{nullptr, (const void*)func, grid, block, 0};
+    if (!exec_) {
+      const CUresult r = launch();
+      if (r == CUDA_SUCCESS) noted(cudaSuccess, n);
+      return r;
+    }
+    const Recording::Node* old = expect(n);
+    if (!driver().GraphExecKernelNodeSetParams) failed = true;
+    if (!old || failed) return CUDA_SUCCESS;
+    CUDA_KERNEL_NODE_PARAMS p = {};
+    p.func = func;
+    p.gridDimX = grid.x; p.gridDimY = grid.y; p.gridDimZ = grid.z;
+    p.blockDimX = block.x; p.blockDimY = block.y; p.blockDimZ = block.z;
+    p.kernelParams = args;
+    const CUresult r = driver().GraphExecKernelNodeSetParams((CUgraphExec)exec_, (CUgraphNode)old->node, &p);
+    if (r != CUDA_SUCCESS) failed = true;
+    return r;
+  }
+
+ private:
+  cudaError_t noted(cudaError_t e, Recording::Node n) {
+    if (e != cudaSuccess || !nodes) return e;
+    cudaStreamCaptureStatus status;
+    const cudaGraphNode_t* last = nullptr;
+    size_t count = 0;
+    e = cudaStreamGetCaptureInfo(x_.c->compute, &status, nullptr, nullptr, &last, &count);
+    if (e == cudaSuccess && count == 1) n.node = last[0];
+    else failed = true;
+    nodes->push_back(n);
+    return e;
+  }
+  const Recording::Node* expect(const Recording::Node& n) {
+    const Recording::Node* old = nodes && next < nodes->size() ? &(*nodes)[next++] : nullptr;
+    auto same = [](const dim3& a, const dim3& b) { return a.x == b.x && a.y == b.y && a.z == b.z; };
+    if (!old || old->func != n.func || old->bytes != n.bytes || !same(old->grid, n.grid) || !same(old->block, n.block)) {
+      failed = true;
+      return nullptr;
+    }
+    return old;
+  }
+  cudaError_t set(cudaError_t e) {
+    if (e != cudaSuccess) failed = true;
+    return e;
+  }
+  ExecCtx& x_;
+  cudaGraphExec_t exec_;
+};
+
 class Recorder {
  public:
-  Recorder(ExecCtx& x, cudaGraph_t graph) : x_(x), graph_(graph) {}
+  Recorder(ExecCtx& x, Recording& rec) : x_(x), rec_(rec), graph_(rec.graph), observer_(x, nullptr) {
+    rec.outer = outer_addresses(x);
+    outer_ = rec.outer;
+    std::sort(outer_.begin(), outer_.end());
+  }
 
   b200_error* step(const Step& s) {
     reads_.clear();
     writes_.clear();
     const bool all = !accesses(s);
+    std::vector<void*> at;
+    touched_addresses(x_, s, at, false);
+    begin(std::move(at));
     return record(all, [&]() { return run_step(x_, s); });
   }
   b200_error* copy(void* dst, const void* src, size_t bytes) {
     reads_.assign(1, {(uintptr_t)src, (uintptr_t)src + bytes});
     writes_.assign(1, {(uintptr_t)dst, (uintptr_t)dst + bytes});
+    begin({dst, (void*)src});
     return record(false, [&]() -> b200_error* {
-      CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, x_.c->compute));
+      CUDA_TRY(copy_on_device(dst, src, bytes, x_.c->compute));
       return nullptr;
     });
   }
+  bool failed() const { return observer_.failed; }
 
  private:
+  // what the next launches belong to: their nodes are kept when they have an argument's or a result's address
+  void begin(std::vector<void*> at) {
+    bool moves = false;
+    for (void* p : at) moves = moves || std::binary_search(outer_.begin(), outer_.end(), p);
+    rec_.order.push_back(moves ? (int)rec_.issues.size() : -1);
+    if (moves) rec_.issues.push_back({std::move(at), {}});
+    observer_.nodes = moves ? &rec_.issues.back().nodes : nullptr;
+  }
   struct Range { uintptr_t lo, hi; };
   struct Memory { Range at; int writer; std::vector<int> readers; };
   struct Node { std::vector<cudaGraphNode_t> ends; std::vector<bool> before; };
@@ -876,12 +1004,144 @@ class Recorder {
     return nullptr;
   }
   ExecCtx& x_;
+  Recording& rec_;
   cudaGraph_t graph_;
+  NodeObserver observer_;
+  std::vector<void*> outer_;           // sorted
   std::vector<Node> nodes_;
   std::vector<Memory> memory_;
   std::vector<Range> reads_, writes_;
   int barrier_ = -1;
 };
+
+// Walks a recording's steps again with the addresses of another call and gives the nodes that hold others the new ones.
+// The edges stay: arguments are only read, a result is a fresh allocation in every call, and which steps meet in the arena
+// does not change. Launches that are on their way keep the parameters they were issued with.
+// Measured on the ResNet18 step, whose 247 launches have 143 with an address of a parameter, a moment or a result: 50 us
+// for giving all of them others, and 30 us more for the launch that follows.
+class Relocator {
+ public:
+  Relocator(ExecCtx& x, Recording& rec) : x_(x), rec_(rec), observer_(x, rec.exec) {}
+  b200_error* step(const Step& s) {
+    at_.clear();
+    if (next()) touched_addresses(x_, s, at_, false);
+    return move([&]() { return run_step(x_, s); });
+  }
+  b200_error* copy(void* dst, const void* src, size_t bytes) {
+    at_.clear();
+    if (next()) at_ = {dst, (void*)src};
+    return move([&]() -> b200_error* {
+      CUDA_TRY(copy_on_device(dst, src, bytes, x_.c->compute));
+      return nullptr;
+    });
+  }
+  bool failed() const { return observer_.failed; }
+
+ private:
+  bool next() {
+    const int k = rec_.order[at_op_++];
+    issue_ = k >= 0 ? &rec_.issues[k] : nullptr;
+    return issue_ != nullptr;
+  }
+  template <typename F>
+  b200_error* move(F&& launch) {
+    if (!issue_ || issue_->at == at_) return nullptr;
+    issue_->at = at_;
+    observer_.nodes = &issue_->nodes;
+    observer_.next = 0;
+    b200_error* err = launch();
+    if (observer_.next != issue_->nodes.size()) observer_.failed = true;
+    return err;
+  }
+  ExecCtx& x_;
+  Recording& rec_;
+  NodeObserver observer_;
+  Recording::Issue* issue_ = nullptr;
+  std::vector<void*> at_;
+  size_t at_op_ = 0;
+};
+
+// What a recording consists of: the steps of a plan, or iterations of a counted loop with the copies and exchanges of its
+// carried values (exchanged pointers are back where they started after an even number).
+template <typename G>
+b200_error* walk(G& g, const Plan& plan) {
+  for (const Step& s : plan.steps)
+    if (auto* e = g.step(s)) return e;
+  return nullptr;
+}
+template <typename G>
+b200_error* walk(G& g, ExecCtx& x, const Step& loop, long long iterations) {
+  for (long long i = 0; i < iterations; i++) {
+    if (auto* e = walk(g, *loop.sub[1])) return e;
+    for (size_t k = 0; k < loop.state.size(); k++) {
+      void *&d = x.ptrs[loop.state[k]], *&src = x.ptrs[loop.next[k]];
+      const size_t b = x.lp->prog->slots[loop.state[k]].type.bytes();
+      if (k < loop.swap.size() && loop.swap[k]) std::swap(d, src);
+      else if (d != src && b)
+        if (auto* e = g.copy(d, src, b)) return e;
+    }
+  }
+  return nullptr;
+}
+
+// Records what `steps` walks; false (and `off`) when that does not go: the caller runs it step by step.
+template <typename F>
+bool record_graph(ExecCtx& x, Recording& rec, F&& steps) {
+  const int before = x.launches;
+  const std::vector<void*> at_start = x.ptrs;
+  b200_error* err = nullptr;
+  cudaError_t ce = cudaGraphCreate(&rec.graph, 0);
+  bool ok = ce == cudaSuccess;
+  if (ok) {
+    Recorder recorder(x, rec);
+    err = steps(recorder);
+    ok = !err && !recorder.failed() && x.ptrs == at_start;
+  }
+  if (ok) ok = (ce = cudaGraphInstantiate(&rec.exec, rec.graph, 0)) == cudaSuccess;
+  rec.launches = x.launches - before;
+  x.launches = before;
+  x.ptrs = at_start;
+  if (ok) {
+    x.lp->recordings++;
+    return true;
+  }
+  logf(1, "a plan could not be recorded and runs step by step: %s", err ? err->message.c_str() : cudaGetErrorString(ce));
+  if (err) b200_error_destroy(err);
+  cudaGetLastError();
+  rec.clear();
+  rec.off = true;
+  return false;
+}
+
+// Gives a recording the addresses of this call; false (and `off`) when it can no longer be used.
+template <typename F>
+bool relocate_graph(ExecCtx& x, Recording& rec, F&& steps) {
+  std::vector<void*> outer = outer_addresses(x);
+  if (outer == rec.outer) return true;
+  const int before = x.launches;
+  const std::vector<void*> at_start = x.ptrs;
+  b200_error* err;
+  bool ok;
+  {
+    Relocator relocator(x, rec);
+    err = steps(relocator);
+    ok = !err && !relocator.failed();
+  }
+  x.launches = before;
+  x.ptrs = at_start;
+  if (ok) {
+    rec.outer = std::move(outer);
+    x.lp->relocations++;
+    return true;
+  }
+  logf(1, "a recording could not take a call's addresses, its plan runs step by step: %s", err ? err->message.c_str() : cudaGetErrorString(cudaPeekAtLastError()));
+  if (err) b200_error_destroy(err);
+  cudaGetLastError();
+  cudaStreamSynchronize(x.c->compute);         // launches of it may be on their way
+  rec.clear();
+  rec.off = true;
+  return false;
+}
 
 b200_error* run_step(ExecCtx& x, const Step& s) {
   b200_client* c = x.c;
@@ -896,8 +1156,10 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
         vals[k] = x.ptrs[s.args[k]];
         argv[k] = &vals[k];
       }
-      CUresult r;
-      if (driver().LaunchKernelEx && !c->sw.no_pdl && !x.plain_launch) {
+      auto launch = [&]() -> CUresult {
+        if (!driver().LaunchKernelEx || c->sw.no_pdl || x.plain_launch)
+          return driver().LaunchKernel(x.lp->functions[s.kernel], s.grid[0], s.grid[1], s.grid[2], s.block[0], s.block[1], s.block[2], 0,
+                                       (CUstream)st, argv, nullptr);
         // programmatic stream serialization: the kernel is scheduled while the one in front of it drains, and waits for
         // it (first statement of every generated kernel) before it reads or writes anything
         CUlaunchConfig cfg = {};
@@ -910,11 +1172,11 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
         attr[0].value.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        r = driver().LaunchKernelEx(&cfg, x.lp->functions[s.kernel], argv, nullptr);
-      } else {
-        r = driver().LaunchKernel(x.lp->functions[s.kernel], s.grid[0], s.grid[1], s.grid[2], s.block[0], s.block[1], s.block[2], 0,
-                                  (CUstream)st, argv, nullptr);
-      }
+        return driver().LaunchKernelEx(&cfg, x.lp->functions[s.kernel], argv, nullptr);
+      };
+      const CUresult r = x.nodes ? x.nodes->generated(x.lp->functions[s.kernel], dim3(s.grid[0], s.grid[1], s.grid[2]),
+                                                      dim3(s.block[0], s.block[1], s.block[2]), argv, launch)
+                                 : launch();
       if (r != CUDA_SUCCESS) {
         const char* msg = nullptr;
         driver().GetErrorString(r, &msg);
@@ -996,7 +1258,7 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
     }
     case Step::MEMCPY: {
       if (s.bytes && x.ptrs[s.args[0]] != x.ptrs[s.args[1]])
-        CUDA_TRY(cudaMemcpyAsync(x.ptrs[s.args[0]], x.ptrs[s.args[1]], s.bytes, cudaMemcpyDeviceToDevice, st));
+        CUDA_TRY(copy_on_device(x.ptrs[s.args[0]], x.ptrs[s.args[1]], s.bytes, st));
       return nullptr;
     }
     case Step::ALL_REDUCE: {
@@ -1041,7 +1303,7 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
       for (size_t k = 0; k < n; k++) {
         void *d = x.ptrs[s.state[k]], *src = x.ptrs[s.init[k]];
         size_t b = x.lp->prog->slots[s.state[k]].type.bytes();
-        if (d != src && b) CUDA_TRY(cudaMemcpyAsync(d, src, b, cudaMemcpyDeviceToDevice, st));
+        if (d != src && b) CUDA_TRY(copy_on_device(d, src, b, st));
       }
       // carried values marked for exchange trade pointers with their next value after every iteration; when the
       // loop ends the pointers go back and a value left in the other buffer is copied home once
@@ -1059,7 +1321,7 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
           }
           void *d = x.ptrs[s.state[k]], *src = x.ptrs[s.next[k]];
           size_t b = x.lp->prog->slots[s.state[k]].type.bytes();
-          if (d != src && b) CUDA_TRY(cudaMemcpyAsync(d, src, b, cudaMemcpyDeviceToDevice, st));
+          if (d != src && b) CUDA_TRY(copy_on_device(d, src, b, st));
         }
         return nullptr;
       };
@@ -1070,7 +1332,7 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
           x.ptrs[s.state[k]] = home_state[k];
           x.ptrs[s.next[k]] = home_next[k];
           size_t b = x.lp->prog->slots[s.state[k]].type.bytes();
-          if (cur != home_state[k] && b) CUDA_TRY(cudaMemcpyAsync(home_state[k], cur, b, cudaMemcpyDeviceToDevice, st));
+          if (cur != home_state[k] && b) CUDA_TRY(copy_on_device(home_state[k], cur, b, st));
         }
         return nullptr;
       };
@@ -1080,80 +1342,32 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
         long long done = 0;
         cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
         CUDA_TRY(cudaStreamIsCapturing(st, &capturing));
-        if (s.trip_count >= 4 && !c->profiling && capturing == cudaStreamCaptureStatusNone && graph_safe(*s.sub[1]) &&
+        if (s.trip_count >= 4 && !c->profiling && !x.nodes && capturing == cudaStreamCaptureStatusNone && graph_safe(*s.sub[1]) &&
             !c->sw.no_loop_graphs) {
-          // An even number of iterations (after which exchanged pointers are back where they started) is recorded once as
-          // a CUDA graph and replayed: the host issues one launch for all of them. As many iterations as make about
-          // kLoopGraphNodes nodes: kernels inside a graph start while their predecessors drain, but a graph waits for the
-          // whole graph in front of it, which costs about 1 us (a loop of one small kernel took 2.1 us an iteration in
-          // graphs of two and takes 0.9 us in long ones).
-          std::vector<void*> touched;                  // what the recording depends on: not the program's other arguments and results
-          touched_addresses(x, s, touched);
-          LoadedProgram::LoopGraph* hit = nullptr;
-          for (auto& g : x.lp->loop_graphs)
-            if (g.step == &s && g.ptrs == touched) { hit = &g; break; }
-          bool record = !hit;
-          if (record && !x.lp->met_before(&s, touched)) {
-            // addresses that are new: a loop of many recordings' length is worth one all the same
-            const int first = x.launches;
-            if (auto* e = iterate()) return e;
-            if (auto* e = iterate()) return e;
-            done = 2;
-            record = (s.trip_count - done) / 2 * std::max(1, x.launches - first) >= 16 * kLoopGraphNodes;
-          }
-          if (record) {
-            if (x.lp->loop_graphs.size() >= 24) {
-              // bounded cache: let the device finish with the oldest graph before it goes
-              CUDA_TRY(cudaStreamSynchronize(st));
-              cudaGraphExecDestroy(x.lp->loop_graphs.front().exec);
-              x.lp->loop_graphs.erase(x.lp->loop_graphs.begin());
-            }
-            const std::vector<void*> at_start = x.ptrs;
+          // An even number of iterations is recorded once as a CUDA graph and replayed: the host issues one launch for all
+          // of them. As many iterations as make about kLoopGraphNodes nodes: kernels inside a graph start while their
+          // predecessors drain, but a graph waits for the whole graph in front of it, which costs about 1 us (a loop of one
+          // small kernel took 2.1 us an iteration in graphs of two and takes 0.9 us in long ones).
+          Recording& rec = x.lp->loop_graphs[&s];
+          if (!rec.exec && !rec.off) {
             // a pair runs directly, so that every kernel of the body has been loaded and configured before anything is
             // recorded, and its launches are known
             const int first = x.launches;
             if (auto* e = iterate()) return e;
             if (auto* e = iterate()) return e;
-            done += 2;
+            done = 2;
             const int per_pair = std::max(1, x.launches - first);
-            const long long pairs = std::max<long long>(1, std::min<long long>((s.trip_count - done) / 2, kLoopGraphNodes / per_pair));
-            const int before = x.launches;
-            cudaGraph_t graph = nullptr;
-            CUDA_TRY(cudaGraphCreate(&graph, 0));
-            b200_error* err = nullptr;
-            {
-              Recorder recorder(x, graph);
-              for (long long i = 0; i < 2 * pairs && !err; i++) {
-                for (const Step& t : s.sub[1]->steps)
-                  if (!err) err = recorder.step(t);
-                for (size_t k = 0; k < n && !err; k++) {
-                  void *&d = x.ptrs[s.state[k]], *&src = x.ptrs[s.next[k]];
-                  const size_t b = x.lp->prog->slots[s.state[k]].type.bytes();
-                  if (k < s.swap.size() && s.swap[k]) std::swap(d, src);
-                  else if (d != src && b) err = recorder.copy(d, src, b);
-                }
-              }
+            const long long left = (s.trip_count - done) / 2;
+            if (left > 0) {
+              rec.iterations = 2 * std::max<long long>(1, std::min<long long>(left, kLoopGraphNodes / per_pair));
+              record_graph(x, rec, [&](auto& g) { return walk(g, x, s, rec.iterations); });
             }
-            if (err) {
-              cudaGraphDestroy(graph);
-              return err;
-            }
-            cudaError_t ce;
-            cudaGraphExec_t exec = nullptr;
-            ce = cudaGraphInstantiate(&exec, graph, 0);
-            cudaGraphDestroy(graph);
-            CUDA_TRY(ce);
-            if (x.ptrs != at_start) {
-              cudaGraphExecDestroy(exec);
-              return make_error(B200_INTERNAL, "loop state pointers did not return after an even number of iterations");
-            }
-            x.lp->loop_graphs.push_back({&s, std::move(touched), exec, x.launches - before, 2 * pairs});
-            x.launches = before;
-            hit = &x.lp->loop_graphs.back();
+          } else if (rec.exec) {
+            relocate_graph(x, rec, [&](auto& g) { return walk(g, x, s, rec.iterations); });
           }
-          for (; hit && done + hit->iterations <= s.trip_count; done += hit->iterations) {
-            CUDA_TRY(cudaGraphLaunch(hit->exec, st));
-            x.launches += hit->launches;
+          for (; rec.exec && done + rec.iterations <= s.trip_count; done += rec.iterations) {
+            CUDA_TRY(cudaGraphLaunch(rec.exec, st));
+            x.launches += rec.launches;
           }
         }
         for (long long i = done; i < s.trip_count; i++)
@@ -1275,14 +1489,14 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
           b200_error_destroy(err);
           cudaGetLastError();
         } else {
-          x.lp->cond_graphs.push_back({&s, touched, exec, recorded, 0});
+          x.lp->cond_graphs.push_back({&s, touched, exec, recorded});
         }
       }
       return nullptr;
     }
     case Step::SCATTER: {
       void *operand = x.ptrs[s.args[0]], *out = x.ptrs[s.args[3]];
-      if (operand != out && s.bytes) CUDA_TRY(cudaMemcpyAsync(out, operand, s.bytes, cudaMemcpyDeviceToDevice, st));
+      if (operand != out && s.bytes) CUDA_TRY(copy_on_device(out, operand, s.bytes, st));
       const int ek = s.dtype == DT::F32 ? 0 : s.dtype == DT::BF16 ? 1 : 2;
       if (s.iparams.size() > 5 && s.iparams[5] == 1) {
         // general form: the key kernel in front of this step has filled the scratch with (destination, update) pairs
@@ -1384,7 +1598,7 @@ b200_error* run_step(ExecCtx& x, const Step& s) {
           b200_error_destroy(err);
           cudaGetLastError();
         } else {
-          x.lp->cond_graphs.push_back({&s, touched, exec, recorded, 0});
+          x.lp->cond_graphs.push_back({&s, touched, exec, recorded});
         }
       }
       return nullptr;
@@ -1523,59 +1737,26 @@ b200_error* run_plan(ExecCtx& x, const Plan& plan) {
 }
 
 // A plan of many small kernels is bound by the host: a launch costs it two to four microseconds, a graph of all of them a
-// few. The addresses of arguments and results are part of a recording, and programs that run in a loop come back to the
-// same few sets of them (results return to the pool and are handed out again), so a set is recorded when it is seen for
-// the second time and replayed from then on; everything else is launched step by step as before. Bounded: at most
-// kPlanGraphs recordings are kept, the least recently used goes first, and a program whose addresses keep changing stops
-// recording (a recording has to pay for itself in replays).
-constexpr size_t kPlanGraphs = 12;
+// few, and a node that is given other addresses less than one. The first call runs step by step, which loads and configures
+// every kernel, and records behind that (capture takes 7 us a launch, instantiation another 3 to 14 ms for plans of 250 to
+// 420 launches; loading took 20 to 30 ms); all later calls replay, whichever buffers they are given.
 constexpr int kReplayLaunches = 6;
 
 b200_error* run_main(ExecCtx& x) {
   LoadedProgram& lp = *x.lp;
   b200_client* c = x.c;
   const Plan& plan = lp.prog->main;
-  if (!lp.replayable || c->profiling || c->sw.no_plan_graphs) return run_plan(x, plan);
-  lp.calls++;
-  std::vector<void*> key;
-  for (size_t s = 0; s < lp.prog->slots.size(); s++)
-    if (lp.prog->slots[s].kind == Slot::ARG || lp.prog->slots[s].kind == Slot::RESULT) key.push_back(x.ptrs[s]);
-  for (auto& g : lp.plan_graphs)
-    if (g.ptrs == key) {
-      g.used = lp.calls;
-      lp.replays++;
-      CUDA_TRY(cudaGraphLaunch(g.exec, c->compute));
-      x.launches += g.launches;
-      return nullptr;
-    }
-  if (!lp.met_before(&plan, key) || lp.recordings > 2 * kPlanGraphs + lp.replays / 16) return run_plan(x, plan);
-  if (lp.plan_graphs.size() >= kPlanGraphs) {
-    auto old = std::min_element(lp.plan_graphs.begin(), lp.plan_graphs.end(), [](auto& a, auto& b) { return a.used < b.used; });
-    CUDA_TRY(cudaStreamSynchronize(c->compute));
-    cudaGraphExecDestroy(old->exec);
-    lp.plan_graphs.erase(old);
+  Recording& rec = lp.main_graph;
+  if (!lp.replayable || c->profiling || c->sw.no_plan_graphs || rec.off) return run_plan(x, plan);
+  auto steps = [&](auto& g) { return walk(g, plan); };
+  if (!rec.exec) {
+    if (auto* e = run_plan(x, plan)) return e;
+    record_graph(x, rec, steps);
+    return nullptr;
   }
-  lp.recordings++;
-  const int before = x.launches;
-  cudaGraph_t graph = nullptr;
-  CUDA_TRY(cudaGraphCreate(&graph, 0));
-  b200_error* err = nullptr;
-  {
-    Recorder recorder(x, graph);
-    for (const Step& st : plan.steps)
-      if (!err) err = recorder.step(st);
-  }
-  if (err) {
-    cudaGraphDestroy(graph);
-    return err;
-  }
-  cudaError_t ce;
-  cudaGraphExec_t exec = nullptr;
-  ce = cudaGraphInstantiate(&exec, graph, 0);
-  cudaGraphDestroy(graph);
-  CUDA_TRY(ce);
-  lp.plan_graphs.push_back({std::move(key), exec, x.launches - before, lp.calls});
-  CUDA_TRY(cudaGraphLaunch(exec, c->compute));
+  if (!relocate_graph(x, rec, steps)) return run_plan(x, plan);
+  CUDA_TRY(cudaGraphLaunch(rec.exec, c->compute));
+  x.launches += rec.launches;
   return nullptr;
 }
 
@@ -2031,6 +2212,8 @@ int64_t b200_executable_temp_bytes(const b200_executable* e) {
   for (auto b : e->lp->prog->arena_bytes) t += (int64_t)b;
   return t;
 }
+int64_t b200_executable_recordings(const b200_executable* e) { return e->lp->recordings; }
+int64_t b200_executable_relocations(const b200_executable* e) { return e->lp->relocations; }
 const char* b200_executable_plan_text(const b200_executable* e) { return e->lp->prog->dump.c_str(); }
 
 b200_error* b200_executable_output_info(const b200_executable* e, size_t i, b200_dtype* dt, const int64_t** dims,

@@ -26,6 +26,7 @@
 #include <algorithm>
 
 #include "kernels.h"
+#include "launch.h"
 #include "tc_util.cuh"
 
 namespace b200 {
@@ -344,8 +345,8 @@ cudaError_t launch(const Tile32Launch& t, const CUtensorMap& tm, const float* im
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = g_programmatic ? 1 : 0;
-  if (t.mode == 3) return cudaLaunchKernelEx(&cfg, tile32_kernel<BN, true>, tm, image, C, partial, ct[0], ct[1], ct[2], error_flag, p);
-  return cudaLaunchKernelEx(&cfg, tile32_kernel<BN, false>, tm, image, C, partial, ct[0], ct[1], ct[2], error_flag, p);
+  if (t.mode == 3) return launch_kernel(cfg, tile32_kernel<BN, true>, tm, image, C, partial, ct[0], ct[1], ct[2], error_flag, p);
+  return launch_kernel(cfg, tile32_kernel<BN, false>, tm, image, C, partial, ct[0], ct[1], ct[2], error_flag, p);
 }
 
 }  // namespace
@@ -365,7 +366,7 @@ cudaError_t launch_split_b(const Tile32Launch& t, bool lanes_n, const void* B, v
   cfg.attrs = attr;
   cfg.numAttrs = g_programmatic ? 1 : 0;
   auto row = (const long long*)b_tables[0], col = (const long long*)b_tables[1], grp = (const long long*)b_tables[2];
-  cudaError_t e = cudaLaunchKernelEx(&cfg, lanes_n ? split_b_kernel<true> : split_b_kernel<false>, (const float*)B, (float*)image, row, col, grp, t.N, t.K,
+  cudaError_t e = launch_kernel(cfg, lanes_n ? split_b_kernel<true> : split_b_kernel<false>, (const float*)B, (float*)image, row, col, grp, t.N, t.K,
                                      t.bn, tiles_n, ktiles, total);
   if (e == cudaSuccess) ++*launches;
   return e;
