@@ -204,7 +204,8 @@ def load_library():
         fn.restype = res
         fn.argtypes = args
     if _hot is None:
-        raise B200Error(f"b200._hot not found beside {p}: build both with `python jax-mps_b200/build.py`", FAILED_PRECONDITION)
+        raise B200Error(f"b200._hot for this Python not found in {Path(__file__).resolve().parent}: build it with "
+                        "`python jax-mps_b200/build.py`", FAILED_PRECONDITION)
     _hot.bind([C.cast(getattr(lib, n), _P).value for n in (
         "b200_executable_execute", "b200_buffer_from_host", "b200_buffer_to_host", "b200_buffer_destroy", "b200_error_destroy",
         "b200_host_alloc", "b200_host_free")], lambda err: _check(err), Buffer)

@@ -12,7 +12,8 @@ from pathlib import Path
 HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 OUT = HERE / "b200" / "libb200core.so"
-HOT = HERE / "b200" / "_hot.so"
+# named for the interpreter it is built for: it uses structures of CPython that differ between versions
+HOT = HERE / "b200" / ("_hot" + sysconfig.get_config_var("EXT_SUFFIX"))
 SOURCES = ["parser.cc", "codegen.cc", "compiler.cc", "runtime.cc", "kernels.cu", "gemm16.cu", "gemm32.cu", "tile32.cu"]
 
 
@@ -70,6 +71,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
                         str(CSRC / "hot.c"), "-o", str(HOT)], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"gcc failed on hot.c:\n{r.stdout}")
+    (HERE / "b200" / "_hot.so").unlink(missing_ok=True)        # of before the interpreter was part of the name
     return OUT
 
 

@@ -51,3 +51,23 @@ def test_initialize_says_what_is_missing(monkeypatch, tmp_path):
         plugin._find_library()
     monkeypatch.delenv("B200_PJRT_LIBRARY_PATH")
     assert plugin._find_library() is None                       # the adapter library is not built on this machine
+
+
+def test_an_installed_package_loads(tmp_path):
+    """What the package data names is all that the library needs: installed elsewhere, it loads."""
+    import shutil
+    import subprocess
+    import b200
+    b200.load_library()                     # built
+    src, to = tmp_path / "src", tmp_path / "site"
+    shutil.copytree(ROOT / "jax-mps_b200", src, ignore=shutil.ignore_patterns("csrc", "build", "__pycache__", "*.egg-info"))
+    r = subprocess.run([sys.executable, "-m", "pip", "install", "-q", "--no-index", "--no-build-isolation", "--no-deps", "--target", str(to), str(src)],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    code = "import b200; b200.load_library(); print(b200.__file__, b200._hot.__file__)"
+    r = subprocess.run([sys.executable, "-c", code], cwd=tmp_path, env={"PYTHONPATH": str(to), "PATH": "/usr/bin:/bin"}, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    files = r.stdout.split()
+    assert all(f.startswith(str(to)) for f in files), files
+    import importlib.machinery
+    assert any(files[1].endswith(s) for s in importlib.machinery.EXTENSION_SUFFIXES if s != ".so"), files[1]
