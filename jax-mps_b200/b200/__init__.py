@@ -16,11 +16,6 @@ from pathlib import Path
 
 import numpy as np
 
-try:
-    from . import _hot                  # the calls of an inner loop (csrc/hot.c); built beside the library
-except ImportError:
-    _hot = None
-
 _LIB_NAME = "libb200core.so"
 
 
@@ -188,6 +183,15 @@ def library_path() -> Path:
     return Path(__file__).resolve().parent / _LIB_NAME
 
 
+def __getattr__(name):
+    # the buffer class derives from a type of the extension module, which a program that only makes or reads program text
+    # (or times something else) does not map
+    if name == "Buffer":
+        load_library()
+        return globals()["Buffer"]
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
+
+
 def load_library():
     """dlopen the core and bind every declared symbol. Raises B200Error when
     the extension has not been built — nothing here falls back to the CPU."""
@@ -203,9 +207,13 @@ def load_library():
         fn = getattr(lib, name)
         fn.restype = res
         fn.argtypes = args
-    if _hot is None:
+    try:
+        from . import _hot                  # the calls of an inner loop (csrc/hot.c)
+    except ImportError as e:
         raise B200Error(f"b200._hot for this Python not found in {Path(__file__).resolve().parent}: build it with "
-                        "`python jax-mps_b200/build.py`", FAILED_PRECONDITION)
+                        "`python jax-mps_b200/build.py`", FAILED_PRECONDITION) from e
+    from .buffer import Buffer
+    globals()["Buffer"] = Buffer
     _hot.bind([C.cast(getattr(lib, n), _P).value for n in (
         "b200_executable_execute", "b200_buffer_from_host", "b200_buffer_to_host", "b200_buffer_destroy", "b200_error_destroy",
         "b200_host_alloc", "b200_host_free")], lambda err: _check(err), Buffer)
@@ -360,76 +368,6 @@ class Event:
         if getattr(self, "_h", None):
             load_library().b200_event_destroy(self._h)
             self._h = None
-
-
-class Buffer(_hot.Handle if _hot else object):
-    """A device array (PJRT_Buffer), made from its client and its handle (`_h`), which it owns."""
-
-    @property
-    def dtype_code(self) -> int:
-        return load_library().b200_buffer_dtype(self._h)
-
-    @property
-    def dtype(self) -> str:
-        return _DT_NAMES[self.dtype_code]
-
-    @property
-    def shape(self) -> tuple:
-        lib = load_library()
-        n = lib.b200_buffer_num_dims(self._h)
-        d = lib.b200_buffer_dims(self._h)
-        return tuple(int(d[i]) for i in range(n))
-
-    @property
-    def nbytes(self) -> int:
-        return load_library().b200_buffer_on_device_size(self._h)
-
-    def device_pointer(self) -> int:
-        return load_library().b200_buffer_device_pointer(self._h) or 0
-
-    def is_deleted(self) -> bool:
-        return bool(load_library().b200_buffer_is_deleted(self._h))
-
-    def delete(self):
-        _check(load_library().b200_buffer_delete(self._h))
-
-    def copy(self) -> "Buffer":
-        out = _P()
-        _check(load_library().b200_buffer_copy(self._h, C.byref(out)))
-        return Buffer(self.client, out.value)
-
-    def block_until_ready(self) -> "Buffer":
-        ev = _P()
-        _check(load_library().b200_buffer_ready_event(self._h, C.byref(ev)))
-        Event(ev.value).wait()
-        return self
-
-    def to_host_async(self, out: np.ndarray) -> Event:
-        """Start a device-to-host copy into `out` (same shape/dtype; pinned memory makes it truly asynchronous)."""
-        size = C.c_size_t(out.nbytes)
-        ev = _P()
-        _check(load_library().b200_buffer_to_host(self._h, out.ctypes.data_as(_P), C.byref(size), C.byref(ev)))
-        return Event(ev.value)
-
-    def to_numpy(self) -> np.ndarray:
-        """bf16 buffers come back as float32 (exactly representable)."""
-        code = self.dtype_code
-        nbytes = self.nbytes
-        if 65536 <= nbytes <= 1 << 24:
-            block = _hot.to_block(self, nbytes)              # page-locked memory, given back with the array
-            if block is not None:
-                out = np.frombuffer(block, dtype=_DT_TO_NP[code]).reshape(self.shape)
-                return (out.astype(np.uint32) << 16).view(np.float32) if code == BF16 else out
-        out = np.empty(self.shape, dtype=_DT_TO_NP[code])
-        size = C.c_size_t(out.nbytes)
-        _check(load_library().b200_buffer_to_host(self._h, out.ctypes.data_as(_P), C.byref(size), None))
-        if code == BF16:
-            return (out.astype(np.uint32) << 16).view(np.float32)
-        return out
-
-    def __array__(self, dtype=None, copy=None):
-        a = self.to_numpy()
-        return a.astype(dtype) if dtype is not None else a
 
 
 class Executable:

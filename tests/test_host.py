@@ -35,6 +35,18 @@ def test_no_cpu_fallback():
     assert "no CPU fallback" in str(e.value)
 
 
+def test_import_maps_no_compiled_code():
+    """Program text, its generators and the PyTorch twin (the benchmark's reference arm) run without this package's libraries."""
+    import subprocess
+    import sys
+    code = ("import b200, oracle.twins\nfrom b200.shlo import programs\nprograms.init_resnet18(0)\n"
+            "import re; print(sorted(set(re.findall(r'\\S*jax-mps_b200\\S*\\.so', open('/proc/self/maps').read()))))")
+    r = subprocess.run([sys.executable, "-c", code], env={**os.environ, "PYTHONPATH": f"{ROOT / 'jax-mps_b200'}:{ROOT}"}, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    assert r.stdout.strip() == "[]", r.stdout
+    assert issubclass(b200.Buffer, b200._hot.Handle)            # and the class is there once it is asked for
+
+
 def test_unsupported_op_is_a_compile_error_naming_all_ops():
     """Like the reference (src/pjrt_plugin/stablehlo_parser.cc:167-184): one error listing every unsupported op."""
     text = """
