@@ -29,12 +29,17 @@ typedef struct {
   PyObject *client, *host;
 } Handle;
 
+/* Without the interpreter: the client's lock may be held by a thread that waits for the device. */
+static void destroy(void* h) {
+  Py_BEGIN_ALLOW_THREADS
+  b200_error* e = api.destroy((b200_buffer*)h);
+  if (e) api.error_destroy(e);
+  Py_END_ALLOW_THREADS
+}
 static void drop(Handle* self) {
-  if (self->h && api.destroy) {
-    b200_error* e = api.destroy((b200_buffer*)self->h);
-    if (e) api.error_destroy(e);
-  }
+  void* h = self->h;
   self->h = NULL;
+  if (h && api.destroy) destroy(h);
 }
 static int handle_traverse(PyObject* o, visitproc visit, void* arg) {
   Py_VISIT(((Handle*)o)->client);
@@ -91,8 +96,7 @@ static PyObject* wrap(void* h, PyObject* client) {
   PyTypeObject* t = (PyTypeObject*)buffer_class;
   Handle* b = (Handle*)t->tp_alloc(t, 0);
   if (!b) {
-    b200_error* e = api.destroy((b200_buffer*)h);
-    if (e) api.error_destroy(e);
+    destroy(h);
     return NULL;
   }
   b->h = h;
@@ -146,10 +150,7 @@ static PyObject* hot_execute(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   for (Py_ssize_t k = 0; k < num_out; k++) {
     PyObject* b = wrap(out[k], a[5]);
     if (!b) {
-      for (Py_ssize_t q = k + 1; q < num_out; q++) {
-        b200_error* e = api.destroy((b200_buffer*)out[q]);
-        if (e) api.error_destroy(e);
-      }
+      for (Py_ssize_t q = k + 1; q < num_out; q++) destroy(out[q]);
       Py_DECREF(bufs);
       goto done;
     }
@@ -218,7 +219,12 @@ typedef struct {
   Py_ssize_t size;
 } Block;
 static void block_dealloc(PyObject* o) {
-  if (((Block*)o)->ptr) api.host_free(((Block*)o)->ptr);
+  void* ptr = ((Block*)o)->ptr;
+  if (ptr) {
+    Py_BEGIN_ALLOW_THREADS                       /* giving page-locked memory back may wait for the device */
+    api.host_free(ptr);
+    Py_END_ALLOW_THREADS
+  }
   Py_TYPE(o)->tp_free(o);
 }
 static int block_buffer(PyObject* o, Py_buffer* v, int flags) {
@@ -238,7 +244,10 @@ static PyObject* hot_to_block(PyObject* self, PyObject* const* a, Py_ssize_t n) 
   if (n != 2 || !PyObject_TypeCheck(a[0], &HandleType)) return PyErr_Format(PyExc_TypeError, "to_block takes a buffer and its size");
   const Py_ssize_t bytes = PyLong_AsSsize_t(a[1]);
   if (bytes < 0) return PyErr_Occurred() ? NULL : PyErr_Format(PyExc_ValueError, "negative size");
-  void* ptr = api.host_alloc((size_t)bytes);
+  void* ptr;
+  Py_BEGIN_ALLOW_THREADS
+  ptr = api.host_alloc((size_t)bytes);
+  Py_END_ALLOW_THREADS
   if (!ptr) Py_RETURN_NONE;
   Block* b = PyObject_New(Block, &BlockType);
   if (!b) { api.host_free(ptr); return NULL; }

@@ -47,6 +47,48 @@ def test_import_maps_no_compiled_code():
     assert issubclass(b200.Buffer, b200._hot.Handle)            # and the class is there once it is asked for
 
 
+@pytest.mark.parametrize("what", ["a buffer's end", "page-locked memory", "a block's end"])
+def test_extension_module_waits_without_the_interpreter(what):
+    """The C calls behind a buffer's end and behind result memory may wait for a lock that another thread holds until the device
+    is done, or for the device itself: other Python threads run on. libc's sleep stands in for each call in turn (its one
+    argument is the handle or the size, its result the null error)."""
+    import subprocess
+    import sys
+    code = f"""
+import ctypes, threading, time
+import b200
+from b200 import _hot
+libc = ctypes.CDLL(None)
+at = lambda n: ctypes.cast(getattr(libc, n), ctypes.c_void_p).value
+slow, quick = at("sleep"), at("abs")            # abs(0) is a null pointer or null error, abs(1) a pointer that is never read
+class B(_hot.Handle): pass
+what = {what!r}
+host_alloc = slow if what == "page-locked memory" else quick
+# execute, from_host, to_host, destroy, error_destroy, host_alloc, host_free
+_hot.bind([quick, quick, at("isdigit") if what == "a block's end" else quick, slow if what == "a buffer's end" else quick, quick,
+           host_alloc, slow if what == "a block's end" else quick], lambda e: None, B)
+def act():
+    if what == "a buffer's end":
+        h = B(None, 1)
+        del h
+    else:
+        _hot.to_block(B(None, 2 if what == "a block's end" else 0), 1)
+t = threading.Thread(target=act)
+gap, last = 0.0, time.monotonic()
+t.start()
+began = last
+while t.is_alive():
+    time.sleep(0.001)
+    now = time.monotonic()
+    gap, last = max(gap, now - last), now
+print(time.monotonic() - began, gap)
+"""
+    r = subprocess.run([sys.executable, "-c", code], env={**os.environ, "PYTHONPATH": str(ROOT / "jax-mps_b200")}, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    took, gap = map(float, r.stdout.split())
+    assert took > 0.9 and gap < 0.5, (took, gap)
+
+
 def test_unsupported_op_is_a_compile_error_naming_all_ops():
     """Like the reference (src/pjrt_plugin/stablehlo_parser.cc:167-184): one error listing every unsupported op."""
     text = """
