@@ -117,16 +117,17 @@ static PyObject* hot_execute(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   if (n != 6) return PyErr_Format(PyExc_TypeError, "execute takes 6 arguments");
   void* exe = PyLong_AsVoidPtr(a[0]);
   if (!exe) return PyErr_Occurred() ? NULL : PyErr_Format(PyExc_ValueError, "the executable has been destroyed");
-  PyObject* seq = PySequence_Fast(a[1], "arguments are a sequence of buffers");
+  /* a tuple of our own: the caller's list may change in another thread while the call runs without the interpreter */
+  PyObject* seq = PySequence_Tuple(a[1]);
   if (!seq) return NULL;
-  const Py_ssize_t num_args = PySequence_Fast_GET_SIZE(seq), num_out = PyLong_AsSsize_t(a[2]);
+  const Py_ssize_t num_args = PyTuple_GET_SIZE(seq), num_out = PyLong_AsSsize_t(a[2]);
   void *small_in[64], *small_out[64];
   void** in = num_args <= 64 ? small_in : PyMem_Malloc(sizeof(void*) * (size_t)num_args);
   void** out = num_out <= 64 ? small_out : PyMem_Malloc(sizeof(void*) * (size_t)num_out);
   PyObject* result = NULL;
   if (!in || !out) { PyErr_NoMemory(); goto done; }
   for (Py_ssize_t k = 0; k < num_args; k++) {
-    PyObject* o = PySequence_Fast_GET_ITEM(seq, k);
+    PyObject* o = PyTuple_GET_ITEM(seq, k);
     if (!PyObject_TypeCheck(o, &HandleType)) {
       PyErr_Format(PyExc_TypeError, "argument %zd is not a buffer", k);
       goto done;

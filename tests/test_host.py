@@ -89,6 +89,32 @@ print(time.monotonic() - began, gap)
     assert took > 0.9 and gap < 0.5, (took, gap)
 
 
+def test_arguments_live_as_long_as_the_call():
+    """Another thread may empty the list that a call was given; libc's sleep stands in for the call."""
+    import subprocess
+    import sys
+    code = """
+import ctypes, threading, time
+import b200
+from b200 import _hot
+libc = ctypes.CDLL(None)
+at = lambda n: ctypes.cast(getattr(libc, n), ctypes.c_void_p).value
+ends = []
+class B(_hot.Handle):
+    def __del__(self): ends.append(time.monotonic())
+_hot.bind([at("sleep")] + [at("abs")] * 6, lambda e: None, B)
+args = [B(None, 7)]
+t = threading.Timer(0.2, args.clear)
+t.start()
+_hot.execute(1, args, 0, False, False, None)
+back = time.monotonic()
+t.join()
+print(len(ends) == 1 and ends[0] >= back - 0.1)
+"""
+    r = subprocess.run([sys.executable, "-c", code], env={**os.environ, "PYTHONPATH": str(ROOT / "jax-mps_b200")}, capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.strip() == "True", r.stdout + r.stderr
+
+
 def test_unsupported_op_is_a_compile_error_naming_all_ops():
     """Like the reference (src/pjrt_plugin/stablehlo_parser.cc:167-184): one error listing every unsupported op."""
     text = """
