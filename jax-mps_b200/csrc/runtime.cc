@@ -2338,40 +2338,52 @@ HostPool& host_pool() {
 }
 }  // namespace
 
+// The pool's lock is not held across the driver's calls: they may wait for a device, and that device for what another
+// thread launches once it has its own result memory.
 void* b200_host_alloc(size_t bytes) {
   if (bytes < kHostMin || bytes > kHostMax) return nullptr;
   size_t n = kHostMin;
   while (n < bytes) n <<= 1;
   HostPool& pool = host_pool();
-  std::lock_guard<std::mutex> l(pool.mu);
-  if (pool.out[n] >= kHostLent) return nullptr;
-  void* p = nullptr;
-  auto it = pool.kept.find(n);
-  if (it != pool.kept.end()) {
-    p = it->second;
-    pool.kept.erase(it);
-    pool.kept_bytes -= n;
-  } else if (cudaHostAlloc(&p, n, cudaHostAllocPortable) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
+  {
+    std::lock_guard<std::mutex> l(pool.mu);
+    if (pool.out[n] >= kHostLent) return nullptr;
+    pool.out[n]++;
+    auto it = pool.kept.find(n);
+    if (it != pool.kept.end()) {
+      void* p = it->second;
+      pool.kept.erase(it);
+      pool.kept_bytes -= n;
+      pool.lent[p] = n;
+      return p;
+    }
   }
-  pool.lent[p] = n;
-  pool.out[n]++;
-  return p;
+  void* p = nullptr;
+  const bool got = cudaHostAlloc(&p, n, cudaHostAllocPortable) == cudaSuccess;
+  if (!got) cudaGetLastError();
+  std::lock_guard<std::mutex> l(pool.mu);
+  if (got) pool.lent[p] = n;
+  else pool.out[n]--;
+  return got ? p : nullptr;
 }
 
 void b200_host_free(void* ptr) {
   if (!ptr) return;
   HostPool& pool = host_pool();
-  std::lock_guard<std::mutex> l(pool.mu);
-  auto it = pool.lent.find(ptr);
-  if (it == pool.lent.end()) return;
-  const size_t n = it->second;
-  pool.lent.erase(it);
-  pool.out[n]--;
-  if (pool.kept_bytes + n > kHostKept) { cudaFreeHost(ptr); return; }
-  pool.kept.emplace(n, ptr);
-  pool.kept_bytes += n;
+  {
+    std::lock_guard<std::mutex> l(pool.mu);
+    auto it = pool.lent.find(ptr);
+    if (it == pool.lent.end()) return;
+    const size_t n = it->second;
+    pool.lent.erase(it);
+    pool.out[n]--;
+    if (pool.kept_bytes + n <= kHostKept) {
+      pool.kept.emplace(n, ptr);
+      pool.kept_bytes += n;
+      return;
+    }
+  }
+  cudaFreeHost(ptr);
 }
 
 b200_error* b200_buffer_to_host(b200_buffer* b, void* dst, size_t* dst_size, b200_event** event) {
