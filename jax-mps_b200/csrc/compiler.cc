@@ -3692,7 +3692,7 @@ struct Planner {
         p.tma_ow = (int)OW; p.tma_oh = (int)OH; p.tma_box_h = (int)box_h; p.tma_box_n = (int)box_n;
         p.tma_kw = (int)KW; p.tma_pad_h = (int)pad[0]; p.tma_pad_w = (int)pad[2];
         p.tma_rdil_h = (int)rdil[0]; p.tma_rdil_w = (int)rdil[1];
-        if (!getenv("B200_NO_TILE32")) {
+        if (opts.tensor_cores && !getenv("B200_NO_TILE32")) {
           Tile32Launch& t = p.tile;
           t.mode = 1;
           t.M = p.M; t.N = p.N; t.K = p.K;
@@ -3829,7 +3829,7 @@ struct Planner {
         double us_tile = 1e30;
         // Below a tile of rows or four k-tiles the FMA pipe stays: a recurrent cell's 64 rows are a chain of launches, and the
         // split of B is one more of them (scan of 100 steps: 6890 us, 7940 with its products by tiled copies).
-        if (g.a_vec && g.M >= 128 && g.K >= 128 && !getenv("B200_NO_TILE32")) {
+        if (g.a_vec && g.M >= 128 && g.K >= 128 && opts.tensor_cores && !getenv("B200_NO_TILE32")) {
           t.mode = g.a_kc ? 2 : 3;
           const long long inner = g.a_kc ? g.K : g.M, outer = g.a_kc ? g.M : g.K;
           t.dims[0] = inner; t.dims[1] = outer; t.dims[2] = g.G; t.dims[3] = 1;

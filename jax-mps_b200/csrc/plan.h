@@ -139,6 +139,7 @@ struct CompiledProgram {
 
 struct CompileOptions {
   bool fuse = true;                   // B200_NO_FUSE=1 turns fusion off (one kernel per op)
+  bool tensor_cores = true;           // B200_NO_TENSOR_CORES=1: fp32 contractions stay on the FMA pipe
   int num_partitions = 1;
   int partition_id = 0;               // this process's partition (stablehlo.partition_id)
 };

@@ -211,6 +211,11 @@ NcclApi& nccl() {
   return api;
 }
 
+bool tensor_cores_allowed() {
+  const char* e = getenv("B200_NO_TENSOR_CORES");
+  return !e || atoi(e) == 0;
+}
+
 size_t dtype_size(b200_dtype d) {
   switch (d) {
     case B200_PRED: case B200_S8: case B200_U8: return 1;
@@ -1846,7 +1851,7 @@ b200_error* create_client(const b200_client_options* o, ncclComm_t given_comm, b
   CUDA_TRY(cudaMallocHost((void**)&c->status_block, sizeof(int) * b200_client::kStatusWords));
   memset(c->status_block, 0, sizeof(int) * b200_client::kStatusWords);
   for (int k = b200_client::kStatusWords - 1; k >= 0; k--) c->free_status.push_back(k);
-  if (const char* e2 = getenv("B200_NO_TENSOR_CORES")) c->tensor_cores = atoi(e2) == 0;
+  c->tensor_cores = tensor_cores_allowed();
   c->sw.no_vec_gather = getenv("B200_NO_VEC_GATHER") != nullptr;
   c->sw.no_seg_gather = getenv("B200_NO_SEG_GATHER") != nullptr;
   c->sw.no_tmem_a = getenv("B200_NO_TMEM_A") != nullptr;
@@ -2013,6 +2018,7 @@ b200_error* b200_client_compile(b200_client* c, const char* code, size_t code_si
   if (auto* e = set_device(c)) return e;
   CompileOptions co;
   co.fuse = !(o && o->disable_fusion) && !(getenv("B200_NO_FUSE") && atoi(getenv("B200_NO_FUSE")));
+  co.tensor_cores = c->tensor_cores;
   co.partition_id = c->rank;
   co.num_partitions = c->nprocs;
   char key[64];
@@ -2107,6 +2113,7 @@ b200_error* b200_compile_to_plan(const char* code, size_t code_size, const b200_
   if (cuda_source) *cuda_source = nullptr;
   CompileOptions co;
   co.fuse = !(o && o->disable_fusion) && !(getenv("B200_NO_FUSE") && atoi(getenv("B200_NO_FUSE")));
+  co.tensor_cores = tensor_cores_allowed();
   co.num_partitions = num_processes > 0 ? num_processes : 1;
   co.partition_id = process_index;
   std::unique_ptr<CompiledProgram> prog;

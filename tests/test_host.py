@@ -464,3 +464,21 @@ def test_all_gather_plans_and_oracle():
     x = b.arg((6, 5), "f32")
     one = b.module([b.all_gather(x, 1, 1)])
     np.testing.assert_array_equal(interp.run_text(one, [shards[0]])[0], shards[0])
+
+
+@pytest.mark.parametrize("what", ["product", "convolution"])
+def test_no_tensor_cores_keeps_fp32_contractions_off_them(monkeypatch, what):
+    """B200_NO_TENSOR_CORES=1: no fp32 contraction by tiled copies, which have no other form (the table-driven ones choose theirs
+    at launch)."""
+    b = Builder()
+    if what == "product":
+        x, w = b.arg((4096, 1024), "f32"), b.arg((1024, 1024), "f32")
+        text = b.module([b.matmul(x, w)])
+    else:
+        text = programs.resnet18_train_step(batch=8, image=32, width=64).text
+    assert " tile mode=" in b200.compile_to_plan(text)[0]
+    monkeypatch.setenv("B200_NO_TENSOR_CORES", "0")
+    assert " tile mode=" in b200.compile_to_plan(text)[0]
+    monkeypatch.setenv("B200_NO_TENSOR_CORES", "1")
+    plan = b200.compile_to_plan(text)[0]
+    assert " tile mode=" not in plan and "split_b" not in plan.lower()
