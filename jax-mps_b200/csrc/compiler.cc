@@ -5620,10 +5620,15 @@ struct Planner {
   int partition_id = 0;
 
   // ---- arena layout ---------------------------------------------------------------
-  // Memory goes to another temporary only so many steps after its last use: recordings run steps side by side that do not
-  // depend on one another, and steps that share memory do.
+  // In a plan that is recorded, memory goes to another temporary only so many steps after its last use: recordings run steps
+  // side by side that do not depend on one another, and steps that share memory do. Not the memory of a temporary above
+  // kReuseAtOnce: a step that writes one keeps the whole chip busy for microseconds and gains nothing from its neighbours.
+  // Measured, arena and step with no distance / this rule / the distance for all: masked-LM bf16 2090 MB 4698 us / 2097 MB
+  // 4571 us / 2644 MB 4515 us; ResNet18 of 128 744 MB 4044 us / 802 MB 3963 us / 878 MB 3958 us, of 20 157 MB 1522 us /
+  // 198 MB 1354 us / 208 MB 1379 us; masked-LM f32 of 462 rows 160 MB 1679 us / 177 MB 1410 us / 239 MB 1430 us.
   static constexpr int kReuseDistance = 8;
-  void layout_arena(Plan& plan) {
+  static constexpr size_t kReuseAtOnce = 8 << 20;
+  void layout_arena(Plan& plan, bool recorded) {
     const int arena = plan.arena;
     // liveness over the step sequence of this plan
     size_t S = plan.steps.size();
@@ -5666,7 +5671,7 @@ struct Planner {
     for (int ps : whole_plan)
       if (live.count(ps)) live[ps] = {0, (int)S};
     for (auto& sub_steps : plan.steps)
-      for (auto& sp : sub_steps.sub) layout_arena(*sp);
+      for (auto& sp : sub_steps.sub) layout_arena(*sp, !recorded && sub_steps.kind == Step::WHILE && sub_steps.trip_count >= 4 && &sp == &sub_steps.sub[1] && graph_safe(*sp));
     // The operands of a run of all-reduces (the gradient leaves of a data-parallel step) are laid out back to back,
     // inputs in one block and outputs in another, so that the runtime can reduce the whole run with one call over
     // one flat buffer instead of one operation per leaf. A pack is placed as a single block that lives from the
@@ -5720,7 +5725,7 @@ struct Planner {
         for (int m : pk->second) need += (prog.slots[m].bytes + 255) & ~(size_t)255;
       }
       // drop blocks that ended before `first`
-      active.erase(std::remove_if(active.begin(), active.end(), [&](const Blk& b) { return b.last + kReuseDistance < first; }), active.end());
+      active.erase(std::remove_if(active.begin(), active.end(), [&](const Blk& b) { return b.last + (recorded && b.size <= kReuseAtOnce ? kReuseDistance : 0) < first; }), active.end());
       std::sort(active.begin(), active.end(), [](const Blk& a, const Blk& b) { return a.off < b.off; });
       size_t off = 0;
       for (auto& b : active) {
@@ -5802,6 +5807,24 @@ uint64_t fnv1a(const std::string& s) {
 
 }  // namespace
 
+bool graph_safe_step(const Step& s) {
+  switch (s.kind) {
+    case Step::KERNEL: case Step::IGEMM: case Step::MEMCPY: case Step::GEMM16: case Step::REPACK16: case Step::TRANSPOSE: case Step::SPLIT_B: return true;
+    case Step::WHILE: return s.trip_count >= 0 && graph_safe(*s.sub[1]);
+    default: return false;
+  }
+}
+bool graph_safe(const Plan& plan) {
+  for (const Step& s : plan.steps)
+    if (!graph_safe_step(s)) return false;
+  return true;
+}
+bool recorded_whole(const Plan& main) {
+  for (const Step& s : main.steps)
+    if (s.kind == Step::WHILE || !(graph_safe_step(s) || s.kind == Step::SCATTER)) return false;
+  return (int)main.steps.size() >= kReplayLaunches;
+}
+
 std::unique_ptr<CompiledProgram> compile_module(Module& m, const CompileOptions& opts) {
   auto prog = std::make_unique<CompiledProgram>();
   prog->name = m.name.empty() ? "main" : m.name;
@@ -5870,7 +5893,7 @@ std::unique_ptr<CompiledProgram> compile_module(Module& m, const CompileOptions&
     }
     prog->results.push_back(ri);
   }
-  pl.layout_arena(prog->main);
+  pl.layout_arena(prog->main, recorded_whole(prog->main));
   // kernels that ended up inside bundles only are not compiled on their own
   {
     std::set<int> used;

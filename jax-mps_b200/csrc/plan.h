@@ -107,6 +107,14 @@ struct Plan {
   int arena = 0;                      // arena holding this plan's temporaries
 };
 
+// A plan can be recorded into a CUDA graph when it only launches kernels and device copies: no host round trip
+// (data-dependent loops, case), no collective. The main plan is recorded as a whole when it has no loop either (counted
+// loops have recordings of their own) and at least kReplayLaunches steps.
+constexpr int kReplayLaunches = 6;
+bool graph_safe_step(const Step& s);
+bool graph_safe(const Plan& plan);
+bool recorded_whole(const Plan& main);
+
 struct KernelSource {
   std::string name;
   std::string body;                   // full __global__ definition

@@ -737,22 +737,6 @@ bool waits_inside(const Plan& plan) {
   return false;
 }
 
-// A plan can be recorded into a CUDA graph when it only launches kernels and device copies: no host round trip
-// (data-dependent loops, case), no collective.
-bool graph_safe(const Plan& plan);
-bool graph_safe_step(const Step& s) {
-  switch (s.kind) {
-    case Step::KERNEL: case Step::IGEMM: case Step::MEMCPY: case Step::GEMM16: case Step::REPACK16: case Step::TRANSPOSE: case Step::SPLIT_B: return true;
-    case Step::WHILE: return s.trip_count >= 0 && graph_safe(*s.sub[1]);
-    default: return false;
-  }
-}
-bool graph_safe(const Plan& plan) {
-  for (const Step& s : plan.steps)
-    if (!graph_safe_step(s)) return false;
-  return true;
-}
-
 // Addresses of every slot a step and the plans below it refer to, in a fixed order.
 void touched_addresses(const ExecCtx& x, const Step& s, std::vector<void*>& out, bool top = true) {
   for (int a : s.args) out.push_back(x.ptrs[a]);
@@ -1745,8 +1729,6 @@ b200_error* run_plan(ExecCtx& x, const Plan& plan) {
 // few, and a node that is given other addresses less than one. The first call runs step by step, which loads and configures
 // every kernel, and records behind that (capture takes 7 us a launch, instantiation another 3 to 14 ms for plans of 250 to
 // 420 launches; loading took 20 to 30 ms); all later calls replay, whichever buffers they are given.
-constexpr int kReplayLaunches = 6;
-
 b200_error* run_main(ExecCtx& x) {
   LoadedProgram& lp = *x.lp;
   b200_client* c = x.c;
@@ -2063,8 +2045,7 @@ b200_error* b200_client_compile(b200_client* c, const char* code, size_t code_si
     }
     if (auto* e = build_kernels(*lp)) return e;
     lp->watched = waits_inside(lp->prog->main);
-    lp->replayable = (int)lp->prog->main.steps.size() >= kReplayLaunches;
-    for (const Step& st : lp->prog->main.steps) lp->replayable = lp->replayable && st.kind != Step::WHILE && (graph_safe_step(st) || st.kind == Step::SCATTER);
+    lp->replayable = recorded_whole(lp->prog->main);
     // constants: one device block, uploaded once
     CompiledProgram& p = *lp->prog;
     size_t total = 0;

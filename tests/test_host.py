@@ -482,3 +482,21 @@ def test_no_tensor_cores_keeps_fp32_contractions_off_them(monkeypatch, what):
     monkeypatch.setenv("B200_NO_TENSOR_CORES", "1")
     plan = b200.compile_to_plan(text)[0]
     assert " tile mode=" not in plan and "split_b" not in plan.lower()
+
+
+@pytest.mark.parametrize("n,tail,blocks", [(256, "recorded", (8, 13)), (256, "loop", (2, 4)), (256, "few", (1, 3)), (2304, "recorded", (2, 4))])
+def test_temporaries_are_kept_apart_only_for_recordings(n, tail, blocks):
+    """A chain of bf16 products needs two temporaries at a time. Plans that are recorded keep small ones apart for eight steps more;
+    plans that cannot be (a data-dependent loop, too few steps) and temporaries above 8 MB do not pay for that."""
+    b = Builder()
+    x, w = b.arg((n, n), "bf16"), b.arg((n, n), "bf16")
+    y = x
+    for _ in range(3 if tail == "few" else 14):
+        y = b.matmul(y, w)
+    outs = [y]
+    if tail == "loop":
+        lim = b.arg((), "f32")
+        outs.append(b.while_([b.full((), 1.0, "f32")], lambda s, v: s.compare(v, lim, "LT"), lambda s, v: [s.add(v, v)])[0])
+    plan = b200.compile_to_plan(b.module(outs))[0]
+    arena = int(re.search(r"arena0 (\d+) bytes", plan).group(1))
+    assert blocks[0] <= arena / (2 * n * n) <= blocks[1], plan[:400]
