@@ -1956,7 +1956,11 @@ struct Planner {
   // with any riders; the merge sort below takes every other comparator. 16 rows of 30522 keys with positions: 114 us as
   // a merge sort, 73 us here; 32 rows of 64000: 377 and 173; 8 rows of 4000: 45 and 28. (One row of 8000 is 57 us both
   // ways, which is where the rule in lower_sort draws the line.)
+  // A tile reads the counts of every tile of its row, which grows with the square of the row: from 2^23 elements on that is
+  // what a pass spends its time on, and the merge sort takes over. One row, radix / merge, us: 2^18 74 / 104, 2^20 168 / 334,
+  // 2^22 1044 / 1358, 2^23 3059 / 3111, 2^24 13418 / 6888; 4 rows of 2^22 3933 / 5846.
   static constexpr int kRadixTile = 4096;
+  static constexpr int64_t kRadixRowMax = 1 << 22;
   bool lower_radix_sort(Op* op, size_t key, bool descending, int64_t rows, int64_t N, Plan& plan, BlockState& st) {
     std::vector<Value*> ins(op->operands.begin(), op->operands.end()), outs(op->results.begin(), op->results.end());
     const int64_t tiles = (N + kRadixTile - 1) / kRadixTile, numel = rows * N;
@@ -2327,7 +2331,7 @@ struct Planner {
     if (rows * tiles >= (1LL << 31)) throw CompileError("stablehlo.sort: too many rows");
     const bool one_tile = tiles == 1;
 
-    if (inner == 1 && N >= 128 && (N <= kRadixTile || N * rows >= 16384)) {
+    if (inner == 1 && N >= 128 && N <= kRadixRowMax && (N <= kRadixTile || N * rows >= 16384)) {
       size_t key = 0;
       bool descending = false;
       if (radix_order(op, key, descending) && lower_radix_sort(op, key, descending, rows, N, plan, st)) return;

@@ -54,3 +54,15 @@ def test_top_k_of_equal_values_keeps_positions(client, fill):
     b = Builder()
     got, _ = run_gpu(client, b.module(b.top_k(b.arg(x.shape, "f32"), 9)), [x])
     np.testing.assert_array_equal(got[1], np.tile(np.arange(9, dtype=np.int32), (2, 1)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1 << 22, (1 << 22) + 1])
+def test_sort_at_the_longest_radix_row(client, n):
+    x = np.random.default_rng(n).integers(-1000, 1000, (1, n)).astype(np.int32)
+    b = Builder()
+    text = b.module(b.sort([b.arg(x.shape, "i32"), b.iota(x.shape, "i32", 1)], 1, comparator=lambda s, a0, b0, a1, b1: s.compare(a0, b0, "LT")))
+    got, _ = run_gpu(client, text, [x])
+    order = np.argsort(x, axis=1, kind="stable").astype(np.int32)
+    np.testing.assert_array_equal(got[1], order)
+    np.testing.assert_array_equal(got[0], np.take_along_axis(x, order, 1))

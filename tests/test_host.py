@@ -500,3 +500,11 @@ def test_temporaries_are_kept_apart_only_for_recordings(n, tail, blocks):
     plan = b200.compile_to_plan(b.module(outs))[0]
     arena = int(re.search(r"arena0 (\d+) bytes", plan).group(1))
     assert blocks[0] <= arena / (2 * n * n) <= blocks[1], plan[:400]
+
+
+@pytest.mark.parametrize("rows,n,radix", [(1, 1 << 22, True), (1, (1 << 22) + 1, False), (3, 1 << 23, False), (2, 5000, False), (4, 5000, True)])
+def test_radix_sort_is_for_bounded_rows(rows, n, radix):
+    b = Builder()
+    x = b.arg((rows, n), "f32")
+    plan = b200.compile_to_plan(b.module(b.sort([x], 1, comparator=lambda s, a0, b0: s.compare(a0, b0, "LT", "TOTALORDER"))))[0]
+    assert ("sort (radix pass" in plan) == radix, plan
