@@ -130,7 +130,12 @@ bool dot16_geometry(Op* op, Dot16& d) {
 int top_k_threads(int64_t n) { return n >= 8192 ? 1024 : n >= 2048 ? 512 : 256; }
 bool few_of_many(const TensorType& t, int64_t k) {
   const int64_t n = t.dims.empty() ? 0 : t.dims.back();
-  return n >= 512 && n < (1LL << 30) && k >= 1 && k <= top_k_threads(n) / 2 && dt_size(t.dt) <= 4 && t.numel() > 0;
+  if (n < 512 || n >= (1LL << 30) || k < 1 || k > top_k_threads(n) / 2 || dt_size(t.dt) > 4 || t.numel() <= 0) return false;
+  // One block reads a row, up to 34 times where many elements share the largest keys, while a sort of the row has the whole
+  // chip. Keys in no order / all equal / sorted, us: 1 x 2^16 20 / 163 / 49, 1 x 2^18 47 / 586 / 64, 1 x 2^20 137 / 2218 / 163,
+  // 16 x 2^18 43 / 578 / 331, 16 x 2^20 150 / 2348 / 1718. So few rows up to where the gain on ordinary keys ends, and from 16
+  // on, which a sort takes one after the other, rows of any length.
+  return n <= (1LL << 18) || t.numel() / n >= 16;
 }
 
 // ---------------------------------------------------------------------------

@@ -66,3 +66,14 @@ def test_sort_at_the_longest_radix_row(client, n):
     order = np.argsort(x, axis=1, kind="stable").astype(np.int32)
     np.testing.assert_array_equal(got[1], order)
     np.testing.assert_array_equal(got[0], np.take_along_axis(x, order, 1))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1 << 18, (1 << 18) + 1])
+def test_top_k_at_the_longest_row_of_a_block(client, n):
+    x = np.random.default_rng(n).integers(-1000, 1000, (1, n)).astype(np.float32)
+    b = Builder()
+    got, _ = run_gpu(client, b.module(b.top_k(b.arg(x.shape, "f32"), 200)), [x])
+    order = np.argsort(-x, axis=1, kind="stable")[:, :200].astype(np.int32)
+    np.testing.assert_array_equal(got[1], order)
+    np.testing.assert_array_equal(got[0], np.take_along_axis(x, order, 1))

@@ -508,3 +508,10 @@ def test_radix_sort_is_for_bounded_rows(rows, n, radix):
     x = b.arg((rows, n), "f32")
     plan = b200.compile_to_plan(b.module(b.sort([x], 1, comparator=lambda s, a0, b0: s.compare(a0, b0, "LT", "TOTALORDER"))))[0]
     assert ("sort (radix pass" in plan) == radix, plan
+
+
+@pytest.mark.parametrize("rows,n,one_block", [(1, 1 << 18, True), (1, (1 << 18) + 1, False), (15, 1 << 20, False), (16, 1 << 20, True), (16, 511, False)])
+def test_selecting_top_k_is_for_bounded_rows(rows, n, one_block):
+    b = Builder()
+    plan = b200.compile_to_plan(b.module(b.top_k(b.arg((rows, n), "f32"), 50)))[0]
+    assert (" top_k" in plan and "sort" not in plan) == one_block, plan
