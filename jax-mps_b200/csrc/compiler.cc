@@ -3468,21 +3468,28 @@ struct Planner {
     return s;
   }
 
-  // Split the contraction over blockIdx.z when the output has too few tiles to fill the GPU. A small cost model
-  // (measured on the ResNet layer shapes: about 0.6 us per 128 x 64 x 32 k-tile, 0.9 us per 128 x 128 x 32 one,
-  // 6 us of fixed cost per wave of CTAs, partial sums written and re-read at about 3 TB/s) picks the split
-  // that minimises waves * time per CTA + reduction time.
-  // Returns the modelled time in microseconds.
-  static double choose_split_k(IGemmParams& p) {
+  // Modelled time in microseconds of a contraction by tables, split `split` ways along K: waves * time per CTA + reduction time,
+  // with (measured on the ResNet layer shapes) about 0.6 us per 128 x 64 x 32 k-tile, 0.9 us per 128 x 128 x 32 one, 6 us of
+  // fixed cost per wave of CTAs, partial sums written and re-read at about 3 TB/s. `copies`: of that many side by side.
+  struct TableShape { long long tiles, ktiles, per_wave; double tile_us; };
+  static TableShape table_shape(const IGemmParams& p) {
     const int bn = p.N >= 128 ? 128 : 64;
-    const long long tiles = (long long)((p.M + 127) / 128) * ((p.N + bn - 1) / bn) * p.groups;
-    const long long ktiles = (p.K + 31) / 32;
     // the scalar-gather kernel (operands without 16-byte structure) spends about 10 us per k-tile and runs two
     // CTAs per SM; the row-gather kernels one CTA per SM
     // 64-wide row-gather tiles run as two half-size CTAs per SM (about 1 us per k-tile each, two at a time)
     const bool half = p.vec && p.seg && bn == 64;
-    const double tile_us = !p.vec ? 10.0 : (bn == 128 ? 0.9 : (half ? 1.0 : 0.6));
-    const long long per_wave = (!p.vec || half) ? 296 : 148;
+    return {(long long)((p.M + 127) / 128) * ((p.N + bn - 1) / bn) * p.groups, (p.K + 31) / 32, (!p.vec || half) ? 296 : 148,
+            !p.vec ? 10.0 : (bn == 128 ? 0.9 : (half ? 1.0 : 0.6))};
+  }
+  static double table_time(const IGemmParams& p, int split, int copies = 1) {
+    const TableShape s = table_shape(p);
+    const long long waves = (copies * s.tiles * split + s.per_wave - 1) / s.per_wave;
+    const double us = (double)waves * ((double)((s.ktiles + split - 1) / split) * s.tile_us + 6.0);
+    return split > 1 ? us + 3.0 + 2.0 * copies * split * (double)p.M * p.N * p.groups * 4.0 / 3e6 : us;
+  }
+  // Splits the contraction over blockIdx.z when the output has too few tiles to fill the GPU. Returns its modelled time.
+  static double choose_split_k(IGemmParams& p) {
+    const auto [tiles, ktiles, per_wave, tile_us] = table_shape(p);
     int best = 1;
     double best_cost = 1e30;
     // a split keeps at least 8 k-tiles, except when the output has so few tiles that even then most of the GPU
@@ -3490,26 +3497,32 @@ struct Planner {
     const long long min_kt = tiles * 8 <= per_wave ? 2 : 8;
     const int max_split = (int)std::min<long long>(592, std::max<long long>(1, ktiles / min_kt));
     for (int split = 1; split <= max_split; split++) {
-      const long long waves = (tiles * split + per_wave - 1) / per_wave;
-      const long long kt = (ktiles + split - 1) / split;
-      double cost = (double)waves * ((double)kt * tile_us + 6.0);
-      if (split > 1) cost += 3.0 + 2.0 * split * (double)p.M * p.N * p.groups * 4.0 / 3e6;
+      const double cost = table_time(p, split);
       if (cost < best_cost * 0.97) { best_cost = cost; best = split; }
     }
     p.split_k = best;
     return best_cost;
   }
 
-  // Tile width and K split of a contraction by tiled copies (tile32.cu), and its modelled time in microseconds. Cycles: 300 per
-  // 64-wide and 500 per 128-wide k-tile, 500 per tile of C, 2000 to launch, fill and drain; a split adds the pass that sums it.
-  // A k-tile really takes 830 and 960, but the table-driven kernels take as much longer than choose_split_k says, and the two are
-  // compared; the constants are those at which encoder steps of 150 to 2048 rows and classifier steps ran fastest (462 rows:
-  // 1540 us without tiled copies, 1400 now).
+  // The three models of an fp32 product's time (this one, fma_product, choose_split_k) are compared with one another, so each
+  // gives microseconds as measured: of a product in a chain of products that is replayed as a graph, with weights as the other
+  // operand. Over 141 such chains from 32 x 64 x 512 to 4096 x 2048 x 2048 the root of the mean squared relative error is 4 %
+  // for the tiled copies, 8 % for the FMA pipe and 8 % for the tables, and the way that is taken is 0.8 % slower than the
+  // fastest of the three on average, 14 % at most. (M x K x N, FMA / tables / tiles, us: 250 x 128 x 512 6.2 / 12.3 / 10.2,
+  // 1024 x 128 x 512 8.0 / 12.4 / 10.4, 462 x 512 x 512 12.4 / 13.9 / 12.4, 250 x 2048 x 2048 76 / 26 / 34,
+  // 462 x 768 x 3072 74 / 30 / 31, 2048 x 1024 x 1024 127 / 37 / 33, 4096 x 768 x 3072 455 / 156 / 109.)
+  // Products that become ready together (the two gradients of a product, the projections of an input) are recorded side by side
+  // and share the SMs; `copies` is then 2, and the shortest time is that of two of them together. f32 encoder steps with every
+  // product modelled alone / as one of two, us: 462 rows 1463 / 1400, 256 rows 1126 / 1102, 462 rows of 256 1019 / 900, 400 rows
+  // of 768 1853 / 1772. A loop body is the other way about, its iterations are one chain: 6900 / 7330 us for a scan of 100 steps.
+  //
+  // Tile width and K split of a contraction by tiled copies (tile32.cu), and its time: 0.42 us per 64-wide and 0.64 per 128-wide
+  // k-tile, 6.9 to launch, fill and drain, 1.9 and the partial sums at 6 TB/s for a split, the image of B at 4.4 TB/s.
   // `b_is_weight`: B is a program input, whose split image is made beside what is in front of the product. The tensor core
   // truncates its sums, so an error grows with the k-tiles one accumulator takes in (36 of them 8e-6, 12 of them 3e-6): a
   // product is split at least as finely as the table-driven kernels would (`split_k`), a convolution exactly so, which gives
   // the same bits.
-  static double tile_product(Tile32Launch& t, bool b_is_weight, int split_k) {
+  static double tile_product(Tile32Launch& t, bool b_is_weight, int split_k, int copies = 1) {
     const long long ktiles = (t.K + 31) / 32, tm = (t.M + 127) / 128, longest = (ktiles + split_k - 1) / split_k;
     double best = 1e30;
     for (int bn : {128, 64}) {
@@ -3519,22 +3532,18 @@ struct Planner {
         const long long kps = (ktiles + want - 1) / want, split = (ktiles + kps - 1) / kps;
         if (split != want || kps > longest || (t.mode == 1 && kps != longest)) continue;
         if (split > 1 && kps < longest && (tiles * split > 2 * 148 || split * t.G * t.M * t.N > (64LL << 20))) break;
-        double cycles = (double)((tiles * split + 147) / 148) * ((double)kps * (bn == 64 ? 300.0 : 500.0) + 500.0) + 2000.0;
-        if (split > 1) cycles += 2000.0 + (double)split * t.G * t.M * t.N * 8.0 / 3000.0;
-        if (cycles < best * 0.98) { best = cycles; t.bn = bn; t.split = (int)split; }
+        double us = (double)((copies * tiles * split + 147) / 148) * (double)kps * (bn == 64 ? 0.415 : 0.637) + 6.9;
+        if (split > 1) us += 1.9 + (double)copies * split * t.G * t.M * t.N * 8.0 / 6.05e6;
+        if (us < best * 0.98) { best = us; t.bn = bn; t.split = (int)split; }
       }
     }
-    const double image = (double)t.G * t.K * t.N * 12.0;
-    return best / 1850.0 + (b_is_weight ? 0.3 : 2.0 + image / 5e6);
+    return best + (double)copies * t.G * t.K * t.N * 12.0 / 4.4e6 + (b_is_weight ? 0.0 : 2.0);
   }
 
-  // Modelled time of a dense fp32 product on the FMA pipe (gemm32.cu), with its tile and split. Cycles of an SM, fitted to
-  // products from 64 x 64 x 64 to 512 x 8003 x 462: 1.7 per row of four warps' FMA
-  // instructions and k when a CTA is alone on its SM (one warp per scheduler) and 1.25 when others fill its stalls, 1500
-  // (900) to fill and drain a CTA, 2500 for the launch, 700 for the sum of warps, 1000 for that of a
-  // cluster. The lines against choose_split_k's model: 462 x 512 x 512 is 7 us here and 19 there, 462 x 2048 x 512 about
-  // 27 both ways, 4096 x 1000 x 784 stays on the tensor cores.
-  static double fma_product(Gemm32Launch& g) {
+  // Modelled time of a dense fp32 product on the FMA pipe (gemm32.cu), with its tile and split: 1.3 ns per row of four warps'
+  // FMA instructions and k when a CTA is alone on its SM (one warp per scheduler) and 0.92 when others fill its stalls, 1.6 us to
+  // launch, fill and drain, 2.2 for every further CTA of an SM, 2.1 for the sum of a cluster.
+  static double fma_product(Gemm32Launch& g, int copies) {
     if (g.G > 65535 || getenv("B200_NO_GEMM32")) return 1e30;
     double best = 1e30;
     for (int tile = 2; tile >= 0; tile--) {
@@ -3542,25 +3551,37 @@ struct Planner {
       const long long tiles = (long long)((g.M + tm - 1) / tm) * ((g.N + tn - 1) / tn) * g.G;
       for (int split = 1; split <= 4; split *= 2) {
         if (split > 1 && g.K < 32 * split) break;
-        const long long per_sm = tiles * split <= gemm32_resident(split) ? 1 : (tiles * split + 147) / 148;
+        const long long per_sm = copies * tiles * split <= gemm32_resident(split) ? 1 : (copies * tiles * split + 147) / 148;
         const long long chunk = ((g.K + split - 1) / split + 3) / 4 * 4;
-        const double row = per_sm == 1 ? 1.7 : 1.25, edge = per_sm == 1 ? 1500.0 : 900.0;
-        const double us = ((double)per_sm * (tm * tn / 128 * row * (double)chunk + edge) + 2500.0 + (split > 1 || tile < 2 ? 700.0 : 0.0) +
-                           (split > 1 ? 1000.0 : 0.0)) / 1850.0;
+        const double us = (double)per_sm * (tm * tn / 128) * (double)chunk * (per_sm == 1 ? 1.3e-3 : 0.92e-3) + 1.6 + 2.2 * (double)(per_sm - 1) +
+                          (split > 1 ? 2.1 : 0.0);
         if (us < best * 0.97) { best = us; g.split = split; g.tile = tile; }
       }
     }
     return best;
   }
   // ... and in the table-driven kernels (choose_split_k).
-  static double table_product(const Gemm32Launch& g, int& split_k) {
+  static double table_product(const Gemm32Launch& g, int& split_k, int copies) {
     IGemmParams t;
     t.M = g.M; t.N = g.N; t.K = g.K; t.groups = g.G;
     t.vec = g.a_vec && g.b_vec;
     t.seg = t.vec && g.K % 32 == 0 && (g.a_kc || g.M % 32 == 0) && (g.b_kc || g.N % 32 == 0);
-    const double us = choose_split_k(t);
+    choose_split_k(t);
     split_k = t.split_k;
-    return us;
+    return table_time(t, split_k, copies);
+  }
+
+  // Whether a product of the main plan has an operand, other than a program input, in common with another contraction.
+  static bool shares_operand(Op* op, BlockState& st) {
+    if (st.block->parent_op) return false;
+    for (Value* v : op->operands) {
+      if (!v->def) continue;
+      auto it = st.users.find(v);
+      if (it == st.users.end()) continue;
+      for (Op* u : it->second)
+        if (u != op && (u->short_name() == "dot_general" || u->short_name() == "convolution")) return true;
+    }
+    return false;
   }
 
   std::vector<Step> before_product;          // steps that go in front of the product being lowered
@@ -3834,11 +3855,15 @@ struct Planner {
         Tile32Launch t;
         t.M = g.M; t.N = g.N; t.K = g.K; t.G = g.G;
         int split_k = 1;
-        const double us_fma = fma_product(g), us_table = table_product(g, split_k);
-        double us_tile = 1e30;
-        // Below a tile of rows or four k-tiles the FMA pipe stays: a recurrent cell's 64 rows are a chain of launches, and the
-        // split of B is one more of them (scan of 100 steps: 6890 us, 7940 with its products by tiled copies).
-        if (g.a_vec && g.M >= 128 && g.K >= 128 && opts.tensor_cores && !getenv("B200_NO_TILE32")) {
+        const int copies = shares_operand(op, st) ? 2 : 1;
+        const double us_fma = fma_product(g, copies);
+        double us_table = table_product(g, split_k, copies), us_tile = 1e30;
+        // the switches that keep products off the tensor cores or tiled copies leave them to the FMA pipe
+        const bool tiles = opts.tensor_cores && !getenv("B200_NO_TILE32");
+        if (!tiles) us_table = 1e30;
+        // Below a tile of rows or four k-tiles tiled copies are never the fastest (M x K x N, FMA / tables / tiles, us:
+        // 96 x 512 x 2048 14.6 / 13.8 / 14.3, 96 x 2048 x 2048 33 / 19 / 29, 2048 x 64 x 512 8.5 / 10.8 / 9.9).
+        if (g.a_vec && g.M >= 128 && g.K >= 128 && tiles) {
           t.mode = g.a_kc ? 2 : 3;
           const long long inner = g.a_kc ? g.K : g.M, outer = g.a_kc ? g.M : g.K;
           t.dims[0] = inner; t.dims[1] = outer; t.dims[2] = g.G; t.dims[3] = 1;
@@ -3846,7 +3871,7 @@ struct Planner {
           t.strides[1] = g.G > 1 ? g.a_gs : t.strides[0] * outer;
           t.strides[2] = t.strides[1] * g.G;
           t.box[0] = 32; t.box[1] = g.a_kc ? 128 : 32; t.box[2] = t.box[3] = 1;
-          us_tile = tile_product(t, !rhs->def && rhs->owner && rhs->owner->parent_op == nullptr, split_k);
+          us_tile = tile_product(t, !rhs->def && rhs->owner && rhs->owner->parent_op == nullptr, split_k, copies);
         }
         if (us_tile < us_fma && us_tile < us_table) p.tile = t;
         else if (us_fma < us_table) {

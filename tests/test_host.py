@@ -515,3 +515,26 @@ def test_selecting_top_k_is_for_bounded_rows(rows, n, one_block):
     b = Builder()
     plan = b200.compile_to_plan(b.module(b.top_k(b.arg((rows, n), "f32"), 50)))[0]
     assert (" top_k" in plan and "sort" not in plan) == one_block, plan
+
+
+@pytest.mark.parametrize("m,k,n,way", [(250, 128, 512, "fma"), (1024, 128, 512, "fma"), (128, 512, 512, "fma"), (128, 2048, 2048, "table"),
+                                       (250, 2048, 2048, "table"), (250, 768, 3072, "table"), (2048, 1024, 1024, "tile"), (4096, 768, 3072, "tile"),
+                                       (1024, 512, 2048, "tile")])
+def test_products_take_the_way_that_measures_fastest(m, k, n, way):
+    """Shapes at which the three ways of an fp32 product are at least 10 % apart; the first six went the wrong way under
+    models that had been fitted to steps instead of products."""
+    b = Builder()
+    plan = b200.compile_to_plan(b.module([b.matmul(b.arg((m, k), "f32"), b.arg((k, n), "f32"))]))[0]
+    assert ("tile" if " tile mode=" in plan else "fma" if " fma tile=" in plan else "table") == way, plan[:300]
+
+
+def test_products_that_become_ready_together_share_the_chip():
+    """Two products of one intermediate value: the one that is quickest alone takes the whole chip for itself."""
+    def plan(shared):
+        b = Builder()
+        x = b.tanh(b.arg((462, 512), "f32"))
+        outs = [b.matmul(x, b.arg((512, 512), "f32"))]
+        if shared:
+            outs.append(b.matmul(x, b.arg((512, 512), "f32")))
+        return b200.compile_to_plan(b.module(outs))[0]
+    assert " fma tile=" in plan(False) and " tile mode=" in plan(True)
