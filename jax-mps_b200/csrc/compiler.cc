@@ -3470,7 +3470,7 @@ struct Planner {
 
   // Modelled time in microseconds of a contraction by tables, split `split` ways along K: waves * time per CTA + reduction time,
   // with (measured on the ResNet layer shapes) about 0.6 us per 128 x 64 x 32 k-tile, 0.9 us per 128 x 128 x 32 one, 6 us of
-  // fixed cost per wave of CTAs, partial sums written and re-read at about 3 TB/s. `copies`: of that many side by side.
+  // fixed cost per wave of CTAs, partial sums written and re-read at about 3 TB/s.
   struct TableShape { long long tiles, ktiles, per_wave; double tile_us; };
   static TableShape table_shape(const IGemmParams& p) {
     const int bn = p.N >= 128 ? 128 : 64;
@@ -3481,11 +3481,11 @@ struct Planner {
     return {(long long)((p.M + 127) / 128) * ((p.N + bn - 1) / bn) * p.groups, (p.K + 31) / 32, (!p.vec || half) ? 296 : 148,
             !p.vec ? 10.0 : (bn == 128 ? 0.9 : (half ? 1.0 : 0.6))};
   }
-  static double table_time(const IGemmParams& p, int split, int copies = 1) {
+  static double table_time(const IGemmParams& p, int split) {
     const TableShape s = table_shape(p);
-    const long long waves = (copies * s.tiles * split + s.per_wave - 1) / s.per_wave;
+    const long long waves = (s.tiles * split + s.per_wave - 1) / s.per_wave;
     const double us = (double)waves * ((double)((s.ktiles + split - 1) / split) * s.tile_us + 6.0);
-    return split > 1 ? us + 3.0 + 2.0 * copies * split * (double)p.M * p.N * p.groups * 4.0 / 3e6 : us;
+    return split > 1 ? us + 3.0 + 2.0 * split * (double)p.M * p.N * p.groups * 4.0 / 3e6 : us;
   }
   // Splits the contraction over blockIdx.z when the output has too few tiles to fill the GPU. Returns its modelled time.
   static double choose_split_k(IGemmParams& p) {
@@ -3504,11 +3504,10 @@ struct Planner {
     return best_cost;
   }
 
-  // The three models of an fp32 product's time (this one, fma_product, choose_split_k) are compared with one another, so each
+  // The three models of an fp32 product's time (this one, fma_product, table_product) are compared with one another, so each
   // gives microseconds as measured: of a product in a chain of products that is replayed as a graph, with weights as the other
   // operand. Over 141 such chains from 32 x 64 x 512 to 4096 x 2048 x 2048 the root of the mean squared relative error is 4 %
-  // for the tiled copies, 8 % for the FMA pipe and 8 % for the tables, and the way that is taken is 0.8 % slower than the
-  // fastest of the three on average, 14 % at most. (M x K x N, FMA / tables / tiles, us: 250 x 128 x 512 6.2 / 12.3 / 10.2,
+  // for the tiled copies, 8 % for the FMA pipe and 5 % for the tables. (M x K x N, FMA / tables / tiles, us: 250 x 128 x 512 6.2 / 12.3 / 10.2,
   // 1024 x 128 x 512 8.0 / 12.4 / 10.4, 462 x 512 x 512 12.4 / 13.9 / 12.4, 250 x 2048 x 2048 76 / 26 / 34,
   // 462 x 768 x 3072 74 / 30 / 31, 2048 x 1024 x 1024 127 / 37 / 33, 4096 x 768 x 3072 455 / 156 / 109.)
   // Products that become ready together (the two gradients of a product, the projections of an input) are recorded side by side
@@ -3540,9 +3539,10 @@ struct Planner {
     return best + (double)copies * t.G * t.K * t.N * 12.0 / 4.4e6 + (b_is_weight ? 0.0 : 2.0);
   }
 
-  // Modelled time of a dense fp32 product on the FMA pipe (gemm32.cu), with its tile and split: 1.3 ns per row of four warps'
-  // FMA instructions and k when a CTA is alone on its SM (one warp per scheduler) and 0.92 when others fill its stalls, 1.6 us to
-  // launch, fill and drain, 2.2 for every further CTA of an SM, 2.1 for the sum of a cluster.
+  // Modelled time of a dense fp32 product on the FMA pipe (gemm32.cu), with its tile and split: 1.02 ns per row of four warps'
+  // FMA instructions and k (6 % less in the widest tile, which reads shared memory least; 12 % more for a B whose k is contiguous
+  // while nothing else on the SM hides its transposition), 2.95 us to launch, fill and drain, 1.3 for every further CTA of an
+  // SM, 1.35 for the sum of a cluster. Every tile and split over 70 chains from 6 x 64 x 256 to 250 x 512 x 1024: 6 % rms error.
   static double fma_product(Gemm32Launch& g, int copies) {
     if (g.G > 65535 || getenv("B200_NO_GEMM32")) return 1e30;
     double best = 1e30;
@@ -3553,14 +3553,16 @@ struct Planner {
         if (split > 1 && g.K < 32 * split) break;
         const long long per_sm = copies * tiles * split <= gemm32_resident(split) ? 1 : (copies * tiles * split + 147) / 148;
         const long long chunk = ((g.K + split - 1) / split + 3) / 4 * 4;
-        const double us = (double)per_sm * (tm * tn / 128) * (double)chunk * (per_sm == 1 ? 1.3e-3 : 0.92e-3) + 1.6 + 2.2 * (double)(per_sm - 1) +
-                          (split > 1 ? 2.1 : 0.0);
+        const double row = 1.02e-3 * (tile == 2 ? 0.94 : 1.0) * (g.b_kc && per_sm == 1 ? 1.12 : 1.0);
+        const double us = (double)per_sm * (tm * tn / 128) * (double)chunk * row + 2.95 + 1.3 * (double)(per_sm - 1) + (split > 1 ? 1.35 : 0.0);
         if (us < best * 0.97) { best = us; g.split = split; g.tile = tile; }
       }
     }
     return best;
   }
-  // ... and in the table-driven kernels (choose_split_k).
+  // ... and in the table-driven kernels, split as choose_split_k would: its k-tiles, 8.5 us for the first wave of CTAs and 4.8
+  // for each further one, the partial sums at 3.3 TB/s (5 % rms error; the 6 us a wave of choose_split_k, which weighs splits
+  // against one another, are 2.5 short for the few k-tiles of small products).
   static double table_product(const Gemm32Launch& g, int& split_k, int copies) {
     IGemmParams t;
     t.M = g.M; t.N = g.N; t.K = g.K; t.groups = g.G;
@@ -3568,7 +3570,10 @@ struct Planner {
     t.seg = t.vec && g.K % 32 == 0 && (g.a_kc || g.M % 32 == 0) && (g.b_kc || g.N % 32 == 0);
     choose_split_k(t);
     split_k = t.split_k;
-    return table_time(t, split_k, copies);
+    const TableShape s = table_shape(t);
+    const long long waves = (copies * s.tiles * split_k + s.per_wave - 1) / s.per_wave;
+    return (double)waves * (double)((s.ktiles + split_k - 1) / split_k) * 0.95 * s.tile_us + 8.5 + 4.8 * (double)(waves - 1) +
+           (split_k > 1 ? (double)copies * split_k * t.M * t.N * t.groups * 8.0 / 3.3e6 : 0.0);
   }
 
   // Whether a product of the main plan has an operand, other than a program input, in common with another contraction.

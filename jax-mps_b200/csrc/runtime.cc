@@ -1087,6 +1087,7 @@ bool record_graph(ExecCtx& x, Recording& rec, F&& steps) {
     ok = !err && !recorder.failed() && x.ptrs == at_start;
   }
   if (ok) ok = (ce = cudaGraphInstantiate(&rec.exec, rec.graph, 0)) == cudaSuccess;
+  if (ok) ok = (ce = cudaGraphUpload(rec.exec, x.c->compute)) == cudaSuccess;      // here and not in its first launch
   rec.launches = x.launches - before;
   x.launches = before;
   x.ptrs = at_start;
