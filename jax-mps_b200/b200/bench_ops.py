@@ -207,14 +207,14 @@ def distilbert_step(client, reps=5, profile=False, verbose=False, **shape):
     return res
 
 
-def gemm(client, m, n, k, reps):
+def gemm(client, m, n, k, reps, dtype="bf16"):
     b = Builder()
-    x, w = b.arg((m, k), "bf16"), b.arg((k, n), "bf16")
+    x, w = b.arg((m, k), dtype), b.arg((k, n), dtype)
     text = b.module([b.matmul(x, w)])
     rng = np.random.default_rng(0)
     exe = client.compile(text)
-    bufs = [client.buffer_from_host(rng.standard_normal((m, k)).astype(np.float32), dtype="bf16"),
-            client.buffer_from_host(rng.standard_normal((k, n)).astype(np.float32), dtype="bf16")]
+    bufs = [client.buffer_from_host(rng.standard_normal((m, k)).astype(np.float32), dtype=dtype),
+            client.buffer_from_host(rng.standard_normal((k, n)).astype(np.float32), dtype=dtype)]
     record = _events(client)
     for _ in range(3):
         exe.execute(bufs)
@@ -225,7 +225,7 @@ def gemm(client, m, n, k, reps):
     e = record()
     client.synchronize()
     ms = a.elapsed_time(e) / reps
-    print(f"gemm bf16 {m}x{n}x{k}: {ms * 1e3:.1f} us, {2.0 * m * n * k / ms / 1e9:.1f} TFLOP/s; plan: "
+    print(f"gemm {dtype} {m}x{n}x{k}: {ms * 1e3:.1f} us, {2.0 * m * n * k / ms / 1e9:.1f} TFLOP/s; plan: "
           + " | ".join(l.strip()[:90] for l in exe.plan_text().splitlines()[1:]))
 
 
@@ -329,7 +329,7 @@ def simple(client, what, dtype, reps):
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("what", choices=["conv", "reduce", "scan", "gemma", "distilbert", "gemm", "gemv", "pointwise", "transpose",
+    ap.add_argument("what", choices=["conv", "reduce", "scan", "gemma", "distilbert", "gemm", "gemm32", "gemv", "pointwise", "transpose",
                                      "softmax", "gather", "scatter", "attention", "sort"])
     ap.add_argument("--dtype", default="f32", choices=["f32", "bf16"])
     ap.add_argument("--layout", default="kc", choices=["kc", "nc"])
@@ -365,9 +365,9 @@ def main():
         m, n, k = (int(v) for v in a.shape.split(","))
         gemv(client, m, n, k, a.layout, a.reps)
         return
-    if a.what == "gemm":
+    if a.what in ("gemm", "gemm32"):
         m, n, k = (int(v) for v in a.shape.split(","))
-        gemm(client, m, n, k, a.reps)
+        gemm(client, m, n, k, a.reps, "f32" if a.what == "gemm32" else "bf16")
         return
     if a.what == "conv":
         xs, ws = CONV_CASES[a.case]
