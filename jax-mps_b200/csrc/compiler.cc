@@ -1324,6 +1324,7 @@ struct Planner {
     std::map<Op*, std::vector<Group*>> group_of;   // a cheap op may be evaluated in several kernels
     std::deque<Group> groups;
     std::set<Op*> dup_materialize;
+    std::map<Op*, int> order;                       // where an operation stands in the block, once has_company asks
   };
 
   static void lift_uses(Block* inner, Op* owner, Block* home, BlockState& st) {
@@ -3511,10 +3512,14 @@ struct Planner {
   // 1024 x 128 x 512 8.0 / 12.4 / 10.4, 462 x 512 x 512 12.4 / 13.9 / 12.4, 250 x 2048 x 2048 76 / 26 / 34,
   // 462 x 768 x 3072 74 / 30 / 31, 2048 x 1024 x 1024 127 / 37 / 33, 4096 x 768 x 3072 455 / 156 / 109.)
   // Products that become ready together (the two gradients of a product, the projections of an input) are recorded side by side
-  // and share the SMs; `copies` is then 2, and the shortest time is that of two of them together. f32 encoder steps with every
+  // and share the SMs; `copies` is then 2, and what counts is the time of two of them together. f32 encoder steps with every
   // product modelled alone / as one of two, us: 462 rows 1463 / 1400, 256 rows 1126 / 1102, 462 rows of 256 1019 / 900, 400 rows
   // of 768 1853 / 1772. A loop body is the other way about, its iterations are one chain: 6900 / 7330 us for a scan of 100 steps.
   //
+  static double in_company(int copies, const std::function<double(int)>& time) {
+    // a third of it as if alone: the one beside it may be much smaller
+    return copies == 1 ? time(1) : 0.65 * time(copies) + 0.35 * time(1);
+  }
   // Tile width and K split of a contraction by tiled copies (tile32.cu), and its time: 0.42 us per 64-wide and 0.64 per 128-wide
   // k-tile, 6.9 to launch, fill and drain, 1.9 and the partial sums at 6 TB/s for a split, the image of B at 4.4 TB/s.
   // `b_is_weight`: B is a program input, whose split image is made beside what is in front of the product. The tensor core
@@ -3531,18 +3536,21 @@ struct Planner {
         const long long kps = (ktiles + want - 1) / want, split = (ktiles + kps - 1) / kps;
         if (split != want || kps > longest || (t.mode == 1 && kps != longest)) continue;
         if (split > 1 && kps < longest && (tiles * split > 2 * 148 || split * t.G * t.M * t.N > (64LL << 20))) break;
-        double us = (double)((copies * tiles * split + 147) / 148) * (double)kps * (bn == 64 ? 0.415 : 0.637) + 6.9;
-        if (split > 1) us += 1.9 + (double)copies * split * t.G * t.M * t.N * 8.0 / 6.05e6;
+        const double us = in_company(copies, [&](int n) {
+          const double alone = (double)((n * tiles * split + 147) / 148) * (double)kps * (bn == 64 ? 0.415 : 0.637) + 6.9;
+          return split > 1 ? alone + 1.9 + (double)n * split * t.G * t.M * t.N * 8.0 / 6.05e6 : alone;
+        });
         if (us < best * 0.98) { best = us; t.bn = bn; t.split = (int)split; }
       }
     }
-    return best + (double)copies * t.G * t.K * t.N * 12.0 / 4.4e6 + (b_is_weight ? 0.0 : 2.0);
+    return best + in_company(copies, [&](int n) { return (double)n * t.G * t.K * t.N * 12.0 / 4.4e6; }) + (b_is_weight ? 0.0 : 2.0);
   }
 
-  // Modelled time of a dense fp32 product on the FMA pipe (gemm32.cu), with its tile and split: 1.02 ns per row of four warps'
-  // FMA instructions and k (6 % less in the widest tile, which reads shared memory least; 12 % more for a B whose k is contiguous
-  // while nothing else on the SM hides its transposition), 2.95 us to launch, fill and drain, 1.3 for every further CTA of an
-  // SM, 1.35 for the sum of a cluster. Every tile and split over 70 chains from 6 x 64 x 256 to 250 x 512 x 1024: 6 % rms error.
+  // Modelled time of a dense fp32 product on the FMA pipe (gemm32.cu), with its tile and split: 0.97 ns per row of four warps'
+  // FMA instructions and k (7 % less in the widest tile, which reads shared memory least; 10 % more for each operand without rows
+  // of 16 bytes; 13 % more for a B whose k is contiguous while nothing else on the SM hides its transposition), 3.4 us to launch,
+  // fill and drain, 1.7 for every further CTA of an SM, 1.13 for the sum of a cluster. Every tile and split over 140 chains from
+  // 6 x 64 x 256 to 1500 x 304 x 1304: 8 % rms error.
   static double fma_product(Gemm32Launch& g, int copies) {
     if (g.G > 65535 || getenv("B200_NO_GEMM32")) return 1e30;
     double best = 1e30;
@@ -3551,10 +3559,12 @@ struct Planner {
       const long long tiles = (long long)((g.M + tm - 1) / tm) * ((g.N + tn - 1) / tn) * g.G;
       for (int split = 1; split <= 4; split *= 2) {
         if (split > 1 && g.K < 32 * split) break;
-        const long long per_sm = copies * tiles * split <= gemm32_resident(split) ? 1 : (copies * tiles * split + 147) / 148;
         const long long chunk = ((g.K + split - 1) / split + 3) / 4 * 4;
-        const double row = 1.02e-3 * (tile == 2 ? 0.94 : 1.0) * (g.b_kc && per_sm == 1 ? 1.12 : 1.0);
-        const double us = (double)per_sm * (tm * tn / 128) * (double)chunk * row + 2.95 + 1.3 * (double)(per_sm - 1) + (split > 1 ? 1.35 : 0.0);
+        const double us = in_company(copies, [&](int n) {
+          const long long per_sm = n * tiles * split <= gemm32_resident(split) ? 1 : (n * tiles * split + 147) / 148;
+          const double row = 0.97e-3 * (tile == 2 ? 0.93 : 1.0) * (g.b_kc && per_sm == 1 ? 1.13 : 1.0) * (g.a_vec ? 1.0 : 1.1) * (g.b_vec ? 1.0 : 1.1);
+          return (double)per_sm * (tm * tn / 128) * (double)chunk * row + 3.4 + 1.7 * (double)(per_sm - 1) + (split > 1 ? 1.13 : 0.0);
+        });
         if (us < best * 0.97) { best = us; g.split = split; g.tile = tile; }
       }
     }
@@ -3571,21 +3581,29 @@ struct Planner {
     choose_split_k(t);
     split_k = t.split_k;
     const TableShape s = table_shape(t);
-    const long long waves = (copies * s.tiles * split_k + s.per_wave - 1) / s.per_wave;
-    return (double)waves * (double)((s.ktiles + split_k - 1) / split_k) * 0.95 * s.tile_us + 8.5 + 4.8 * (double)(waves - 1) +
-           (split_k > 1 ? (double)copies * split_k * t.M * t.N * t.groups * 8.0 / 3.3e6 : 0.0);
+    return in_company(copies, [&](int n) {
+      const long long waves = (n * s.tiles * split_k + s.per_wave - 1) / s.per_wave;
+      return (double)waves * (double)((s.ktiles + split_k - 1) / split_k) * 0.95 * s.tile_us + 8.5 + 4.8 * (double)(waves - 1) +
+             (split_k > 1 ? (double)n * split_k * t.M * t.N * t.groups * 8.0 / 3.3e6 : 0.0);
+    });
   }
 
-  // Whether a product of the main plan has an operand, other than a program input, in common with another contraction.
-  static bool shares_operand(Op* op, BlockState& st) {
+  // The operand of a product that is made last; null when both are program inputs. Products that wait for the same value become
+  // ready together.
+  static Value* waits_for(Op* op, BlockState& st) {
+    Value* last = nullptr;
+    for (Value* v : op->operands)
+      if (v->def && v->def->parent == st.block && (!last || st.order[last->def] < st.order[v->def])) last = v;
+    return last;
+  }
+  static bool has_company(Op* op, BlockState& st) {
     if (st.block->parent_op) return false;
-    for (Value* v : op->operands) {
-      if (!v->def) continue;
-      auto it = st.users.find(v);
-      if (it == st.users.end()) continue;
-      for (Op* u : it->second)
-        if (u != op && (u->short_name() == "dot_general" || u->short_name() == "convolution")) return true;
-    }
+    if (st.order.empty())
+      for (size_t k = 0; k < st.ops.size(); k++) st.order[st.ops[k]] = (int)k;
+    Value* v = waits_for(op, st);
+    if (!v) return false;
+    for (Op* u : st.users[v])
+      if (u != op && (u->short_name() == "dot_general" || u->short_name() == "convolution") && waits_for(u, st) == v) return true;
     return false;
   }
 
@@ -3595,6 +3613,7 @@ struct Planner {
     Value *lhs = op->operands[0], *rhs = op->operands[1], *out = op->results[0];
     if (lhs->type.dt != DT::F32 || rhs->type.dt != DT::F32 || out->type.dt != DT::F32)
       throw CompileError("stablehlo.convolution: only f32 operands are supported so far, got " + lhs->type.str());
+    prog.tensor_saving = 1e30;
     std::string dn = op->attr("dimension_numbers");
     // '#stablehlo.conv<[b, 0, 1, f]x[0, 1, i, o]->[b, 0, 1, f]>' (also accepts the 'raw' keyword-less form)
     auto parse_spec = [&](const std::string& s) {
@@ -3764,6 +3783,7 @@ struct Planner {
       repacked[key] = tmp;
       return tmp;
     };
+    prog.tensor_saving = 1e30;
     Step s;
     s.kind = Step::GEMM16;
     s.label = op->name;
@@ -3838,6 +3858,7 @@ struct Planner {
     IGemmParams p;
     p.M = (int)M; p.N = (int)N; p.K = (int)K; p.groups = (int)G;
     p.needs_mask = 0;
+    bool dense = false;
     {
       // a strided matrix per group on both sides, with one of its two indices contiguous
       long long mv, kv, nv, kv2, gv, gv2;
@@ -3860,7 +3881,7 @@ struct Planner {
         Tile32Launch t;
         t.M = g.M; t.N = g.N; t.K = g.K; t.G = g.G;
         int split_k = 1;
-        const int copies = shares_operand(op, st) ? 2 : 1;
+        const int copies = has_company(op, st) ? 2 : 1;
         const double us_fma = fma_product(g, copies);
         double us_table = table_product(g, split_k, copies), us_tile = 1e30;
         // the switches that keep products off the tensor cores or tiled copies leave them to the FMA pipe
@@ -3878,6 +3899,9 @@ struct Planner {
           t.box[0] = 32; t.box[1] = g.a_kc ? 128 : 32; t.box[2] = t.box[3] = 1;
           us_tile = tile_product(t, !rhs->def && rhs->owner && rhs->owner->parent_op == nullptr, split_k, copies);
         }
+        if (us_tile < us_fma || us_table <= us_fma)
+          prog.tensor_saving += st.block->parent_op ? 1e30 : us_fma - std::min(us_tile, us_table);       // a loop's saving counts every time
+        dense = true;
         if (us_tile < us_fma && us_tile < us_table) p.tile = t;
         else if (us_fma < us_table) {
           p.fma = g;
@@ -3893,6 +3917,7 @@ struct Planner {
         }
       }
     }
+    if (!dense) prog.tensor_saving = 1e30;
     auto am = offsets(lhs->type.dims, sl, lfree, M), ak = offsets(lhs->type.dims, sl, lcd, K);
     auto bk = offsets(rhs->type.dims, sr, rcd, K), bn = offsets(rhs->type.dims, sr, rfree, N);
     auto ag = offsets(lhs->type.dims, sl, lbd, G), bg = offsets(rhs->type.dims, sr, rbd, G);
@@ -5862,6 +5887,20 @@ bool recorded_whole(const Plan& main) {
   for (const Step& s : main.steps)
     if (s.kind == Step::WHILE || !(graph_safe_step(s) || s.kind == Step::SCATTER)) return false;
   return (int)main.steps.size() >= kReplayLaunches;
+}
+
+std::unique_ptr<CompiledProgram> compile_text(const char* text, size_t size, Module& m, const CompileOptions& opts) {
+  auto p = compile_module(m, opts);
+  // Tensor-core kernels have bounded waits that can run out, so every execution of a plan with one reads the device's error word
+  // back: 8 us of a small program (classifier step of 2000 x 64 x 64: 41.7 us without, 49.8 with one product by tables that
+  // is 2 us quicker than on the FMA pipe).
+  if (opts.tensor_cores && p->tensor_saving > 0.0 && p->tensor_saving < 8.0) {
+    CompileOptions o = opts;
+    o.tensor_cores = false;
+    auto again = parse_module(text, size);
+    p = compile_module(*again, o);
+  }
+  return p;
 }
 
 std::unique_ptr<CompiledProgram> compile_module(Module& m, const CompileOptions& opts) {

@@ -143,6 +143,9 @@ struct CompiledProgram {
   int num_partitions = 1, num_replicas = 1;
   int launches_per_execute = -1;      // static count when the plan has no data-dependent control flow
   std::string dump;                   // human-readable plan (B200_DUMP_PLAN)
+  // Modelled microseconds that the fp32 products on the tensor cores save against the FMA pipe, 1e30 when something of the
+  // plan has no other way than the tensor cores.
+  double tensor_saving = 0.0;
 };
 
 struct CompileOptions {
@@ -154,6 +157,9 @@ struct CompileOptions {
 
 // StableHLO module -> plan. Throws CompileError (unsupported op, malformed attribute...).
 std::unique_ptr<CompiledProgram> compile_module(Module& m, const CompileOptions& opts);
+// The same for the module `m` parsed from `text`; a plan that would gain less from the tensor cores than watching them costs is
+// made without them.
+std::unique_ptr<CompiledProgram> compile_text(const char* text, size_t size, Module& m, const CompileOptions& opts);
 
 // The device-function library every generated kernel is compiled with.
 const char* codegen_prelude();

@@ -2034,7 +2034,7 @@ b200_error* b200_client_compile(b200_client* c, const char* code, size_t code_si
       if (np > 1 && np != c->nprocs)
         return make_error(B200_INVALID_ARGUMENT, "program wants " + std::to_string(np) + " partitions but the job has " +
                                                      std::to_string(c->nprocs) + " processes");
-      lp->prog = compile_module(*m, co);
+      lp->prog = compile_text(code, code_size, *m, co);
     } catch (const CompileError& e) {
       return make_error(B200_INVALID_ARGUMENT, e.what());
     } catch (const std::exception& e) {
@@ -2101,7 +2101,7 @@ b200_error* b200_compile_to_plan(const char* code, size_t code_size, const b200_
   std::unique_ptr<CompiledProgram> prog;
   try {
     auto m = parse_module(code, code_size);
-    prog = compile_module(*m, co);
+    prog = compile_text(code, code_size, *m, co);
   } catch (const CompileError& e) {
     return make_error(B200_INVALID_ARGUMENT, e.what());
   } catch (const std::exception& e) {

@@ -533,8 +533,21 @@ def test_products_that_become_ready_together_share_the_chip():
     def plan(shared):
         b = Builder()
         x = b.tanh(b.arg((462, 512), "f32"))
-        outs = [b.matmul(x, b.arg((512, 512), "f32"))]
+        outs = [b.matmul(x, b.arg((512, 512), "f32")), b.matmul(b.arg((2048, 2048), "f32"), b.arg((2048, 2048), "f32"))]
         if shared:
             outs.append(b.matmul(x, b.arg((512, 512), "f32")))
         return b200.compile_to_plan(b.module(outs))[0]
-    assert " fma tile=" in plan(False) and " tile mode=" in plan(True)
+    ways = [re.findall(r"M=462 N=512 .*? (fma|tile) ", plan(shared)) for shared in (False, True)]
+    assert ways == [["fma"], ["tile", "tile"]]
+
+
+def test_a_plan_that_gains_little_from_tensor_cores_does_without():
+    """Plans with tensor-core kernels read the device's error word back after every execution."""
+    b = Builder()
+    x, y = b.arg((2000, 64), "f32"), b.arg((2000, 64), "f32")
+    small = b.dot_general(x, y, ((0,), (0,)))
+    assert " fma tile=" in b200.compile_to_plan(b.module([small]))[0]
+    b = Builder()
+    x, y, big = b.arg((2000, 64), "f32"), b.arg((2000, 64), "f32"), b.arg((2048, 2048), "f32")
+    plan = b200.compile_to_plan(b.module([b.dot_general(x, y, ((0,), (0,))), b.matmul(big, big)]))[0]
+    assert " fma tile=" not in plan
