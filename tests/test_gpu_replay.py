@@ -131,3 +131,24 @@ def test_a_training_loop_is_recorded_once(client, by_steps, name):
         assert exe.recordings - before <= (max(1, _loops(name)) if c is client else 0)
     for g, w in zip(*losses):
         np.testing.assert_array_equal(g, w)
+
+
+@pytest.mark.gpu
+def test_arguments_may_be_one_buffer(client, by_steps):
+    """A recording made while two arguments were one buffer serves calls in which they are two, and the other way about."""
+    b = Builder()
+    x, y = b.arg((96, 96), "f32"), b.arg((96, 96), "f32")
+    h = b.matmul(b.tanh(b.matmul(x, y)), x)
+    text = b.module([b.matmul(b.sub(h, y), y), b.reduce_sum(b.mul(h, x), (0,)), x, y, b.transpose(b.add(x, h), (1, 0))])
+    exe, plain = client.compile(text), by_steps.compile(text)
+    rng = np.random.default_rng(3)
+    for k, one in enumerate([True, True, False, False, True, False]):
+        a, c = (rng.standard_normal((96, 96)).astype(np.float32) for _ in range(2))
+        got, want = [], []
+        for to, cl, e in ((got, client, exe), (want, by_steps, plain)):
+            u = cl.buffer_from_host(a)
+            v = u if one else cl.buffer_from_host(c)
+            to += [o.to_numpy() for o in e.execute([u, v])]
+        for g, w in zip(got, want):
+            np.testing.assert_array_equal(g, w)
+    assert exe.recordings == 1 and exe.relocations >= 2
