@@ -102,6 +102,13 @@ bool is_elementwise_op(const std::string& s) {
 void Emitter::line(const std::string& s) { os_ << std::string(indent_, ' ') << s << "\n"; }
 std::string Emitter::fresh(const char* p) { return name_prefix + p + std::to_string(nvar_++); }
 
+std::string Emitter::shifted(const std::string& base, int64_t by) {
+  if (by == 0) return base;
+  const std::string v = fresh("x");
+  line("const " + idx_t + " " + v + " = " + base + " + (" + std::to_string(by) + ");");
+  return v;
+}
+
 std::string Emitter::input_name(Value* v) {
   auto it = in_index_.find(v);
   if (it == in_index_.end()) {
@@ -112,16 +119,42 @@ std::string Emitter::input_name(Value* v) {
   return "in" + std::to_string(it->second);
 }
 
+std::string wide_move(const std::string& arr, const std::string& ptr, int W, int es, bool is_load, int indent, const std::string& at) {
+  std::ostringstream o;
+  const int bytes = W * es;
+  const char* piece = bytes >= 16 ? "uint4" : (bytes == 8 ? "uint2" : "unsigned int");
+  const int pb = bytes >= 16 ? 16 : bytes;
+  for (int q = 0; q < bytes / pb; q++) {
+    const std::string mem = "reinterpret_cast<" + std::string(is_load ? "const " : "") + piece + "*>(" + ptr + " + " + at + ")[" + std::to_string(q) + "]";
+    const std::string loc = "reinterpret_cast<" + std::string(is_load ? "" : "const ") + piece + "*>(" + arr + ")[" + std::to_string(q) + "]";
+    o << std::string(indent, ' ') << (is_load ? loc + " = " + mem : mem + " = " + loc) << ";\n";
+  }
+  return o.str();
+}
+
+std::string Emitter::run_arrays(int indent) const {
+  std::string s;
+  for (auto& a : arrays_) s += std::string(indent, ' ') + a + "\n";
+  return s;
+}
+
 void Emitter::ensure_idx(Ctx& c) {
   if (c.idx.size() == c.shape.size()) return;
   c.idx.assign(c.shape.size(), "0");
   int64_t stride = 1;
   std::vector<int64_t> strides(c.shape.size());
   for (int d = (int)c.shape.size() - 1; d >= 0; d--) { strides[d] = stride; stride *= c.shape[d]; }
+  // a run along the linear index lies along the innermost dimension where that is a multiple of the run long
+  int along = -1;
+  if (run && !c.lin_base.empty()) {
+    for (int d = (int)c.shape.size() - 1; d >= 0 && along < 0; d--)
+      if (c.shape[d] != 1) along = d;
+    if (along >= 0 && c.shape[along] % run != 0) along = -1;
+  }
   for (size_t d = 0; d < c.shape.size(); d++) {
     if (c.shape[d] == 1) continue;
     std::string v = fresh("x");
-    std::string e = c.lin;
+    std::string e = along >= 0 ? c.lin_base : c.lin;
     if (strides[d] != 1) e = "(" + e + " / " + std::to_string(strides[d]) + ")";
     if (d != 0) {
       bool leading_all_one = true;
@@ -129,6 +162,12 @@ void Emitter::ensure_idx(Ctx& c) {
       if (!leading_all_one) e = "(" + e + " % " + std::to_string(c.shape[d]) + ")";
     }
     line("const " + idx_t + " " + v + " = " + e + ";");
+    if ((int)d == along) {
+      c.run_dim = along;
+      c.run_base = v;
+      v = fresh("x");
+      line("const " + idx_t + " " + v + " = " + c.run_base + " + " + run_var + ";");
+    }
     c.idx[d] = v;
   }
 }
@@ -136,18 +175,32 @@ void Emitter::ensure_idx(Ctx& c) {
 std::string Emitter::lin_of(Ctx& c) {
   if (!c.lin.empty()) return c.lin;
   if (c.shape.empty()) { c.lin = "0"; return c.lin; }
+  // whole runs stay whole when memory runs along their dimension and every line starts on a multiple of the run
+  bool runs = run && c.run_dim >= 0;
+  for (int d = 0; d < (int)c.shape.size() && runs; d++)
+    runs = d < c.run_dim ? (c.shape[d] == 1 || c.shape[c.run_dim] % run == 0) : d == c.run_dim || c.shape[d] == 1;
   std::string e;
   int64_t stride = 1;
   std::vector<std::string> terms;
   for (int d = (int)c.shape.size() - 1; d >= 0; d--) {
-    if (c.shape[d] != 1 && c.idx[d] != "0")
-      terms.push_back(stride == 1 ? c.idx[d] : "(" + idx_t + ")" + c.idx[d] + " * " + std::to_string(stride));
+    const std::string& ix = runs && d == c.run_dim ? c.run_base : c.idx[d];
+    if (c.shape[d] != 1 && ix != "0")
+      terms.push_back(stride == 1 ? ix : "(" + idx_t + ")" + ix + " * " + std::to_string(stride));
     stride *= c.shape[d];
   }
-  if (terms.empty()) { c.lin = "0"; return c.lin; }
+  if (terms.empty()) {
+    c.lin = "0";
+    if (!runs) return c.lin;
+    terms.push_back("0");
+  }
   for (size_t k = 0; k < terms.size(); k++) e += (k ? " + " : "") + terms[k];
   std::string v = fresh("l");
   line("const " + idx_t + " " + v + " = " + e + ";");
+  if (runs) {
+    c.lin_base = v;
+    v = fresh("l");
+    line("const " + idx_t + " " + v + " = " + c.lin_base + " + " + run_var + ";");
+  }
   c.lin = v;
   return v;
 }
@@ -165,6 +218,16 @@ std::string Emitter::load(Value* v, Ctx& c) {
   DT d = v->type.dt;
   std::string var = fresh("v");
   std::string e = p + "[" + at + "]";
+  if (run && !c.lin_base.empty() && at != "lin" && wide_size(run, (int)dt_size(d))) {
+    // the whole run at its first position, in the widest pieces. (Read one element at a time, a bias along the rows of a bf16
+    // tensor took eight 2-byte loads for every 16-byte load of the tensor.)
+    const std::string arr = fresh("w");
+    arrays_.push_back(std::string("__align__(16) ") + s_type(d) + " " + arr + "[" + std::to_string(run) + "];");
+    line("if (" + run_var + " == 0) {");
+    os_ << wide_move(arr, p, run, (int)dt_size(d), true, indent_ + 2, c.lin_base);
+    line("}");
+    e = arr + "[" + run_var + "]";
+  }
   if (d == DT::BF16) e = "bf16_to_f(" + e + ")";
   else if (d == DT::F16) e = "f16_to_f(" + e + ")";
   else if (d == DT::PRED) e = "(" + e + " != 0)";
@@ -272,7 +335,7 @@ std::string Emitter::emit(Value* v, Ctx c) {
   std::string var;
   auto same_ctx = [&](Value* o) -> Ctx {
     if (o->type.dims == c.shape) return c;
-    if (o->type.rank() == 0) { Ctx s; s.lin = "0"; return s; }
+    if (o->type.rank() == 0) return Ctx::scalar();
     throw CompileError(d->name + ": operand shape differs from result shape");
   };
   if (is_elementwise_op(sh)) {
@@ -300,12 +363,17 @@ std::string Emitter::emit(Value* v, Ctx c) {
     for (size_t i = 0; i < dims.size(); i++)
       oc.idx[i] = (o->type.dims[i] == 1) ? "0" : c.idx[dims[i]];
     if (oc.shape.empty()) oc.lin = "0";
+    oc.run_dim = c.run_dim >= 0 ? Ctx::kSame : c.run_dim;
+    for (size_t i = 0; i < dims.size(); i++)
+      if (c.run_dim >= 0 && dims[i] == c.run_dim && o->type.dims[i] != 1) { oc.run_dim = (int)i; oc.run_base = c.run_base; }
     return emit(o, oc);
   } else if (sh == "reshape") {
     Value* o = d->operands[0];
     Ctx oc;
     oc.shape = o->type.dims;
     oc.lin = lin_of(c);
+    oc.lin_base = c.lin_base;
+    oc.run_dim = c.run_dim == Ctx::kSame ? Ctx::kSame : Ctx::kUnknown;
     return emit(o, oc);
   } else if (sh == "transpose") {
     ensure_idx(c);
@@ -315,14 +383,18 @@ std::string Emitter::emit(Value* v, Ctx c) {
     oc.shape = o->type.dims;
     oc.idx.resize(perm.size());
     for (size_t i = 0; i < perm.size(); i++) oc.idx[perm[i]] = c.idx[i];
+    oc.run_dim = c.run_dim >= 0 ? (int)perm[c.run_dim] : c.run_dim;
+    oc.run_base = c.run_base;
     return emit(o, oc);
   } else if (sh == "reverse") {
     ensure_idx(c);
     auto dims = attr_i64s(d->attr("dimensions"));
     Ctx oc = c;
     oc.lin.clear();
+    oc.lin_base.clear();
     for (auto dd : dims) {
       if (c.shape[dd] == 1) continue;
+      if (dd == oc.run_dim) oc.run_dim = Ctx::kUnknown;
       std::string nv = fresh("x");
       line("const " + idx_t + " " + nv + " = " + std::to_string(c.shape[dd] - 1) + " - " + c.idx[dd] + ";");
       oc.idx[dd] = nv;
@@ -336,9 +408,15 @@ std::string Emitter::emit(Value* v, Ctx c) {
     Ctx oc;
     oc.shape = o->type.dims;
     oc.idx = c.idx;
+    oc.run_dim = c.run_dim;
+    oc.run_base = c.run_base;
     for (size_t i = 0; i < st.size(); i++) {
       if (st[i] == 0 && sd[i] == 1) continue;
       if (c.shape[i] == 1) { oc.idx[i] = std::to_string(st[i]); continue; }
+      if ((int)i == c.run_dim) {
+        if (sd[i] == 1 && st[i] % run == 0) oc.run_base = shifted(c.run_base, st[i]);
+        else oc.run_dim = Ctx::kUnknown;
+      }
       std::string nv = fresh("x");
       line("const " + idx_t + " " + nv + " = " + c.idx[i] + " * " + std::to_string(sd[i]) + " + " + std::to_string(st[i]) + ";");
       oc.idx[i] = nv;
@@ -349,18 +427,23 @@ std::string Emitter::emit(Value* v, Ctx c) {
     auto lo = attr_i64s(d->attr("edge_padding_low"));
     auto in = attr_i64s(d->attr("interior_padding"));
     Value* o = d->operands[0];
-    Ctx sc;
-    sc.lin = "0";
+    Ctx sc = Ctx::scalar();
     std::string pv = emit(d->operands[1], sc);
     Ctx oc;
     oc.shape = o->type.dims;
     oc.idx = c.idx;
+    oc.run_dim = c.run_dim;
+    oc.run_base = c.run_base;
     std::string ok = fresh("ok");
     line("bool " + ok + " = true;");
     for (size_t i = 0; i < lo.size(); i++) {
       int64_t step = in[i] + 1;
       bool trivial = lo[i] == 0 && step == 1 && o->type.dims[i] == c.shape[i];
       if (trivial) continue;
+      if ((int)i == c.run_dim) {                     // a run is inside or outside as a whole, or it is taken apart
+        if (step == 1 && lo[i] % run == 0 && o->type.dims[i] % run == 0) oc.run_base = shifted(c.run_base, -lo[i]);
+        else oc.run_dim = Ctx::kUnknown;
+      }
       std::string t = fresh("x");
       line("const " + idx_t + " " + t + " = " + c.idx[i] + " - (" + std::to_string(lo[i]) + ");");
       std::string q = t;
@@ -386,6 +469,11 @@ std::string Emitter::emit(Value* v, Ctx c) {
     var = fresh("v");
     line(ct + " " + var + ";");
     int64_t off = 0;
+    bool whole = c.run_dim != dim;                   // no run reaches over the border of two operands
+    if (!whole) {
+      whole = true;
+      for (auto* o : d->operands) whole = whole && o->type.dims[dim] % run == 0;
+    }
     for (size_t k = 0; k < d->operands.size(); k++) {
       Value* o = d->operands[k];
       int64_t sz = o->type.dims[dim];
@@ -398,6 +486,8 @@ std::string Emitter::emit(Value* v, Ctx c) {
       Ctx oc;
       oc.shape = o->type.dims;
       oc.idx = c.idx;
+      oc.run_dim = whole ? c.run_dim : Ctx::kUnknown;
+      oc.run_base = c.run_dim == dim ? shifted(c.run_base, -off) : c.run_base;
       if (off != 0) {
         std::string nv = fresh("x");
         line("const " + idx_t + " " + nv + " = " + c.idx[dim] + " - " + std::to_string(off) + ";");
@@ -416,8 +506,7 @@ std::string Emitter::emit(Value* v, Ctx c) {
     size_t first = upd ? 2 : 1;
     const std::vector<int64_t>& win = upd ? d->operands[1]->type.dims : c.shape;
     std::vector<std::string> starts;
-    Ctx sc;
-    sc.lin = "0";
+    Ctx sc = Ctx::scalar();
     for (size_t i = 0; i < o->type.dims.size(); i++) {
       std::string s = emit(d->operands[first + i], sc);
       std::string nv = fresh("s");
@@ -435,8 +524,12 @@ std::string Emitter::emit(Value* v, Ctx c) {
         line("const " + idx_t + " " + nv + " = " + c.idx[i] + " + " + starts[i] + ";");
         oc.idx[i] = nv;
       }
+      // along the run's dimension the window starts anywhere, unless it is as long as the operand
+      oc.run_dim = c.run_dim >= 0 && o->type.dims[c.run_dim] != win[c.run_dim] ? Ctx::kUnknown : c.run_dim;
+      oc.run_base = c.run_base;
       return emit(o, oc);
     }
+    const bool apart = c.run_dim == Ctx::kUnknown || (c.run_dim >= 0 && o->type.dims[c.run_dim] != win[c.run_dim]);   // parts of a run in and out of the window
     Value* u = d->operands[1];
     std::string in = fresh("ok");
     line("bool " + in + " = true;");
@@ -449,6 +542,8 @@ std::string Emitter::emit(Value* v, Ctx c) {
       line(in + " = " + in + " && " + nv + " >= 0 && " + nv + " < " + std::to_string(u->type.dims[i]) + ";");
       uc.idx[i] = nv;
     }
+    uc.run_dim = apart ? Ctx::kUnknown : c.run_dim;
+    uc.run_base = c.run_base;
     var = fresh("v");
     line(ct + " " + var + ";");
     line("if (" + in + ") {");
@@ -458,6 +553,7 @@ std::string Emitter::emit(Value* v, Ctx c) {
     line("} else {");
     push_scope();
     Ctx oc = c;
+    if (apart) { oc.run_dim = Ctx::kUnknown; oc.lin_base.clear(); }
     line(var + " = " + emit(o, oc) + ";");
     pop_scope();
     line("}");
@@ -480,12 +576,15 @@ std::string Emitter::emit(Value* v, Ctx c) {
     for (int q = 0; q < indices->type.rank(); q++)
       if (q != ivd) idx_batch_dims.push_back(q);
     std::vector<std::string> full(operand->type.rank(), "0");
+    const bool by_offset = c.run_dim == Ctx::kSame || (c.run_dim >= 0 && std::find(offset_dims.begin(), offset_dims.end(), (int64_t)c.run_dim) != offset_dims.end());
+    int oc_run = c.run_dim == Ctx::kSame ? Ctx::kSame : Ctx::kUnknown;
     for (size_t kk = 0; kk < smap.size(); kk++) {
       Ctx ic;
       ic.shape = indices->type.dims;
       ic.idx.assign(indices->type.rank(), "0");
       for (size_t q = 0; q < idx_batch_dims.size(); q++) ic.idx[idx_batch_dims[q]] = c.idx[batch_out[q]];
       if (ivd < indices->type.rank()) ic.idx[ivd] = std::to_string(kk);
+      if (by_offset) ic.run_dim = Ctx::kSame;        // every position of the run takes the same index
       std::string s = emit(indices, ic);
       int od = (int)smap[kk];
       std::string nv = fresh("g");
@@ -501,6 +600,8 @@ std::string Emitter::emit(Value* v, Ctx c) {
     for (int od = 0; od < operand->type.rank(); od++) {
       if (std::find(collapsed.begin(), collapsed.end(), od) != collapsed.end()) continue;
       if (std::find(obatch.begin(), obatch.end(), od) != obatch.end()) continue;
+      // a run along an offset dimension stays one in the operand where the slice is as long as the operand (it starts at 0)
+      if (by_offset && c.run_dim >= 0 && offset_dims[w] == c.run_dim && sizes[od] == operand->type.dims[od]) oc_run = od;
       std::string o_idx = c.idx[offset_dims[w++]];
       if (full[od] == "0") full[od] = o_idx;
       else if (o_idx != "0") {
@@ -512,6 +613,8 @@ std::string Emitter::emit(Value* v, Ctx c) {
     Ctx oc;
     oc.shape = operand->type.dims;
     oc.idx = full;
+    oc.run_dim = oc_run;
+    oc.run_base = c.run_base;
     return emit(operand, oc);
   } else {
     throw CompileError("internal: op " + d->name + " cannot be generated inside a fusion");

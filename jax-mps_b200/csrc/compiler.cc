@@ -1602,20 +1602,6 @@ struct Planner {
     return any;
   }
 
-  // moves W elements of `es` bytes between a thread's array `arr` and `ptr + base` in the widest aligned pieces
-  static std::string wide_move(const std::string& arr, const std::string& ptr, int W, int es, bool is_load, int indent = 2) {
-    std::ostringstream o;
-    const int bytes = W * es;
-    const char* piece = bytes >= 16 ? "uint4" : (bytes == 8 ? "uint2" : "unsigned int");
-    const int pb = bytes >= 16 ? 16 : bytes;
-    for (int q = 0; q < bytes / pb; q++) {
-      const std::string mem = "reinterpret_cast<" + std::string(is_load ? "const " : "") + piece + "*>(" + ptr + " + base)[" + std::to_string(q) + "]";
-      const std::string loc = "reinterpret_cast<" + std::string(is_load ? "" : "const ") + piece + "*>(" + arr + ")[" + std::to_string(q) + "]";
-      o << std::string(indent, ' ') << (is_load ? loc + " = " + mem : mem + " = " + loc) << ";\n";
-    }
-    return o.str();
-  }
-
   static constexpr int kEPT = 4;       // elements per thread of a pointwise kernel
   static constexpr int kThreads = 256;
 
@@ -1634,21 +1620,11 @@ struct Planner {
       for (auto* o : m->operands) all.push_back(o);
     }
     em.idx_t = idx_type_for(all, n + kThreads * 8);
-    Ctx root;
-    root.shape = rt.dims;
-    root.lin = "lin";
-    em.ensure_idx(root);
-    std::vector<std::string> vals;
-    for (auto* o : outs) vals.push_back(em.emit(o, root));
-    for (size_t k = 0; k < outs.size(); k++)
-      em.line("out" + std::to_string(k) + "[lin] = " + store_expr(outs[k]->type.dt, vals[k]) + ";");
-    std::ostringstream src;
-    src << "extern \"C\" __global__ void __launch_bounds__(" << kThreads << ") @NAME@(" << signature(outs, em.inputs)
-        << ") {\n";
     // Wide accesses: a thread takes W consecutive elements (8 when a 2-byte type is among the outputs and the element
     // count allows it, else 4). Inputs read at the kernel's own linear index (same-shaped tensors) are fetched with
     // 16-byte loads (one for 8 two-byte or 4 four-byte elements, two for 8 four-byte ones), the outputs leave the
-    // same way. Other operands (broadcast vectors, gathers) keep their scalar loads.
+    // same way. Other operands (broadcast vectors, transposes, slices, gathered rows) are too where the emitter finds that the
+    // W elements lie in one aligned piece, and the index arithmetic is then that of one element.
     auto esize = [](DT d) -> int {
       switch (d) {
         case DT::F32: case DT::I32: case DT::U32: return 4;
@@ -1667,6 +1643,18 @@ struct Planner {
     const int W = (two_byte_out && n % 8 == 0) ? 8 : 4;
     for (auto* o : outs) wide_ok = wide_ok && (W * esize(o->type.dt)) % 4 == 0;
     const bool vec4 = wide_ok && n % W == 0 && !getenv("B200_NO_WIDE_POINTWISE");
+    Ctx root;
+    root.shape = rt.dims;
+    root.lin = "lin";
+    if (vec4) { em.run = W; root.lin_base = "base"; }
+    em.ensure_idx(root);
+    std::vector<std::string> vals;
+    for (auto* o : outs) vals.push_back(em.emit(o, root));
+    for (size_t k = 0; k < outs.size(); k++)
+      em.line("out" + std::to_string(k) + "[lin] = " + store_expr(outs[k]->type.dt, vals[k]) + ";");
+    std::ostringstream src;
+    src << "extern \"C\" __global__ void __launch_bounds__(" << kThreads << ") @NAME@(" << signature(outs, em.inputs)
+        << ") {\n";
     Launch L;
     if (vec4) {
       std::string body = em.str();
@@ -1687,7 +1675,7 @@ struct Planner {
       }
       src << "  const " << em.idx_t << " base = ((" << em.idx_t << ")blockIdx.x * " << kThreads << " + threadIdx.x) * " << W << ";\n";
       src << "  if (base >= (" << em.idx_t << ")" << n << "LL) return;\n";
-      src << loads.str();
+      src << loads.str() << em.run_arrays(2);
       src << "  #pragma unroll\n  for (int e = 0; e < " << W << "; ++e) {\n";
       src << "    const " << em.idx_t << " lin = base + e;\n";
       src << body;
@@ -3173,7 +3161,23 @@ struct Planner {
   // `epilogue`: pointwise groups over the kept index space that are evaluated by the thread holding the final
   // value of each output (second pass of a split reduction only); `bound_results` are the reduce results their
   // expressions refer to, in accumulator order.
-  static bool use_col4(int64_t Nk) { return Nk % 4 == 0 && Nk >= 64 && !getenv("B200_NO_COL4"); }
+  // consecutive kept indices per thread of a column reduction
+  static int col_run(int64_t Nk) {
+    if (Nk < 64 || getenv("B200_NO_COL4")) return 1;
+    return Nk % 4 == 0 ? 4 : Nk % 2 == 0 ? 2 : 1;
+  }
+
+  // does evaluating `v` read a tensor of 2-byte elements as large as the reduction's index space?
+  static bool reads_two_bytes(Value* v, const std::function<bool(Op*)>& internal, int64_t total) {
+    std::set<Value*> seen;
+    std::function<bool(Value*)> walk = [&](Value* x) -> bool {
+      if (!seen.insert(x).second) return false;
+      if (!x->def || !internal(x->def)) return x->type.numel() == total && dt_size(x->type.dt) == 2;
+      for (Value* o : x->def->operands) if (walk(o)) return true;
+      return false;
+    };
+    return walk(v);
+  }
 
   Launch gen_reduce_kernel(const ReduceGen& rg, std::function<bool(Op*)> internal, int splits, bool col,
                            std::vector<Value*> outs, const std::vector<Group*>* epilogue = nullptr,
@@ -3202,6 +3206,24 @@ struct Planner {
     int64_t total = Nk * std::max<int64_t>(Nr, 1);
     em.idx_t = total >= (1LL << 31) - 65536 ? "i64" : "int";
     em.indent_ = 6;
+    // Q consecutive kept indices per thread (column form), or V consecutive reduced ones (row form, where the reduced
+    // dimensions are the innermost): 16-byte pieces of what is read along memory, 8-byte ones of 2-byte types in columns.
+    const int Q = col ? col_run(Nk) : 1;
+    // T threads cooperate on one output; the reduced range is contiguous-ish along threads
+    // a block per output from 128 reduced elements on: second passes over a few hundred partial rows are latency-
+    // bound, and 256 threads fetch them in one or two rounds of loads where a warp would need ten to twenty
+    const int T = Nr >= 128 ? 256 : 32;
+    int V = 1;
+    bool two_bytes = false;
+    for (auto& part : rg.parts)
+      for (auto* v : part.operands) two_bytes = two_bytes || reads_two_bytes(v, internal, total);
+    if (!col && !getenv("B200_NO_WIDE_ROWS")) {
+      bool suffix = true;
+      for (size_t d = 0; d < rg.in_shape.size(); d++)
+        suffix = suffix && ((d + rg.dims.size() >= rg.in_shape.size()) == (std::find(rg.dims.begin(), rg.dims.end(), (int64_t)d) != rg.dims.end()));
+      if (suffix) V = two_bytes && Nr % 8 == 0 ? 8 : Nr % 4 == 0 ? 4 : Nr % 2 == 0 ? 2 : 1;
+      while (V > 1 && (int64_t)T * V * splits > Nr) V /= 2;
+    }
     // contexts
     Ctx kc;
     kc.shape = kept_shape;
@@ -3211,6 +3233,15 @@ struct Planner {
     rc.lin = "r";
     std::ostringstream pre;       // code before the loop (kept index decomposition, init loads)
     Emitter pe;
+    if (Q > 1) {
+      pe.run = em.run = Q;
+      pe.run_var = em.run_var = "q";
+      kc.lin_base = "o4";
+    } else if (V > 1) {
+      em.run = V;
+      rc.lin_base = "rb";
+      kc.run_dim = Ctx::kSame;
+    }
     pe.is_internal = [](Op*) { return false; };
     pe.idx_t = em.idx_t;
     pe.name_prefix = "k";
@@ -3226,6 +3257,12 @@ struct Planner {
       for (size_t d = 0; d < rg.in_shape.size(); d++) {
         if (std::find(rg.dims.begin(), rg.dims.end(), (int64_t)d) == rg.dims.end()) oc.idx[d] = kc.idx[ki++];
         else oc.idx[d] = rc.idx[ri++];
+        const bool kept = std::find(rg.dims.begin(), rg.dims.end(), (int64_t)d) == rg.dims.end();
+        const Ctx& from = kept ? kc : rc;
+        if ((Q > 1) == kept && from.run_dim == (int)(kept ? ki : ri) - 1) {
+          oc.run_dim = (int)d;
+          oc.run_base = from.run_base;
+        }
       }
     }
     std::vector<std::string> vals;
@@ -3310,43 +3347,48 @@ struct Planner {
     Launch L;
     L.outs = outs;
     L.ins = ins;
-    const bool col4 = col && use_col4(Nk);
-    if (col4) {
-      // Column strategy with four consecutive kept indices per thread: four times the bytes in flight per thread
+    if (Q > 1) {
+      // Column strategy with four (two) consecutive kept indices per thread: as many times the bytes in flight per thread
       // and, for inputs read at their own position, neighbouring loads the compiler can merge into 16-byte ones
       // (every slot and buffer starts on a 256-byte boundary). The per-index code is the scalar one, instantiated
-      // four times with the accumulators indexed by q.
-      const int TX = (int)std::min<int64_t>(32, Nk / 4), TY = 256 / TX;
-      const int unroll_r = 2;      // measured on the ResNet18 step: 1 -> 5.20 ms, 2 -> 5.15, 4 -> 5.18 (scalar form 5.21)
+      // as many times with the accumulators indexed by q.
+      const int TX = (int)std::min<int64_t>(32, Nk / Q), TY = 256 / TX;
+      // 16 bytes per thread and row, measured on the ResNet18 step: 1 -> 5.20 ms, 2 -> 5.15, 4 -> 5.18 (scalar form 5.21);
+      // twice as many rows in flight where a row gives a thread 8 bytes
+      const int unroll_r = Q == 4 && !two_bytes ? 2 : 4;
       auto per_q = [](std::string text) {
         return std::regex_replace(text, std::regex("\\bacc(\\d+)\\b"), "acc$1[q]");
       };
       src << "extern \"C\" __global__ void __launch_bounds__(256) @NAME@(" << signature(outs, ins) << ") {\n";
       for (size_t k = 0; k < ins.size(); k++)
-        if (dt_size(ins[k]->type.dt) == 4 && ins[k]->type.numel() % 4 == 0)
-          src << "  in" << k << " = (const " << s_type(ins[k]->type.dt) << "*)__builtin_assume_aligned(in" << k << ", 16);\n";
+        if (dt_size(ins[k]->type.dt) == 4 && ins[k]->type.numel() % Q == 0)
+          src << "  in" << k << " = (const " << s_type(ins[k]->type.dt) << "*)__builtin_assume_aligned(in" << k << ", " << 4 * Q << ");\n";
       for (size_t k = 0; k < n; k++)
-        src << "  __shared__ " << c_type(dts[k]) << " sm" << k << "[" << TY << "][" << TX * 4 + 4 << "];\n";
-      src << "  const " << it << " o4 = ((" << it << ")blockIdx.x * " << TX << " + threadIdx.x) * 4;\n";
+        src << "  __shared__ " << c_type(dts[k]) << " sm" << k << "[" << TY << "][" << TX * Q + 4 << "];\n";
+      src << "  const " << it << " o4 = ((" << it << ")blockIdx.x * " << TX << " + threadIdx.x) * " << Q << ";\n";
       src << "  const bool live = o4 < (" << it << ")" << Nk << "LL;\n";
       for (size_t k = 0; k < n; k++)
-        src << "  " << c_type(dts[k]) << " acc" << k << "[4] = {" << init_names[k] << ", " << init_names[k] << ", "
-            << init_names[k] << ", " << init_names[k] << "};\n";
+        {
+          src << "  " << c_type(dts[k]) << " acc" << k << "[" << Q << "] = {";
+          for (int q = 0; q < Q; q++) src << (q ? ", " : "") << init_names[k];
+          src << "};\n";
+        }
       src << "  if (live) {\n";
       src << "    #pragma unroll " << unroll_r << "\n";
       src << "    for (" << it << " r = (" << it << ")blockIdx.y * " << TY << " + threadIdx.y; r < (" << it << ")" << Nr
           << "LL; r += " << TY << " * (" << it << ")gridDim.y) {\n";
-      src << "      #pragma unroll\n      for (int q = 0; q < 4; ++q) {\n        const " << it << " o = o4 + q;\n";
+      src << em.run_arrays(6);
+      src << "      #pragma unroll\n      for (int q = 0; q < " << Q << "; ++q) {\n        const " << it << " o = o4 + q;\n";
       src << pe.str() << per_q(em.str());
       src << "      }\n    }\n  }\n";
-      src << "  #pragma unroll\n  for (int q = 0; q < 4; ++q) {\n";
-      for (size_t k = 0; k < n; k++) src << "    sm" << k << "[threadIdx.y][threadIdx.x * 4 + q] = acc" << k << "[q];\n";
+      src << "  #pragma unroll\n  for (int q = 0; q < " << Q << "; ++q) {\n";
+      for (size_t k = 0; k < n; k++) src << "    sm" << k << "[threadIdx.y][threadIdx.x * " << Q << " + q] = acc" << k << "[q];\n";
       src << "  }\n  __syncthreads();\n";
       src << "  if (threadIdx.y == 0 && live) {\n";
-      src << "    #pragma unroll\n    for (int q = 0; q < 4; ++q) {\n      const " << it << " o = o4 + q;\n";
+      src << "    #pragma unroll\n    for (int q = 0; q < " << Q << "; ++q) {\n      const " << it << " o = o4 + q;\n";
       src << "      for (int y = 1; y < " << TY << "; ++y) {\n";
       for (size_t k = 0; k < n; k++)
-        src << "        const " << c_type(dts[k]) << " oth" << k << " = sm" << k << "[y][threadIdx.x * 4 + q];\n";
+        src << "        const " << c_type(dts[k]) << " oth" << k << " = sm" << k << "[y][threadIdx.x * " << Q << " + q];\n";
       {
         Emitter te;
         te.idx_t = em.idx_t;
@@ -3361,7 +3403,7 @@ struct Planner {
             << store_expr(outs[k]->type.dt, "acc" + std::to_string(k) + "[q]") << ";\n";
       src << per_q(epi);
       src << "    }\n  }\n}\n";
-      L.grid[0] = (unsigned)((Nk + TX * 4 - 1) / (TX * 4)); L.grid[1] = (unsigned)splits; L.grid[2] = 1;
+      L.grid[0] = (unsigned)((Nk + TX * Q - 1) / (TX * Q)); L.grid[1] = (unsigned)splits; L.grid[2] = 1;
       L.block[0] = TX; L.block[1] = TY; L.block[2] = 1;
     } else if (col) {
       // threads along the kept index (coalesced), rows of the reduced range over threadIdx.y and blockIdx.y
@@ -3399,10 +3441,6 @@ struct Planner {
       L.grid[0] = (unsigned)((Nk + TX - 1) / TX); L.grid[1] = (unsigned)splits; L.grid[2] = 1;
       L.block[0] = TX; L.block[1] = TY; L.block[2] = 1;
     } else {
-      // T threads cooperate on one output; the reduced range is contiguous-ish along threads
-      // a block per output from 128 reduced elements on: second passes over a few hundred partial rows are latency-
-      // bound, and 256 threads fetch them in one or two rounds of loads where a warp would need ten to twenty
-      int T = Nr >= 128 ? 256 : 32;
       int per_block = 256 / T;
       src << "extern \"C\" __global__ void __launch_bounds__(256) @NAME@(" << signature(outs, ins) << ") {\n";
       if (T == 256)
@@ -3412,11 +3450,17 @@ struct Planner {
       src << "  const bool live = o < (" << it << ")" << Nk << "LL;\n";
       for (size_t k = 0; k < n; k++) src << "  " << c_type(dts[k]) << " acc" << k << " = " << init_names[k] << ";\n";
       src << "  if (live) {\n" << pe.str();
-      src << "    #pragma unroll 4\n";
-      src << "    for (" << it << " r = (" << it << ")blockIdx.y * " << T << " + lane; r < (" << it << ")" << Nr
-          << "LL; r += " << T << " * (" << it << ")gridDim.y) {\n";
+      src << "    #pragma unroll " << (V > 4 ? 2 : 4) << "\n";
+      if (V > 1) {
+        src << "    for (" << it << " rb = ((" << it << ")blockIdx.y * " << T << " + lane) * " << V << "; rb < (" << it << ")" << Nr
+            << "LL; rb += " << T * V << " * (" << it << ")gridDim.y) {\n" << em.run_arrays(6);
+        src << "      #pragma unroll\n      for (int e = 0; e < " << V << "; ++e) {\n      const " << it << " r = rb + e;\n";
+      } else {
+        src << "    for (" << it << " r = (" << it << ")blockIdx.y * " << T << " + lane; r < (" << it << ")" << Nr
+            << "LL; r += " << T << " * (" << it << ")gridDim.y) {\n";
+      }
       src << em.str();
-      src << "    }\n  }\n";
+      src << (V > 1 ? "      }\n" : "") << "    }\n  }\n";
       src << "  #pragma unroll\n  for (int m = 16; m >= 1; m >>= 1) {\n";
       for (size_t k = 0; k < n; k++)
         src << "    const " << c_type(dts[k]) << " oth" << k << " = shfl_xor(acc" << k << ", m);\n";
@@ -4424,7 +4468,9 @@ struct Planner {
     const int64_t warp_max = wm ? atoll(wm) : 1024;
     const int T = (Nr <= 64 || (Nr <= warp_max && Nk >= 1184)) ? 32 : 256, per_block = 256 / T;
     // V consecutive elements of the row per thread and round, moved with 16-byte accesses where a tensor is read or
-    // written at the row element's own position: 8 when the row's tensors include 2-byte types, else 4
+    // written at the row element's own position: 8 when the row's tensors include 2-byte types, else 4; fewer when that
+    // would leave half of the threads without an element (128 elements of a softmax row in pieces of eight: 31 us for
+    // 49152 rows, 16 of 32 lanes idle)
     int V = 1;
     if (!getenv("B200_NO_WIDE_ROWS")) {
       bool two = false;
@@ -4435,7 +4481,17 @@ struct Planner {
         }
       if (two && Nr % 8 == 0) V = 8;
       else if (Nr % 4 == 0) V = 4;
+      else if (Nr % 2 == 0) V = 2;
+      while (V > 2 && T * V >= 2 * Nr) V /= 2;
     }
+    // Rows of up to 32 elements per thread stay in registers: the operands of all stages are fetched once, together, and the
+    // loops over the row are unrolled, so that what several stages compute from them is computed once. With the runs of the
+    // emitter: a layer norm of 4096 x 768 bf16 with a bias in front 17 us before, a softmax of 49152 x 128 31 us (ncu; both are
+    // 3 to 4 us of memory traffic), the masked-LM step of 4096 tokens 4544 -> 3916 us, the ResNet18 step 3945 -> 3797.
+    const int64_t rounds = (Nr + T * V - 1) / (T * V);
+    const bool hold = V > 1 && rounds * V <= 32 && !getenv("B200_NO_HELD_ROWS");
+    std::map<size_t, DT> held;         // input number -> type, of those kept in registers
+    int64_t held_bytes = 0;
     const std::string it = "int";
     std::set<Op*> chain_members;
     for (Group* g : rc.stages) chain_members.insert(g->members.begin(), g->members.end());
@@ -4470,11 +4526,16 @@ struct Planner {
     Ctx kc;
     kc.shape = rc.kept_shape;
     kc.lin = "o";
+    kc.run_dim = Ctx::kSame;
     pe.ensure_idx(kc);
     std::vector<Value*> ins, outs;
     std::ostringstream decl, body;
     std::set<Op*> members_so_far;
     std::map<Value*, std::string> bound;
+    const std::string row_rounds = hold
+        ? "    #pragma unroll\n    for (int t = 0; t < " + std::to_string(rounds) + "; ++t) {\n      const " + it + " rb = (t * " + std::to_string(T) + " + lane) * " +
+              std::to_string(V) + ";\n" + (Nr % (T * V) ? "      if (rb >= " + std::to_string(Nr) + ") continue;\n" : "")
+        : "    for (" + it + " rb = lane * " + std::to_string(V) + "; rb < " + std::to_string(Nr) + "; rb += " + std::to_string(T * V) + ") {\n";
     std::string label = "row{";
     int stage_no = 0;
     for (Group* g : rc.stages) {
@@ -4493,12 +4554,16 @@ struct Planner {
       Ctx rctx;
       rctx.shape = rc.red_shape;
       rctx.lin = "r";
+      if (V > 1) { em.run = V; rctx.lin_base = "rb"; }
       em.ensure_idx(rctx);
       Ctx oc;
       oc.shape = rc.in_shape;
       oc.idx = kc.idx;
       oc.idx.insert(oc.idx.end(), rctx.idx.begin(), rctx.idx.end());
       oc.lin = "lin";
+      if (V > 1) oc.lin_base = "base";
+      oc.run_dim = rctx.run_dim >= 0 ? (int)rc.kept_shape.size() + rctx.run_dim : rctx.run_dim;
+      oc.run_base = rctx.run_base;
       // the loop over the row's elements around a stage's code; `stage_outs` are the (output number, value) pairs the
       // stage stores at the element's own position
       auto row_loop = [&](Emitter& e2, const std::vector<std::pair<size_t, Value*>>& stage_outs) -> std::string {
@@ -4512,9 +4577,15 @@ struct Planner {
           const int es = dt_size(in->type.dt);
           if (in->type.numel() != Nk * Nr || (es != 1 && es != 2 && es != 4) || (V * es) % 4 != 0) continue;
           const std::string nm = "in" + std::to_string(k);
+          if (hold && (held.count(k) || held_bytes + rounds * V * es <= 256)) {
+            if (!replace_word(inner, nm + "[lin]", "h" + nm + "[t][e]")) continue;
+            if (held.emplace(k, in->type.dt).second) held_bytes += rounds * V * es;
+            continue;
+          }
           if (!replace_word(inner, nm + "[lin]", "v" + nm + "[e]")) continue;
           pre << "      __align__(16) " << s_type(in->type.dt) << " v" << nm << "[" << V << "];\n" << wide_move("v" + nm, nm, V, es, true, 6);
         }
+        pre << e2.run_arrays(6);
         for (auto& so : stage_outs) {
           const int es = dt_size(so.second->type.dt);
           if ((es != 1 && es != 2 && es != 4) || (V * es) % 4 != 0) continue;
@@ -4523,8 +4594,7 @@ struct Planner {
           pre << "      __align__(16) " << s_type(so.second->type.dt) << " v" << nm << "[" << V << "];\n";
           post << wide_move("v" + nm, nm, V, es, false, 6);
         }
-        return "    for (" + it + " rb = lane * " + std::to_string(V) + "; rb < " + std::to_string(Nr) + "; rb += " + std::to_string(T * V) +
-               ") {\n      const " + it + " base = o * " + std::to_string(Nr) + " + rb;\n" + pre.str() +
+        return row_rounds + "      const " + it + " base = o * " + std::to_string(Nr) + " + rb;\n" + pre.str() +
                "      #pragma unroll\n      for (int e = 0; e < " + std::to_string(V) + "; ++e) {\n      const " + it + " r = rb + e;\n      const " +
                it + " lin = base + e;\n" + inner + "      }\n" + post.str() + "    }\n";
       };
@@ -4655,7 +4725,15 @@ struct Planner {
     src << "  const bool live = o_raw < " << Nk << ";\n";
     src << "  const " << it << " o = live ? o_raw : " << Nk - 1 << ";\n";
     src << "  const int lane = threadIdx.x % " << T << ";\n";
-    src << pe.str() << decl.str() << body.str() << "}\n";
+    src << pe.str() << decl.str();
+    for (auto& h : held)
+      src << "  __align__(16) " << s_type(h.second) << " hin" << h.first << "[" << rounds << "][" << V << "];\n";
+    if (!held.empty()) {
+      src << row_rounds << "      const " << it << " base = o * " << Nr << " + rb;\n";
+      for (auto& h : held) src << wide_move("hin" + std::to_string(h.first) + "[t]", "in" + std::to_string(h.first), V, (int)dt_size(h.second), true, 6);
+      src << "    }\n";
+    }
+    src << body.str() << "}\n";
     Launch L;
     L.kernel = add_kernel(src.str(), "row");
     L.grid[0] = (unsigned)((Nk + per_block - 1) / per_block); L.grid[1] = L.grid[2] = 1;
