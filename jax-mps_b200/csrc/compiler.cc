@@ -3560,9 +3560,10 @@ struct Planner {
   // product modelled alone / as one of two, us: 462 rows 1463 / 1400, 256 rows 1126 / 1102, 462 rows of 256 1019 / 900, 400 rows
   // of 768 1853 / 1772. A loop body is the other way about, its iterations are one chain: 6900 / 7330 us for a scan of 100 steps.
   //
-  static double in_company(int copies, const std::function<double(int)>& time) {
-    // a third of it as if alone: the one beside it may be much smaller
-    return copies == 1 ? time(1) : 0.65 * time(copies) + 0.35 * time(1);
+  static double in_company(int copies, const std::function<double(int)>& time, double share = 0.65) {
+    // a third of it as if alone: the one beside it may be much smaller (a tenth on the FMA pipe, where one product already keeps
+    // the SMs that it is on busy)
+    return copies == 1 ? time(1) : share * time(copies) + (1.0 - share) * time(1);
   }
   // Tile width and K split of a contraction by tiled copies (tile32.cu), and its time: 0.42 us per 64-wide and 0.64 per 128-wide
   // k-tile, 6.9 to launch, fill and drain, 1.9 and the partial sums at 6 TB/s for a split, the image of B at 4.4 TB/s.
@@ -3590,29 +3591,38 @@ struct Planner {
     return best + in_company(copies, [&](int n) { return (double)n * t.G * t.K * t.N * 12.0 / 4.4e6; }) + (b_is_weight ? 0.0 : 2.0);
   }
 
-  // Modelled time of a dense fp32 product on the FMA pipe (gemm32.cu), with its tile and split: 0.97 ns per row of four warps'
-  // FMA instructions and k (7 % less in the widest tile, which reads shared memory least; 10 % more for each operand without rows
-  // of 16 bytes; 13 % more for a B whose k is contiguous while nothing else on the SM hides its transposition), 3.4 us to launch,
-  // fill and drain, 1.7 for every further CTA of an SM, 1.13 for the sum of a cluster. Every tile and split over 140 chains from
-  // 6 x 64 x 256 to 1500 x 304 x 1304: 8 % rms error.
+  // Modelled time of a dense fp32 product on the FMA pipe (gemm32.cu), with its tile and split: 0.87 ns per row of four warps'
+  // FMA instructions and k (1.07 in the smallest tile, which reads shared memory most; 25 % more for a B whose k is contiguous, 10 %
+  // more for each operand without rows of 16 bytes), 1.75 us to launch, fill and drain, 3.7 for every further wave, 1.45 for the
+  // sum of a cluster. The tile of four warps, two CTAs of which share an SM, starts later and hides the fill and drain of one CTA
+  // behind the other: 2.75 us, 0.76 ns from the second CTA of an SM on, 1.8 for each. Every tile and split over 114 chains from
+  // 6 x 256 x 512 to 250 x 784 x 1000 and 180 from 250 x 784 x 1000 to 2019 x 174 x 3490: 8 % rms error.
   static double fma_product(Gemm32Launch& g, int copies) {
     if (g.G > 65535 || getenv("B200_NO_GEMM32")) return 1e30;
     double best = 1e30;
-    for (int tile = 2; tile >= 0; tile--) {
-      const int tm = tile == 0 ? 32 : 64, tn = tile == 2 ? 128 : 64;
+    for (int tile = 3; tile >= 0; tile--) {
+      const int tm = tile == 0 ? 32 : 64, tn = tile >= 2 ? 128 : 64;
       const long long tiles = (long long)((g.M + tm - 1) / tm) * ((g.N + tn - 1) / tn) * g.G;
-      for (int split = 1; split <= 4; split *= 2) {
+      for (int split = 1; split <= 8; split *= 2) {
         if (split > 1 && g.K < 32 * split) break;
         const long long chunk = ((g.K + split - 1) / split + 3) / 4 * 4;
         const double us = in_company(copies, [&](int n) {
-          const long long per_sm = n * tiles * split <= gemm32_resident(split) ? 1 : (n * tiles * split + 147) / 148;
-          const double row = 0.97e-3 * (tile == 2 ? 0.93 : 1.0) * (g.b_kc && per_sm == 1 ? 1.13 : 1.0) * (g.a_vec ? 1.0 : 1.1) * (g.b_vec ? 1.0 : 1.1);
-          return (double)per_sm * (tm * tn / 128) * (double)chunk * row + 3.4 + 1.7 * (double)(per_sm - 1) + (split > 1 ? 1.13 : 0.0);
-        });
+          const double odd = (g.a_vec ? 1.0 : 1.1) * (g.b_vec ? 1.0 : 1.1), sum = split > 1 ? (tile == 3 ? 1.25 : 1.45) : 0.0;
+          if (tile == 3) {
+            const long long per_sm = n * tiles * split <= gemm32_resident(split) ? 1 : (n * tiles * split + 147) / 148;
+            const double row = (per_sm == 1 ? 0.87e-3 : 0.76e-3) * (g.b_kc ? 1.19 : 1.0) * odd;
+            return (double)per_sm * (tm * tn / 128) * (double)chunk * row + 2.75 + 1.8 * (double)(per_sm - 1) + sum;
+          }
+          const long long waves = (n * tiles * split + gemm32_resident(split) - 1) / gemm32_resident(split);
+          const double row = (tile == 0 ? 1.07e-3 : 0.87e-3) * (g.b_kc ? 1.25 : 1.0) * odd;
+          return (double)waves * (tm * tn / 128) * (double)chunk * row + 1.75 + 3.7 * (double)(waves - 1) + sum;
+        }, 0.9);
         if (us < best * 0.97) { best = us; g.split = split; g.tile = tile; }
       }
     }
-    return best;
+    // One of several that run side by side holds whole SMs that the step's chain of kernels waits for: 17 weight gradients of
+    // 512 x 462 x 512 at a modelled 14.6 us here and 15.9 in the table-driven kernels made an f32 encoder step 1316 us, not 1286.
+    return copies > 1 ? 1.15 * best : best;
   }
   // ... and in the table-driven kernels, split as choose_split_k would: its k-tiles, 8.5 us for the first wave of CTAs and 4.8
   // for each further one, the partial sums at 3.3 TB/s (5 % rms error; the 6 us a wave of choose_split_k, which weighs splits

@@ -4,16 +4,20 @@
 // five times the arithmetic rate, but a CTA of theirs spends about 8 us on its way through table look-ups, tensor-memory
 // allocation, conversion and read-back before and after a handful of k-tiles, and their K splits need a second launch to
 // be added up. A recurrent cell's products (64 x 1024 x 512: 34 M multiply-adds, 1 us of the FMA pipe of the whole chip)
-// are all overhead there. Here a warp computes 32 x 64 outputs, 8 x 8 per thread, which makes every 16-byte shared load
-// feed 32 multiply-adds; the four warps of a CTA stand side by side (64 x 128 tile), or share the k of a stage between
-// two or four of them (64 x 64, 32 x 64), and two or four CTAs of one thread-block cluster may split K on top of that and
-// add their tiles through distributed shared memory, all sums in a fixed order and in the same launch. (Clusters of eight
-// do not fill the chip: with an SM per CTA 15 of them are resident, against 33 of four and 74 of two.) Operand tiles move
-// by cp.async (16 bytes where the layout allows, single floats otherwise) through a ring of three stages and stay in
+// are all overhead there. Here a warp computes 32 x 64 outputs, 8 x 8 per thread, two columns per FMA instruction; the eight
+// warps of a CTA share the k of a stage between two, four or eight of them (64 x 128, 64 x 64, 32 x 64 tiles; a grid of several
+// waves takes 64 x 128 tiles of four warps that do not, two CTAs to an SM), and two, four or
+// eight CTAs of one thread-block cluster may split K on top of that. The warps' tiles are added up in shared memory, every CTA
+// sends each of the others its part of the sum (stores to distributed shared memory, behind a barrier that was begun when the
+// kernel started), and adds what it was sent: one barrier to wait for, all sums in a fixed order, in the same launch. Operand
+// tiles move by cp.async (16 bytes where the layout allows, single floats otherwise) through a ring of three stages and stay in
 // shared memory as they lie in global memory: k-contiguous rows are read four k at a time, row-contiguous ones four rows
-// at a time, so neither layout is transposed. Bound by issue (64 FMA and 4 shared loads per k and thread, 1.3 - 1.7 times
-// the FMA floor) and, for the small ones, by the latency of the first loads and of the sums. Inside a replayed loop:
-// 64 x 512 x 512 5.6 us (10.3 as two tensor-core launches), 64 x 64 x 64 2.9 (6.3), 256 x 256 x 256 4.8 (11.4).
+// at a time, so neither layout is transposed. Bound by what shared memory gives to the registers (64 bytes per thread and k, 64
+// cycles of the SM's 128 bytes per cycle for the 64 cycles that the FMA instructions of four warps take: 0.87 ns per k and 64
+// instructions where either alone would take 0.52) and, for the small ones, by the latency of the first loads and of the sums.
+// Chains of products replayed as a graph, us a product, before (four warps, the other CTAs' tiles read behind a first and kept
+// until a second barrier) and now: 64 x 1024 x 512 7.6 / 6.1, 64 x 288 x 1024 7.1 / 5.8, 6 x 256 x 512 5.4 / 4.0,
+// 128 x 512 x 512 6.5 / 5.3, 250 x 784 x 1000 18.7 / 16.4; four k contiguous in B 8.1 / 7.6, 7.6 / 7.1, 5.8 / 4.2, 7.0 / 6.3, 20.8 / 19.3.
 #include <cuda_runtime.h>
 #include <cstdint>
 
@@ -24,25 +28,27 @@
 namespace b200 {
 namespace {
 
-constexpr int FSTAGES = 3, FTHREADS = 128;
+constexpr int FSTAGES = 3;
 
 // WM x WN warps side by side, WK of them sharing the k of a stage; FK: depth of a stage.
 template <int WM_, int WN_, int WK_>
 struct FmaCfg {
   static constexpr int WM = WM_, WN = WN_, WK = WK_;
-  static_assert(WM * WN * WK * 32 == FTHREADS, "four warps");
-  static constexpr int TM = 32 * WM, TN = 64 * WN, FK = WK == 4 ? 64 : 32;
+  static constexpr int THREADS = WM * WN * WK * 32;
+  static constexpr int TM = 32 * WM, TN = 64 * WN, FK = WK >= 4 ? 64 : 32;
   static constexpr int KROW = FK + 4;                           // row stride of k-contiguous tiles: 16-byte rows, spread over banks
   static constexpr int AROW = TM + 4, BROW = TN + 4;            // the same for row-contiguous ones
   static constexpr int A_FLOATS = TM * KROW > FK * AROW ? TM * KROW : FK * AROW;
   static constexpr int B_FLOATS = TN * KROW > FK * BROW ? TN * KROW : FK * BROW;
   static constexpr int STAGE = A_FLOATS + B_FLOATS;
-  static constexpr int SMEM = FSTAGES * STAGE * 4;
-  static_assert(FSTAGES * STAGE >= WK * TM * BROW, "the warps' partial tiles reuse the stages");
+  static constexpr int RING = FSTAGES * STAGE, INBOX = TM * TN;  // floats; the inbox takes the sums of the cluster's other CTAs
+  static constexpr int smem(int split) { return (RING + (split > 1 ? INBOX : 0)) * 4; }
+  static_assert(RING >= WK * TM * BROW, "the warps' partial tiles reuse the stages");
 };
 // Asked for instead when every CTA can have an SM to itself: the CTAs of a cluster are otherwise packed two to an SM while
 // other SMs stand idle.
 constexpr int F_SMEM_ALONE = 118 * 1024;
+static_assert(FmaCfg<1, 1, 8>::smem(2) <= F_SMEM_ALONE && FmaCfg<2, 1, 4>::smem(2) <= F_SMEM_ALONE && FmaCfg<2, 2, 2>::smem(2) <= F_SMEM_ALONE, "");
 
 bool g_programmatic = true;
 
@@ -53,15 +59,26 @@ __device__ __forceinline__ void copy4(uint32_t dst, const float* src, bool valid
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(valid ? 4 : 0) : "memory");
 }
 
+// c += a * (bx, by), each product and sum rounded as fmaf does. PAIR: in one instruction (fma.rn.f32x2), where bx and by were
+// loaded side by side; packing them first costs more than it saves.
+template <bool PAIR>
+__device__ __forceinline__ void fma2(float2& c, float a, float bx, float by) {
+  if (PAIR)
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %2};\n\tmov.b64 y, {%3, %4};\n\tmov.b64 z, {%0, %1};\n\t"
+        "fma.rn.f32x2 z, x, y, z;\n\tmov.b64 {%0, %1}, z;\n\t}"
+        : "+f"(c.x), "+f"(c.y) : "f"(a), "f"(bx), "f"(by));
+  else { c.x = fmaf(a, bx, c.x); c.y = fmaf(a, by, c.y); }
+}
+
 // One operand's tile of T outer indices (m or n) by FK k, stage after stage. KC: k is contiguous (outer stride `ld`), else
 // the outer index is (k stride `ld`). VEC: 16-byte copies. What does not change from stage to stage is worked out once.
-template <int T, int FK, bool KC, bool VEC>
+template <int T, int FK, bool KC, bool VEC, int THREADS>
 struct Loader {
   static constexpr int PER = VEC ? 4 : 1;                       // floats per copy
-  static constexpr int COUNT = T * FK / PER / FTHREADS;
+  static constexpr int COUNT = T * FK / PER / THREADS;
   static constexpr int LINE = (KC ? FK : T) / PER;              // copies along memory
-  static constexpr int STEP = FTHREADS / LINE;                  // lines between a thread's copies
-  static_assert(FTHREADS % LINE == 0, "a thread keeps its place in the line");
+  static constexpr int STEP = THREADS / LINE;                  // lines between a thread's copies
+  static_assert(THREADS % LINE == 0, "a thread keeps its place in the line");
   const float *src, *at;                                        // a valid address; this thread's first element of the next stage
   long long step, advance;
   uint32_t dst, fine = 0;                                       // fine: which copies have their outer index inside
@@ -92,10 +109,10 @@ struct Loader {
 };
 
 template <class Cfg, bool AKC, bool BKC, bool AVEC, bool BVEC>
-__global__ void __launch_bounds__(FTHREADS) gemm32_kernel(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C,
+__global__ void __launch_bounds__(Cfg::THREADS) gemm32_kernel(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C,
                                                         Gemm32Launch p) {
   extern __shared__ __align__(16) float f_smem[];
-  constexpr int TM = Cfg::TM, TN = Cfg::TN, FK = Cfg::FK, KROW = Cfg::KROW;
+  constexpr int TM = Cfg::TM, TN = Cfg::TN, FK = Cfg::FK, KROW = Cfg::KROW, THREADS = Cfg::THREADS;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lx = lane & 7, ly = lane >> 3;
   const int wk = warp % Cfg::WK, wm = warp / Cfg::WK % Cfg::WM, wn = warp / (Cfg::WK * Cfg::WM);
   const int S = p.split, rank = blockIdx.x % S, tile = blockIdx.x / S;
@@ -110,8 +127,9 @@ __global__ void __launch_bounds__(FTHREADS) gemm32_kernel(const float* __restric
   // (neighbouring lanes read neighbouring rows), else two runs of four
   auto row = [&](int i) { return 32 * wm + (AKC ? ly + 4 * i : 16 * (i >> 2) + 4 * ly + (i & 3)); };
   auto col = [&](int j) { return 64 * wn + (BKC ? lx + 8 * j : 32 * (j >> 2) + 4 * lx + (j & 3)); };
-  Loader<TM, FK, AKC, AVEC> la(Ag, p.a_ld, m0, p.M, kbeg, tid);
-  Loader<TN, FK, BKC, BVEC> lb(Bg, p.b_ld, n0, p.N, kbeg, tid);
+  Loader<TM, FK, AKC, AVEC, THREADS> la(Ag, p.a_ld, m0, p.M, kbeg, tid);
+  Loader<TN, FK, BKC, BVEC, THREADS> lb(Bg, p.b_ld, n0, p.N, kbeg, tid);
+  if (S > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");    // every CTA of the cluster is there: waited for in front of the exchange
   pdl_prologue();
   auto load = [&](int s) {
     if (s < steps) {
@@ -121,11 +139,11 @@ __global__ void __launch_bounds__(FTHREADS) gemm32_kernel(const float* __restric
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  float acc[8][8];
+  float2 acc[8][4];                                  // two columns each
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
 #pragma unroll
   for (int s = 0; s < FSTAGES - 1; ++s) load(s);
   for (int s = 0; s < steps; ++s) {
@@ -153,7 +171,7 @@ __global__ void __launch_bounds__(FTHREADS) gemm32_kernel(const float* __restric
 #pragma unroll
         for (int i = 0; i < 8; ++i)
 #pragma unroll
-          for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i][k], b[j][k], acc[i][j]);
+          for (int j = 0; j < 4; ++j) fma2<!BKC>(acc[i][j], a[i][k], b[2 * j][k], b[2 * j + 1][k]);
     }
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
@@ -168,60 +186,68 @@ __global__ void __launch_bounds__(FTHREADS) gemm32_kernel(const float* __restric
     if (n + 2 < p.N) out[2] = v.z;
     if (n + 3 < p.N) out[3] = v.w;
   };
-  if (S == 1 && Cfg::WK == 1) {
+  if (Cfg::WK == 1 && S == 1) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int m = m0 + row(i);
-      if (!BKC) {
 #pragma unroll
-        for (int j = 0; j < 8; j += 4) store4(m, n0 + col(j), make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]));
-      } else {
+      for (int j = 0; j < 8; j += 4) {
+        const float2 u = acc[i][j / 2], v = acc[i][j / 2 + 1];
+        if (!BKC) store4(m, n0 + col(j), make_float4(u.x, u.y, v.x, v.y));
+        else {
+          const float w[4] = {u.x, u.y, v.x, v.y};
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if (m < p.M && n0 + col(j) < p.N) Cg[(long long)m * p.N + n0 + col(j)] = acc[i][j];
+          for (int q = 0; q < 4; ++q)
+            if (m < p.M && n0 + col(j + q) < p.N) Cg[(long long)m * p.N + n0 + col(j + q)] = w[q];
+        }
       }
     }
     return;
   }
-  // the partial tiles of the WK warps and of the cluster's CTAs, in shared memory; CTA r adds rows TM / S * r .. of all
-  // of them, by rank and then by warp
+  // the WK warps' partial tiles meet in shared memory, a thread adds up its quads of them in the order of the warps
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     float* to = f_smem + (wk * TM + row(i)) * Cfg::BROW;
 #pragma unroll
     for (int j = 0; j < 8; j += 4) {
-      if (!BKC) *reinterpret_cast<float4*>(to + col(j)) = make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
-      else { to[col(j)] = acc[i][j]; to[col(j + 1)] = acc[i][j + 1]; to[col(j + 2)] = acc[i][j + 2]; to[col(j + 3)] = acc[i][j + 3]; }
+      const float2 u = acc[i][j / 2], v = acc[i][j / 2 + 1];
+      if (!BKC) *reinterpret_cast<float4*>(to + col(j)) = make_float4(u.x, u.y, v.x, v.y);
+      else { to[col(j)] = u.x; to[col(j + 1)] = u.y; to[col(j + 2)] = v.x; to[col(j + 3)] = v.y; }
     }
   }
-  if (S > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-  else __syncthreads();
-  const int rows = TM / S;
-  for (int e = tid; e < rows * (TN / 4); e += FTHREADS) {
-    const int r = rank * rows + e / (TN / 4), c = (e % (TN / 4)) * 4;
-    const uint32_t at = smem_u32(f_smem + r * Cfg::BROW + c);
-    float4 v[4][Cfg::WK];                            // all loads in flight together
+  __syncthreads();
+  if (S > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  const int rows = TM / S;                           // CTA r of the cluster gives out rows `rows` * r ..
+  float* inbox = f_smem + Cfg::RING;                 // [sender][row][column]
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if (q >= S) break;
-      uint32_t peer = at;
-      if (S > 1) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(at), "r"(q));
+  for (int e0 = 0; e0 < TM * (TN / 4); e0 += THREADS) {
+    const int e = e0 + tid, r = e / (TN / 4), c = (e % (TN / 4)) * 4;
+    float4 sum = *reinterpret_cast<const float4*>(f_smem + r * Cfg::BROW + c);
 #pragma unroll
-      for (int w = 0; w < Cfg::WK; ++w)
-        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                     : "=f"(v[q][w].x), "=f"(v[q][w].y), "=f"(v[q][w].z), "=f"(v[q][w].w) : "r"(peer + (uint32_t)(w * TM * Cfg::BROW * 4)) : "memory");
+    for (int w = 1; w < Cfg::WK; ++w) {
+      const float4 v = *reinterpret_cast<const float4*>(f_smem + (w * TM + r) * Cfg::BROW + c);
+      sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
     }
-    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if (q >= S) break;
-#pragma unroll
-      for (int w = 0; w < Cfg::WK; ++w) { sum.x += v[q][w].x; sum.y += v[q][w].y; sum.z += v[q][w].z; sum.w += v[q][w].w; }
-    }
-    store4(m0 + r, n0 + c, sum);
+    if (S == 1) { store4(m0 + r, n0 + c, sum); continue; }
+    uint32_t to;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(smem_u32(inbox + (rank * rows + r % rows) * TN + c)), "r"(r / rows));
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to), "f"(sum.x), "f"(sum.y), "f"(sum.z), "f"(sum.w) : "memory");
   }
-  if (S > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // nobody leaves while its tile is read
+  if (S == 1) return;
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  for (int e = tid; e < rows * (TN / 4); e += THREADS) {
+    const int r = e / (TN / 4), c = (e % (TN / 4)) * 4;
+    float4 v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (q < S) v[q] = *reinterpret_cast<const float4*>(inbox + (q * rows + r) * TN + c);
+    float4 sum = v[0];
+#pragma unroll
+    for (int q = 1; q < 8; ++q)
+      if (q < S) { sum.x += v[q].x; sum.y += v[q].y; sum.z += v[q].z; sum.w += v[q].w; }
+    store4(m0 + rank * rows + r, n0 + c, sum);
+  }
 }
 
 template <class Cfg, bool AKC, bool BKC, bool AVEC, bool BVEC>
@@ -232,8 +258,8 @@ cudaError_t launch(const Gemm32Launch& p, const float* A, const float* B, float*
     if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F_SMEM_ALONE)) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(((p.M + Cfg::TM - 1) / Cfg::TM) * (long long)((p.N + Cfg::TN - 1) / Cfg::TN) * p.split), (unsigned)p.G, 1);
-  cfg.blockDim = dim3(FTHREADS, 1, 1);
-  cfg.dynamicSmemBytes = (long long)cfg.gridDim.x * p.G <= gemm32_resident(p.split) ? F_SMEM_ALONE : Cfg::SMEM;
+  cfg.blockDim = dim3(Cfg::THREADS, 1, 1);
+  cfg.dynamicSmemBytes = (long long)cfg.gridDim.x * p.G <= gemm32_resident(p.split) ? F_SMEM_ALONE : Cfg::smem(p.split);
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   int n = 0;
@@ -271,8 +297,9 @@ void set_gemm32_programmatic_launch(bool on) { g_programmatic = on; }
 cudaError_t launch_gemm32(const Gemm32Launch& p, const void* A, const void* B, void* C, cudaStream_t stream, int* launches) {
   if (p.G > 65535) return cudaErrorInvalidValue;
   const float *a = (const float*)A, *b = (const float*)B;
-  cudaError_t e = p.tile == 0   ? launch_layout<FmaCfg<1, 1, 4>>(p, a, b, (float*)C, stream)
-                  : p.tile == 1 ? launch_layout<FmaCfg<2, 1, 2>>(p, a, b, (float*)C, stream)
+  cudaError_t e = p.tile == 0   ? launch_layout<FmaCfg<1, 1, 8>>(p, a, b, (float*)C, stream)
+                  : p.tile == 1 ? launch_layout<FmaCfg<2, 1, 4>>(p, a, b, (float*)C, stream)
+                  : p.tile == 2 ? launch_layout<FmaCfg<2, 2, 2>>(p, a, b, (float*)C, stream)
                                 : launch_layout<FmaCfg<2, 2, 1>>(p, a, b, (float*)C, stream);
   if (e == cudaSuccess) ++*launches;
   return e;
