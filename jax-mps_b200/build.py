@@ -14,7 +14,7 @@ CSRC = HERE / "csrc"
 OUT = HERE / "b200" / "libb200core.so"
 # named for the interpreter it is built for: it uses structures of CPython that differ between versions
 HOT = HERE / "b200" / ("_hot" + sysconfig.get_config_var("EXT_SUFFIX"))
-SOURCES = ["parser.cc", "codegen.cc", "compiler.cc", "runtime.cc", "kernels.cu", "gemm16.cu", "gemm32.cu", "tile32.cu"]
+SOURCES = ["parser.cc", "codegen.cc", "compiler.cc", "loops.cc", "runtime.cc", "kernels.cu", "gemm16.cu", "gemm32.cu", "tile32.cu"]
 
 
 def _nccl_include() -> str:

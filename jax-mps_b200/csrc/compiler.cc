@@ -22,6 +22,7 @@
 #include <sstream>
 
 #include "codegen.h"
+#include "loops.h"
 #include "plan.h"
 
 namespace b200 {
@@ -3939,7 +3940,7 @@ struct Planner {
         const double us_fma = fma_product(g, copies);
         double us_table = table_product(g, split_k, copies), us_tile = 1e30;
         // the switches that keep products off the tensor cores or tiled copies leave them to the FMA pipe
-        const bool tiles = opts.tensor_cores && !getenv("B200_NO_TILE32");
+        const bool tiles = opts.tensor_cores && !getenv("B200_NO_TILE32") && !op->has("b200.fma");
         if (!tiles) us_table = 1e30;
         // Below a tile of rows or four k-tiles tiled copies are never the fastest (M x K x N, FMA / tables / tiles, us:
         // 96 x 512 x 2048 14.6 / 13.8 / 14.3, 96 x 2048 x 2048 33 / 19 / 29, 2048 x 64 x 512 8.5 / 10.8 / 9.9).
@@ -6000,6 +6001,7 @@ std::unique_ptr<CompiledProgram> compile_module(Module& m, const CompileOptions&
   Inliner inl(m);
   inl.run(f->body.get());
   fix_region_operands(f->body.get(), inl);
+  if (opts.fuse && !getenv("B200_NO_LOOP_SPLIT")) split_counted_loops(m, f->body.get());
   SkinnyWeightHoist(m).run(f->body.get());
   DecodeAttentionFusion(m).run(f->body.get());
   // unsupported-op check names every offender at once (src/pjrt_plugin/stablehlo_parser.cc:167-184)
