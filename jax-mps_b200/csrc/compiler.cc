@@ -5566,7 +5566,7 @@ struct Planner {
       if (v->def && v->def->parent == block && is_dup(v->def)) { materialize_dup(v->def, plan, st); continue; }
       throw CompileError("internal: returned value without storage: " + v->name);
     }
-    bundle_independent_kernels(plan);
+    bundle_independent_kernels(plan, block->parent_op && block->parent_op->short_name() == "while" && graph_safe(plan));
   }
 
   // ---- bundling of independent pointwise kernels --------------------------------------
@@ -5620,8 +5620,31 @@ struct Planner {
     return add_kernel(src.str(), "bundle");
   }
 
-  void bundle_independent_kernels(Plan& plan) {
+  // The iterations of a recorded loop body run into one another as far as their dependences allow, and a bundle waits for what
+  // any of its parts waits for: there only parts become one that wait for the same last kernel of the iteration and for the same
+  // carried tensors (scalars, loop counters and positions, are there early). A scan of two recurrent layers bundled by adjacency
+  // ran the layers of all steps one after the other, 5390 us for forward and reverse; with this the second layer of a step runs
+  // beside the first layer of the next, 4617 us.
+  void bundle_independent_kernels(Plan& plan, bool recorded_body) {
     if (getenv("B200_NO_BUNDLES")) return;
+    std::vector<std::set<int>> waits(recorded_body ? plan.steps.size() : 0);       // slots carried or made in front of the loop; -1 - the last kernel
+    if (recorded_body) {
+      std::map<int, int> writer;
+      for (size_t k = 0; k < plan.steps.size(); k++) {
+        const Step& s = plan.steps[k];
+        int last = -1;
+        for (size_t a = s.kind == Step::KERNEL ? s.n_outs : 0; a < s.args.size(); a++) {
+          auto it = writer.find(s.args[a]);
+          const Slot& sl = prog.slots[s.args[a]];
+          if (it != writer.end()) last = std::max(last, it->second);
+          else if (sl.kind == Slot::TEMP && sl.arena != plan.arena && sl.type.numel() > 1) waits[k].insert(s.args[a]);
+        }
+        waits[k].insert(-1 - last);
+        if (s.kind == Step::KERNEL)
+          for (int a = 0; a < s.n_outs; a++) writer[s.args[a]] = (int)k;
+        else for (int a : s.args) writer[a] = (int)k;
+      }
+    }
     auto eligible = [&](const Step& s) {
       return s.kind == Step::KERNEL && s.block[0] == (unsigned)kThreads && s.block[1] == 1 && s.block[2] == 1 && s.grid[1] == 1 &&
              s.grid[2] == 1 && s.n_outs > 0 && prog.kernels[s.kernel].name.rfind("fused_", 0) == 0;
@@ -5636,6 +5659,7 @@ struct Planner {
       for (; j < plan.steps.size() && j - i < 16; j++) {
         const Step& s = plan.steps[j];
         if (!eligible(s) || nargs + s.args.size() > 256 || (uint64_t)blocks + s.grid[0] > (1u << 30)) break;
+        if (recorded_body && waits[j] != waits[i]) break;
         bool clash = false;
         for (size_t a = 0; a < s.args.size(); a++) {
           const bool w = (int)a < s.n_outs;
