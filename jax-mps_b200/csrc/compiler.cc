@@ -2708,7 +2708,7 @@ struct Planner {
   // on its way; then every row below is a thread that substitutes through the diagonal block; then all threads subtract
   // the panel's product from the trailing triangle, which stays in the result (L2), in tiles of 4 x 4 or, near the end,
   // 2 x 2. Panels pass between memory and shared memory by rows, so that both sides are coalesced. 160 x 160, eight
-  // matrices: 756 us for a block that updated the trailing triangle element by element after each column, 43 us now
+  // matrices: 756 us for a block that updated the trailing triangle element by element after each column, 43 us this way
   // (per panel 3.0 us diagonal, 1.4 us rows below, 1 - 6 us triangle). NB is 32 while NB columns fit static shared memory.
   // Only the named triangle of the input is read; the other triangle of the result is zero. A matrix that is not
   // positive definite gives NaN from its first bad pivot on.
@@ -2733,6 +2733,235 @@ struct Planner {
     while (nb > 1 && nb * np * es + nb * (nb + 2) * es > 46 * 1024) nb /= 2;
     const bool paneled = nb >= 4;                          // narrower panels than that (n above 2800 in f32): column by column
     const int threads = !paneled ? kThreads : n <= 32 ? 64 : n <= 96 || es > 4 ? 256 : 640;
+    // f32 matrices of 33 to 208 rows stay in the registers of their block from the first load on, as pieces of 4 rows x 8 columns
+    // of the lower triangle, column by column over the tile warps, at most two a thread (8 columns to 4 rows, so that three
+    // 16-byte reads of shared memory feed 32 multiply-adds: with 4 x 4 tiles those reads set the time of the first panels); a
+    // thread of the row warps stands for a row. The time is the chain of pivots, so nothing is exchanged along it: for every panel
+    // of eight columns each row thread takes the 8 x 8 diagonal block and factors it for itself, its own row on the way (a pivot is a
+    // root, a quotient and a multiply-add behind the one before), and brings its row of the next panel up to date, while the tile
+    // warps do that for the columns behind it. Two block barriers a panel. 160 x 160, eight matrices: 48.7 us with panels of 32 and the
+    // trailing triangle in L2 (below, which larger and f64 matrices keep: beyond 208 rows the pieces do not fit the registers), 28.5 us
+    // so; whole solves of 34 rows 18.9 -> 11.1 us, 100 rows 46.8 -> 23.9, 208 rows 139 -> 96.
+    const int64_t nt = (n + 3) / 4, tiles = nt + (nt / 2) * ((nt - 1) / 2), row_warps = (n + 31) / 32, tile_warps = std::min<int64_t>(18 - row_warps, (tiles + 31) / 32);
+    if (es == 4 && n > 32 && tiles <= 2 * 32 * tile_warps) {
+      std::ostringstream rs;
+      const int64_t th = 32 * (row_warps + tile_warps);
+      rs << "extern \"C\" __global__ void __launch_bounds__(" << th << ") @NAME@(" << signature({out}, {a}) << ") {\n";
+      rs << "#define AT(i, j) (" << at << ")\n  typedef " << T << " T;\n  const int N = " << n << ", NT = " << nt << ", NB = 8, NP = " << np << ", RT = " << 32 * row_warps << ", TT = " << 32 * tile_warps
+         << ", TPT = " << (tiles + 32 * tile_warps - 1) / (32 * tile_warps) << ";\n";
+      rs << "  const bool LOWER = " << (lower ? "true" : "false") << ", ALIGNED = " << (n % 4 == 0 ? "true" : "false") << ";\n";
+      rs << "  T* o = out0 + (long long)blockIdx.x * N * N;\n  const T* a = in0 + (long long)blockIdx.x * N * N;\n";
+      rs << R"SRC(  struct alignas(16) V4 { T v[4]; };
+  __shared__ V4 raw4[2][NB * NP / 4 + 1];            // columns of the next panel less what panels before this one take: [column][row of the matrix]
+  __shared__ V4 final4[2][NB * NP / 4 + 1];          // columns of the factor, this panel's and the one's in front
+  __shared__ V4 diag4[NB * NB / 4];                  // [column][row] of the panel's diagonal block
+  const int tid = threadIdx.x;
+  if (tid < RT) {
+    // ---- row warps ----
+    const int i = tid;
+    T x[NB];                                         // this thread's row of the panel
+    auto write = [&](int c0, const T* x) {           // the panel's columns of this row, zero behind the diagonal
+      if (i >= N) return;
+      if (LOWER && ALIGNED) {
+#pragma unroll
+        for (int h = 0; h < NB; h += 4) {
+          V4 t;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) t.v[k] = c0 + h + k <= i ? x[h + k] : (T)0;
+          if (c0 + h < N) *(V4*)&o[AT(i, c0 + h)] = t;
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < NB; ++k)
+          if (c0 + k < N) o[AT(i, c0 + k)] = c0 + k <= i ? x[k] : (T)0;
+      }
+    };
+    __syncthreads();
+    if (i < N) {
+#pragma unroll
+      for (int k = 0; k < NB; ++k) {
+        x[k] = ((const T*)raw4[0])[k * NP + i];
+        if (i < NB) ((T*)diag4)[k * NB + i] = x[k];
+      }
+    }
+    __syncthreads();
+    for (int c0 = 0; c0 < N; c0 += NB) {
+      T* F = (T*)final4[(c0 / NB) & 1];
+      if ((tid | 31) >= c0) {
+        T m[NB][NB], xr[NB];                         // the diagonal block, of the identity past the matrix; the row as it was
+        bool fine = true;
+        auto fetch = [&]() {
+#pragma unroll
+          for (int k = 0; k < NB; ++k) {
+            const V4 lo = diag4[k * (NB / 4)], hi = diag4[k * (NB / 4) + 1];
+#pragma unroll
+            for (int r = 0; r < NB; ++r)
+              if (r >= k) m[r][k] = c0 + r < N ? (r < 4 ? lo.v[r] : hi.v[r - 4]) : (T)(r == k ? 1 : 0);
+          }
+        };
+        fetch();
+#pragma unroll
+        for (int k = 0; k < NB; ++k) xr[k] = x[k];
+#pragma unroll
+        for (int j = 0; j < NB; ++j) {
+          T root, inv;
+          fine = lin_pivot(m[j][j], root, inv) && fine;
+#pragma unroll
+          for (int r = j + 1; r < NB; ++r) m[r][j] = lin_quotient(m[r][j], root, inv);
+          x[j] = i == c0 + j ? root : lin_quotient(x[j], root, inv);
+#pragma unroll
+          for (int k = j + 1; k < NB; ++k) {
+            x[k] = x[k] - x[j] * m[k][j];
+#pragma unroll
+            for (int r = k; r < NB; ++r) m[r][k] = m[r][k] - m[r][j] * m[k][j];
+          }
+        }
+        if (!fine) {                                 // the same with plain roots and divisions
+          fetch();
+#pragma unroll
+          for (int k = 0; k < NB; ++k) x[k] = xr[k];
+#pragma unroll 1
+          for (int j = 0; j < NB; ++j) {
+            T root = (T)0, xj = (T)0, col[NB];
+#pragma unroll
+            for (int q = 0; q < NB; ++q)
+              if (q == j) {
+                root = op_sqrt(m[q][q]);
+                xj = i == c0 + q ? root : x[q] / root;
+                x[q] = xj;
+#pragma unroll
+                for (int r = 0; r < NB; ++r) col[r] = r > q ? m[r][q] / root : (T)0;
+              }
+#pragma unroll
+            for (int k = 1; k < NB; ++k)
+              if (k > j) {
+                x[k] = x[k] - xj * col[k];
+#pragma unroll
+                for (int r = 1; r < NB; ++r)
+                  if (r >= k) m[r][k] = m[r][k] - col[r] * col[k];
+              }
+          }
+        }
+        if (i >= c0 && i < N) {
+#pragma unroll
+          for (int k = 0; k < NB; ++k) F[k * NP + i] = x[k];
+        }
+      }
+      __syncthreads();
+      // the next panel's columns of this row, less what this panel takes
+      T next[NB];
+#pragma unroll
+      for (int k = 0; k < NB; ++k) next[k] = (T)0;
+      if (c0 + NB < N && i >= c0 + NB && i < N) {
+        const V4* G = final4[(c0 / NB) & 1];
+        const T* R = (const T*)raw4[(c0 / NB + 1) & 1];
+#pragma unroll
+        for (int k = 0; k < NB; ++k) next[k] = R[k * NP + i];
+#pragma unroll
+        for (int j = 0; j < NB; ++j) {
+          const V4 lo = G[(j * NP + c0 + NB) / 4], hi = G[(j * NP + c0 + NB) / 4 + 1];
+#pragma unroll
+          for (int k = 0; k < NB; ++k) next[k] = next[k] - x[j] * (k < 4 ? lo.v[k] : hi.v[k - 4]);
+        }
+        if (i < c0 + 2 * NB) {
+#pragma unroll
+          for (int k = 0; k < NB; ++k) ((T*)diag4)[k * NB + i - c0 - NB] = next[k];
+        }
+      }
+      __syncthreads();
+      write(c0, x);
+#pragma unroll
+      for (int k = 0; k < NB; ++k) x[k] = next[k];
+    }
+    return;
+  }
+  // ---- tile warps ----
+  const int u = tid - RT;
+  int ti[TPT], tp[TPT];                              // this thread's pieces: rows 4 ti .., columns 8 tp .. (tp < 0: none)
+  T c[TPT][2][4][4];
+#pragma unroll
+  for (int q = 0; q < TPT; ++q) {
+    // columns of NT, NT - 2, NT - 4 .. pieces
+    int e = u + q * TT, p = 0;
+    while (p < (NT + 1) / 2 && e >= NT - 2 * p) { e -= NT - 2 * p; ++p; }
+    const bool mine = p < (NT + 1) / 2;
+    tp[q] = mine ? p : -1;
+    ti[q] = mine ? 2 * p + e : 0;
+    const int i0 = 4 * ti[q];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int k0 = 8 * p + 4 * h;
+      if (ALIGNED) {                                 // lines of four in memory; what lies behind the diagonal is loaded and not used
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+          V4 t = {{(T)0, (T)0, (T)0, (T)0}};
+          if (mine && k0 < N) t = *(const V4*)&a[LOWER ? AT(i0 + l, k0) : AT(i0, k0 + l)];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) c[q][h][LOWER ? l : e][LOWER ? e : l] = t.v[e];
+        }
+      } else {
+#pragma unroll
+        for (int y = 0; y < 4; ++y)
+#pragma unroll
+          for (int x = 0; x < 4; ++x) c[q][h][y][x] = (mine && i0 + y < N && k0 + x <= i0 + y) ? a[AT(i0 + y, k0 + x)] : (T)0;
+      }
+    }
+  }
+  // rows past the matrix are zero in every panel
+  for (int e = u; e < 2 * NB * (NP - N); e += TT) ((T*)final4[0])[(e / (NP - N)) * NP + N + e % (NP - N)] = (T)0;
+  auto update = [&](int q, const V4* from) {         // piece q less what the panel's columns take from it
+#pragma unroll
+    for (int k = 0; k < NB; ++k) {
+      const V4 pi = from[k * (NP / 4) + ti[q]];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const V4 pk = from[k * (NP / 4) + 2 * tp[q] + h];
+#pragma unroll
+        for (int y = 0; y < 4; ++y)
+#pragma unroll
+          for (int x = 0; x < 4; ++x) c[q][h][y][x] = c[q][h][y][x] - pi.v[y] * pk.v[x];
+      }
+    }
+  };
+  auto publish = [&](int q) {
+    V4* to = raw4[tp[q] & 1];
+#pragma unroll
+    for (int k = 0; k < NB; ++k) {
+      V4 t;
+#pragma unroll
+      for (int y = 0; y < 4; ++y) t.v[y] = c[q][k / 4][y][k % 4];
+      to[k * (NP / 4) + ti[q]] = t;
+    }
+  };
+#pragma unroll
+  for (int q = 0; q < TPT; ++q)
+    if (tp[q] == 0 || tp[q] == 1) publish(q);
+  __syncthreads();
+  __syncthreads();
+  for (int p = 0; p * NB < N; ++p) {
+    __syncthreads();                                 // the panel is final
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < TPT; ++q)
+      if (tp[q] > p + 1) {
+        update(q, final4[p & 1]);
+        if (tp[q] == p + 2) publish(q);
+      }
+  }
+#undef AT
+}
+)SRC";
+      Step s;
+      s.kind = Step::KERNEL;
+      s.kernel = add_kernel(rs.str(), "cholesky");
+      s.label = op->name;
+      s.grid[0] = (unsigned)batch; s.grid[1] = s.grid[2] = 1;
+      s.block[0] = (unsigned)th; s.block[1] = s.block[2] = 1;
+      s.args = {slot_of.at(out), slot_of.at(a)};
+      s.n_outs = 1;
+      plan.steps.push_back(std::move(s));
+      return;
+    }
     std::ostringstream src;
     src << "extern \"C\" __global__ void __launch_bounds__(" << threads << ") @NAME@(" << signature({out}, {a}) << ") {\n";
     src << "#define AT(i, j) (" << at << ")\n";
@@ -2935,13 +3164,14 @@ struct Planner {
   }
 
   // stablehlo.triangular_solve (src/pjrt_plugin/ops/linalg.cc:573-660 of the reference): op(A) X = B or X op(A) = B for a
-  // batch of triangular A. A warp per right-hand-side vector: lane l owns the unknowns l, l + 32, ... in registers, and
-  // step j hands unknown j to all lanes by a shuffle, which subtract its column from the rows they own. The chain per
-  // unknown is one shuffle and four dependent multiply-adds, whatever n is, as long as the matrix is at hand: its
-  // columns come in panels of NB through shared memory, the next panel in flight in registers meanwhile. A block holds
-  // four or eight vectors of one matrix: more would queue for shared memory (n / 32 reads a step and warp). 160 x 160,
-  // eight matrices, twelve vectors: 712 us for a thread per vector that read the matrix and its unknowns back from
-  // memory, 15 us now. Above n = 1024 (32 unknowns in a lane) the thread per vector stays. As in the reference, a
+  // batch of triangular A. A warp per right-hand-side vector: lane l owns the unknowns l, l + 32, ... in registers. Eight
+  // right-hand sides at a time are handed to all lanes by shuffles, every lane solves for the eight unknowns itself and
+  // subtracts their columns from the rows it owns: the chain per unknown is a quotient and a multiply-add, whatever n is, as
+  // long as the matrix is at hand: its columns come in panels of NB through shared memory, the next panel in flight in
+  // registers meanwhile. Pivots too small or large for the quick quotient (a branch in the chain otherwise) go one by one. The
+  // loop over the eights stays rolled: unrolled, the instructions of a kernel that runs them once came too slowly (22 us). A
+  // block holds four or eight vectors of one matrix: more would queue for shared memory (n / 32 reads a step and warp). 160 x
+  // 160, eight matrices, twelve vectors: 13.9 us with a shuffle between one unknown and the next, 9.2 us now. Above n = 1024 (32 unknowns in a lane) the thread per vector stays. As in the reference, a
   // matrix with a zero on a diagonal that counts gives NaN for its whole solution.
   void lower_triangular_solve(Op* op, Plan& plan, BlockState& st) {
     if (op->operands.size() != 2 || op->results.size() != 1) throw CompileError("stablehlo.triangular_solve: malformed operands");
@@ -2977,7 +3207,7 @@ struct Planner {
       int64_t nb = 32;
       while (nb > 1 && nb * np * es > 46 * 1024) nb /= 2;
       const int64_t groups = (vecs_per + per_block - 1) / per_block;
-      src << "  typedef " << T << " T;\n  const int NB = " << nb << ", NP = " << np << ", NR = " << (n + 31) / 32 << ", VB = " << per_block << ", TH = " << kThreads << ";\n";
+      src << "  typedef " << T << " T;\n  const int NB = " << nb << ", NP = " << np << ", SB = NB < 8 ? NB : 8, NR = " << (n + 31) / 32 << ", VB = " << per_block << ", TH = " << kThreads << ";\n";
       src << "  const long long g = blockIdx.x / " << groups << "u;\n  const int v = (int)(blockIdx.x % " << groups << "u) * VB + (int)(threadIdx.x >> 5);\n";
       src << "  const T* A = in0 + g * N * N;\n";
       // unknowns in the order they are found: U(i) is the row of unknown i
@@ -2987,9 +3217,10 @@ struct Planner {
       src << "#define COL(q) " << (flip ? "((q) / N)" : "((q) % NB)") << "\n#define ROW(q) " << (flip ? "((q) % N)" : "((q) / NB)") << "\n";
       src << "#define M(i, j) A[" << (flip ? "(long long)U(j) * N + U(i)" : "(long long)U(i) * N + U(j)") << "]\n";
       src << "  const bool UNIT = " << (unit ? "true" : "false") << ";\n";
-      src << R"SRC(  __shared__ T panel[NB * NP];                       // [column of the panel][row]
+      src << R"SRC(  __shared__ T panel[NB * NP + 32];                  // [column of the panel][row]; rows past the matrix are read and not used
   const int tid = threadIdx.x, lane = tid & 31;
   const bool mine = (tid >> 5) < VB && v < )SRC" << vecs_per << R"SRC(;
+  __shared__ T pivot[NB], inverse[NB];
   __shared__ int singular;
   if (tid == 0) singular = 0;
   bool zero = false;
@@ -2999,13 +3230,14 @@ struct Planner {
 #pragma unroll
   for (int r = 0; r < NR; ++r) acc[r] = (mine && lane + 32 * r < N) ? in1[X(lane + 32 * r)] : (T)0;
   const int PF = (NB * N + TH - 1) / TH;             // elements of a panel per thread
-  T next[PF];
+  T next[PF], pv = (T)1;
   auto fetch = [&](int c0) {
 #pragma unroll
     for (int k = 0; k < PF; ++k) {
       const int q = tid + k * TH, c = c0 + COL(q), i = ROW(q);
       next[k] = (q < NB * N && c < N && i >= c) ? M(i, c) : (T)0;
     }
+    pv = (!UNIT && tid < NB && c0 + tid < N) ? M(c0 + tid, c0 + tid) : (T)1;       // the pivots, of the identity past the matrix
   };
   fetch(0);
   __syncthreads();
@@ -3023,24 +3255,46 @@ struct Planner {
           const int q = tid + k * TH;
           if (q < NB * N) panel[COL(q) * NP + ROW(q)] = next[k];
         }
+        if (tid < NB) { pivot[tid] = pv; inverse[tid] = (T)1 / pv; }
         __syncthreads();
         if (c0 + NB < N) fetch(c0 + NB);
         if (mine) {
-          const int own = lane - h * NB;             // column of the panel that holds this lane's pivot
-          const T d = (!UNIT && own >= 0 && own < NB && 32 * p + lane < N) ? panel[own * NP + 32 * p + lane] : (T)1;
-          const T inv = (T)1 / d;
-          const bool reg = lin_regular(inv);
-          const int cols = N - c0 < NB ? N - c0 : NB;
-#pragma unroll 4
-          for (int j = 0; j < cols; ++j) {
-            const T* col = panel + j * NP;
-            const T sol = UNIT ? acc[p] : lin_div(acc[p], d, inv, reg);
-            const T xj = __shfl_sync(0xFFFFFFFFu, sol, h * NB + j);
-            if (lane == h * NB + j) x = xj;
-            if (32 * p + lane < N) acc[p] = acc[p] - (lane > h * NB + j ? col[32 * p + lane] : (T)0) * xj;
+          const bool regular = UNIT || __ballot_sync(0xFFFFFFFFu, lane >= NB || lin_regular(inverse[lane < NB ? lane : 0])) == 0xFFFFFFFFu;
+          if (regular) {
+#pragma unroll 1
+            for (int j0 = 0; j0 < NB && c0 + j0 < N; j0 += SB) {
+              // SB unknowns at a time: every lane takes the SB right-hand sides and solves for all of them, without an exchange
+              // between one and the next
+              const int l0 = h * NB + j0;            // the lane of the first
+              const T* blk = panel + j0 * NP + 32 * p + l0;
+              T y[SB];
 #pragma unroll
-            for (int r = p + 1; r < NR; ++r)
-              if (32 * r + lane < N) acc[r] = acc[r] - col[32 * r + lane] * xj;
+              for (int s = 0; s < SB; ++s) y[s] = __shfl_sync(0xFFFFFFFFu, acc[p], l0 + s);
+#pragma unroll
+              for (int s = 0; s < SB; ++s) {
+                if (!UNIT) y[s] = lin_div(y[s], pivot[j0 + s], inverse[j0 + s], true);
+#pragma unroll
+                for (int t = s + 1; t < SB; ++t) y[t] = y[t] - blk[s * NP + t] * y[s];
+                if (lane == l0 + s) x = y[s];
+              }
+#pragma unroll
+              for (int s = 0; s < SB; ++s) {
+                const T* col = panel + (j0 + s) * NP + 32 * p + lane;
+                acc[p] = acc[p] - (lane >= l0 + SB ? col[0] : (T)0) * y[s];
+#pragma unroll
+                for (int r = p + 1; r < NR; ++r) acc[r] = acc[r] - col[32 * (r - p)] * y[s];
+              }
+            }
+          } else {
+#pragma unroll 1
+            for (int j = 0; j < NB && c0 + j < N; ++j) {
+              const T* col = panel + j * NP + 32 * p + lane;
+              const T xj = lin_div(__shfl_sync(0xFFFFFFFFu, acc[p], h * NB + j), pivot[j], inverse[j], lin_regular(inverse[j]));
+              if (lane == h * NB + j) x = xj;
+              acc[p] = acc[p] - (lane > h * NB + j ? col[0] : (T)0) * xj;
+#pragma unroll
+              for (int r = p + 1; r < NR; ++r) acc[r] = acc[r] - col[32 * (r - p)] * xj;
+            }
           }
         }
       }
