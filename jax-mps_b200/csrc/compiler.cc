@@ -3860,6 +3860,9 @@ struct Planner {
       const long long tiles = (long long)((g.M + tm - 1) / tm) * ((g.N + tn - 1) / tn) * g.G;
       for (int split = 1; split <= 8; split *= 2) {
         if (split > 1 && g.K < 32 * split) break;
+        // eight to a cluster where that makes a few clusters at least; a long K of one or two tiles is split over more CTAs by the
+        // table-driven kernels
+        if (split == 8 && tiles < 4) break;
         const long long chunk = ((g.K + split - 1) / split + 3) / 4 * 4;
         const double us = in_company(copies, [&](int n) {
           const double odd = (g.a_vec ? 1.0 : 1.1) * (g.b_vec ? 1.0 : 1.1), sum = split > 1 ? (tile == 3 ? 1.25 : 1.45) : 0.0;

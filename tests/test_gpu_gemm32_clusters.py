@@ -7,7 +7,7 @@ from b200.shlo.builder import Builder
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("m,k,n", [(31, 1024, 63), (20, 1000, 10), (32, 4096, 65), (64, 1024, 288), (33, 901, 130), (1, 1100, 61)])
+@pytest.mark.parametrize("m,k,n", [(31, 1024, 250), (20, 1000, 200), (120, 4096, 65), (64, 1024, 288), (33, 901, 130), (1, 1100, 251)])
 @pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
 def test_cluster_of_eight(client, monkeypatch, m, k, n, ta, tb):
     monkeypatch.setenv("B200_NO_TILE32", "1")
