@@ -132,6 +132,12 @@ std::string wide_move(const std::string& arr, const std::string& ptr, int W, int
   return o.str();
 }
 
+std::string Emitter::run_array(DT d) {
+  const std::string arr = fresh("w");
+  arrays_.push_back(std::string("__align__(16) ") + s_type(d) + " " + arr + "[" + std::to_string(run) + "];");
+  return arr;
+}
+
 std::string Emitter::run_arrays(int indent) const {
   std::string s;
   for (auto& a : arrays_) s += std::string(indent, ' ') + a + "\n";
@@ -221,8 +227,7 @@ std::string Emitter::load(Value* v, Ctx& c) {
   if (run && !c.lin_base.empty() && at != "lin" && wide_size(run, (int)dt_size(d))) {
     // the whole run at its first position, in the widest pieces. (Read one element at a time, a bias along the rows of a bf16
     // tensor took eight 2-byte loads for every 16-byte load of the tensor.)
-    const std::string arr = fresh("w");
-    arrays_.push_back(std::string("__align__(16) ") + s_type(d) + " " + arr + "[" + std::to_string(run) + "];");
+    const std::string arr = run_array(d);
     line("if (" + run_var + " == 0) {");
     os_ << wide_move(arr, p, run, (int)dt_size(d), true, indent_ + 2, c.lin_base);
     line("}");

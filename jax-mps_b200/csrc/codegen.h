@@ -61,6 +61,7 @@ class Emitter {
   void pop_scope() { memo_.pop_back(); indent_ -= 2; }
   std::string str() const { return os_.str(); }
   std::string run_arrays(int indent) const;    // declarations in front of the loop over run_var
+  std::string run_array(DT d);                 // one of them, `run` elements of storage type `d`: its name
   // Evaluates a region whose operations are all scalar elementwise ops.
   std::vector<std::string> emit_scalar_region(Block* b, const std::vector<std::string>& args);
   int indent_ = 4;

@@ -1406,6 +1406,26 @@ struct Planner {
     return cheap.count(op->short_name()) != 0;
   }
 
+  // A large exponential of 2-byte data is computed again by every kernel that needs it: its f32 values are twice the bytes of what
+  // it is made of, written once and read back by each. (The softmax of 4096 x 30522 logits, its column sums and its gradient:
+  // with stored values 229 us for the rows and 257 for columns and gradient, 147 and 229 so.)
+  static bool recomputed(Op* op) {
+    Value* v = op->results[0];
+    if (op->short_name() != "exponential" || v->type.dt != DT::F32 || v->type.numel() < (1LL << 25)) return false;
+    bool any = false;
+    std::set<Value*> seen;
+    std::function<bool(Value*)> two_bytes = [&](Value* x) -> bool {
+      if (!seen.insert(x).second || x->type.numel() < v->type.numel()) return true;
+      if (x->def && x->type.dims == v->type.dims && (cheap_to_duplicate(x->def) || categorize(x->def) == Cat::DUP)) {
+        for (Value* o : x->def->operands) if (!two_bytes(o)) return false;
+        return true;
+      }
+      any = true;
+      return dt_size(x->type.dt) == 2;
+    };
+    return two_bytes(op->operands[0]) && any;
+  }
+
   bool identity_in(Group* g, Op* op, BlockState& st) {
     Value* v = op->results[0];
     for (auto* u : st.users[v])
@@ -1464,7 +1484,7 @@ struct Planner {
         else if (identity_in(g, op, st)) g->identity.insert(op);
       };
       if (ext.empty() && !returned && gs.size() == 1) { join(gs[0], false); continue; }
-      if (ext.empty() && !returned && gs.size() > 1 && cheap_to_duplicate(op)) {
+      if (ext.empty() && !returned && gs.size() > 1 && (cheap_to_duplicate(op) || recomputed(op))) {
         bool small = true;
         for (auto* g : gs) small &= g->members.size() < 48;
         // a chain of duplicated operations (the residual stream of a deep network: x4 = x3 + o3 = x2 + o2 + o3 ...)
@@ -3422,6 +3442,16 @@ struct Planner {
     return Nk % 4 == 0 ? 4 : Nk % 2 == 0 ? 2 : 1;
   }
 
+  // Runs of them per thread, 32 threads apart: what a row has for all its columns (a label, a scale) is read once for all of them.
+  // Where a run is 8 bytes or less, and where the pass has a tensor to write as well.
+  static int col_groups(int64_t Nk, int64_t Nr, bool stores) {
+    const int Q = col_run(Nk);
+    return Nk < 1024 || Nr < 128 || Q == 1 ? 1 : Q == 2 ? 4 : stores ? 2 : 1;
+  }
+
+  // A value over the index space of a column reduction that its first pass stores as it goes, in rows `ld` elements apart.
+  struct FullOut { Value* v; int64_t ld; };
+
   // does evaluating `v` read a tensor of 2-byte elements as large as the reduction's index space?
   static bool reads_two_bytes(Value* v, const std::function<bool(Op*)>& internal, int64_t total) {
     std::set<Value*> seen;
@@ -3436,7 +3466,7 @@ struct Planner {
 
   Launch gen_reduce_kernel(const ReduceGen& rg, std::function<bool(Op*)> internal, int splits, bool col,
                            std::vector<Value*> outs, const std::vector<Group*>* epilogue = nullptr,
-                           const std::vector<Value*>* bound_results = nullptr, BlockState* est = nullptr) {
+                           const std::vector<Value*>* bound_results = nullptr, BlockState* est = nullptr, const std::vector<FullOut>* full = nullptr) {
     size_t n = 0;
     std::vector<DT> dts;
     std::vector<Value*> all_inits;
@@ -3463,7 +3493,7 @@ struct Planner {
     em.indent_ = 6;
     // Q consecutive kept indices per thread (column form), or V consecutive reduced ones (row form, where the reduced
     // dimensions are the innermost): 16-byte pieces of what is read along memory, 8-byte ones of 2-byte types in columns.
-    const int Q = col ? col_run(Nk) : 1;
+    const int Q = col ? col_run(Nk) : 1, H = col ? col_groups(Nk, Nr, full && !full->empty()) : 1;
     // T threads cooperate on one output; the reduced range is contiguous-ish along threads
     // a block per output from 128 reduced elements on: second passes over a few hundred partial rows are latency-
     // bound, and 256 threads fetch them in one or two rounds of loads where a warp would need ten to twenty
@@ -3491,7 +3521,7 @@ struct Planner {
     if (Q > 1) {
       pe.run = em.run = Q;
       pe.run_var = em.run_var = "q";
-      kc.lin_base = "o4";
+      kc.lin_base = "o4h";
     } else if (V > 1) {
       em.run = V;
       rc.lin_base = "rb";
@@ -3523,6 +3553,20 @@ struct Planner {
     std::vector<std::string> vals;
     for (auto& part : rg.parts)
       for (auto* v : part.operands) vals.push_back(em.emit(v, oc));
+    if (full)
+      for (const FullOut& fo : *full) {
+        const std::string val = em.emit(fo.v, oc), name = "out" + std::to_string(outs.size()), arr = em.run_array(fo.v->type.dt);
+        outs.push_back(fo.v);
+        em.line(arr + "[" + em.run_var + "] = " + store_expr(fo.v->type.dt, val) + ";");
+        const int last = (int)oc.shape.size() - 1;
+        std::string at = oc.run_base;
+        int64_t stride = fo.ld;
+        for (int d = last - 1; d >= 0; stride *= oc.shape[d--])
+          if (oc.shape[d] != 1) at += " + (" + em.idx_t + ")" + oc.idx[d] + " * " + std::to_string(stride);
+        em.line("if (" + em.run_var + " == " + std::to_string(Q - 1) + ") {");
+        em.line(wide_move(arr, name, Q, (int)dt_size(fo.v->type.dt), false, 0, at));
+        em.line("}");
+      }
     // combine(acc, val), part by part
     em.round_small_floats = false;
     {
@@ -3610,40 +3654,43 @@ struct Planner {
       const int TX = (int)std::min<int64_t>(32, Nk / Q), TY = 256 / TX;
       // 16 bytes per thread and row, measured on the ResNet18 step: 1 -> 5.20 ms, 2 -> 5.15, 4 -> 5.18 (scalar form 5.21);
       // twice as many rows in flight where a row gives a thread 8 bytes
-      const int unroll_r = Q == 4 && !two_bytes ? 2 : 4;
-      auto per_q = [](std::string text) {
-        return std::regex_replace(text, std::regex("\\bacc(\\d+)\\b"), "acc$1[q]");
+      const int unroll_r = H > 1 ? 1 : Q == 4 && !two_bytes ? 2 : 4;
+      const std::string at_q = H > 1 ? "h * " + std::to_string(Q) + " + q" : "q";
+      auto per_q = [&](std::string text) {
+        return std::regex_replace(text, std::regex("\\bacc(\\d+)\\b"), "acc$1[" + at_q + "]");
       };
       src << "extern \"C\" __global__ void __launch_bounds__(256) @NAME@(" << signature(outs, ins) << ") {\n";
       for (size_t k = 0; k < ins.size(); k++)
         if (dt_size(ins[k]->type.dt) == 4 && ins[k]->type.numel() % Q == 0)
           src << "  in" << k << " = (const " << s_type(ins[k]->type.dt) << "*)__builtin_assume_aligned(in" << k << ", " << 4 * Q << ");\n";
       for (size_t k = 0; k < n; k++)
-        src << "  __shared__ " << c_type(dts[k]) << " sm" << k << "[" << TY << "][" << TX * Q + 4 << "];\n";
-      src << "  const " << it << " o4 = ((" << it << ")blockIdx.x * " << TX << " + threadIdx.x) * " << Q << ";\n";
+        src << "  __shared__ " << c_type(dts[k]) << " sm" << k << "[" << TY << "][" << TX * Q * H + 4 << "];\n";
+      src << "  const " << it << " o4 = ((" << it << ")blockIdx.x * " << TX << " * " << H << " + threadIdx.x) * " << Q << ";\n";
       src << "  const bool live = o4 < (" << it << ")" << Nk << "LL;\n";
       for (size_t k = 0; k < n; k++)
         {
-          src << "  " << c_type(dts[k]) << " acc" << k << "[" << Q << "] = {";
-          for (int q = 0; q < Q; q++) src << (q ? ", " : "") << init_names[k];
+          src << "  " << c_type(dts[k]) << " acc" << k << "[" << H * Q << "] = {";
+          for (int q = 0; q < H * Q; q++) src << (q ? ", " : "") << init_names[k];
           src << "};\n";
         }
+      const std::string runs = "      #pragma unroll\n      for (int h = 0; h < " + std::to_string(H) + "; ++h) {\n        const " + em.idx_t + " o4h = o4 + h * " + std::to_string(TX * Q) + ";\n" +
+                               (H > 1 ? "        if (o4h >= (" + em.idx_t + ")" + std::to_string(Nk) + "LL) break;\n" : "");
+      const std::string each = "      #pragma unroll\n      for (int q = 0; q < " + std::to_string(Q) + "; ++q) {\n        const " + em.idx_t + " o = o4h + q;\n";
+      const std::string column = "h * " + std::to_string(TX * Q) + " + threadIdx.x * " + std::to_string(Q) + " + q";
       src << "  if (live) {\n";
       src << "    #pragma unroll " << unroll_r << "\n";
       src << "    for (" << it << " r = (" << it << ")blockIdx.y * " << TY << " + threadIdx.y; r < (" << it << ")" << Nr
           << "LL; r += " << TY << " * (" << it << ")gridDim.y) {\n";
-      src << em.run_arrays(6);
-      src << "      #pragma unroll\n      for (int q = 0; q < " << Q << "; ++q) {\n        const " << it << " o = o4 + q;\n";
-      src << pe.str() << per_q(em.str());
-      src << "      }\n    }\n  }\n";
-      src << "  #pragma unroll\n  for (int q = 0; q < " << Q << "; ++q) {\n";
-      for (size_t k = 0; k < n; k++) src << "    sm" << k << "[threadIdx.y][threadIdx.x * " << Q << " + q] = acc" << k << "[q];\n";
-      src << "  }\n  __syncthreads();\n";
+      src << runs << em.run_arrays(6) << each << pe.str() << per_q(em.str());
+      src << "      }\n      }\n    }\n  }\n";
+      src << runs << each;
+      for (size_t k = 0; k < n; k++) src << "    sm" << k << "[threadIdx.y][" << column << "] = acc" << k << "[" << at_q << "];\n";
+      src << "      }\n      }\n  __syncthreads();\n";
       src << "  if (threadIdx.y == 0 && live) {\n";
-      src << "    #pragma unroll\n    for (int q = 0; q < " << Q << "; ++q) {\n      const " << it << " o = o4 + q;\n";
+      src << runs << each;
       src << "      for (int y = 1; y < " << TY << "; ++y) {\n";
       for (size_t k = 0; k < n; k++)
-        src << "        const " << c_type(dts[k]) << " oth" << k << " = sm" << k << "[y][threadIdx.x * " << Q << " + q];\n";
+        src << "        const " << c_type(dts[k]) << " oth" << k << " = sm" << k << "[y][" << column << "];\n";
       {
         Emitter te;
         te.idx_t = em.idx_t;
@@ -3655,10 +3702,10 @@ struct Planner {
       src << "      }\n";
       for (size_t k = 0; k < n; k++)
         src << "      out" << k << "[(" << it << ")blockIdx.y * " << Nk << " + o] = "
-            << store_expr(outs[k]->type.dt, "acc" + std::to_string(k) + "[q]") << ";\n";
+            << store_expr(outs[k]->type.dt, per_q("acc" + std::to_string(k))) << ";\n";
       src << per_q(epi);
-      src << "    }\n  }\n}\n";
-      L.grid[0] = (unsigned)((Nk + TX * Q - 1) / (TX * Q)); L.grid[1] = (unsigned)splits; L.grid[2] = 1;
+      src << "    }\n    }\n  }\n}\n";
+      L.grid[0] = (unsigned)((Nk + TX * Q * H - 1) / (TX * Q * H)); L.grid[1] = (unsigned)splits; L.grid[2] = 1;
       L.block[0] = TX; L.block[1] = TY; L.block[2] = 1;
     } else if (col) {
       // threads along the kept index (coalesced), rows of the reduced range over threadIdx.y and blockIdx.y
@@ -4647,7 +4694,8 @@ struct Planner {
     rc.Nk = rc.Nr = 1;
     for (auto v : rc.kept_shape) rc.Nk *= v;
     for (auto v : rc.red_shape) rc.Nr *= v;
-    if (rc.Nr < 32 || rc.Nr > 16384 || rc.Nk < 1 || rc.Nk * rc.Nr >= (1LL << 31)) return false;
+    // a row is one block's: longer ones only where there are enough of them for the SMs
+    if (rc.Nr < 32 || rc.Nr > (rc.Nk >= 148 ? 65536 : 16384) || rc.Nk < 1 || rc.Nk * rc.Nr >= (1LL << 31)) return false;
     for (Op* root : g->roots) {
       if (root->operands[0]->type.dims != shape) return false;
       auto d2 = attr_i64s(root->attr("dimensions"));
@@ -4734,7 +4782,8 @@ struct Planner {
     // (with few rows a block per row is what spreads the work over the SMs)
     const char* wm = getenv("B200_ROW_WARP_MAX");
     const int64_t warp_max = wm ? atoll(wm) : 1024;
-    const int T = (Nr <= 64 || (Nr <= warp_max && Nk >= 1184)) ? 32 : 256, per_block = 256 / T;
+    // (rows beyond 8192 elements: a block of 1024 threads, which still holds up to 32768 of them in registers)
+    const int T = (Nr <= 64 || (Nr <= warp_max && Nk >= 1184)) ? 32 : Nr <= 8192 ? 256 : 1024, TB = std::max(256, T), per_block = TB / T;
     // V consecutive elements of the row per thread and round, moved with 16-byte accesses where a tensor is read or
     // written at the row element's own position: 8 when the row's tensors include 2-byte types, else 4; fewer when that
     // would leave half of the threads without an element (128 elements of a softmax row in pieces of eight: 31 us for
@@ -4902,7 +4951,7 @@ struct Planner {
         const std::string sn = std::to_string(stage_no);
         for (size_t k = 0; k < n; k++) {
           decl << "  " << c_type(dts[k]) << " S" << sn << "_" << k << ";\n";
-          if (T == 256) decl << "  __shared__ " << c_type(dts[k]) << " sm" << sn << "_" << k << "[8];\n";
+          if (T >= 256) decl << "  __shared__ " << c_type(dts[k]) << " sm" << sn << "_" << k << "[" << T / 32 << "];\n";
         }
         body << "  {\n";
         for (size_t k = 0; k < n; k++) body << "    " << c_type(dts[k]) << " acc" << k << " = " << inits[k] << ";\n";
@@ -4919,13 +4968,19 @@ struct Planner {
           body << te.str();
         }
         body << "    }\n";
-        if (T == 256) {
+        if (T >= 256) {
           body << "    if ((threadIdx.x & 31) == 0) {";
           for (size_t k = 0; k < n; k++) body << " sm" << sn << "_" << k << "[threadIdx.x >> 5] = acc" << k << ";";
           body << " }\n    __syncthreads();\n";
-          for (size_t k = 0; k < n; k++) body << "    acc" << k << " = sm" << sn << "_" << k << "[0];\n";
-          body << "    for (int w = 1; w < 8; ++w) {\n";
-          for (size_t k = 0; k < n; k++) body << "      const " << c_type(dts[k]) << " oth" << k << " = sm" << sn << "_" << k << "[w];\n";
+          if (T == 256) {
+            for (size_t k = 0; k < n; k++) body << "    acc" << k << " = sm" << sn << "_" << k << "[0];\n";
+            body << "    for (int w = 1; w < 8; ++w) {\n";
+            for (size_t k = 0; k < n; k++) body << "      const " << c_type(dts[k]) << " oth" << k << " = sm" << sn << "_" << k << "[w];\n";
+          } else {                                     // the 32 warps' values by another tree of shuffles, in every warp
+            for (size_t k = 0; k < n; k++) body << "    acc" << k << " = sm" << sn << "_" << k << "[threadIdx.x & 31];\n";
+            body << "    #pragma unroll\n    for (int m = 16; m >= 1; m >>= 1) {\n";
+            for (size_t k = 0; k < n; k++) body << "      const " << c_type(dts[k]) << " oth" << k << " = shfl_xor(acc" << k << ", m);\n";
+          }
           Emitter te;
           te.idx_t = it;
           te.name_prefix = em.name_prefix + "u";
@@ -4987,7 +5042,7 @@ struct Planner {
     }
     label += "}";
     std::ostringstream src;
-    src << "extern \"C\" __global__ void __launch_bounds__(256) @NAME@(" << signature(outs, ins) << ") {\n";
+    src << "extern \"C\" __global__ void __launch_bounds__(" << TB << ") @NAME@(" << signature(outs, ins) << ") {\n";
     // rows past the end (the last block of the warp-per-row form) work on the last row and store nothing
     src << "  const " << it << " o_raw = (" << it << ")blockIdx.x * " << per_block << " + threadIdx.x / " << T << ";\n";
     src << "  const bool live = o_raw < " << Nk << ";\n";
@@ -5005,7 +5060,7 @@ struct Planner {
     Launch L;
     L.kernel = add_kernel(src.str(), "row");
     L.grid[0] = (unsigned)((Nk + per_block - 1) / per_block); L.grid[1] = L.grid[2] = 1;
-    L.block[0] = 256; L.block[1] = L.block[2] = 1;
+    L.block[0] = TB; L.block[1] = L.block[2] = 1;
     L.outs = outs;
     L.ins = ins;
     if (outs.empty()) return;
@@ -5086,6 +5141,68 @@ struct Planner {
     return true;
   }
 
+  // The row length in which nothing but 16-bit products reads `v`, all of them after the same padding of its rows; 0 otherwise.
+  int64_t padded_rows(Value* v, BlockState& st) {
+    if (st.returned.count(v) || v->type.rank() < 2 || dt_size(v->type.dt) != 2 || st.users[v].empty()) return 0;
+    int64_t ld = 0;
+    for (Op* u : st.users[v]) {
+      Dot16 d;
+      if (u->parent != st.block || categorize(u) != Cat::DOT || !dot16_geometry(u, d)) return 0;
+      for (int side = 0; side < 2; side++) {
+        if (u->operands[side] != v) continue;
+        const Dot16::Repack& r = side ? d.rb : d.ra;
+        if (!r.needed || r.cols != v->type.dims.back() || r.src_ld != r.cols || r.rows * r.cols != v->type.numel() || (ld && ld != r.dst_ld)) return 0;
+        ld = r.dst_ld;
+      }
+    }
+    return ld;
+  }
+
+  // A pointwise group that can be stored by the first pass of the column reduction `g`: over the same elements, reading a tensor
+  // of that size that `g` reads too, everything it reads at hand, nothing of it from `g`.
+  Group* partner_of(Group* g, const ReduceGen& rg, BlockState& st) {
+    int64_t total = 1;
+    for (auto d : rg.in_shape) total *= d;
+    const int Q = col_run([&] { int64_t nk = 1; for (size_t d = 0; d < rg.in_shape.size(); d++) if (std::find(rg.dims.begin(), rg.dims.end(), (int64_t)d) == rg.dims.end()) nk *= rg.in_shape[d]; return nk; }());
+    if (!opts.fuse || total < (1 << 22) || rg.in_shape.back() % Q || std::find(rg.dims.begin(), rg.dims.end(), (int64_t)rg.in_shape.size() - 1) != rg.dims.end()) return nullptr;
+    // the tensors a group reads; false when one of them is not there yet
+    auto reads = [&](Group* q, std::set<Value*>& in) {
+      bool there = true;
+      std::set<Value*> seen;
+      std::function<void(Value*)> walk = [&](Value* v) {
+        if (!seen.insert(v).second) return;
+        Op* d = v->def;
+        if (d && d->parent == st.block && (q->members.count(d) || (is_dup(d) && !st.dup_materialize.count(d) && !slot_of.count(v)))) {
+          for (Value* o : d->operands) walk(o);
+          return;
+        }
+        in.insert(v);
+        there = there && slot_of.count(v);
+      };
+      for (Op* mop : q->members)
+        for (Value* o : mop->operands)
+          if (!(o->def && q->members.count(o->def))) walk(o);
+      return there;
+    };
+    std::set<Value*> mine;
+    reads(g, mine);
+    for (auto& cand : st.groups) {
+      Group* e = &cand;
+      if (e == g || e->is_reduce || e->members.empty() || e->members.size() > 24 || emitted.count(e) || absorbed.count(e)) continue;
+      bool ok = true;
+      for (Op* r : e->roots)
+        ok = ok && r->results.size() == 1 && r->results[0]->type.dims == rg.in_shape && !window_updates.count(r) && !slot_of.count(r->results[0]) &&
+             wide_size(Q, (int)dt_size(r->results[0]->type.dt)) && r->results[0]->type.dt != DT::PRED;
+      for (Op* mop : e->members) ok = ok && (categorize(mop) == Cat::ELEMENTWISE || is_dup(mop));
+      std::set<Value*> in;
+      if (!ok || !reads(e, in)) continue;
+      bool shared = false;
+      for (Value* v : in) shared = shared || (mine.count(v) && v->type.numel() == total);
+      if (shared) return e;
+    }
+    return nullptr;
+  }
+
   void emit_group(Group* g, Plan& plan, BlockState& st) {
     if (!g->is_reduce) {
       // a lone reshape of a value that already lives in memory is a view
@@ -5145,7 +5262,10 @@ struct Planner {
     bool col = trailing >= 16;
     // parallelism: split the reduced range over blockIdx.y when there are few outputs
     // (the row strategy gives an output a whole block from 128 reduced elements on, a warp below)
+    Group* beside = col && col_run(Nk) > 1 ? partner_of(g, rg, st) : nullptr;
+    const int64_t wide = col ? col_groups(Nk, Nr, beside != nullptr) : 1;
     int64_t blocks = col ? (Nk + 31) / 32 : (Nr >= 128 ? Nk : (Nk + 7) / 8);
+    if (wide > 1) blocks = (Nk + 32 * wide * col_run(Nk) - 1) / (32 * wide * col_run(Nk));
     // enough blocks to fill 148 SMs with 2048 threads each (1184 blocks of 256 threads), each split keeping
     // at least a few unrolled iterations per thread
     int64_t per_split_min = col ? 64 : (Nr >= 1024 ? 2048 : 256);
@@ -5157,12 +5277,31 @@ struct Planner {
     }
     // a few thousand elements in all: a second launch costs more than the parallelism of a split returns
     if (Nk * Nr <= 32768) splits = 1;
-    auto internal = [this, g, &st](Op* o) {
-      return (g->members.count(o) && categorize(o) != Cat::REDUCE) || (is_dup(o) && !st.dup_materialize.count(o) && !slot_of.count(o->results[0]));
+    // A pointwise kernel over the same elements that reads the same large tensor is done on the way (the gradient of the logits
+    // beside the sum of its columns, 4096 x 30522: two passes of 146 and 122 us from stored exponentials, one of 229 us that makes
+    // them, bound by its instructions; the rows padded for the products, which took 71 us as a pass of its own).
+    std::vector<FullOut> full;
+    if (beside)
+      for (Op* r : beside->roots) {
+        Value* v = r->results[0];
+        const int64_t ld = padded_rows(v, st);
+        if (ld) {
+          TensorType t = v->type;
+          t.dims = {v->type.numel() / v->type.dims.back(), ld};
+          slot_of[v] = new_slot(Slot::TEMP, t, st.arena);
+          repacked[std::make_tuple(st.block, v, (long long)ld)] = slot_of.at(v);
+        }
+        full.push_back({v, ld ? ld : v->type.dims.back()});
+      }
+    auto internal = [this, g, beside, &st](Op* o) {
+      return (g->members.count(o) && categorize(o) != Cat::REDUCE) || (beside && beside->members.count(o)) ||
+             (is_dup(o) && !st.dup_materialize.count(o) && !slot_of.count(o->results[0]));
     };
+    const std::string and_more = beside ? "+" + group_label(beside) : "";
+    if (beside) absorbed.insert(beside);
     if (splits == 1) {
-      Launch L = gen_reduce_kernel(rg, internal, 1, col, outs);
-      add_launch(plan, L, group_label(g), st);
+      Launch L = gen_reduce_kernel(rg, internal, 1, col, outs, nullptr, nullptr, nullptr, &full);
+      add_launch(plan, L, group_label(g) + and_more, st);
       return;
     }
     // pass 1 -> partials [splits, kept...]; pass 2 reduces dim 0 with the same combiners
@@ -5184,8 +5323,8 @@ struct Planner {
       p2.dts = part.dts;
       r2.parts.push_back(std::move(p2));
     }
-    Launch L1 = gen_reduce_kernel(rg, internal, splits, col, partials);
-    add_launch(plan, L1, group_label(g) + ".partial", st);
+    Launch L1 = gen_reduce_kernel(rg, internal, splits, col, partials, nullptr, nullptr, nullptr, &full);
+    add_launch(plan, L1, group_label(g) + ".partial" + and_more, st);
     r2.in_shape = partials[0]->type.dims;
     r2.dims = {0};
     // Pointwise kernels over the reduced shape whose inputs are all at hand once the sums exist (the per-channel
