@@ -132,6 +132,15 @@ std::string wide_move(const std::string& arr, const std::string& ptr, int W, int
   return o.str();
 }
 
+std::string Emitter::stored(DT d, const std::string& e) const {
+  auto it = bits_.find(e);
+  if (it != bits_.end() && (d == DT::BF16 || d == DT::F16)) return it->second;
+  if (d == DT::BF16) return "f_to_bf16(" + e + ")";
+  if (d == DT::F16) return "f_to_f16(" + e + ")";
+  if (d == DT::PRED) return "(u8)(" + e + ")";
+  return e;
+}
+
 std::string Emitter::run_array(DT d) {
   const std::string arr = fresh("w");
   arrays_.push_back(std::string("__align__(16) ") + s_type(d) + " " + arr + "[" + std::to_string(run) + "];");
@@ -233,6 +242,7 @@ std::string Emitter::load(Value* v, Ctx& c) {
     line("}");
     e = arr + "[" + run_var + "]";
   }
+  if (d == DT::BF16 || d == DT::F16) bits_[var] = e;
   if (d == DT::BF16) e = "bf16_to_f(" + e + ")";
   else if (d == DT::F16) e = "f16_to_f(" + e + ")";
   else if (d == DT::PRED) e = "(" + e + " != 0)";
@@ -347,7 +357,15 @@ std::string Emitter::emit(Value* v, Ctx c) {
     std::vector<std::string> a;
     for (auto* o : d->operands) a.push_back(emit(o, same_ctx(o)));
     var = fresh("v");
-    line("const " + ct + " " + var + " = " + elementwise(d, a) + ";");
+    std::string e = elementwise(d, a);
+    const std::string to = rt == DT::BF16 ? "bf16" : "f16", round = "r" + to + "(";
+    if ((rt == DT::BF16 || rt == DT::F16) && e.compare(0, round.size(), round) == 0) {
+      // round as r..() does, and keep the bits: what is only stored needs no second conversion
+      line("const u16 " + var + "h = f_to_" + to + e.substr(round.size() - 1) + ";");
+      bits_[var] = var + "h";
+      e = to + "_to_f(" + var + "h)";
+    }
+    line("const " + ct + " " + var + " = " + e + ";");
   } else if (sh == "constant") {
     DenseValue dv = attr_dense(d->attr("value"));
     if (!dv.splat) throw CompileError("internal: non-splat constant inside a fusion");

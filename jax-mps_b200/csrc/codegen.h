@@ -52,6 +52,8 @@ class Emitter {
 
   std::string emit(Value* v, Ctx c);
   std::string input_name(Value* v);
+  // The value `e` of type `d` as it is stored. A value that was just rounded to 16 bits, or loaded, is stored as those bits.
+  std::string stored(DT d, const std::string& e) const;
   void seed_inputs(const std::vector<Value*>& vs) { for (Value* v : vs) input_name(v); }   // fix the first parameters
   void line(const std::string& s);
   std::string fresh(const char* prefix);
@@ -75,6 +77,7 @@ class Emitter {
   std::vector<std::map<std::string, std::string>> memo_{1};
   std::map<Value*, int> in_index_;
   std::vector<std::string> arrays_;
+  std::map<std::string, std::string> bits_;    // variable of a 16-bit float type -> its bits
   int nvar_ = 0;
 };
 

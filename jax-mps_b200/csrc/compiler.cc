@@ -1672,7 +1672,7 @@ struct Planner {
     std::vector<std::string> vals;
     for (auto* o : outs) vals.push_back(em.emit(o, root));
     for (size_t k = 0; k < outs.size(); k++)
-      em.line("out" + std::to_string(k) + "[lin] = " + store_expr(outs[k]->type.dt, vals[k]) + ";");
+      em.line("out" + std::to_string(k) + "[lin] = " + em.stored(outs[k]->type.dt, vals[k]) + ";");
     std::ostringstream src;
     src << "extern \"C\" __global__ void __launch_bounds__(" << kThreads << ") @NAME@(" << signature(outs, em.inputs)
         << ") {\n";
@@ -3557,7 +3557,7 @@ struct Planner {
       for (const FullOut& fo : *full) {
         const std::string val = em.emit(fo.v, oc), name = "out" + std::to_string(outs.size()), arr = em.run_array(fo.v->type.dt);
         outs.push_back(fo.v);
-        em.line(arr + "[" + em.run_var + "] = " + store_expr(fo.v->type.dt, val) + ";");
+        em.line(arr + "[" + em.run_var + "] = " + em.stored(fo.v->type.dt, val) + ";");
         const int last = (int)oc.shape.size() - 1;
         std::string at = oc.run_base;
         int64_t stride = fo.ld;
@@ -5030,7 +5030,7 @@ struct Planner {
         if (!stores.empty()) {
           std::vector<std::pair<size_t, Value*>> stage_outs;
           for (auto& sv : stores) {
-            em.line("out" + std::to_string(outs.size()) + "[lin] = " + store_expr(sv.first->type.dt, sv.second) + ";");
+            em.line("out" + std::to_string(outs.size()) + "[lin] = " + em.stored(sv.first->type.dt, sv.second) + ";");
             stage_outs.push_back({outs.size(), sv.first});
             outs.push_back(sv.first);
           }
