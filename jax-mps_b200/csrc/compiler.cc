@@ -305,6 +305,29 @@ struct Inliner {
         sh = "reshape";
       }
     }
+    // a pointwise result that is reshaped and rounded to 16 bits is rounded first: the reshape is then a name, and the rounding part
+    // of the kernel that makes the result
+    if (sh == "convert" && op->operands.size() == 1 && dt_size(op->results[0]->type.dt) == 2 && dt_is_float(op->results[0]->type.dt) && op->operands[0]->def &&
+        op->operands[0]->def->short_name() == "reshape" && op->operands[0]->def->parent == b) {
+      Value* inner = op->operands[0]->def->operands[0];
+      if (inner->def && inner->def->parent == b && is_elementwise_op(inner->def->short_name()) && inner->type.dt == DT::F32) {
+        auto cv = std::make_unique<Op>();
+        cv->name = op->name;
+        cv->attrs = op->attrs;
+        cv->operands = {inner};
+        TensorType t = inner->type;
+        t.dt = op->results[0]->type.dt;
+        Value* v = m.new_value(t, "");
+        v->def = cv.get();
+        v->def_index = 0;
+        cv->results.push_back(v);
+        process(std::move(cv), b);
+        op->name = "stablehlo.reshape";
+        op->attrs.clear();
+        op->operands = {res(v)};
+        sh = "reshape";
+      }
+    }
     // x + broadcast(0), x * broadcast(1), x - broadcast(0), x / broadcast(1) -> x
     // (src/pjrt_plugin/passes/canonicalize_broadcast_identity.cc)
     if ((sh == "add" || sh == "multiply" || sh == "subtract" || sh == "divide") && op->operands.size() == 2 &&
@@ -1400,6 +1423,10 @@ struct Planner {
   }
 
   static bool cheap_to_duplicate(Op* op) {
+    if (op->short_name() == "reshape") {                   // the same linear index, of what is cheap or in memory anyway
+      Op* d = op->operands[0]->def;
+      return !d || cheap_to_duplicate(d) || (categorize(d) != Cat::ELEMENTWISE && categorize(d) != Cat::INDEXING);
+    }
     if (categorize(op) != Cat::ELEMENTWISE) return false;
     static const std::set<std::string> cheap = {"add", "subtract", "multiply", "maximum", "minimum", "negate", "abs",
                                                 "compare", "select", "convert", "and", "or", "xor", "not", "clamp", "sign"};
@@ -1434,6 +1461,7 @@ struct Planner {
     return false;
   }
 
+  std::set<Op*> views;                 // reshapes that name their operand's memory
   void build_groups(BlockState& st) {
     for (int i = (int)st.ops.size() - 1; i >= 0; i--) {
       Op* op = st.ops[i];
@@ -1472,7 +1500,7 @@ struct Planner {
       bool returned = st.returned.count(v) != 0;
       for (auto* u : st.users[v]) {
         auto it = st.group_of.find(u);
-        if (opts.fuse && it != st.group_of.end() && can_fuse_into(op, v, u)) {
+        if (opts.fuse && it != st.group_of.end() && can_fuse_into(op, v, u) && !views.count(u)) {
           for (auto* g : it->second)
             if (std::find(gs.begin(), gs.end(), g) == gs.end()) gs.push_back(g);
         } else ext.push_back(u);
@@ -1501,11 +1529,16 @@ struct Planner {
           continue;
         }
       }
+      // a reshape that has to be in memory is another name for its operand there, which keeps the kernel that makes it in the
+      // operand's shape: a softmax over [heads, queries, keys] is one row kernel although the products name its sides otherwise
+      if (opts.fuse && op->short_name() == "reshape" && op->operands[0]->def && op->operands[0]->def->parent == st.block &&
+          categorize(op->operands[0]->def) == Cat::ELEMENTWISE)
+        views.insert(op);
       // written to memory: as an extra output of a consumer kernel when it shares that kernel's index space
       std::sort(gs.begin(), gs.end(), [](Group* a, Group* b) { return a->max_pos < b->max_pos; });
       bool placed = false;
       for (auto* g : gs) {
-        if (g->is_reduce || !identity_in(g, op, st)) continue;
+        if (g->is_reduce || views.count(op) || !identity_in(g, op, st)) continue;
         // consumers that will read the value from memory: non-fusable users, and every other group
         // holding one of its users
         std::vector<Op*> others = ext;
@@ -4695,7 +4728,8 @@ struct Planner {
     for (auto v : rc.kept_shape) rc.Nk *= v;
     for (auto v : rc.red_shape) rc.Nr *= v;
     // a row is one block's: longer ones only where there are enough of them for the SMs
-    if (rc.Nr < 32 || rc.Nr > (rc.Nk >= 148 ? 65536 : 16384) || rc.Nk < 1 || rc.Nk * rc.Nr >= (1LL << 31)) return false;
+    // (short ones, a softmax over ten classes, where latency is all there is: a warp a row leaves most of its lanes idle)
+    if (rc.Nr < (rc.Nk * rc.Nr <= 32768 ? 2 : 32) || rc.Nr > (rc.Nk >= 148 ? 65536 : 16384) || rc.Nk < 1 || rc.Nk * rc.Nr >= (1LL << 31)) return false;
     for (Op* root : g->roots) {
       if (root->operands[0]->type.dims != shape) return false;
       auto d2 = attr_i64s(root->attr("dimensions"));
@@ -4909,7 +4943,8 @@ struct Planner {
           const std::string nm = "out" + std::to_string(so.first);
           if (!replace_word(inner, nm + "[lin]", "v" + nm + "[e]")) continue;
           pre << "      __align__(16) " << s_type(so.second->type.dt) << " v" << nm << "[" << V << "];\n";
-          post << wide_move("v" + nm, nm, V, es, false, 6);
+          const int64_t ld = rc.red_shape.size() == 1 ? store_padded(so.second, st) : 0;
+          post << wide_move("v" + nm, nm, V, es, false, 6, ld ? "(long long)o * " + std::to_string(ld) + " + rb" : "base");
         }
         return row_rounds + "      const " + it + " base = o * " + std::to_string(Nr) + " + rb;\n" + pre.str() +
                "      #pragma unroll\n      for (int e = 0; e < " + std::to_string(V) + "; ++e) {\n      const " + it + " r = rb + e;\n      const " +
@@ -5158,6 +5193,17 @@ struct Planner {
     return ld;
   }
 
+  // Gives `v` memory in such rows; their length, or 0.
+  int64_t store_padded(Value* v, BlockState& st) {
+    const int64_t ld = slot_of.count(v) ? 0 : padded_rows(v, st);
+    if (!ld) return 0;
+    TensorType t = v->type;
+    t.dims = {v->type.numel() / v->type.dims.back(), ld};
+    slot_of[v] = new_slot(Slot::TEMP, t, st.arena);
+    repacked[std::make_tuple(st.block, v, (long long)ld)] = slot_of.at(v);
+    return ld;
+  }
+
   // A pointwise group that can be stored by the first pass of the column reduction `g`: over the same elements, reading a tensor
   // of that size that `g` reads too, everything it reads at hand, nothing of it from `g`.
   Group* partner_of(Group* g, const ReduceGen& rg, BlockState& st) {
@@ -5284,13 +5330,7 @@ struct Planner {
     if (beside)
       for (Op* r : beside->roots) {
         Value* v = r->results[0];
-        const int64_t ld = padded_rows(v, st);
-        if (ld) {
-          TensorType t = v->type;
-          t.dims = {v->type.numel() / v->type.dims.back(), ld};
-          slot_of[v] = new_slot(Slot::TEMP, t, st.arena);
-          repacked[std::make_tuple(st.block, v, (long long)ld)] = slot_of.at(v);
-        }
+        const int64_t ld = store_padded(v, st);
         full.push_back({v, ld ? ld : v->type.dims.back()});
       }
     auto internal = [this, g, beside, &st](Op* o) {
@@ -5636,8 +5676,9 @@ struct Planner {
             take(u.group);
             // units that stand between the stages but read nothing of the chain (a constant, the scale vector of a
             // norm) go out in front of it
-            std::vector<size_t> before;
-            size_t last_stage = oi, n_before_at_last = 0;
+            std::vector<size_t> before, behind;
+            std::set<Value*> late;                   // what units behind the chain make: they read it, but not by rows
+            size_t last_stage = oi, n_before_at_last = 0, n_behind_at_last = 0;
             const bool dbg = getenv("B200_DEBUG_ROWS") != nullptr;
             for (size_t oj = oi + 1; oj < order.size() && oj < oi + 16 && rc.stages.size() < 8; oj++) {
               Unit& nu = units[order[oj]];
@@ -5661,23 +5702,28 @@ struct Planner {
               }
               Group* g = nu.group;
               if (g->roots.size() == 1 && window_updates.count(g->roots[0])) break;
-              if (!reads_any(g, produced, st)) { before.push_back(oj); continue; }
-              if (g->is_reduce) {
+              bool joins = !reads_any(g, late, st);
+              if (joins && !reads_any(g, produced, st)) { before.push_back(oj); continue; }
+              if (joins && g->is_reduce) {
                 RowChain r2;
-                if (!row_form(g, r2) || r2.in_shape != rc.in_shape || r2.kept_shape != rc.kept_shape) {
-                  if (dbg) fprintf(stderr, "row chain stops: %s has another row form\n", group_label(g).c_str());
-                  break;
-                }
+                joins = row_form(g, r2) && r2.in_shape == rc.in_shape && r2.kept_shape == rc.kept_shape;
+                if (dbg && !joins) fprintf(stderr, "row chain goes around: %s has another row form\n", group_label(g).c_str());
               }
-              std::set<Op*> m2 = members;
-              m2.insert(g->members.begin(), g->members.end());
-              if (!row_safe(g, rc, m2, reduced, st)) {
-                if (dbg) fprintf(stderr, "row chain stops: %s is not row safe\n", group_label(g).c_str());
-                break;
+              if (joins) {
+                std::set<Op*> m2 = members;
+                m2.insert(g->members.begin(), g->members.end());
+                joins = row_safe(g, rc, m2, reduced, st);
+                if (dbg && !joins) fprintf(stderr, "row chain goes around: %s is not row safe\n", group_label(g).c_str());
+              }
+              if (!joins) {
+                behind.push_back(oj);
+                for (Op* r : g->roots) late.insert(r->results.begin(), r->results.end());
+                continue;
               }
               take(g);
               last_stage = oj;
               n_before_at_last = before.size();
+              n_behind_at_last = behind.size();
             }
             if (rc.stages.size() >= 2) {
               before.resize(n_before_at_last);
@@ -5688,6 +5734,12 @@ struct Planner {
               }
               emit_row_chain(rc, plan, st);
               for (Group* g : rc.stages) emitted.insert(g);
+              behind.resize(n_behind_at_last);
+              for (size_t ob : behind) {
+                Group* bg = units[order[ob]].group;
+                if (!absorbed.count(bg)) emit_group(bg, plan, st);
+                emitted.insert(bg);
+              }
               oi = last_stage;
               continue;
             }

@@ -28,8 +28,8 @@ def test_cross_entropy_over_a_vocabulary(client, rows, vocab):
     text = b.module([loss, *b.grad(loss, [hv, wv, bv])], name=f"jit_ce_{rows}_{vocab}")
     plan = client.compile(text).plan_text()
     assert "block=1024x1 row{" in plan and "repack16" not in plan, plan
-    stored = next(line for line in plan.splitlines() if ".partial+fusion{" in line)
-    assert ("exponential" in stored) == (rows * vocab >= 1 << 25), plan
+    stored = next(line for line in plan.splitlines() if "row{" in line)
+    assert (stored.count("exponential") > 1) == (rows * vocab >= 1 << 25), plan
     got, _ = run_gpu(client, text, [h, w, bias, label], ["bf16", "bf16", None, None])
     z64 = _bf16(h.astype(np.float64) @ w.astype(np.float64).T).astype(np.float64) + bias
     z64 -= z64.max(1, keepdims=True)
