@@ -1453,6 +1453,28 @@ struct Planner {
     return two_bytes(op->operands[0]) && any;
   }
 
+  // In a loop body, whose iterations are a chain of kernels, a small value made of a few tensors in memory is computed again by each
+  // of its readers whatever it costs: it takes a fraction of a microsecond on idle SMs, a kernel in front of them two. (The gates
+  // of a recurrent cell, read by the gradient of the pre-activations and by that of the state, and the state
+  // itself, read by the next layer: a step of 100 iterations forth and back 4592 -> 4376 us.)
+  bool again_in_loop(Op* op, BlockState& st) {
+    if (!st.block->parent_op || st.block->parent_op->short_name() != "while" || op->results[0]->type.numel() > 65536 || getenv("B200_NO_LOOP_SPLIT")) return false;
+    auto inline_op = [&](Op* d) {
+      if (!d || d->parent != st.block || d->results.size() != 1) return false;
+      const std::string sh = d->short_name();
+      return categorize(d) == Cat::ELEMENTWISE || is_dup(d) || sh == "slice" || sh == "dynamic_slice" || sh == "reshape";
+    };
+    if (!inline_op(op)) return false;
+    std::set<Value*> seen, leaves;
+    std::function<bool(Value*)> walk = [&](Value* v) -> bool {
+      if (!seen.insert(v).second) return true;
+      if (!inline_op(v->def)) { leaves.insert(v); return leaves.size() <= 8; }
+      for (Value* o : v->def->operands) if (!walk(o)) return false;
+      return true;
+    };
+    return walk(op->results[0]);
+  }
+
   bool identity_in(Group* g, Op* op, BlockState& st) {
     Value* v = op->results[0];
     for (auto* u : st.users[v])
@@ -1512,9 +1534,10 @@ struct Planner {
         else if (identity_in(g, op, st)) g->identity.insert(op);
       };
       if (ext.empty() && !returned && gs.size() == 1) { join(gs[0], false); continue; }
-      if (ext.empty() && !returned && gs.size() > 1 && (cheap_to_duplicate(op) || recomputed(op))) {
+      const bool again = ext.empty() && !returned && gs.size() > 1 && again_in_loop(op, st);
+      if (ext.empty() && !returned && gs.size() > 1 && (cheap_to_duplicate(op) || recomputed(op) || again)) {
         bool small = true;
-        for (auto* g : gs) small &= g->members.size() < 48;
+        for (auto* g : gs) small &= g->members.size() < (again ? 96 : 48);
         // a chain of duplicated operations (the residual stream of a deep network: x4 = x3 + o3 = x2 + o2 + o3 ...)
         // would be re-evaluated from ever more inputs by every later kernel: after four links the value is written
         int depth = 1;
@@ -1522,7 +1545,7 @@ struct Planner {
           auto du = dup_depth.find(u);
           if (du != dup_depth.end()) depth = std::max(depth, du->second + 1);
         }
-        if (depth > 8) small = false;
+        if (depth > 8 && !again) small = false;
         if (small) {
           dup_depth[op] = depth;
           for (auto* g : gs) join(g, false);
@@ -1555,6 +1578,9 @@ struct Planner {
         placed = true;
         break;
       }
+      if (opts.fuse && returned && ext.empty() && again_in_loop(op, st))       // carried, and made again for the readers in this iteration
+        for (auto* g : gs)
+          if (g->members.size() < 96 && !g->members.count(op)) join(g, false);
       if (placed) continue;
       st.groups.emplace_back();
       Group* g = &st.groups.back();
