@@ -3983,10 +3983,12 @@ struct Planner {
   // sum of a cluster. The tile of four warps, two CTAs of which share an SM, starts later and hides the fill and drain of one CTA
   // behind the other: 2.75 us, 0.76 ns from the second CTA of an SM on, 1.8 for each. Every tile and split over 114 chains from
   // 6 x 256 x 512 to 250 x 784 x 1000 and 180 from 250 x 784 x 1000 to 2019 x 174 x 3490: 8 % rms error.
-  static double fma_product(Gemm32Launch& g, int copies) {
+  // `deep`: products and sums of all iterations of a loop, which keep chains of additions as short as an iteration's: a tile that at
+  // least four warps share.
+  static double fma_product(Gemm32Launch& g, int copies, bool deep = false) {
     if (g.G > 65535 || getenv("B200_NO_GEMM32")) return 1e30;
     double best = 1e30;
-    for (int tile = 3; tile >= 0; tile--) {
+    for (int tile = deep ? 1 : 3; tile >= 0; tile--) {
       const int tm = tile == 0 ? 32 : 64, tn = tile >= 2 ? 128 : 64;
       const long long tiles = (long long)((g.M + tm - 1) / tm) * ((g.N + tn - 1) / tn) * g.G;
       for (int split = 1; split <= 8; split *= 2) {
@@ -4325,7 +4327,7 @@ struct Planner {
         t.M = g.M; t.N = g.N; t.K = g.K; t.G = g.G;
         int split_k = 1;
         const int copies = has_company(op, st) ? 2 : 1;
-        const double us_fma = fma_product(g, copies);
+        const double us_fma = fma_product(g, copies, op->has("b200.fma"));
         double us_table = table_product(g, split_k, copies), us_tile = 1e30;
         // the switches that keep products off the tensor cores or tiled copies leave them to the FMA pipe
         const bool tiles = opts.tensor_cores && !getenv("B200_NO_TILE32") && !op->has("b200.fma");
