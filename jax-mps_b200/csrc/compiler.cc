@@ -3536,12 +3536,12 @@ struct Planner {
   // A value over the index space of a column reduction that its first pass stores as it goes, in rows `ld` elements apart.
   struct FullOut { Value* v; int64_t ld; };
 
-  // does evaluating `v` read a tensor of 2-byte elements as large as the reduction's index space?
-  static bool reads_two_bytes(Value* v, const std::function<bool(Op*)>& internal, int64_t total) {
+  // does evaluating `v` read a tensor of `size`-byte elements as large as the reduction's index space?
+  static bool reads_size(Value* v, size_t size, const std::function<bool(Op*)>& internal, int64_t total) {
     std::set<Value*> seen;
     std::function<bool(Value*)> walk = [&](Value* x) -> bool {
       if (!seen.insert(x).second) return false;
-      if (!x->def || !internal(x->def)) return x->type.numel() == total && dt_size(x->type.dt) == 2;
+      if (!x->def || !internal(x->def)) return x->type.numel() == total && dt_size(x->type.dt) == size;
       for (Value* o : x->def->operands) if (walk(o)) return true;
       return false;
     };
@@ -3577,16 +3577,22 @@ struct Planner {
     em.indent_ = 6;
     // Q consecutive kept indices per thread (column form), or V consecutive reduced ones (row form, where the reduced
     // dimensions are the innermost): 16-byte pieces of what is read along memory, 8-byte ones of 2-byte types in columns.
-    const int Q = col ? col_run(Nk) : 1, H = col ? col_groups(Nk, Nr, full && !full->empty()) : 1;
+    const int Q = col ? col_run(Nk) : 1;
+    int H = col ? col_groups(Nk, Nr, full && !full->empty()) : 1;
+    auto shared_bytes = [&](int h) { size_t b = 0; for (DT d : dts) b += dt_size(d) * 8 * (32 * Q * h + 4); return b; };
+    while (H > 1 && shared_bytes(H) > 40 * 1024) H /= 2;         // several accumulators, or wide ones
     // T threads cooperate on one output; the reduced range is contiguous-ish along threads
     // a block per output from 128 reduced elements on: second passes over a few hundred partial rows are latency-
     // bound, and 256 threads fetch them in one or two rounds of loads where a warp would need ten to twenty
     const int T = Nr >= 128 ? 256 : 32;
     int V = 1;
-    bool two_bytes = false;
+    bool two_bytes = false, eight_bytes = false;
     for (auto& part : rg.parts)
-      for (auto* v : part.operands) two_bytes = two_bytes || reads_two_bytes(v, internal, total);
-    if (!col && !getenv("B200_NO_WIDE_ROWS")) {
+      for (auto* v : part.operands) {
+        two_bytes = two_bytes || reads_size(v, 2, internal, total);
+        eight_bytes = eight_bytes || reads_size(v, 8, internal, total);
+      }
+    if (!col && !eight_bytes && !getenv("B200_NO_WIDE_ROWS")) {
       bool suffix = true;
       for (size_t d = 0; d < rg.in_shape.size(); d++)
         suffix = suffix && ((d + rg.dims.size() >= rg.in_shape.size()) == (std::find(rg.dims.begin(), rg.dims.end(), (int64_t)d) != rg.dims.end()));

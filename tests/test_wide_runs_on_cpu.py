@@ -115,3 +115,16 @@ def test_reductions_of_runs(shape, dim, dt):
     y = b.add(x, b.bcast(bias, shape, tuple(range(1, len(shape)))))
     y = b.convert(y, "f32") if dt != "f32" else y
     _check(b.module([b.reduce_sum(y, (dim,)), b.reduce_max(y, (dim,))]), [r.integers(-4, 5, s).astype(np.float32) for s in (shape, shape[1:])], 1e-6)
+
+
+def test_many_wide_accumulators_fit_shared_memory():
+    """Four sums in f64 over columns in runs of two, several runs a thread: fewer runs where their tiles would not fit."""
+    import b200
+    b = Builder()
+    x = b.arg((600, 1026), "f64")
+    sums = [b.reduce_sum(y, (0,)) for y in (x, b.mul(x, x), b.mul(x, b.mul(x, x)), b.neg(x))]
+    plan, src = b200.compile_to_plan(b.module(sums), validate=True)
+    import re
+    for body in src.split('extern "C"')[1:]:
+        tiles = re.findall(r"__shared__ double sm\d+\[(\d+)\]\[(\d+)\]", body)
+        assert sum(int(r) * int(c) * 8 for r, c in tiles) <= 48 * 1024
