@@ -1669,6 +1669,7 @@ struct Planner {
     int kernel;
     unsigned grid[3], block[3];
     std::vector<Value*> outs, ins;
+    std::set<Value*> pads;             // those of `outs` that it stores in the padded rows of store_padded
   };
 
   std::string idx_type_for(const std::vector<Value*>& vals, int64_t extra = 0) {
@@ -3641,12 +3642,14 @@ struct Planner {
       }
     }
     std::vector<std::string> vals;
+    std::set<Value*> pads;
     for (auto& part : rg.parts)
       for (auto* v : part.operands) vals.push_back(em.emit(v, oc));
     if (full)
       for (const FullOut& fo : *full) {
         const std::string val = em.emit(fo.v, oc), name = "out" + std::to_string(outs.size()), arr = em.run_array(fo.v->type.dt);
         outs.push_back(fo.v);
+        if (padded.count(fo.v)) pads.insert(fo.v);
         em.line(arr + "[" + em.run_var + "] = " + em.stored(fo.v->type.dt, val) + ";");
         const int last = (int)oc.shape.size() - 1;
         std::string at = oc.run_base;
@@ -3736,6 +3739,7 @@ struct Planner {
     Launch L;
     L.outs = outs;
     L.ins = ins;
+    L.pads = pads;
     if (Q > 1) {
       // Column strategy with four (two) consecutive kept indices per thread: as many times the bytes in flight per thread
       // and, for inputs read at their own position, neighbouring loads the compiler can merge into 16-byte ones
@@ -4270,6 +4274,7 @@ struct Planner {
     plan.steps.push_back(std::move(s));
   }
   std::map<std::tuple<Block*, Value*, long long>, int> repacked;   // padded copies of operands, per block
+  std::set<Value*> padded;                                         // values that exist in padded rows only
 
   Step lower_dot(Op* op, BlockState& st) {
     Value *lhs = op->operands[0], *rhs = op->operands[1], *out = op->results[0];
@@ -4722,6 +4727,7 @@ struct Planner {
 
   // ---- block -> steps ----------------------------------------------------------------
   void ensure_slot(Value* v, BlockState& st) {
+    if (padded.count(v)) throw CompileError("internal: " + v->name + " has padded rows, and a second writer that does not pad them");
     if (slot_of.count(v)) return;
     if (v->type.dt == DT::TOKEN) {
       TensorType t;
@@ -4738,9 +4744,13 @@ struct Planner {
     s.kernel = L.kernel;
     s.label = label;
     for (int k = 0; k < 3; k++) { s.grid[k] = L.grid[k]; s.block[k] = L.block[k]; }
-    for (auto* o : L.outs) { ensure_slot(o, st); s.args.push_back(slot_of.at(o)); }
+    for (auto* o : L.outs) {
+      if (!L.pads.count(o)) ensure_slot(o, st);
+      s.args.push_back(slot_of.at(o));
+    }
     s.n_outs = (int)L.outs.size();
     for (auto* i : L.ins) {
+      if (padded.count(i)) throw CompileError("internal: " + i->name + " has padded rows, and a reader that does not know of them (" + label + ")");
       if (!slot_of.count(i)) throw CompileError("internal: kernel input without storage: " + i->name + " (" + label + ")");
       s.args.push_back(slot_of.at(i));
     }
@@ -4939,6 +4949,7 @@ struct Planner {
     kc.run_dim = Ctx::kSame;
     pe.ensure_idx(kc);
     std::vector<Value*> ins, outs;
+    std::set<Value*> pads;
     std::ostringstream decl, body;
     std::set<Op*> members_so_far;
     std::map<Value*, std::string> bound;
@@ -5003,6 +5014,7 @@ struct Planner {
           if (!replace_word(inner, nm + "[lin]", "v" + nm + "[e]")) continue;
           pre << "      __align__(16) " << s_type(so.second->type.dt) << " v" << nm << "[" << V << "];\n";
           const int64_t ld = rc.red_shape.size() == 1 ? store_padded(so.second, st) : 0;
+          if (ld) pads.insert(so.second);
           post << wide_move("v" + nm, nm, V, es, false, 6, ld ? "(long long)o * " + std::to_string(ld) + " + rb" : "base");
         }
         return row_rounds + "      const " + it + " base = o * " + std::to_string(Nr) + " + rb;\n" + pre.str() +
@@ -5157,6 +5169,7 @@ struct Planner {
     L.block[0] = TB; L.block[1] = L.block[2] = 1;
     L.outs = outs;
     L.ins = ins;
+    L.pads = pads;
     if (outs.empty()) return;
     add_launch(plan, L, label, st);
   }
@@ -5252,7 +5265,7 @@ struct Planner {
     return ld;
   }
 
-  // Gives `v` memory in such rows; their length, or 0.
+  // Gives `v` memory in such rows; their length, or 0. The kernel that asked is the only one to write them (Launch::pads).
   int64_t store_padded(Value* v, BlockState& st) {
     const int64_t ld = slot_of.count(v) ? 0 : padded_rows(v, st);
     if (!ld) return 0;
@@ -5260,6 +5273,7 @@ struct Planner {
     t.dims = {v->type.numel() / v->type.dims.back(), ld};
     slot_of[v] = new_slot(Slot::TEMP, t, st.arena);
     repacked[std::make_tuple(st.block, v, (long long)ld)] = slot_of.at(v);
+    padded.insert(v);
     return ld;
   }
 
@@ -5786,13 +5800,14 @@ struct Planner {
             }
             if (rc.stages.size() >= 2) {
               before.resize(n_before_at_last);
+              for (Group* g : rc.stages) emitted.insert(g);      // the chain's: no unit in front of it may take them
               for (size_t ob : before) {
                 Unit& bu = units[order[ob]];
-                if (bu.kind == Unit::CONST_MAT) materialize_dup(bu.op, plan, st);
-                else { emit_group(bu.group, plan, st); emitted.insert(bu.group); }
+                if (bu.kind == Unit::CONST_MAT) { materialize_dup(bu.op, plan, st); continue; }
+                if (!absorbed.count(bu.group)) emit_group(bu.group, plan, st);      // a reduction in front of it may have stored it
+                emitted.insert(bu.group);
               }
               emit_row_chain(rc, plan, st);
-              for (Group* g : rc.stages) emitted.insert(g);
               behind.resize(n_behind_at_last);
               for (size_t ob : behind) {
                 Group* bg = units[order[ob]].group;

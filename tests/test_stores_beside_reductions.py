@@ -1,0 +1,45 @@
+"""A column sum whose first pass also stores a pointwise result over the same elements, in front of a chain of row kernels: the
+result is made once, in the rows that the 16-bit product behind it reads (padded where their length is no multiple of eight), and
+so is what the second pass makes of the sums. On the GPU held to float64: tanh and the product are rounded to 8 bits once each
+(2e-2 of the result's scale), the sums of 4096 values are fp32."""
+import numpy as np
+import pytest
+
+import b200
+from b200.shlo.builder import Builder, f32_to_bf16_bits
+from util import run_gpu
+
+
+def program(rows, cols, lanes=128):
+    b = Builder()
+    g, t, w = b.arg((rows, cols), "bf16"), b.arg((rows, lanes), "f32"), b.arg((cols, 64), "bf16")
+    m = b.reduce_max(t, (1,))
+    sums = b.reduce_sum(b.convert(g, "f32"), (0,))
+    y, scaled = b.tanh(g), b.sin(sums)
+    e = b.exp(b.sub(t, b.bcast(m, t.shape, (0,))))
+    z = b.div(e, b.bcast(b.reduce_sum(e, (1,)), t.shape, (0,)))
+    return b.module([sums, scaled, z, b.matmul(y, w)], name=f"jit_beside_{rows}_{cols}")
+
+
+@pytest.mark.parametrize("cols", [1024, 1026, 1030, 2050])
+def test_made_once(cols):
+    plan = b200.compile_to_plan(program(4096, cols))[0]
+    assert plan.count("tanh") == 1 and plan.count("sine") == 1 and "repack16" not in plan, plan
+    first = next(line for line in plan.splitlines() if "tanh" in line)
+    assert "reduce_" in first and plan.index(first) < plan.index("row{"), plan
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cols", [1024, 1026, 1030, 2050])
+def test_values(client, cols):
+    r = np.random.default_rng(cols)
+    def bf16(*shape): return (f32_to_bf16_bits(r.standard_normal(shape).astype(np.float32)).astype(np.uint32) << 16).view(np.float32)
+    g, t, w = bf16(4096, cols), r.standard_normal((4096, 128)).astype(np.float32), bf16(cols, 64)
+    (sums, scaled, z, o), _ = run_gpu(client, program(4096, cols), [g, t, w], ["bf16", None, "bf16"])
+    want = g.astype(np.float64).sum(0)
+    np.testing.assert_allclose(sums, want, rtol=1e-5, atol=1e-5 * np.abs(want).max())
+    np.testing.assert_allclose(scaled, np.sin(sums.astype(np.float64)), rtol=1e-5, atol=1e-5)
+    e = np.exp(t.astype(np.float64) - t.max(1, keepdims=True))
+    np.testing.assert_allclose(z, e / e.sum(1, keepdims=True), rtol=1e-5, atol=1e-7)
+    want = np.tanh(g.astype(np.float64)) @ w.astype(np.float64)
+    np.testing.assert_allclose(np.asarray(o, np.float64), want, rtol=2e-2, atol=2e-2 * np.abs(want).max())
