@@ -1678,6 +1678,19 @@ struct Planner {
     return mx >= (1LL << 31) - 1024 ? "i64" : "int";
   }
 
+  // Elements of the largest tensor in memory that evaluating `vals` reads: a slice or a gather reads a larger one than it makes.
+  static int64_t largest_read(const std::vector<Value*>& vals, const std::function<bool(Op*)>& internal) {
+    int64_t mx = 0;
+    std::set<Value*> seen;
+    std::function<void(Value*)> walk = [&](Value* v) {
+      if (!seen.insert(v).second) return;
+      if (!v->def || !internal(v->def)) { mx = std::max<int64_t>(mx, v->type.numel()); return; }
+      for (Value* o : v->def->operands) walk(o);
+    };
+    for (Value* v : vals) walk(v);
+    return mx;
+  }
+
   std::string store_expr(DT d, const std::string& e) {
     if (d == DT::BF16) return "f_to_bf16(" + e + ")";
     if (d == DT::F16) return "f_to_f16(" + e + ")";
@@ -3574,7 +3587,15 @@ struct Planner {
     em.is_internal = internal;
     em.round_small_floats = true;
     int64_t total = Nk * std::max<int64_t>(Nr, 1);
-    em.idx_t = total >= (1LL << 31) - 65536 ? "i64" : "int";
+    // 32-bit indices only where they reach whatever is read, and rows stored with padding between them
+    int64_t reach = total;
+    for (auto& part : rg.parts) reach = std::max(reach, largest_read(part.operands, internal));
+    if (full)
+      for (const FullOut& fo : *full) reach = std::max({reach, largest_read({fo.v}, internal), fo.v->type.numel() / fo.v->type.dims.back() * fo.ld});
+    if (epilogue)
+      for (Group* eg : *epilogue)
+        for (Op* r : eg->roots) reach = std::max(reach, largest_read(r->results, [&](Op* o) { return eg->members.count(o) || is_dup(o); }));
+    em.idx_t = reach >= (1LL << 31) - 65536 ? "i64" : "int";
     em.indent_ = 6;
     // Q consecutive kept indices per thread (column form), or V consecutive reduced ones (row form, where the reduced
     // dimensions are the innermost): 16-byte pieces of what is read along memory, 8-byte ones of 2-byte types in columns.
@@ -4912,9 +4933,12 @@ struct Planner {
     const bool hold = V > 1 && rounds * V <= 32 && !getenv("B200_NO_HELD_ROWS");
     std::map<size_t, DT> held;         // input number -> type, of those kept in registers
     int64_t held_bytes = 0;
-    const std::string it = "int";
     std::set<Op*> chain_members;
     for (Group* g : rc.stages) chain_members.insert(g->members.begin(), g->members.end());
+    int64_t reach = 0;                 // the rows' own elements are below 2^31 (row_form); what a slice of them reads need not be
+    for (Group* g : rc.stages)
+      for (Op* r : g->roots) reach = std::max(reach, largest_read(r->operands, [&](Op* o) { return chain_members.count(o) || is_dup(o); }));
+    const std::string it = reach >= (1LL << 31) - 65536 ? "i64" : "int";
     // a value needs memory when somebody outside the chain reads it (looking through the broadcasts and other
     // duplicable operations that are evaluated inline by their users)
     std::function<bool(Value*)> stored = [&](Value* v) -> bool {

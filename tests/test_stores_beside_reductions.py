@@ -43,3 +43,35 @@ def test_values(client, cols):
     np.testing.assert_allclose(z, e / e.sum(1, keepdims=True), rtol=1e-5, atol=1e-7)
     want = np.tanh(g.astype(np.float64)) @ w.astype(np.float64)
     np.testing.assert_allclose(np.asarray(o, np.float64), want, rtol=2e-2, atol=2e-2 * np.abs(want).max())
+
+
+def _kernel(src, name):
+    body = src[src.index(f" {name}("):]
+    return body[:body.index("\n}\n")]
+
+
+@pytest.mark.parametrize("rows,wide", [(2_080_000, False), (2_090_000, True)])
+def test_padded_rows_past_32_bits(rows, wide):
+    """2 090 000 rows of 1026 elements are below 2^31, 1032 apart they are not."""
+    assert rows * 1026 < 2**31 - 65536 and (rows * 1032 >= 2**31) == wide
+    b = Builder()
+    g, w = b.arg((rows, 1026), "bf16"), b.arg((1026, 64), "bf16")
+    plan, src = b200.compile_to_plan(b.module([b.reduce_sum(b.convert(g, "f32"), (0,)), b.matmul(b.tanh(g), w)]), validate=True)
+    assert "partial+fusion{tanh}" in plan, plan
+    assert ("(i64)x0 * 1032" if wide else "(int)x0 * 1032") in _kernel(src, "reduce_0")
+
+
+@pytest.mark.parametrize("kind", ["rows", "columns", "chain", "chain of two reads"])
+def test_slices_of_a_tensor_past_32_bits(kind):
+    """10 000 of 3 000 000 rows of 1024: the reduction is small, where it reads is not."""
+    b = Builder()
+    x = b.arg((3_000_000, 1024), "bf16")
+    y = b.convert(b.slice(x, [2_990_000, 0], [3_000_000, 1024]), "f32")
+    s = b.reduce_sum(y, (0 if kind == "columns" else 1,))
+    outs = [b.rsqrt(s), b.tanh(s)] if kind == "chain" else [s]
+    if kind == "chain of two reads":
+        outs = [b.mul(b.bcast(s, y.shape, (0,)), b.convert(b.slice(x, [1_990_000, 0], [2_000_000, 1024]), "f32"))]
+    plan, src = b200.compile_to_plan(b.module(outs), validate=True)
+    assert ("row{" in plan) == kind.startswith("chain"), plan
+    readers = [k for k in src.split('extern "C"')[1:] if "const u16* __restrict__ in" in k]
+    assert readers and all("const i64 " in k for k in readers)
