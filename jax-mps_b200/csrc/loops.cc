@@ -15,7 +15,9 @@
 // and one per iteration. Against 64 bits, the gradients of four LSTM steps (100 x 64 x 32 x 256 and smaller), norm of the
 // difference over the norm: 2.0e-7 to 2.9e-7 before, 1.8e-7 to 2.6e-7 now; over 512 rows in one chain the largest was 5.3e-7.
 // Taken when the loop's trip count is known and at least 8, an iteration's product is below 2^30 multiply-adds (larger ones
-// fill the chip by themselves) and all stacks together are below 512 MB.
+// fill the chip by themselves) and all that is written in front of a loop, by its iterations and behind it for the sake of the
+// split is below 512 MB: stacks, the operands they are made of, partial sums. A sum over an operand that is the same in all
+// iterations stays in the loop: its stack would be as many copies of one tensor.
 #include "loops.h"
 
 #include <algorithm>
@@ -318,8 +320,32 @@ struct Splitter {
     w->results.push_back(res);
     return carried_[v] = res;
   }
-  int64_t history_bytes(Value* v) { return fixed(v) || carried_.count(v) || stack_.count(v) ? 0 : trips * (int64_t)v->type.bytes(); }
-  bool fits(int64_t more) { return bytes + more <= kMaxStackBytes; }
+  // What stacked(v) and history(v) write that is not there yet. Each step counts as a tensor in memory, although kernels take
+  // pointwise ones in; `seen` holds what the same sum has counted already.
+  int64_t stacked_bytes(Value* v, std::set<Value*>& seen) {
+    if (stack_.count(v) || !seen.insert(v).second) return 0;
+    const int64_t all = trips * (int64_t)v->type.bytes();
+    if (fixed(v)) return all;
+    Op* d = v->def;
+    const std::string sh = d->short_name();
+    if (sh == "dynamic_slice") {
+      long long base, slope;
+      affine(d->operands[1], base, slope);
+      return all * ((fixed(d->operands[0])->type.dims[0] != trips) + (slope < 0));        // a slice, reversed
+    }
+    int64_t n = sh == "reshape" ? 0 : all;
+    for (size_t k = 0; k < (sh == "dot_general" ? 1 : d->operands.size()); k++) n += stacked_bytes(d->operands[k], seen);
+    return n;
+  }
+  int64_t history_bytes(Value* v, std::set<Value*>& seen) {
+    if (known(v)) return stacked_bytes(v, seen);
+    return carried_.count(v) || !seen.insert(v).second ? 0 : 2 * trips * (int64_t)v->type.bytes();      // zeros to begin with, and the stack
+  }
+  bool fits(int64_t more) {
+    if (bytes + more > kMaxStackBytes) return false;
+    bytes += more;
+    return true;
+  }
 
   Value* sum_over(Value* v, const std::vector<int64_t>& dims, const TensorType& t) {
     TensorType scalar;
@@ -379,9 +405,8 @@ struct Splitter {
     for (size_t i = 0; i < body->ops.size(); i++) {
       Op* d = body->ops[i].get();
       if (d->short_name() != "dot_general" || d->results.size() != 1 || !known(d->results[0]) || product_size(d) >= (1LL << 30)) continue;
-      const int64_t more = trips * (int64_t)(d->results[0]->type.bytes() + d->operands[0]->type.bytes());
-      if (!fits(more)) continue;
-      bytes += more;
+      std::set<Value*> seen;
+      if (!fits(stacked_bytes(d->results[0], seen))) continue;
       Value* all = stacked(d->results[0]);
       need_indices();
       TensorType row = d->results[0]->type;
@@ -416,10 +441,12 @@ struct Splitter {
         Value *A = d->operands[0], *B = d->operands[1];
         if (A->type.rank() != 2 || B->type.rank() != 2 || A->type.dt != DT::F32 || B->type.dt != DT::F32 || A == B || product_size(d) >= (1LL << 30) || product_size(d) == 0) continue;
         if (!f["lhs_batching_dimensions"].empty() || f["lhs_contracting_dimensions"] != std::vector<int64_t>{0} || f["rhs_contracting_dimensions"] != std::vector<int64_t>{0}) continue;
-        const int64_t per = std::max<int64_t>(1, kSumRows / A->type.dims[0]);
-        const int64_t more = history_bytes(A) + history_bytes(B) + (trips / per + 1) * (int64_t)term->type.bytes();
+        if (fixed(A) || fixed(B)) continue;
+        const int64_t per = std::min<int64_t>(trips, std::max<int64_t>(1, kSumRows / A->type.dims[0]));
+        std::set<Value*> seen;
+        int64_t more = history_bytes(A, seen) + history_bytes(B, seen) + (trips / per + 3) * (int64_t)term->type.bytes();
+        if (trips % per) more += trips * (int64_t)(A->type.bytes() + B->type.bytes());      // the whole sums' iterations, sliced
         if (!fits(more)) continue;
-        bytes += more;
         sum = sum_of_products(history(A), history(B), term->type);
       } else if (d->short_name() == "reduce" && d->operands.size() == 2) {
         Op* z = d->operands[1]->def;
@@ -429,8 +456,8 @@ struct Splitter {
         float zero_value = 1.f;
         if (dv.type.dt != DT::F32 || dv.type.numel() != 1) continue;
         memcpy(&zero_value, dv.data.data(), 4);
-        if (zero_value != 0.f || d->operands[0]->type.dt != DT::F32 || !fits(history_bytes(d->operands[0]))) continue;
-        bytes += history_bytes(d->operands[0]);
+        std::set<Value*> seen;
+        if (zero_value != 0.f || d->operands[0]->type.dt != DT::F32 || fixed(d->operands[0]) || !fits(history_bytes(d->operands[0], seen))) continue;
         std::vector<int64_t> dims{0};
         for (int64_t x : attr_i64s(d->attr("dimensions"))) dims.push_back(x + 1);
         sum = sum_over(history(d->operands[0]), dims, term->type);

@@ -1,0 +1,72 @@
+"""What a counted loop costs in memory when its sums leave it: 512 MB at most, whatever the operands of a sum are made of, and
+nothing where one of them is the same in all iterations. Plans only: no step of these sizes is run."""
+import re
+
+import pytest
+
+import b200
+from b200.shlo.builder import Builder
+
+
+def sums(T, R, I, N, form):
+    """dw += a^T g[t], db += the rows of g[t], over t; `a` is a tensor that does not change ("same"), a function of one ("made"),
+    the slice x[t] ("rows"), x[T-1-t] ("reversed"), or carried from iteration to iteration ("carried")."""
+    b = Builder()
+    x, g = b.arg((R, I) if form in ("same", "made", "carried") else (T, R, I), "f32"), b.arg((T, R, N), "f32")
+
+    def at(s, v, t): return s.reshape(s.dynamic_slice(v, [t, s.const(0, "i32"), s.const(0, "i32")], (1, *v.shape[1:])), v.shape[1:])
+
+    def body(s, k, dw, db, h):
+        gt = at(s, g, s.sub(s.const(T - 1, "i32"), k) if form == "reversed" else k)
+        a = {"same": lambda: x, "made": lambda: s.tanh(x), "rows": lambda: at(s, x, k), "reversed": lambda: at(s, x, s.sub(s.const(T - 1, "i32"), k)),
+             "carried": lambda: h}[form]()
+        return [s.add(k, s.const(1, "i32")), s.add(dw, s.dot_general(a, gt, ((0,), (0,)))), s.add(db, s.reduce_sum(gt, (0,))), s.tanh(h)]
+    start = x if form == "carried" else b.full((1, 1), 0.5, "f32")
+    _, dw, db, h = b.while_([b.const(0, "i32"), b.full((I, N), 0.0, "f32"), b.full((N,), 0.0, "f32"), start], lambda s, k, *r: s.compare(k, s.const(T, "i32"), "LT"), body)
+    return b.module([dw, db, h], name=f"jit_sums_{T}_{R}_{I}_{N}_{form}")
+
+
+def _arena(plan):
+    return int(re.search(r"arena0 (\d+) bytes", plan).group(1))
+
+
+# whether the product over all iterations stands behind the loop
+CASES = [("same", 400, 4096, 1024, 64, False), ("same", 12000, 4096, 1024, 2, False), ("same", 16, 64, 64, 64, False), ("made", 16, 64, 64, 64, True),
+         ("made", 400, 4096, 1024, 64, False), ("rows", 1000, 64, 1024, 16, True), ("rows", 1001, 64, 1024, 16, True), ("rows", 2001, 64, 1024, 16, False),
+         ("rows", 65536, 2, 64, 64, True), ("reversed", 1000, 64, 1024, 16, True), ("reversed", 1800, 64, 1024, 16, True), ("reversed", 1900, 64, 1024, 16, False),
+         ("carried", 100, 64, 256, 64, True), ("carried", 900, 64, 1024, 16, True), ("carried", 1100, 64, 1024, 16, False)]
+
+
+@pytest.mark.parametrize("form,T,R,I,N,taken", CASES)
+def test_scratch_of_sums_behind_a_loop(monkeypatch, form, T, R, I, N, taken):
+    text = sums(T, R, I, N, form)
+    split = b200.compile_to_plan(text)[0]
+    monkeypatch.setenv("B200_NO_LOOP_SPLIT", "1")
+    whole = b200.compile_to_plan(text)[0]
+    assert _arena(split) - _arena(whole) <= 512 << 20, split
+    assert any(line.startswith("  igemm") for line in split.splitlines()) == taken, split
+    assert taken or _arena(split) <= _arena(whole), (split, whole)
+
+
+def recurrence(T, R, I, N):
+    """h = tanh([x[t], y[T-1-t]] w + h): the product is made in front of the loop from a concatenation of a slice and a reversed one."""
+    b = Builder()
+    x, y, w, h0 = b.arg((T, R, I), "f32"), b.arg((T, R, I), "f32"), b.arg((2 * I, N), "f32"), b.arg((R, N), "f32")
+
+    def at(s, v, t): return s.reshape(s.dynamic_slice(v, [t, s.const(0, "i32"), s.const(0, "i32")], (1, *v.shape[1:])), v.shape[1:])
+
+    def body(s, k, h):
+        a = s.concatenate([at(s, x, k), at(s, y, s.sub(s.const(T - 1, "i32"), k))], 1)
+        return [s.add(k, s.const(1, "i32")), s.tanh(s.add(s.matmul(a, w), h))]
+    return b.module([b.while_([b.const(0, "i32"), h0], lambda s, k, *r: s.compare(k, s.const(T, "i32"), "LT"), body)[1]], name=f"jit_front_{T}_{R}_{I}_{N}")
+
+
+@pytest.mark.parametrize("T,R,I,N,taken", [(100, 64, 32, 1024, True), (900, 64, 256, 1024, True), (1300, 64, 256, 1024, False), (2500, 64, 256, 16, True),
+                                           (6000, 64, 256, 16, False)])
+def test_scratch_of_a_product_in_front_of_a_loop(monkeypatch, T, R, I, N, taken):
+    text = recurrence(T, R, I, N)
+    split = b200.compile_to_plan(text)[0]
+    monkeypatch.setenv("B200_NO_LOOP_SPLIT", "1")
+    whole = b200.compile_to_plan(text)[0]
+    assert any(line.startswith("  igemm") for line in split.splitlines()) == taken, split
+    assert _arena(split) - _arena(whole) <= (512 << 20 if taken else 0), split
