@@ -3026,7 +3026,9 @@ struct Planner {
     }
   }
   // rows past the matrix are zero in every panel
-  for (int e = u; e < 2 * NB * (NP - N); e += TT) ((T*)final4[0])[(e / (NP - N)) * NP + N + e % (NP - N)] = (T)0;
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    for (int e = u; e < NB * (NP - N); e += TT) ((T*)final4[h])[(e / (NP - N)) * NP + N + e % (NP - N)] = (T)0;
   auto update = [&](int q, const V4* from) {         // piece q less what the panel's columns take from it
 #pragma unroll
     for (int k = 0; k < NB; ++k) {

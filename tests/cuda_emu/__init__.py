@@ -41,6 +41,14 @@ DEV u16 f_to_f16(float f) { _Float16 v = (_Float16)f; u16 h; std::memcpy(&h, &v,
 '''
 
 
+# where the kernels' shared memory lies (the symbols are the linker's, absent where no kernel has any)
+_SHARED_BOUNDS = '''
+extern char __start_emu_shared[] __attribute__((weak)), __stop_emu_shared[] __attribute__((weak));
+extern "C" void* emu_shared_begin() { return __start_emu_shared; }
+extern "C" void* emu_shared_end() { return __stop_emu_shared; }
+'''
+
+
 def _host_source(src: str) -> str:
     """The generated translation unit with its four inline-PTX helpers replaced by C++."""
     out, skip = [], False
@@ -58,7 +66,7 @@ def _host_source(src: str) -> str:
     text = "\n".join(out)
     at = text.index("#define DEV")
     at = text.index("\n", at) + 1
-    return '#include "shim.h"\n' + text[:at] + _HOST_CONVERSIONS + text[at:]
+    return '#include "shim.h"\n' + text[:at] + _HOST_CONVERSIONS + text[at:] + _SHARED_BOUNDS
 
 
 def _cache_dir() -> Path:
@@ -78,9 +86,9 @@ def _runner() -> Path:
     key = hashlib.sha256(((HERE / "shim.h").read_text() + (HERE / "runner.cc").read_text()).encode()).hexdigest()[:24]
     so = _cache_dir() / f"libemu_runner_{key}.so"
     if not so.exists():
-        _compile(["g++", "-std=c++17", "-O1", "-g0", "-w", "-fPIC", "-shared", "-pthread", f"-I{HERE}", str(HERE / "runner.cc"), "-o", str(so) + ".tmp"],
+        _compile(["g++", "-std=c++17", "-O1", "-g0", "-w", "-fPIC", "-shared", "-pthread", f"-I{HERE}", str(HERE / "runner.cc"), "-o", f"{so}.{os.getpid()}.tmp"],
                  "the runner")
-        os.replace(str(so) + ".tmp", so)
+        os.replace(f"{so}.{os.getpid()}.tmp", so)
     return so
 
 
@@ -93,8 +101,8 @@ def _build(src: str):
         cu = _cache_dir() / f"k{key}.cc"
         cu.write_text(host)
         _compile(["g++", "-std=c++17", "-O0", "-g0", "-w", "-fPIC", "-shared", f"-I{HERE}", str(cu), str(runner), f"-Wl,-rpath,{runner.parent}",
-                  "-o", str(so) + ".tmp"], "the generated source")
-        os.replace(str(so) + ".tmp", so)
+                  "-o", f"{so}.{os.getpid()}.tmp"], "the generated source")
+        os.replace(f"{so}.{os.getpid()}.tmp", so)
     return C.CDLL(str(runner), mode=C.RTLD_GLOBAL), C.CDLL(str(so))
 
 
@@ -140,10 +148,11 @@ def _scatter_elems(slots, numel, updates, computation, nbytes, args):
                 o[k] = fold(o[k], u[q])
 
 
-def run_plan_on_cpu(text: str, inputs: list) -> list:
+def run_plan_on_cpu(text: str, inputs: list, edit=None) -> list:
     """Compiles `text`, runs the plan's kernel steps on host threads and returns the results as NumPy arrays (bf16
-    results as float32)."""
+    results as float32). `edit` changes the source first: a test adds its own checks to a kernel."""
     plan, src = b200.compile_to_plan(text, slots=True)
+    src = edit(src) if edit else src
     _, table = plan.split("slots:\n")
     table, launches = table.split("launches:\n")
     steps = []
@@ -185,8 +194,11 @@ def run_plan_on_cpu(text: str, inputs: list) -> list:
         if m:                            # a result may be a reshaped view of a slot: its own type counts
             results[int(m.group(1))] = (int(m.group(2)), tuple(int(v) for v in m.group(3).split("x") if v), m.group(4))
     runner, lib = _build(src)
-    runner.emu_launch.argtypes = [C.c_void_p, C.c_int, C.POINTER(C.c_void_p), C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int]
+    runner.emu_launch.argtypes = [C.c_void_p, C.c_int, C.POINTER(C.c_void_p), C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_longlong]
     runner.emu_launch.restype = None
+    lib.emu_shared_begin.restype = lib.emu_shared_end.restype = C.c_void_p
+    shared = lib.emu_shared_begin() or 0
+    shared_bytes = (lib.emu_shared_end() or 0) - shared
     for kind, name, dims, args in steps:
         if kind == "memcpy":
             slots[args[0]][0][:name] = slots[args[1]][0][:name]
@@ -196,7 +208,7 @@ def run_plan_on_cpu(text: str, inputs: list) -> list:
             continue
         fn = C.cast(getattr(lib, name), C.c_void_p)
         ptrs = (C.c_void_p * len(args))(*[slots[a][0].ctypes.data for a in args])
-        runner.emu_launch(fn, len(args), ptrs, *dims)
+        runner.emu_launch(fn, len(args), ptrs, *dims, shared, shared_bytes)
     outs = []
     for k in sorted(results):
         sid, shape, dt = results[k]

@@ -73,7 +73,7 @@ void call(void* fn, int n, void** a) {
 }
 }  // namespace
 
-extern "C" void emu_launch(void* fn, int nargs, void** args, int gx, int gy, int gz, int bx, int by, int bz) {
+extern "C" void emu_launch(void* fn, int nargs, void** args, int gx, int gy, int gz, int bx, int by, int bz, void* shared, long long shared_bytes) {
   using namespace emu;
   const int nthreads = bx * by * bz, nwarps = (nthreads + 31) / 32;
   g_block_dim = {(unsigned)bx, (unsigned)by, (unsigned)bz};
@@ -88,6 +88,7 @@ extern "C" void emu_launch(void* fn, int nargs, void** args, int gx, int gy, int
       warps[w].lanes = std::min(32, nthreads - 32 * w);
       warps[w].bar.reset(warps[w].lanes);
     }
+    if (shared_bytes) memset(shared, 0xFF, (size_t)shared_bytes);
   };
   arm();
   std::vector<std::thread> team;

@@ -18,7 +18,8 @@ using std::signbit;
 #define __host__
 #define __forceinline__ inline __attribute__((always_inline))
 #define __launch_bounds__(...)
-#define __shared__ static
+// all of it in one section, which the runner fills with NaNs (all bits set) in front of every block
+#define __shared__ static __attribute__((section("emu_shared")))
 #define __align__(n) __attribute__((aligned(n)))
 
 struct alignas(8) uint2 { unsigned x, y; };
@@ -110,4 +111,4 @@ static inline double erfinv(double y) {
 }
 static inline float erfinvf(float y) { return (float)erfinv((double)y); }
 
-extern "C" void emu_launch(void* fn, int nargs, void** args, int gx, int gy, int gz, int bx, int by, int bz);
+extern "C" void emu_launch(void* fn, int nargs, void** args, int gx, int gy, int gz, int bx, int by, int bz, void* shared, long long shared_bytes);

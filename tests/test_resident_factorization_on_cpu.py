@@ -30,6 +30,24 @@ def test_resident_cholesky(n, scale, lower):
     np.testing.assert_allclose(got, want, rtol=0, atol=n * 2.0 ** -23 * np.abs(want).max())
 
 
+@pytest.mark.parametrize("n", [33, 50, 67, 141])
+def test_rows_past_the_matrix_are_zero(n):
+    """... in both panels that the tile warps read, of shared memory that is full of NaNs to begin with."""
+    check = """  if (u == 0)
+    for (int h = 0; h < 2; ++h)
+      for (int k = 0; k < NB; ++k)
+        for (int r = N; r < NP; ++r)
+          if (((const T*)final4[h])[k * NP + r] != (T)0) o[0] = __uint_as_float(0x7FC00000u);
+"""
+    def edit(src):
+        at = src.index("#undef AT", src.index("final4"))
+        return src[:at] + check + src[at:]
+    b = Builder()
+    a = _spd(n)
+    got = run_plan_on_cpu(b.module([b.cholesky(b.arg(a.shape, "f32"))]), [a], edit)[0]
+    np.testing.assert_allclose(got, np.linalg.cholesky(a.astype(np.float64)), rtol=0, atol=n * 2.0 ** -23 * 4)
+
+
 def test_resident_cholesky_of_an_indefinite_matrix():
     n = 52
     a = _spd(n)
