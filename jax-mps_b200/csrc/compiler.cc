@@ -5782,17 +5782,21 @@ struct Planner {
             for (size_t oj = oi + 1; oj < order.size() && oj < oi + 16 && rc.stages.size() < 8; oj++) {
               Unit& nu = units[order[oj]];
               if (nu.kind == Unit::CONST_MAT) {
-                std::set<Value*> seen;
-                std::function<bool(Value*)> dep = [&](Value* v) -> bool {
-                  if (produced.count(v)) return true;
-                  if (!seen.insert(v).second || !v->def || v->def->parent != block || !is_dup(v->def)) return false;
-                  for (Value* o : v->def->operands) if (dep(o)) return true;
+                auto made_of = [&](const std::set<Value*>& these) {
+                  std::set<Value*> seen;
+                  std::function<bool(Value*)> dep = [&](Value* v) -> bool {
+                    if (these.count(v)) return true;
+                    if (!seen.insert(v).second || !v->def || v->def->parent != block || !is_dup(v->def)) return false;
+                    for (Value* o : v->def->operands) if (dep(o)) return true;
+                    return false;
+                  };
+                  for (Value* o : nu.op->operands) if (dep(o)) return true;
                   return false;
                 };
-                bool d = false;
-                for (Value* o : nu.op->operands) d = d || dep(o);
-                if (d) break;
-                before.push_back(oj);
+                if (made_of(produced)) break;
+                const bool after = made_of(late);
+                (after ? behind : before).push_back(oj);
+                if (after) late.insert(nu.op->results.begin(), nu.op->results.end());
                 continue;
               }
               if (nu.kind != Unit::GROUP || absorbed.count(nu.group) || nu.group->roots.empty()) {
@@ -5836,9 +5840,10 @@ struct Planner {
               emit_row_chain(rc, plan, st);
               behind.resize(n_behind_at_last);
               for (size_t ob : behind) {
-                Group* bg = units[order[ob]].group;
-                if (!absorbed.count(bg)) emit_group(bg, plan, st);
-                emitted.insert(bg);
+                Unit& bu = units[order[ob]];
+                if (bu.kind == Unit::CONST_MAT) { materialize_dup(bu.op, plan, st); continue; }
+                if (!absorbed.count(bu.group)) emit_group(bu.group, plan, st);
+                emitted.insert(bu.group);
               }
               oi = last_stage;
               continue;

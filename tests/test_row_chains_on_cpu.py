@@ -1,4 +1,4 @@
-"""Chains of row kernels: rows of a few elements, units between two stages that read the chain but not by rows, reshapes on both
+"""Chains of row kernels: rows of a few elements, units between two stages that read the chain but not by rows and what is filled with them, reshapes on both
 sides of a softmax, rows of one block of 1024 threads. The generated kernels run on the CPU and are held to the interpreter."""
 import shutil
 
@@ -58,3 +58,18 @@ def test_a_block_of_1024_threads():
     text = b.module([b.div(e, b.bcast(b.reduce_sum(e, (1,)), x.shape, (0,)))])
     assert "block=1024x1" in b200.compile_to_plan(text)[0]
     _check(text, [r.standard_normal((2, 8194)).astype(np.float32)], 1e-6)
+
+
+@pytest.mark.parametrize("rows,cols", [(64, 64), (7, 33)])
+def test_a_broadcast_of_what_stands_behind_the_chain(rows, cols):
+    """The sum over all rows is made behind the chain of rows, and so is the tensor filled with it."""
+    r = np.random.default_rng(rows)
+    b = Builder()
+    t = b.arg((rows, cols), "f32")
+    s = b.reduce_sum(t, (1,))
+    q = b.reduce_sum(b.mul(s, s), (0,))
+    filled = b.bcast(q, (rows, cols), ())
+    text = b.module([b.sub(t, b.bcast(s, t.shape, (0,))), filled])
+    plan = b200.compile_to_plan(text)[0]
+    assert plan.count(" row{") == 1, plan
+    _check(text, [r.standard_normal((rows, cols)).astype(np.float32)], 1e-5)
