@@ -3597,6 +3597,8 @@ struct Planner {
     if (epilogue)
       for (Group* eg : *epilogue)
         for (Op* r : eg->roots) reach = std::max(reach, largest_read(r->results, [&](Op* o) { return eg->members.count(o) || is_dup(o); }));
+    // ... and up to where a thread's index stands when it leaves its row: a step (of 256 threads, eight elements each) past the end
+    if (!col) reach += 256LL * 8 * splits;
     em.idx_t = reach >= (1LL << 31) - 65536 ? "i64" : "int";
     em.indent_ = 6;
     // Q consecutive kept indices per thread (column form), or V consecutive reduced ones (row form, where the reduced

@@ -75,3 +75,16 @@ def test_slices_of_a_tensor_past_32_bits(kind):
     assert ("row{" in plan) == kind.startswith("chain"), plan
     readers = [k for k in src.split('extern "C"')[1:] if "const u16* __restrict__ in" in k]
     assert readers and all("const i64 " in k for k in readers)
+
+
+@pytest.mark.parametrize("n,wide", [(2**31 - 3_000_000, False), (2**31 - 2_000_000, True), (2**31 - 100_000, True)])
+def test_the_step_past_the_end_of_a_row(n, wide):
+    """A row shared by a thousand blocks: the index that ends a thread's loop lies up to two million elements past the row."""
+    b = Builder()
+    plan, src = b200.compile_to_plan(b.module([b.reduce_sum(b.arg((n,), "f32"), (0,))]), validate=True)
+    splits = int(plan.split("grid=1x")[1].split()[0])
+    assert splits > 1000, plan
+    loop = next(line for line in _kernel(src, "reduce_0").splitlines() if "gridDim.y" in line and "for (" in line)
+    step = 256 * (4 if "* 4;" in loop else 1) * splits
+    assert (n + step >= 2**31) <= wide
+    assert loop.strip().startswith("for (i64 " if wide else "for (int "), loop
