@@ -4301,25 +4301,120 @@ struct Planner {
   std::map<std::tuple<Block*, Value*, long long>, int> repacked;   // padded copies of operands, per block
   std::set<Value*> padded;                                         // values that exist in padded rows only
 
+  // The sides of a product: their batch, free and contracting dimensions, and the strides of the tensors.
+  struct DotSides {
+    std::vector<int64_t> lbd, rbd, lcd, rcd, lfree, rfree, sl, sr;
+    int64_t G, M, N, K;
+    explicit DotSides(Op* op) {
+      Value *lhs = op->operands[0], *rhs = op->operands[1];
+      auto f = attr_struct(op->attr("dot_dimension_numbers"));
+      lbd = f["lhs_batching_dimensions"], rbd = f["rhs_batching_dimensions"];
+      lcd = f["lhs_contracting_dimensions"], rcd = f["rhs_contracting_dimensions"];
+      auto in = [](const std::vector<int64_t>& v, int64_t x) { return std::find(v.begin(), v.end(), x) != v.end(); };
+      for (int d = 0; d < lhs->type.rank(); d++) if (!in(lbd, d) && !in(lcd, d)) lfree.push_back(d);
+      for (int d = 0; d < rhs->type.rank(); d++) if (!in(rbd, d) && !in(rcd, d)) rfree.push_back(d);
+      sl = strides_of(lhs->type.dims), sr = strides_of(rhs->type.dims);
+      auto extent = [](const std::vector<int64_t>& dims, const std::vector<int64_t>& which) {
+        int64_t n = 1;
+        for (auto d : which) n *= dims[d];
+        return n;
+      };
+      G = extent(lhs->type.dims, lbd), M = extent(lhs->type.dims, lfree), K = extent(lhs->type.dims, lcd);
+      N = extent(rhs->type.dims, rfree);
+    }
+  };
+
+  // An fp32 product as a strided matrix per group on both sides, with one of its two indices contiguous; false when it is not one.
+  static bool dense_product(Op* op, const DotSides& d, Gemm32Launch& g) {
+    Value *lhs = op->operands[0], *rhs = op->operands[1];
+    const int64_t G = d.G, M = d.M, N = d.N, K = d.K;
+    long long mv, kv, nv, kv2, gv, gv2;
+    long long ms = 0, ks = 0, ns = 0, ks2 = 0;
+    if (!(M > 0 && N > 0 && K > 0 && G > 0 && collapse_dims(lhs->type.dims, d.sl, d.lfree, mv, ms) && collapse_dims(lhs->type.dims, d.sl, d.lcd, kv, ks) &&
+          collapse_dims(rhs->type.dims, d.sr, d.rfree, nv, ns) && collapse_dims(rhs->type.dims, d.sr, d.rcd, kv2, ks2) &&
+          collapse_dims(lhs->type.dims, d.sl, d.lbd, gv, g.a_gs) && collapse_dims(rhs->type.dims, d.sr, d.rbd, gv2, g.b_gs) &&
+          (ks == 1 || ms == 1 || K == 1 || M == 1) && (ks2 == 1 || ns == 1 || K == 1 || N == 1)))
+      return false;
+    g.M = (int)M; g.N = (int)N; g.K = (int)K; g.G = (int)G;
+    // an index of extent one is contiguous whatever its stride
+    g.a_kc = (ks == 1 || K == 1) ? 1 : 0;
+    g.a_ld = g.a_kc ? ms : ks;
+    g.b_kc = (ns == 1 || N == 1) ? 0 : 1;
+    g.b_ld = g.b_kc ? ns : ks2;
+    auto rows16 = [](int extent, long long ld, long long gs) { return extent % 4 == 0 && ld % 4 == 0 && gs % 4 == 0; };
+    g.a_vec = rows16(g.a_kc ? g.K : g.M, g.a_ld, g.a_gs);
+    g.b_vec = rows16(g.b_kc ? g.K : g.N, g.b_ld, g.b_gs);
+    return true;
+  }
+
+  // The three ways of a dense fp32 product: the FMA pipe, tiled copies, the table-driven kernels. Their modelled times (us, 1e30
+  // where a way is closed), the tile and split of the first two.
+  struct ProductWays {
+    Gemm32Launch fma;
+    Tile32Launch tiles;
+    double us_fma = 1e30, us_tile = 1e30, us_table = 1e30;
+    bool by_fma() const { return !by_tiles() && us_fma < us_table; }
+    bool by_tiles() const { return us_tile < us_fma && us_tile < us_table; }
+  };
+  static ProductWays product_ways(Op* op, const Gemm32Launch& dense, bool tensor_cores, int copies) {
+    ProductWays w;
+    Gemm32Launch& g = w.fma = dense;
+    Tile32Launch& t = w.tiles;
+    Value* rhs = op->operands[1];
+    t.M = g.M; t.N = g.N; t.K = g.K; t.G = g.G;
+    int split_k = 1;
+    w.us_fma = fma_product(g, copies, op->has("b200.fma"));
+    w.us_table = table_product(g, split_k, copies);
+    // the switches that keep products off the tensor cores or tiled copies leave them to the FMA pipe
+    const bool tiles = tensor_cores && !getenv("B200_NO_TILE32") && !op->has("b200.fma");
+    if (!tiles) w.us_table = 1e30;
+    // Below a tile of rows or four k-tiles tiled copies are never the fastest (M x K x N, FMA / tables / tiles, us:
+    // 96 x 512 x 2048 14.6 / 13.8 / 14.3, 96 x 2048 x 2048 33 / 19 / 29, 2048 x 64 x 512 8.5 / 10.8 / 9.9).
+    if (g.a_vec && g.M >= 128 && g.K >= 128 && tiles) {
+      t.mode = g.a_kc ? 2 : 3;
+      const long long inner = g.a_kc ? g.K : g.M, outer = g.a_kc ? g.M : g.K;
+      t.dims[0] = inner; t.dims[1] = outer; t.dims[2] = g.G; t.dims[3] = 1;
+      t.strides[0] = outer > 1 ? g.a_ld : (inner + 3) / 4 * 4;
+      t.strides[1] = g.G > 1 ? g.a_gs : t.strides[0] * outer;
+      t.strides[2] = t.strides[1] * g.G;
+      t.box[0] = 32; t.box[1] = g.a_kc ? 128 : 32; t.box[2] = t.box[3] = 1;
+      w.us_tile = tile_product(t, !rhs->def && rhs->owner && rhs->owner->parent_op == nullptr, split_k, copies);
+    }
+    return w;
+  }
+
+  // What the loop split weighs (loops.h).
+  static LoopProductModel loop_product_model(bool tensor_cores) {
+    LoopProductModel lm;
+    lm.in_loop = [tensor_cores](Op* op) {
+      Gemm32Launch g;
+      if (!dense_product(op, DotSides(op), g)) return -1.0;
+      const ProductWays w = product_ways(op, g, tensor_cores, 1);
+      return w.us_fma >= 1e30 ? -1.0 : std::min({w.us_fma, w.us_tile, w.us_table});
+    };
+    lm.in_front = [](Op* op, int64_t trips) {
+      Gemm32Launch g;
+      if (!dense_product(op, DotSides(op), g) || !g.a_kc || g.M * trips >= (1LL << 31)) return 1e30;
+      g.M = (int)(g.M * trips);
+      return fma_product(g, 1, true);
+    };
+    lm.behind = [](int64_t M, int64_t N, int64_t K, int64_t G) {
+      Gemm32Launch g;
+      g.M = (int)M; g.N = (int)N; g.K = (int)K; g.G = (int)G;
+      g.a_kc = g.b_kc = 0;
+      g.a_vec = M % 4 == 0;
+      g.b_vec = N % 4 == 0;
+      return fma_product(g, 1, true);
+    };
+    return lm;
+  }
+
   Step lower_dot(Op* op, BlockState& st) {
     Value *lhs = op->operands[0], *rhs = op->operands[1], *out = op->results[0];
     if (lhs->type.dt != DT::F32 || rhs->type.dt != DT::F32 || out->type.dt != DT::F32)
       throw CompileError("stablehlo.dot_general: only f32 operands are supported so far, got " + lhs->type.str());
-    auto f = attr_struct(op->attr("dot_dimension_numbers"));
-    auto lbd = f["lhs_batching_dimensions"], rbd = f["rhs_batching_dimensions"];
-    auto lcd = f["lhs_contracting_dimensions"], rcd = f["rhs_contracting_dimensions"];
-    auto in = [](const std::vector<int64_t>& v, int64_t x) { return std::find(v.begin(), v.end(), x) != v.end(); };
-    std::vector<int64_t> lfree, rfree;
-    for (int d = 0; d < lhs->type.rank(); d++) if (!in(lbd, d) && !in(lcd, d)) lfree.push_back(d);
-    for (int d = 0; d < rhs->type.rank(); d++) if (!in(rbd, d) && !in(rcd, d)) rfree.push_back(d);
-    auto sl = strides_of(lhs->type.dims), sr = strides_of(rhs->type.dims);
-    auto extent = [](const std::vector<int64_t>& dims, const std::vector<int64_t>& which) {
-      int64_t n = 1;
-      for (auto d : which) n *= dims[d];
-      return n;
-    };
-    int64_t G = extent(lhs->type.dims, lbd), M = extent(lhs->type.dims, lfree), K = extent(lhs->type.dims, lcd),
-            N = extent(rhs->type.dims, rfree);
+    const DotSides d(op);
+    const int64_t G = d.G, M = d.M, N = d.N, K = d.K;
     // offset of the multi-index (row-major over `which`) in a tensor with strides s
     auto offsets = [](const std::vector<int64_t>& dims, const std::vector<int64_t>& s, const std::vector<int64_t>& which,
                       int64_t count) {
@@ -4339,69 +4434,28 @@ struct Planner {
     IGemmParams p;
     p.M = (int)M; p.N = (int)N; p.K = (int)K; p.groups = (int)G;
     p.needs_mask = 0;
-    bool dense = false;
-    {
-      // a strided matrix per group on both sides, with one of its two indices contiguous
-      long long mv, kv, nv, kv2, gv, gv2;
-      long long ms = 0, ks = 0, ns = 0, ks2 = 0;
-      Gemm32Launch g;
-      if (M > 0 && N > 0 && K > 0 && G > 0 && collapse_dims(lhs->type.dims, sl, lfree, mv, ms) && collapse_dims(lhs->type.dims, sl, lcd, kv, ks) &&
-          collapse_dims(rhs->type.dims, sr, rfree, nv, ns) && collapse_dims(rhs->type.dims, sr, rcd, kv2, ks2) &&
-          collapse_dims(lhs->type.dims, sl, lbd, gv, g.a_gs) && collapse_dims(rhs->type.dims, sr, rbd, gv2, g.b_gs) &&
-          (ks == 1 || ms == 1 || K == 1 || M == 1) && (ks2 == 1 || ns == 1 || K == 1 || N == 1)) {
-        g.M = (int)M; g.N = (int)N; g.K = (int)K; g.G = (int)G;
-        // an index of extent one is contiguous whatever its stride
-        g.a_kc = (ks == 1 || K == 1) ? 1 : 0;
-        g.a_ld = g.a_kc ? ms : ks;
-        g.b_kc = (ns == 1 || N == 1) ? 0 : 1;
-        g.b_ld = g.b_kc ? ns : ks2;
-        auto rows16 = [](int extent, long long ld, long long gs) { return extent % 4 == 0 && ld % 4 == 0 && gs % 4 == 0; };
-        g.a_vec = rows16(g.a_kc ? g.K : g.M, g.a_ld, g.a_gs);
-        g.b_vec = rows16(g.b_kc ? g.K : g.N, g.b_ld, g.b_gs);
-        // three ways: the FMA pipe, tiled copies, the table-driven kernels
-        Tile32Launch t;
-        t.M = g.M; t.N = g.N; t.K = g.K; t.G = g.G;
-        int split_k = 1;
-        const int copies = has_company(op, st) ? 2 : 1;
-        const double us_fma = fma_product(g, copies, op->has("b200.fma"));
-        double us_table = table_product(g, split_k, copies), us_tile = 1e30;
-        // the switches that keep products off the tensor cores or tiled copies leave them to the FMA pipe
-        const bool tiles = opts.tensor_cores && !getenv("B200_NO_TILE32") && !op->has("b200.fma");
-        if (!tiles) us_table = 1e30;
-        // Below a tile of rows or four k-tiles tiled copies are never the fastest (M x K x N, FMA / tables / tiles, us:
-        // 96 x 512 x 2048 14.6 / 13.8 / 14.3, 96 x 2048 x 2048 33 / 19 / 29, 2048 x 64 x 512 8.5 / 10.8 / 9.9).
-        if (g.a_vec && g.M >= 128 && g.K >= 128 && tiles) {
-          t.mode = g.a_kc ? 2 : 3;
-          const long long inner = g.a_kc ? g.K : g.M, outer = g.a_kc ? g.M : g.K;
-          t.dims[0] = inner; t.dims[1] = outer; t.dims[2] = g.G; t.dims[3] = 1;
-          t.strides[0] = outer > 1 ? g.a_ld : (inner + 3) / 4 * 4;
-          t.strides[1] = g.G > 1 ? g.a_gs : t.strides[0] * outer;
-          t.strides[2] = t.strides[1] * g.G;
-          t.box[0] = 32; t.box[1] = g.a_kc ? 128 : 32; t.box[2] = t.box[3] = 1;
-          us_tile = tile_product(t, !rhs->def && rhs->owner && rhs->owner->parent_op == nullptr, split_k, copies);
-        }
-        if (us_tile < us_fma || us_table <= us_fma)
-          prog.tensor_saving += st.block->parent_op ? 1e30 : us_fma - std::min(us_tile, us_table);       // a loop's saving counts every time
-        dense = true;
-        if (us_tile < us_fma && us_tile < us_table) p.tile = t;
-        else if (us_fma < us_table) {
-          p.fma = g;
-          p.a_contig = g.a_kc ? 0 : 1;
-          p.b_contig = g.b_kc;
-          p.vec = g.a_vec && g.b_vec;
-          Step s;
-          s.kind = Step::IGEMM;
-          s.label = op->name;
-          s.ig = p;
-          s.args = {slot_of.at(lhs), slot_of.at(rhs), slot_of.at(out)};
-          return s;
-        }
+    Gemm32Launch g;
+    if (dense_product(op, d, g)) {
+      const ProductWays w = product_ways(op, g, opts.tensor_cores, has_company(op, st) ? 2 : 1);
+      if (w.us_tile < w.us_fma || w.us_table <= w.us_fma)
+        prog.tensor_saving += st.block->parent_op ? 1e30 : w.us_fma - std::min(w.us_tile, w.us_table);       // a loop's saving counts every time
+      if (w.by_tiles()) p.tile = w.tiles;
+      else if (w.by_fma()) {
+        p.fma = w.fma;
+        p.a_contig = g.a_kc ? 0 : 1;
+        p.b_contig = g.b_kc;
+        p.vec = g.a_vec && g.b_vec;
+        Step s;
+        s.kind = Step::IGEMM;
+        s.label = op->name;
+        s.ig = p;
+        s.args = {slot_of.at(lhs), slot_of.at(rhs), slot_of.at(out)};
+        return s;
       }
-    }
-    if (!dense) prog.tensor_saving = 1e30;
-    auto am = offsets(lhs->type.dims, sl, lfree, M), ak = offsets(lhs->type.dims, sl, lcd, K);
-    auto bk = offsets(rhs->type.dims, sr, rcd, K), bn = offsets(rhs->type.dims, sr, rfree, N);
-    auto ag = offsets(lhs->type.dims, sl, lbd, G), bg = offsets(rhs->type.dims, sr, rbd, G);
+    } else prog.tensor_saving = 1e30;
+    auto am = offsets(lhs->type.dims, d.sl, d.lfree, M), ak = offsets(lhs->type.dims, d.sl, d.lcd, K);
+    auto bk = offsets(rhs->type.dims, d.sr, d.rcd, K), bn = offsets(rhs->type.dims, d.sr, d.rfree, N);
+    auto ag = offsets(lhs->type.dims, d.sl, d.lbd, G), bg = offsets(rhs->type.dims, d.sr, d.rbd, G);
     std::vector<RowEnt> arow(M);
     std::vector<ColEnt> acol(K);
     std::vector<long long> crow(M), cn(N), cg(G);
@@ -6591,7 +6645,8 @@ std::unique_ptr<CompiledProgram> compile_module(Module& m, const CompileOptions&
     count(f->body.get());
     turn_transposed_products(f->body.get(), uses);
   }
-  if (opts.fuse && !getenv("B200_NO_LOOP_SPLIT")) split_counted_loops(m, f->body.get());
+  if (opts.fuse && !getenv("B200_NO_LOOP_SPLIT"))
+    split_counted_loops(m, f->body.get(), Planner::loop_product_model(opts.tensor_cores));
   SkinnyWeightHoist(m).run(f->body.get());
   DecodeAttentionFusion(m).run(f->body.get());
   // unsupported-op check names every offender at once (src/pjrt_plugin/stablehlo_parser.cc:167-184)

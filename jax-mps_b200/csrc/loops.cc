@@ -9,15 +9,21 @@
 // The chain of an LSTM training step of two layers (64 x 256, 100 steps) shrinks from 15 kernels per reverse iteration to
 // 6, and 400 products of 64 rows become 2 of 6400 rows and 2 of 25 groups.
 //
-// Nothing is computed with less precision: the products stay on the FMA pipe, as those of an iteration do ("b200.fma"), and a
-// sum over iterations is made of partial products over at most 256 rows each, all with the k of a tile shared by at least four
-// warps, which are then added up: chains of 64 additions, where an iteration's product and the additions over iterations made chains of 16
-// and one per iteration. Against 64 bits, the gradients of four LSTM steps (100 x 64 x 32 x 256 and smaller), norm of the
-// difference over the norm: 2.0e-7 to 2.9e-7 before, 1.8e-7 to 2.6e-7 now; over 512 rows in one chain the largest was 5.3e-7.
-// Taken when the loop's trip count is known and at least 8, an iteration's product is below 2^30 multiply-adds (larger ones
-// fill the chip by themselves) and all that is written in front of a loop, by its iterations and behind it for the sake of the
-// split is below 512 MB: stacks, the operands they are made of, partial sums. A sum over an operand that is the same in all
-// iterations stays in the loop: its stack would be as many copies of one tensor.
+// Nothing is computed with less precision: these products go to the FMA pipe ("b200.fma"), whatever pipe an iteration's would
+// take, and a sum over iterations is made of partial products over at most 256 rows each, all with the k of a tile shared by at
+// least four warps, which are then added up: chains of 64 additions, where an iteration's product and the additions over iterations
+// made chains of 16 and one per iteration. Against 64 bits, the gradients of four LSTM steps (100 x 64 x 32 x 256 and smaller),
+// norm of the difference over the norm: 2.0e-7 to 2.9e-7 before, 1.8e-7 to 2.6e-7 now; over 512 rows in one chain the largest was
+// 5.3e-7.
+//
+// Taken when the loop's trip count is known and at least 8, for each product that the time models (compiler.cc) give no more
+// time so than all iterations' own products, and as long as all that is written in front of a loop, by its iterations and behind it
+// for the sake of the split is below 512 MB: stacks, the operands they are made of, partial sums. A sum over an operand that is the same in all
+// iterations stays in the loop: its stack would be as many copies of one tensor. Sums of rows leave only where what they read is
+// stacked for a product. Training steps of two recurrent layers and 50 iterations, batch x hidden, us, products in the
+// loop / split: 16 x 256 2603 / 1620, 64 x 256 3030 / 2307, 128 x 256 3750 / 3030, 256 x 256 5230 / 4660, 64 x 512 5200 / 4230,
+// 256 x 512 8170 / 8020, 512 x 512 (20 iterations) 4575 / 4570, 16 x 1024 8055 / 5150, 64 x 1024 11230 / 10410, 256 x 1024 15510 / 15450. (All products below
+// 2^30 multiply-adds split and all sums of rows: 4910 at 512 x 512, 15660 at 256 x 1024.)
 #include "loops.h"
 
 #include <algorithm>
@@ -86,12 +92,13 @@ struct Splitter {
   Op* w;
   Block *cond, *body;
   Op* next;                                          // the body's return
+  const LoopProductModel& model;
   int counter = -1;
   long long first = 0, trips = 0;
   std::vector<std::unique_ptr<Op>> front, back;      // in front of the loop, behind it
-  int64_t bytes = 0;
   bool changed = false;
   std::map<Value*, bool> known_;                     // can be stacked in front of the loop
+  std::map<Op*, bool> quicker_;
   std::map<Value*, Value*> stack_, outside_;
   std::map<Value*, Value*> carried_;                 // stacked by the loop itself: the loop's result
 
@@ -164,6 +171,26 @@ struct Splitter {
     return outside_[v] = r;
   }
 
+  // Products of all iterations stay on the FMA pipe, whatever pipe an iteration's would take: they leave where that is no slower.
+  double in_loop_us(Op* d) {
+    if (d->operands[0]->type.dt != DT::F32 || d->operands[1]->type.dt != DT::F32 || d->results[0]->type.dt != DT::F32) return -1.0;
+    return (double)trips * model.in_loop(d);
+  }
+  bool quicker_in_front(Op* d) {
+    auto it = quicker_.find(d);
+    if (it != quicker_.end()) return it->second;
+    const double us = in_loop_us(d);
+    return quicker_[d] = us > 0 && model.in_front(d, trips) <= us;
+  }
+  // The sum of A^T B: partial products, what remains of them, and their sum, against a product and an addition an iteration.
+  bool quicker_behind(Op* d, int64_t per) {
+    const int64_t M = d->operands[0]->type.dims[1], N = d->operands[1]->type.dims[1], rows = d->operands[0]->type.dims[0], groups = trips / per, left = trips % per;
+    const double us = in_loop_us(d), mb = (double)M * N * 4e-6;
+    if (us <= 0) return false;
+    return model.behind(M, N, per * rows, groups) + (left ? model.behind(M, N, left * rows, 1) : 0.0) + (groups > 1 ? 2.0 + 2.0 * groups * mb / 6.0 : 0.0) <=
+           us + (double)trips * std::max(2.0, 3.0 * mb / 6.0);
+  }
+
   // Can all iterations' values of `v` be made in front of the loop?
   bool known(Value* v) {
     if (fixed(v)) return true;
@@ -196,7 +223,7 @@ struct Splitter {
     if (sh == "dot_general") {
       auto f = attr_struct(d->attr("dot_dimension_numbers"));
       return known_[v] = f["lhs_batching_dimensions"].empty() && f["rhs_batching_dimensions"].empty() && known(d->operands[0]) && !fixed(d->operands[0]) &&
-                         fixed(d->operands[1]) && v->type.dt == DT::F32 && d->operands[0]->type.dt == DT::F32 && d->operands[1]->type.dt == DT::F32;
+                         fixed(d->operands[1]) && quicker_in_front(d);
     }
     return false;
   }
@@ -266,13 +293,6 @@ struct Splitter {
     return stack_[v] = r;
   }
 
-  int64_t product_size(Op* d) {                       // multiply-adds of one iteration
-    auto f = attr_struct(d->attr("dot_dimension_numbers"));
-    int64_t n = d->results[0]->type.numel();
-    for (int64_t x : f["lhs_contracting_dimensions"]) n *= d->operands[0]->type.dims[x];
-    return n;
-  }
-
   // The iteration number as the type of the counter, in the body.
   std::vector<std::unique_ptr<Op>> body_ops;
   Value* zero_index = nullptr;
@@ -320,30 +340,43 @@ struct Splitter {
     w->results.push_back(res);
     return carried_[v] = res;
   }
-  // What stacked(v) and history(v) write that is not there yet. Each step counts as a tensor in memory, although kernels take
-  // pointwise ones in; `seen` holds what the same sum has counted already.
-  int64_t stacked_bytes(Value* v, std::set<Value*>& seen) {
-    if (stack_.count(v) || !seen.insert(v).second) return 0;
+  // Memory that the split asks for: stacks that live across the loop, what they are made of in front of it (each step counts as a
+  // tensor, although kernels take pointwise ones in; and so does what a carried stack is to begin with), and what a sum behind it
+  // needs while it is made, one after the other. `Claim` is what would come on top.
+  struct Claim { std::set<Value*> stacks, steps; int64_t behind = 0; };
+  Value* unshaped(Value* v) { return known(v) && !fixed(v) && v->def->short_name() == "reshape" ? unshaped(v->def->operands[0]) : v; }
+  void claim_steps(Value* v, Claim& c) {
+    v = unshaped(v);
+    if (!c.steps.insert(v).second || fixed(v) || v->def->short_name() == "dynamic_slice") return;
+    for (size_t k = 0; k < (v->def->short_name() == "dot_general" ? 1 : v->def->operands.size()); k++) claim_steps(v->def->operands[k], c);
+  }
+  void claim(Value* v, Claim& c) {
+    c.stacks.insert(unshaped(v));
+    if (known(v)) claim_steps(v, c);
+  }
+  int64_t step_bytes(Value* v) {
     const int64_t all = trips * (int64_t)v->type.bytes();
-    if (fixed(v)) return all;
-    Op* d = v->def;
-    const std::string sh = d->short_name();
-    if (sh == "dynamic_slice") {
-      long long base, slope;
-      affine(d->operands[1], base, slope);
-      return all * ((fixed(d->operands[0])->type.dims[0] != trips) + (slope < 0));        // a slice, reversed
+    if (fixed(v) || v->def->short_name() != "dynamic_slice") return all;
+    long long base, slope;
+    affine(v->def->operands[1], base, slope);
+    return all * ((fixed(v->def->operands[0])->type.dims[0] != trips) + (slope < 0));        // a slice, reversed
+  }
+  Claim taken;
+  bool fits(const Claim& more) {
+    Claim c = taken;
+    c.stacks.insert(more.stacks.begin(), more.stacks.end());
+    c.steps.insert(more.steps.begin(), more.steps.end());
+    c.behind = std::max(c.behind, more.behind);
+    int64_t stacks = 0, front = 0;
+    for (Value* v : c.stacks) {
+      const int64_t all = trips * (int64_t)v->type.bytes(), written = c.steps.count(v) ? step_bytes(v) : 2 * all;       // carried: zeros, and the stack
+      stacks += std::min(all, written);
+      front += written - std::min(all, written);
     }
-    int64_t n = sh == "reshape" ? 0 : all;
-    for (size_t k = 0; k < (sh == "dot_general" ? 1 : d->operands.size()); k++) n += stacked_bytes(d->operands[k], seen);
-    return n;
-  }
-  int64_t history_bytes(Value* v, std::set<Value*>& seen) {
-    if (known(v)) return stacked_bytes(v, seen);
-    return carried_.count(v) || !seen.insert(v).second ? 0 : 2 * trips * (int64_t)v->type.bytes();      // zeros to begin with, and the stack
-  }
-  bool fits(int64_t more) {
-    if (bytes + more > kMaxStackBytes) return false;
-    bytes += more;
+    for (Value* v : c.steps)
+      if (!c.stacks.count(v)) front += step_bytes(v);
+    if (stacks + std::max(front, c.behind) > kMaxStackBytes) return false;
+    taken = std::move(c);
     return true;
   }
 
@@ -404,9 +437,10 @@ struct Splitter {
   void products_in_front() {
     for (size_t i = 0; i < body->ops.size(); i++) {
       Op* d = body->ops[i].get();
-      if (d->short_name() != "dot_general" || d->results.size() != 1 || !known(d->results[0]) || product_size(d) >= (1LL << 30)) continue;
-      std::set<Value*> seen;
-      if (!fits(stacked_bytes(d->results[0], seen))) continue;
+      if (d->short_name() != "dot_general" || d->results.size() != 1 || !known(d->results[0])) continue;
+      Claim c;
+      claim(d->results[0], c);
+      if (!fits(c)) continue;
       Value* all = stacked(d->results[0]);
       need_indices();
       TensorType row = d->results[0]->type;
@@ -426,29 +460,35 @@ struct Splitter {
   }
 
   void sums_behind() {
-    std::vector<int> gone;
+    std::set<int> gone;
     const int n = (int)body->args.size();
-    for (int k = 0; k < n; k++) {
+    // products first: sums of rows leave where what they read is known in front of the loop or stacked for a product anyway
+    for (int i = 0; i < 2 * n; i++) {
+      const int k = i % n;
+      const bool products = i < n;
       Value *a = body->args[k], *r = next->operands[k];
       Op* s = r->def;
-      if (k == counter || a->type.dt != DT::F32 || !s || s->parent != body || s->short_name() != "add" || count_uses(cond, cond->args[k])) continue;
+      if (k == counter || gone.count(k) || a->type.dt != DT::F32 || !s || s->parent != body || s->short_name() != "add" || count_uses(cond, cond->args[k])) continue;
       Value* term = s->operands[0] == a ? s->operands[1] : s->operands[1] == a ? s->operands[0] : nullptr;
       if (!term || term == a || count_uses(body, a) != 1 || count_uses(body, r) != 1 || !term->def || term->def->parent != body || count_uses(body, term) != 1) continue;
       Op* d = term->def;
       Value* sum = nullptr;
-      if (d->short_name() == "dot_general") {
+      if (products && d->short_name() == "dot_general") {
         auto f = attr_struct(d->attr("dot_dimension_numbers"));
         Value *A = d->operands[0], *B = d->operands[1];
-        if (A->type.rank() != 2 || B->type.rank() != 2 || A->type.dt != DT::F32 || B->type.dt != DT::F32 || A == B || product_size(d) >= (1LL << 30) || product_size(d) == 0) continue;
+        if (A->type.rank() != 2 || B->type.rank() != 2 || A->type.dt != DT::F32 || B->type.dt != DT::F32 || A == B) continue;
         if (!f["lhs_batching_dimensions"].empty() || f["lhs_contracting_dimensions"] != std::vector<int64_t>{0} || f["rhs_contracting_dimensions"] != std::vector<int64_t>{0}) continue;
-        if (fixed(A) || fixed(B)) continue;
+        if (fixed(A) || fixed(B) || d->results[0]->type.numel() * A->type.dims[0] == 0) continue;
         const int64_t per = std::min<int64_t>(trips, std::max<int64_t>(1, kSumRows / A->type.dims[0]));
-        std::set<Value*> seen;
-        int64_t more = history_bytes(A, seen) + history_bytes(B, seen) + (trips / per + 3) * (int64_t)term->type.bytes();
-        if (trips % per) more += trips * (int64_t)(A->type.bytes() + B->type.bytes());      // the whole sums' iterations, sliced
-        if (!fits(more)) continue;
+        if (!quicker_behind(d, per)) continue;
+        Claim c;
+        claim(A, c);
+        claim(B, c);
+        c.behind = (trips / per + 3) * (int64_t)term->type.bytes();
+        if (trips % per) c.behind += trips * (int64_t)(A->type.bytes() + B->type.bytes());      // the whole sums' iterations, sliced
+        if (!fits(c)) continue;
         sum = sum_of_products(history(A), history(B), term->type);
-      } else if (d->short_name() == "reduce" && d->operands.size() == 2) {
+      } else if (!products && d->short_name() == "reduce" && d->operands.size() == 2) {
         Op* z = d->operands[1]->def;
         Block* rb = d->regions[0].get();
         if (!z || z->short_name() != "constant" || rb->ops.size() != 2 || rb->ops[0]->short_name() != "add" || rb->ops[0]->operands[0] == rb->ops[0]->operands[1]) continue;
@@ -456,20 +496,23 @@ struct Splitter {
         float zero_value = 1.f;
         if (dv.type.dt != DT::F32 || dv.type.numel() != 1) continue;
         memcpy(&zero_value, dv.data.data(), 4);
-        std::set<Value*> seen;
-        if (zero_value != 0.f || d->operands[0]->type.dt != DT::F32 || fixed(d->operands[0]) || !fits(history_bytes(d->operands[0], seen))) continue;
+        Claim c;
+        if (zero_value != 0.f || d->operands[0]->type.dt != DT::F32 || fixed(d->operands[0])) continue;
+        if (!known(d->operands[0]) && !carried_.count(d->operands[0])) continue;
+        claim(d->operands[0], c);
+        if (!fits(c)) continue;
         std::vector<int64_t> dims{0};
         for (int64_t x : attr_i64s(d->attr("dimensions"))) dims.push_back(x + 1);
         sum = sum_over(history(d->operands[0]), dims, term->type);
       } else continue;
       Value* total = add(back, outer, "add", {w->operands[k], sum}, term->type);
       replace_uses(outer, w->results[k], total);
-      gone.push_back(k);
+      gone.insert(k);
       changed = true;
     }
     // the accumulators leave the loop
-    for (size_t q = gone.size(); q-- > 0;) {
-      const int k = gone[q];
+    for (auto it = gone.rbegin(); it != gone.rend(); ++it) {
+      const int k = *it;
       w->operands.erase(w->operands.begin() + k);
       w->results.erase(w->results.begin() + k);
       next->operands.erase(next->operands.begin() + k);
@@ -494,11 +537,11 @@ struct Splitter {
 
 }  // namespace
 
-void split_counted_loops(Module& m, Block* b) {
+void split_counted_loops(Module& m, Block* b, const LoopProductModel& model) {
   for (size_t i = 0; i < b->ops.size(); i++) {
     Op* op = b->ops[i].get();
     if (op->short_name() != "while" || op->regions.size() != 2 || op->regions[1]->ops.empty()) continue;
-    Splitter s{m, b, op, op->regions[0].get(), op->regions[1].get(), op->regions[1]->ops.back().get()};
+    Splitter s{m, b, op, op->regions[0].get(), op->regions[1].get(), op->regions[1]->ops.back().get(), model};
     s.run();
     const size_t f = s.front.size(), k = s.back.size();
     b->ops.insert(b->ops.begin() + i + 1, std::make_move_iterator(s.back.begin()), std::make_move_iterator(s.back.end()));

@@ -1,10 +1,12 @@
 """What a counted loop costs in memory when its sums leave it: 512 MB at most, whatever the operands of a sum are made of, and
-nothing where one of them is the same in all iterations. Plans only: no step of these sizes is run."""
+nothing where one of them is the same in all iterations; and which products leave: those that take less time as one. Plans only: no
+step of these sizes is run."""
 import re
 
 import pytest
 
 import b200
+from b200.shlo import programs
 from b200.shlo.builder import Builder
 
 
@@ -70,3 +72,34 @@ def test_scratch_of_a_product_in_front_of_a_loop(monkeypatch, T, R, I, N, taken)
     whole = b200.compile_to_plan(text)[0]
     assert any(line.startswith("  igemm") for line in split.splitlines()) == taken, split
     assert _arena(split) - _arena(whole) <= (512 << 20 if taken else 0), split
+
+
+# batch and hidden size of a two-layer recurrent training step, products made in front of the reverse loop, sums of products behind it
+STEPS = [(4, 32, 2, 2), (16, 256, 2, 2), (64, 256, 2, 2), (64, 512, 2, 2), (16, 1024, 2, 2), (256, 256, 2, 0), (256, 512, 1, 0), (256, 1024, 0, 0), (512, 512, 0, 0)]
+
+
+@pytest.mark.parametrize("batch,hidden,front,behind", STEPS)
+def test_products_leave_where_that_is_quicker(monkeypatch, batch, hidden, front, behind):
+    text = programs.lstm_scan_train_step(steps=50, batch=batch, in_dim=8, hidden=hidden).text
+    split = b200.compile_to_plan(text)[0]
+    monkeypatch.setenv("B200_NO_LOOP_SPLIT", "1")
+    whole = b200.compile_to_plan(text)[0]
+    assert _arena(split) - _arena(whole) <= 512 << 20
+    outside = [line for line in split.splitlines() if line.startswith("  igemm")]
+    assert all(" fma " in line for line in outside), split
+    assert sum(f"M={50 * batch} " in line for line in outside) == front, split
+    assert len({line.split("N=")[1].split()[0] + line.split("M=")[1].split()[0] for line in outside if f"M={50 * batch} " not in line}) == behind, split
+
+
+def test_a_product_of_a_transposed_operand_stays():
+    """x[t]^T w: all iterations' of them are not one matrix, and would not run where an iteration's do."""
+    T, R, I, N = 20, 32, 64, 48
+    b = Builder()
+    x, w, h0 = b.arg((T, R, I), "f32"), b.arg((R, N), "f32"), b.arg((I, N), "f32")
+
+    def body(s, k, h):
+        xt = s.reshape(s.dynamic_slice(x, [k, s.const(0, "i32"), s.const(0, "i32")], (1, R, I)), (R, I))
+        return [s.add(k, s.const(1, "i32")), s.tanh(s.add(s.dot_general(xt, w, ((0,), (0,))), h))]
+    plan = b200.compile_to_plan(b.module([b.while_([b.const(0, "i32"), h0], lambda s, k, *r: s.compare(k, s.const(T, "i32"), "LT"), body)[1]]))[0]
+    assert [line for line in plan.splitlines() if "igemm" in line and " fma " in line and line.startswith("    ")], plan
+    assert not any(line.startswith("  igemm") for line in plan.splitlines()), plan
