@@ -1481,9 +1481,11 @@ struct Planner {
   // In a loop body, whose iterations are a chain of kernels, a small value made of a few tensors in memory is computed again by each
   // of its readers whatever it costs: it takes a fraction of a microsecond on idle SMs, a kernel in front of them two. (The gates
   // of a recurrent cell, read by the gradient of the pre-activations and by that of the state, and the state
-  // itself, read by the next layer: a step of 100 iterations forth and back 4592 -> 4376 us.)
+  // itself, read by the next layer: a step of 100 iterations forth and back 4592 -> 4376 us.) Small is what a block of a pointwise
+  // kernel on each SM covers. Steps of 50 iterations, batch x hidden, with values of up to 65536 / 131072 / 262144 elements made
+  // again, us: 128 x 256 3025 / 2920 / 2925, 64 x 512 4263 / 4157 / 4160, 256 x 256 4665 / 4655 / 5355, 512 x 512 (20 iterations) 4560 / 4555 / 4790.
   bool again_in_loop(Op* op, BlockState& st) {
-    if (!st.block->parent_op || st.block->parent_op->short_name() != "while" || op->results[0]->type.numel() > 65536 || getenv("B200_NO_LOOP_SPLIT")) return false;
+    if (!st.block->parent_op || st.block->parent_op->short_name() != "while" || op->results[0]->type.numel() > 148 * kThreads * kEPT || getenv("B200_NO_LOOP_RECOMPUTE")) return false;
     auto inline_op = [&](Op* d) {
       if (!d || d->parent != st.block || d->results.size() != 1) return false;
       const std::string sh = d->short_name();
@@ -4047,7 +4049,9 @@ struct Planner {
       }
     }
     // One of several that run side by side holds whole SMs that the step's chain of kernels waits for: 17 weight gradients of
-    // 512 x 462 x 512 at a modelled 14.6 us here and 15.9 in the table-driven kernels made an f32 encoder step 1316 us, not 1286.
+    // 512 x 462 x 512 at a modelled 14.6 us here and 15.9 in the table-driven kernels made an f32 encoder step 1307 us, not 1265.
+    // Steps of four layers with this factor 1 / 1.15 / 1.3, us: 462 rows of 512 1307 / 1265 / 1301, 462 of 256 812 / 819 / 829, 400 of 768
+    // 1770 / 1772 / 1772, 128 of 512 764 / 764 / 765, 1024 of 512 1707 / 1717 / 1804, 150 of 768 1072 / 1028 / 1034.
     return copies > 1 ? 1.15 * best : best;
   }
   // ... and in the table-driven kernels, split as choose_split_k would: its k-tiles, 8.5 us for the first wave of CTAs and 4.8

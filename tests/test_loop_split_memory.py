@@ -103,3 +103,22 @@ def test_a_product_of_a_transposed_operand_stays():
     plan = b200.compile_to_plan(b.module([b.while_([b.const(0, "i32"), h0], lambda s, k, *r: s.compare(k, s.const(T, "i32"), "LT"), body)[1]]))[0]
     assert [line for line in plan.splitlines() if "igemm" in line and " fma " in line and line.startswith("    ")], plan
     assert not any(line.startswith("  igemm") for line in plan.splitlines()), plan
+
+
+@pytest.mark.parametrize("rows,again", [(1, True), (100, True), (148, True), (149, False), (256, False)])
+def test_small_values_of_a_body_are_made_again(monkeypatch, rows, again):
+    """Two carried tensors made of one exponential: each of their kernels makes it for itself while a block on each of 148 SMs covers
+    it (151 552 elements), beyond that it is made once. The switch of the split is not the one of this."""
+    b = Builder()
+    x, y = b.arg((rows, 1024), "f32"), b.arg((1024, rows), "f32")
+
+    def body(s, k, h, t):
+        e = s.exp(s.tanh(h))
+        return [s.add(k, s.const(1, "i32")), s.mul(e, s.full(e.shape, 0.5, "f32")), s.add(s.transpose(e, (1, 0)), t)]
+    text = b.module(b.while_([b.const(0, "i32"), x, y], lambda s, k, *r: s.compare(k, s.const(10, "i32"), "LT"), body)[1:])
+    for name in (None, "B200_NO_LOOP_SPLIT", "B200_NO_LOOP_RECOMPUTE"):
+        with monkeypatch.context() as m:
+            if name:
+                m.setenv(name, "1")
+            plan = b200.compile_to_plan(text)[0]
+        assert plan.count("exponential") == (2 if again and name != "B200_NO_LOOP_RECOMPUTE" else 1), (name, plan)
