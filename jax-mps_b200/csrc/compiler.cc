@@ -6629,6 +6629,18 @@ std::unique_ptr<CompiledProgram> compile_text(const char* text, size_t size, Mod
   return p;
 }
 
+std::string planning_switches() {
+  static const char* names[] = {
+      "B200_ALL_REDUCE_CUTS", "B200_DEBUG_NO_REUSE", "B200_DEBUG_ROWS", "B200_NO_ALL_REDUCE_OVERLAP", "B200_NO_ATTENTION_FUSION", "B200_NO_BUNDLES", "B200_NO_COL4", "B200_NO_CSE",
+      "B200_NO_FLAT_ALL_REDUCE", "B200_NO_GEMM16", "B200_NO_GEMM32", "B200_NO_HELD_ROWS", "B200_NO_HOIST", "B200_NO_LICM", "B200_NO_LOOP_RECOMPUTE", "B200_NO_LOOP_SPLIT",
+      "B200_NO_ROW_FUSION", "B200_NO_TILE32", "B200_NO_TILED_TRANSPOSE", "B200_NO_TMA_A", "B200_NO_WEIGHT_HOIST", "B200_NO_WIDE_POINTWISE", "B200_NO_WIDE_ROWS",
+      "B200_NO_WINDOW_UPDATE", "B200_ROW_WARP_MAX"};
+  std::string s;
+  for (const char* n : names)
+    if (const char* v = getenv(n)) s += std::string(n) + "=" + v + ";";
+  return s;
+}
+
 std::unique_ptr<CompiledProgram> compile_module(Module& m, const CompileOptions& opts) {
   auto prog = std::make_unique<CompiledProgram>();
   prog->name = m.name.empty() ? "main" : m.name;

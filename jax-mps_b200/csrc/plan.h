@@ -159,6 +159,9 @@ struct CompileOptions {
 std::unique_ptr<CompiledProgram> compile_module(Module& m, const CompileOptions& opts);
 // The same for the module `m` parsed from `text`; a plan that would gain less from the tensor cores than watching them costs is
 // made without them.
+// The environment variables that the planner reads, with their values: part of the key of a cached plan.
+std::string planning_switches();
+
 std::unique_ptr<CompiledProgram> compile_text(const char* text, size_t size, Module& m, const CompileOptions& opts);
 
 // The device-function library every generated kernel is compiled with.

@@ -2004,20 +2004,10 @@ b200_error* b200_client_compile(b200_client* c, const char* code, size_t code_si
   co.tensor_cores = c->tensor_cores;
   co.partition_id = c->rank;
   co.num_partitions = c->nprocs;
-  char key[64];
-  // planning switches read from the environment are part of the key (a plan made with one setting must not answer
-  // for another)
-  unsigned env_bits = 0;
-  {
-    static const char* names[] = {"B200_NO_WINDOW_UPDATE", "B200_NO_FLAT_ALL_REDUCE", "B200_NO_GEMM16", "B200_NO_ROW_FUSION",
-                                  "B200_NO_WEIGHT_HOIST", "B200_NO_LOOP_SPLIT", "B200_NO_LICM", "B200_NO_CSE", "B200_NO_HOIST", "B200_NO_BUNDLES",
-                                  "B200_NO_TILED_TRANSPOSE", "B200_NO_ALL_REDUCE_OVERLAP", "B200_DEBUG_NO_REUSE", "B200_NO_COL4",
-                                  "B200_NO_ATTENTION_FUSION", "B200_NO_WIDE_POINTWISE", "B200_NO_WIDE_ROWS", "B200_NO_GEMM32", "B200_NO_TILE32"};
-    for (size_t k = 0; k < sizeof names / sizeof names[0]; k++)
-      if (getenv(names[k])) env_bits |= 1u << k;
-  }
-  snprintf(key, sizeof key, "%016llx-%d-%d-%d-%x", (unsigned long long)hash_text(code, code_size, 0), (int)co.fuse, c->rank,
-           c->nprocs, env_bits);
+  // a plan made with one setting of the planner's switches must not answer for another
+  char head[64];
+  snprintf(head, sizeof head, "%016llx-%d-%d-%d-", (unsigned long long)hash_text(code, code_size, 0), (int)co.fuse, c->rank, c->nprocs);
+  const std::string key = head + planning_switches();
   auto hit = c->cache.find(key);
   std::shared_ptr<LoadedProgram> lp;
   if (hit != c->cache.end()) {
