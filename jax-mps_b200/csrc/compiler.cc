@@ -3547,12 +3547,12 @@ struct Planner {
     return Nk % 4 == 0 ? 4 : Nk % 2 == 0 ? 2 : 1;
   }
 
-  // Runs of them per thread, 32 threads apart: what a row has for all its columns (a label, a scale) is read once for all of them.
-  // Where a run is 8 bytes or less, and where the pass has a tensor to write as well.
-  static int col_groups(int64_t Nk, int64_t Nr, bool stores) {
-    const int Q = col_run(Nk);
-    return Nk < 1024 || Nr < 128 || Q == 1 ? 1 : Q == 2 ? 4 : stores ? 2 : 1;
-  }
+  // Runs of them per thread, 32 threads apart, where the pass has a tensor to write as well and enough columns for it. Sum and tanh of
+  // rows x columns, one run a thread / two, us: f32 8192 x 1024 14.7 / 12.5, 8192 x 2048 43 / 30, 4096 x 30524 224 / 177; bf16 10.7 / 11.6,
+  // 22.8 / 21.3, 141 / 125. Runs of two elements stay single: four of them a thread, which read a row's own values once, made the sum
+  // of 4096 x 30522 143 us (f32 158) and not 49 (75), sum and tanh 221 (291) and not 123 (193), the column sums and gradient of a
+  // softmax of it with its product 494 and not 401.
+  static int col_groups(int64_t Nk, int64_t Nr, bool stores) { return stores && Nk >= 1024 && Nr >= 128 && col_run(Nk) == 4 ? 2 : 1; }
 
   // A value over the index space of a column reduction that its first pass stores as it goes, in rows `ld` elements apart.
   struct FullOut { Value* v; int64_t ld; };
@@ -3686,7 +3686,7 @@ struct Planner {
         int64_t stride = fo.ld;
         for (int d = last - 1; d >= 0; stride *= oc.shape[d--])
           if (oc.shape[d] != 1) at += " + (" + em.idx_t + ")" + oc.idx[d] + " * " + std::to_string(stride);
-        em.line("if (" + em.run_var + " == " + std::to_string(Q - 1) + ") {");
+        em.line("if (" + em.run_var + " == " + std::to_string(Q - 1) + (H > 1 ? " && o4h == o4 + h * " + std::to_string(std::min<int64_t>(32, Nk / Q) * Q) : "") + ") {");
         em.line(wide_move(arr, name, Q, (int)dt_size(fo.v->type.dt), false, 0, at));
         em.line("}");
       }
@@ -3777,8 +3777,9 @@ struct Planner {
       // as many times with the accumulators indexed by q.
       const int TX = (int)std::min<int64_t>(32, Nk / Q), TY = 256 / TX;
       // 16 bytes per thread and row, measured on the ResNet18 step: 1 -> 5.20 ms, 2 -> 5.15, 4 -> 5.18 (scalar form 5.21);
-      // twice as many rows in flight where a row gives a thread 8 bytes
-      const int unroll_r = H > 1 ? 1 : Q == 4 && !two_bytes ? 2 : 4;
+      // twice as many rows in flight where a row gives a thread 8 bytes. Two rows of two runs: sum and tanh of f32 4096 x 30524 213 us with
+      // one row, 177 with two, 196 with three, bf16 157, 125, 137; 8192 x 2048 35.5, 29.7, 29.4 and 22.5, 21.3, 21.7.
+      const int unroll_r = H > 1 || (Q == 4 && !two_bytes) ? 2 : 4;
       const std::string at_q = H > 1 ? "h * " + std::to_string(Q) + " + q" : "q";
       auto per_q = [&](std::string text) {
         return std::regex_replace(text, std::regex("\\bacc(\\d+)\\b"), "acc$1[" + at_q + "]");
@@ -3797,15 +3798,17 @@ struct Planner {
           for (int q = 0; q < H * Q; q++) src << (q ? ", " : "") << init_names[k];
           src << "};\n";
         }
-      const std::string runs = "      #pragma unroll\n      for (int h = 0; h < " + std::to_string(H) + "; ++h) {\n        const " + em.idx_t + " o4h = o4 + h * " + std::to_string(TX * Q) + ";\n" +
-                               (H > 1 ? "        if (o4h >= (" + em.idx_t + ")" + std::to_string(Nk) + "LL) break;\n" : "");
+      // runs past the last column take the last one again, without a branch between the loads of a thread; nothing of theirs is stored
+      const std::string each_run = "      #pragma unroll\n      for (int h = 0; h < " + std::to_string(H) + "; ++h) {\n", run_at = "o4 + h * " + std::to_string(TX * Q), end = "(" + em.idx_t + ")" + std::to_string(Nk) + "LL";
+      const std::string all_runs = each_run + "        const " + em.idx_t + " o4h = " + (H > 1 ? "min(" + run_at + ", " + end + " - " + std::to_string(Q) + ")" : run_at) + ";\n";
+      const std::string runs = each_run + "        const " + em.idx_t + " o4h = " + run_at + ";\n" + (H > 1 ? "        if (o4h >= " + end + ") break;\n" : "");
       const std::string each = "      #pragma unroll\n      for (int q = 0; q < " + std::to_string(Q) + "; ++q) {\n        const " + em.idx_t + " o = o4h + q;\n";
       const std::string column = "h * " + std::to_string(TX * Q) + " + threadIdx.x * " + std::to_string(Q) + " + q";
       src << "  if (live) {\n";
       src << "    #pragma unroll " << unroll_r << "\n";
       src << "    for (" << it << " r = (" << it << ")blockIdx.y * " << TY << " + threadIdx.y; r < (" << it << ")" << Nr
           << "LL; r += " << TY << " * (" << it << ")gridDim.y) {\n";
-      src << runs << em.run_arrays(6) << each << pe.str() << per_q(em.str());
+      src << all_runs << em.run_arrays(6) << each << pe.str() << per_q(em.str());
       src << "      }\n      }\n    }\n  }\n";
       src << runs << each;
       for (size_t k = 0; k < n; k++) src << "    sm" << k << "[threadIdx.y][" << column << "] = acc" << k << "[" << at_q << "];\n";

@@ -2,6 +2,8 @@
 result is made once, in the rows that the 16-bit product behind it reads (padded where their length is no multiple of eight), and
 so is what the second pass makes of the sums. On the GPU held to float64: tanh and the product are rounded to 8 bits once each
 (2e-2 of the result's scale), the sums of 4096 values are fp32."""
+import re
+
 import numpy as np
 import pytest
 
@@ -30,7 +32,7 @@ def test_made_once(cols):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("cols", [1024, 1026, 1030, 2050])
+@pytest.mark.parametrize("cols", [1024, 1026, 1028, 1030, 1284, 2050])
 def test_values(client, cols):
     r = np.random.default_rng(cols)
     def bf16(*shape): return (f32_to_bf16_bits(r.standard_normal(shape).astype(np.float32)).astype(np.uint32) << 16).view(np.float32)
@@ -88,3 +90,28 @@ def test_the_step_past_the_end_of_a_row(n, wide):
     step = 256 * (4 if "* 4;" in loop else 1) * splits
     assert (n + step >= 2**31) <= wide
     assert loop.strip().startswith("for (i64 " if wide else "for (int "), loop
+
+
+@pytest.mark.parametrize("cols,groups", [(1022, 1), (1024, 2), (1026, 1), (1028, 2), (30522, 1), (30524, 2)])
+def test_one_run_of_columns_a_thread(cols, groups):
+    """Two runs a thread only where the pass stores a tensor as well and a run is 16 bytes of f32; no branch between the loads of a
+    thread."""
+    for stores in (False, True):
+        b = Builder()
+        g = b.arg((8192, cols), "f32")
+        plan, src = b200.compile_to_plan(b.module([b.reduce_sum(g, (0,))] + ([b.tanh(g)] if stores else [])), validate=True)
+        kernel = _kernel(src, "reduce_0")
+        assert plan.splitlines()[1].endswith("args=[2,3,0]" if stores else "args=[2,0]"), plan
+        assert f"float acc0[{(4 if cols % 4 == 0 else 2) * (groups if stores else 1)}]" in kernel
+        rows = kernel[kernel.index("for (int r = "):]
+        assert "break" not in rows[:rows.index("\n  }\n")]
+
+
+def test_two_runs_of_wide_accumulators_fit_shared_memory():
+    b = Builder()
+    x = b.arg((4096, 1028), "f32")
+    y = b.convert(x, "f64")
+    plan, src = b200.compile_to_plan(b.module([b.reduce_sum(v, (0,)) for v in (y, b.mul(y, y), b.mul(y, b.mul(y, y)), b.neg(y))] + [b.tanh(x)]), validate=True)
+    assert "+fusion{tanh}" in plan, plan
+    tiles = re.findall(r"__shared__ double sm\d+\[(\d+)\]\[(\d+)\]", _kernel(src, "reduce_0"))
+    assert len(tiles) == 4 and sum(int(r) * int(c) * 8 for r, c in tiles) <= 48 * 1024
