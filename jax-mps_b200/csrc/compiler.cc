@@ -5372,10 +5372,19 @@ struct Planner {
   // A pointwise group that can be stored by the first pass of the column reduction `g`: over the same elements, reading a tensor
   // of that size that `g` reads too, everything it reads at hand, nothing of it from `g`.
   Group* partner_of(Group* g, const ReduceGen& rg, BlockState& st) {
-    int64_t total = 1;
-    for (auto d : rg.in_shape) total *= d;
-    const int Q = col_run([&] { int64_t nk = 1; for (size_t d = 0; d < rg.in_shape.size(); d++) if (std::find(rg.dims.begin(), rg.dims.end(), (int64_t)d) == rg.dims.end()) nk *= rg.in_shape[d]; return nk; }());
+    int64_t total = 1, Nk = 1;
+    for (size_t d = 0; d < rg.in_shape.size(); d++) {
+      total *= rg.in_shape[d];
+      if (std::find(rg.dims.begin(), rg.dims.end(), (int64_t)d) == rg.dims.end()) Nk *= rg.in_shape[d];
+    }
+    const int Q = col_run(Nk);
     if (!opts.fuse || total < (1 << 22) || rg.in_shape.back() % Q || std::find(rg.dims.begin(), rg.dims.end(), (int64_t)rg.in_shape.size() - 1) != rg.dims.end()) return nullptr;
+    // Rows that fill the threads that walk down them: runs for a part of a warp that 32 is a multiple of, or for two thirds of the blocks'
+    // at least. Sum and tanh of rows x columns, apart / in one pass, us, f32 and bf16: 131072 x 66 (33 runs, two blocks) 16.8 / 20.2,
+    // 14.8 / 19.4; 100000 x 100 (25 runs) 20.1 / 25.4, 13.3 / 12.6; 32768 x 130 (65 runs) 9.1 / 9.1, 9.1 / 9.1; 65536 x 64 (16 runs)
+    // 9.4 / 7.5, 9.0 / 7.5; 16384 x 514 15.8 / 14.3, 12.8 / 13.4; 8192 x 1024 16.1 / 12.5, 11.8 / 11.6; 4096 x 30522 241 / 193, 152 / 123.
+    const int64_t runs = Nk / Q;
+    if (runs < 32 ? 32 % runs : 3 * runs < 2 * 32 * ((runs + 31) / 32)) return nullptr;
     // the tensors a group reads; false when one of them is not there yet
     auto reads = [&](Group* q, std::set<Value*>& in) {
       bool there = true;

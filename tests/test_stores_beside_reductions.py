@@ -115,3 +115,12 @@ def test_two_runs_of_wide_accumulators_fit_shared_memory():
     assert "+fusion{tanh}" in plan, plan
     tiles = re.findall(r"__shared__ double sm\d+\[(\d+)\]\[(\d+)\]", _kernel(src, "reduce_0"))
     assert len(tiles) == 4 and sum(int(r) * int(c) * 8 for r, c in tiles) <= 48 * 1024
+
+
+@pytest.mark.parametrize("rows,cols,one_pass", [(65536, 64, True), (131072, 66, False), (100000, 100, False), (65536, 128, True), (32768, 130, True), (49152, 86, True), (45000, 94, True),
+                                                (32768, 132, False), (16384, 514, True)])
+def test_one_pass_where_rows_fill_its_threads(rows, cols, one_pass):
+    b = Builder()
+    x = b.arg((rows, cols), "f32")
+    plan = b200.compile_to_plan(b.module([b.reduce_sum(x, (0,)), b.tanh(x)]))[0]
+    assert ("+fusion{tanh}" in plan) == one_pass, plan
