@@ -4071,9 +4071,13 @@ struct Planner {
     choose_split_k(t);
     split_k = t.split_k;
     const TableShape s = table_shape(t);
+    // Single floats in tiles 64 wide: 15 us and 3.1 a k-tile (M x K x N, FMA / tables, us: 200 x 24323 x 16 54 / 37, 64 x 7034 x 64
+    // 32 / 23, 8 x 6495 x 16 36 / 23, 256 x 7938 x 16 25 / 26, 64 x 3742 x 32 19 / 22, 30 x 2289 x 64 16 / 22).
+    const bool thin = !t.vec && t.N <= 64;
+    const double first_us = thin ? 15.0 : 8.5, tile_us = thin ? 3.1 : 0.95 * s.tile_us;
     return in_company(copies, [&](int n) {
       const long long waves = (n * s.tiles * split_k + s.per_wave - 1) / s.per_wave;
-      return (double)waves * (double)((s.ktiles + split_k - 1) / split_k) * 0.95 * s.tile_us + 8.5 + 4.8 * (double)(waves - 1) +
+      return (double)waves * (double)((s.ktiles + split_k - 1) / split_k) * tile_us + first_us + 4.8 * (double)(waves - 1) +
              (split_k > 1 ? (double)n * split_k * t.M * t.N * t.groups * 8.0 / 3.3e6 : 0.0);
     });
   }
