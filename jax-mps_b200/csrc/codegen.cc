@@ -324,6 +324,19 @@ std::vector<std::string> Emitter::emit_scalar_region(Block* b, const std::vector
   throw CompileError("region without return");
 }
 
+// does evaluating `v` in this kernel take more than a handful of instructions?
+bool Emitter::expensive(Value* v) {
+  static const std::set<std::string> cheap = {"add", "subtract", "multiply", "maximum", "minimum", "negate", "abs", "compare", "select", "convert", "and", "or", "xor", "not",
+                                              "clamp", "sign", "constant", "iota"};
+  std::set<Value*> seen;
+  std::function<bool(Value*)> walk = [&](Value* x) {
+    if (!seen.insert(x).second || !x->def || !is_internal(x->def)) return false;
+    const std::string sh = x->def->short_name();
+    return (is_elementwise_op(sh) && !cheap.count(sh)) || std::any_of(x->def->operands.begin(), x->def->operands.end(), walk);
+  };
+  return walk(v);
+}
+
 std::string Emitter::emit(Value* v, Ctx c) {
   auto bit = bound.find(v);
   if (bit != bound.end()) return bit->second;
@@ -475,7 +488,8 @@ std::string Emitter::emit(Value* v, Ctx c) {
         line("const " + idx_t + " " + q + " = " + t + " / " + std::to_string(step) + ";");
         line(ok + " = " + ok + " && (" + t + " % " + std::to_string(step) + " == 0);");
       }
-      line(ok + " = " + ok + " && " + t + " >= 0 && " + q + " < " + std::to_string(o->type.dims[i]) + ";");
+      const bool whole = (int)i == oc.run_dim;       // one branch for all of a run
+      line(ok + " = " + ok + " && " + (whole ? oc.run_base : t) + " >= 0 && " + (whole ? oc.run_base : q) + " < " + std::to_string(o->type.dims[i]) + ";");
       oc.idx[i] = q;
     }
     var = fresh("v");
@@ -492,10 +506,21 @@ std::string Emitter::emit(Value* v, Ctx c) {
     var = fresh("v");
     line(ct + " " + var + ";");
     int64_t off = 0;
-    bool whole = c.run_dim != dim;                   // no run reaches over the border of two operands
+    bool whole = c.run_dim != dim;                   // no run reaches over the border of two operands: one branch for all of it
     if (!whole) {
       whole = true;
-      for (auto* o : d->operands) whole = whole && o->type.dims[dim] % run == 0;
+      int64_t at = 0, inside = 0;                    // borders that lie inside a warp's runs, per row
+      for (auto* o : d->operands) {
+        at += o->type.dims[dim];
+        whole = whole && at % run == 0;
+        inside += at % (32 * run) != 0;
+      }
+      // A warp with a border inside goes through both sides. One element at a time that costs a load and little else (the compiler
+      // selects the address), run by run all that is computed of them: rows of two parts with a tanh of each, whole runs / apart,
+      // us: f32 30000 x 200 8.9 / 6.8, 8192 x 768 (a border in one of six warps) 7.7 / 7.1; bf16 30000 x 200 10.5 / 9.5, 8192 x 768 (in one
+      // of three) 8.8 / 10.3; without the tanh f32 30000 x 200 5.3 / 6.4, bf16 3.7 / 5.8. Whole runs of eight up to a border in every second warp.
+      if (inside && (run < 8 || 2 * inside * 32 * run > at))
+        whole = whole && std::none_of(d->operands.begin(), d->operands.end(), [&](Value* o) { return expensive(o); });
     }
     for (size_t k = 0; k < d->operands.size(); k++) {
       Value* o = d->operands[k];
@@ -503,7 +528,7 @@ std::string Emitter::emit(Value* v, Ctx c) {
       if (sz == 0) continue;
       bool last = true;
       for (size_t q = k + 1; q < d->operands.size(); q++) last &= d->operands[q]->type.dims[dim] == 0;
-      std::string cond = last ? "" : "if (" + c.idx[dim] + " < " + std::to_string(off + sz) + ") ";
+      std::string cond = last ? "" : "if (" + (whole && c.run_dim == dim ? c.run_base : c.idx[dim]) + " < " + std::to_string(off + sz) + ") ";
       line((off == 0 ? "" : "else ") + cond + "{");
       push_scope();
       Ctx oc;

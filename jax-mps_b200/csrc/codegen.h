@@ -72,6 +72,7 @@ class Emitter {
   std::string shifted(const std::string& base, int64_t by);
   std::string elementwise(Op* op, const std::vector<std::string>& a);
   std::string load(Value* v, Ctx& c);
+  bool expensive(Value* v);
   std::string key(Value* v, Ctx& c);
   std::ostringstream os_;
   std::vector<std::map<std::string, std::string>> memo_{1};

@@ -128,3 +128,22 @@ def test_many_wide_accumulators_fit_shared_memory():
     for body in src.split('extern "C"')[1:]:
         tiles = re.findall(r"__shared__ double sm\d+\[(\d+)\]\[(\d+)\]", body)
         assert sum(int(r) * int(c) * 8 for r, c in tiles) <= 48 * 1024
+
+
+@pytest.mark.parametrize("dt,parts,tanh,whole", [("f32", (96, 104), False, True), ("f32", (96, 104), True, False), ("f32", (128, 128), True, True), ("f32", (64, 64), True, False), ("bf16", (96, 104), True, False),
+                                                 ("bf16", (384, 384), True, True), ("bf16", (256, 512), True, True), ("bf16", (96, 104), False, True), ("bf16", (100, 100), False, False), ("f32", (90, 110), False, False)])
+def test_concatenations_of_runs(dt, parts, tanh, whole):
+    """Two parts of a row: run by run where no run and few warps have the border inside, or where there is little to compute; each branch
+    is then taken by a whole run. The values are those of the interpreter either way."""
+    import re
+
+    import b200
+    rows = -(-151552 // sum(parts)) // 8 * 8 + 8
+    r = np.random.default_rng(parts[0])
+    b = Builder()
+    xs = [b.arg((rows, n), dt) for n in parts]
+    text = b.module([b.concatenate([b.tanh(x) if tanh else x for x in xs], 1)])
+    src = b200.compile_to_plan(text, validate=True)[1]
+    kernel = src[src.index('extern "C"'):]
+    assert bool(re.search(r"reinterpret_cast<const uint4\*>\(in0 \+ l\d+\)", kernel)) == whole, kernel
+    _check(text, [(np.round(r.standard_normal((rows, n)) * 8) / 8).astype(np.float32) for n in parts], 2e-2 if dt == "bf16" else 1e-6)
