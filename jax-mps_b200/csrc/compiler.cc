@@ -1460,13 +1460,10 @@ struct Planner {
 
   // A large exponential of 2-byte data is computed again by every kernel that needs it: its f32 values are twice the bytes of what
   // it is made of, written once and read back by each. (The softmax of 4096 x 30522 logits, its column sums and its gradient:
-  // with stored values 229 us for the rows and 257 for columns and gradient, 147 and 229 so.) Large from 2^22 elements on. One-layer
-  // masked-LM steps of rows x vocabulary, stored / again, us: 4096 x 30522 972 / 865, 2048 x 582 / 524, 1024 x 407 / 369, 512 x 288 / 267,
-  // 256 x 224 / 217, 4096 x 2000 326 / 323; with the line at 2^20 the exponentials of the attention (1 M and 2 M) too: the first two
-  // 868 and 528, the last 314, two layers of 768 at 4096 x 1000 1029 instead of 1035; below that no difference of more than 2 %.
+  // with stored values 229 us for the rows and 257 for columns and gradient, 147 and 229 so.)
   static bool recomputed(Op* op) {
     Value* v = op->results[0];
-    if (op->short_name() != "exponential" || v->type.dt != DT::F32 || v->type.numel() < (1LL << 22)) return false;
+    if (op->short_name() != "exponential" || v->type.dt != DT::F32 || v->type.numel() < (1LL << 25)) return false;
     bool any = false;
     std::set<Value*> seen;
     std::function<bool(Value*)> two_bytes = [&](Value* x) -> bool {
