@@ -1830,7 +1830,7 @@ b200_error* create_client(const b200_client_options* o, ncclComm_t given_comm, b
   CUDA_TRY(cudaMallocHost((void**)&c->pred_host, 64));
   CUDA_TRY(cudaMalloc((void**)&c->error_flag, sizeof(int)));
   CUDA_TRY(cudaMalloc((void**)&c->loop_guard, sizeof(unsigned long long)));
-  CUDA_TRY(cudaMemset(c->error_flag, 0, sizeof(int)));
+  CUDA_TRY(cudaMemsetAsync(c->error_flag, 0, sizeof(int), c->compute));
   CUDA_TRY(cudaMallocHost((void**)&c->status_block, sizeof(int) * b200_client::kStatusWords));
   memset(c->status_block, 0, sizeof(int) * b200_client::kStatusWords);
   for (int k = b200_client::kStatusWords - 1; k >= 0; k--) c->free_status.push_back(k);
@@ -2050,7 +2050,9 @@ b200_error* b200_client_compile(b200_client* c, const char* code, size_t code_si
       std::vector<uint8_t> host(total, 0);
       for (size_t k = 0; k < p.consts.size(); k++)
         memcpy(host.data() + offs[k], p.consts[k].bytes.data(), p.consts[k].bytes.size());
-      CUDA_TRY(cudaMemcpy(lp->const_block, host.data(), total, cudaMemcpyHostToDevice));
+      // On the stream that reads them: a copy from pageable memory returns once the data is staged, and the compute stream does not wait
+      // for the default one. (Behind other transfers the tables of a product arrived after its kernel had begun.)
+      CUDA_TRY(cudaMemcpyAsync(lp->const_block, host.data(), total, cudaMemcpyHostToDevice, c->compute));
     }
     for (size_t k = 0; k < p.consts.size(); k++) lp->const_ptrs.push_back((char*)lp->const_block + offs[k]);
     for (size_t a = 0; a < p.arena_bytes.size(); a++) {
