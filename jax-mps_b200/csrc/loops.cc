@@ -21,9 +21,9 @@
 // for the sake of the split is below 512 MB: stacks, the operands they are made of, partial sums. A sum over an operand that is the same in all
 // iterations stays in the loop: its stack would be as many copies of one tensor. Sums of rows leave only where what they read is
 // stacked for a product. Training steps of two recurrent layers and 50 iterations, batch x hidden, us, products in the
-// loop / split: 16 x 256 2603 / 1620, 64 x 256 3030 / 2307, 128 x 256 3750 / 3030, 256 x 256 5230 / 4660, 64 x 512 5200 / 4230,
-// 256 x 512 8170 / 8020, 512 x 512 (20 iterations) 4575 / 4570, 16 x 1024 8055 / 5150, 64 x 1024 11230 / 10410, 256 x 1024 15510 / 15450. (All products below
-// 2^30 multiply-adds split and all sums of rows: 4910 at 512 x 512, 15660 at 256 x 1024.)
+// loop / split: 16 x 256 2610 / 1615, 64 x 256 3030 / 2305, 128 x 256 3820 / 2925, 256 x 256 5220 / 4670, 64 x 512 4980 / 4160,
+// 256 x 512 8170 - 8760 / 8050, 512 x 512 (20 iterations) 4565 / 4560, 16 x 1024 8000 / 5200, 64 x 1024 11270 / 10505, 256 x 1024 15520 / 15515.
+// (All products below 2^30 multiply-adds split and all sums of rows: 4910 at 512 x 512, 15660 at 256 x 1024.)
 #include "loops.h"
 
 #include <algorithm>
